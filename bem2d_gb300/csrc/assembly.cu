@@ -1,11 +1,7 @@
-// Galerkin assembly kernels for sm_103a (FP64 path).
+// Galerkin assembly kernels for sm_103a: node tables, near field, mass matrix
+// and right-hand sides (FP64 far field and potentials: far_fp64.cu).
 //
 //  node_table_kernel  per (unknown, Gauss node): Map, Normal, |J| w phi
-//  far_fp64_kernel    one CTA per 32 x 32 tile of (test, trial) unknowns;
-//                     the tile's node data staged in shared memory; tensor
-//                     Gauss rule (Integrate<kernel,Gauss2D>,
-//                     lib/bem2d_quadrature.h:37-65, selected for non-adjacent
-//                     elements at :283-287); coalesced column-major stores
 //  near_kernel        one warp per self/adjacent pair: graded rules
 //                     (IntegrateIdent :67-109 with AdaptedGauss1; Integrate
 //                     with AdaptedGauss3 / AdaptedGauss2 for next / prev,
@@ -69,145 +65,6 @@ void launch_node_table(const DevGeom& g, const DevRules& r, NodeTable t,
                        const NodeTableFF* tf, cudaStream_t s) {
   NodeTableFF z{};
   node_table_kernel<<<(g.n_unk + 127) / 128, 128, 0, s>>>(g, r, t, tf ? *tf : z, tf ? 1 : 0);
-}
-
-// ---------------------------------------------------------------------------
-// Far field.  Tile: 32 test unknowns (rows, one per lane) x 32 trial unknowns
-// (columns, 4 per warp).  Shared memory holds, per node q and tile row /
-// column: x, y, nx, ny, w  ([field][q][32]) plus the element links.
-constexpr int kTile = 32;
-constexpr int kFarThreads = 256;
-
-// CK: complex wavenumber k + i ki (complex-argument Hankel functions).
-template <int KERNEL, int NG, bool CK>
-__global__ void __launch_bounds__(kFarThreads)
-far_fp64_kernel(DevGeom g, NodeTable t, int ng_rt, double k, double ki, double eta,
-                double alpha, double2* __restrict__ out, long long ld) {
-  const int ng = NG > 0 ? NG : ng_rt;
-  extern __shared__ double smem[];
-  double* rs = smem;                     // rows: 5 * ng * 32
-  double* cs = smem + 5 * ng * kTile;    // cols: 5 * ng * 32
-  long long* links = reinterpret_cast<long long*>(cs + 5 * ng * kTile);
-  long long* r_idx = links;              // [32]
-  long long* r_next = links + kTile;
-  long long* r_prev = links + 2 * kTile;
-  long long* c_idx = links + 3 * kTile;
-
-  const int row0 = blockIdx.x * kTile, col0 = blockIdx.y * kTile;
-  const int n = g.n_unk;
-  // stage node data
-  for (int v = threadIdx.x; v < ng * kTile; v += blockDim.x) {
-    const int q = v / kTile, l = v - q * kTile;
-    const int ur = min(row0 + l, n - 1), uc = min(col0 + l, n - 1);
-    const size_t ir = (size_t)ur * ng + q, ic = (size_t)uc * ng + q;
-    const int o = q * kTile + l;
-    rs[0 * ng * kTile + o] = t.x[ir];
-    rs[1 * ng * kTile + o] = t.y[ir];
-    rs[2 * ng * kTile + o] = t.nx[ir];
-    rs[3 * ng * kTile + o] = t.ny[ir];
-    rs[4 * ng * kTile + o] = t.w[ir];
-    cs[0 * ng * kTile + o] = t.x[ic];
-    cs[1 * ng * kTile + o] = t.y[ic];
-    cs[2 * ng * kTile + o] = t.nx[ic];
-    cs[3 * ng * kTile + o] = t.ny[ic];
-    cs[4 * ng * kTile + o] = t.w[ic];
-  }
-  if (threadIdx.x < kTile) {
-    const int l = threadIdx.x;
-    const int er = g.unk_elem[min(row0 + l, n - 1)];
-    const int ec = g.unk_elem[min(col0 + l, n - 1)];
-    r_idx[l] = g.index[er];
-    r_next[l] = g.next[er];
-    r_prev[l] = g.prev[er];
-    c_idx[l] = g.index[ec];
-  }
-  __syncthreads();
-
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int row = row0 + lane;
-  const double kq = 0.25 * k, eq = 0.25 * eta;
-  const long long ri = r_idx[lane], rn = r_next[lane], rp = r_prev[lane];
-  const int SZ = ng * kTile;
-
-#pragma unroll 1
-  for (int cc = warp; cc < kTile; cc += kFarThreads / 32) {
-    const int col = col0 + cc;
-    const long long ci = c_idx[cc];
-    const bool near = (ri == ci) || (rn == ci) || (rp == ci);
-    if (row >= n || col >= n || near) continue;
-    double acc_re = 0.0, acc_im = 0.0;
-#pragma unroll 1
-    for (int q1 = 0; q1 < ng; ++q1) {
-      const int o1 = q1 * kTile + lane;
-      const double x1 = rs[o1], y1 = rs[SZ + o1], n1x = rs[2 * SZ + o1],
-                   n1y = rs[3 * SZ + o1], w1 = rs[4 * SZ + o1];
-#pragma unroll
-      for (int q2 = 0; q2 < ng; ++q2) {  // fully unrolled when NG > 0
-        const int o2 = q2 * kTile + cc;
-        double re, im;
-        if (CK)
-          kernel_c<KERNEL>(k, ki, eq, x1, y1, cs[o2], cs[SZ + o2], n1x, n1y,
-                           cs[2 * SZ + o2], cs[3 * SZ + o2], &re, &im);
-        else
-          kernel_d<KERNEL>(k, kq, eq, x1, y1, cs[o2], cs[SZ + o2], n1x, n1y,
-                           cs[2 * SZ + o2], cs[3 * SZ + o2], &re, &im);
-        const double ww = w1 * cs[4 * SZ + o2];
-        acc_re = fma(re, ww, acc_re);
-        acc_im = fma(im, ww, acc_im);
-      }
-    }
-    out[(size_t)col * ld + row] = make_double2(alpha * acc_re, alpha * acc_im);
-  }
-}
-
-template <int KERNEL, bool CK>
-static void launch_far_k(const DevGeom& g, const NodeTable& t, int ng, double k, double ki,
-                         double eta, double alpha, double2* out, long long ld,
-                         cudaStream_t s) {
-  const size_t smem = sizeof(double) * 10 * ng * kTile + sizeof(long long) * 4 * kTile;
-  dim3 grid((g.n_unk + kTile - 1) / kTile, (g.n_unk + kTile - 1) / kTile);
-  if constexpr (!CK) {  // the complex-k kernel keeps its node loop rolled
-    if (ng == 5) {
-      far_fp64_kernel<KERNEL, 5, false><<<grid, kFarThreads, smem, s>>>(g, t, ng, k, ki, eta,
-                                                                        alpha, out, ld);
-      return;
-    }
-  }
-  auto fn = far_fp64_kernel<KERNEL, 0, CK>;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  fn<<<grid, kFarThreads, smem, s>>>(g, t, ng, k, ki, eta, alpha, out, ld);
-}
-
-template <bool CK>
-static void launch_far_any(const DevGeom& g, const NodeTable& t, int ng, int kernel, double k,
-                           double ki, double eta, double alpha, double2* out, long long ld,
-                           cudaStream_t s) {
-  switch (kernel) {
-    case BEM2D_KERNEL_SINGLE:
-      launch_far_k<BEM2D_KERNEL_SINGLE, CK>(g, t, ng, k, ki, eta, alpha, out, ld, s);
-      break;
-    case BEM2D_KERNEL_DOUBLE:
-      launch_far_k<BEM2D_KERNEL_DOUBLE, CK>(g, t, ng, k, ki, eta, alpha, out, ld, s);
-      break;
-    case BEM2D_KERNEL_CONJDOUBLE:
-      launch_far_k<BEM2D_KERNEL_CONJDOUBLE, CK>(g, t, ng, k, ki, eta, alpha, out, ld, s);
-      break;
-    default:
-      launch_far_k<BEM2D_KERNEL_COMBINED, CK>(g, t, ng, k, ki, eta, alpha, out, ld, s);
-  }
-}
-
-void launch_far_fp64(const DevGeom& g, const NodeTable& t, int ng, int kernel,
-                     double k, double eta, double alpha, double2* out,
-                     long long ld, cudaStream_t s) {
-  launch_far_any<false>(g, t, ng, kernel, k, 0.0, eta, alpha, out, ld, s);
-}
-
-void launch_far_fp64_ck(const DevGeom& g, const NodeTable& t, int ng, int kernel, double k,
-                        double ki, double eta, double alpha, double2* out, long long ld,
-                        cudaStream_t s) {
-  launch_far_any<true>(g, t, ng, kernel, k, ki, eta, alpha, out, ld, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -567,90 +424,6 @@ void launch_rhs(const DevGeom& g, const NodeTable& t, int ng, int fun, double k,
                 cudaStream_t s, double ki) {
   rhs_kernel<<<(g.n_unk + 127) / 128, 128, 0, s>>>(g.n_unk, t, ng, fun, k, ki, dx, dy,
                                                    eta, scale, out);
-}
-
-// ---------------------------------------------------------------------------
-// Potential of a density at points (EvalKernel, lib/bem2d_quadrature.h:184-228):
-// out[p] = sum_u c_u sum_q K(x_p, y_uq) W_uq, both normals the source node's.
-// One thread per point; unknowns staged through shared memory in chunks.
-// CK: complex wavenumber k + i ki.
-template <int KERNEL, bool CK>
-__global__ void __launch_bounds__(128)
-potential_kernel(int nunk, NodeTable t, int ng, double k, double ki, double eta,
-                 const double2* __restrict__ coef, int npts, const double* __restrict__ pts,
-                 double2* __restrict__ out) {
-  __shared__ double sx[128], sy[128], snx[128], sny[128], sw[128];
-  __shared__ double2 sc[128];
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const double px = p < npts ? pts[2 * p] : 0.0, py = p < npts ? pts[2 * p + 1] : 0.0;
-  const double kq = 0.25 * k, eq = 0.25 * eta;
-  double ar = 0.0, ai = 0.0;
-  const int total = nunk * ng;
-  for (int base = 0; base < total; base += 128) {
-    const int v = base + threadIdx.x;
-    __syncthreads();
-    if (v < total) {
-      sx[threadIdx.x] = t.x[v];
-      sy[threadIdx.x] = t.y[v];
-      snx[threadIdx.x] = t.nx[v];
-      sny[threadIdx.x] = t.ny[v];
-      sw[threadIdx.x] = t.w[v];
-      sc[threadIdx.x] = coef[v / ng];
-    }
-    __syncthreads();
-    const int cnt = min(128, total - base);
-    if (p < npts) {
-      for (int i = 0; i < cnt; ++i) {
-        double kvr, kvi;
-        if (CK)
-          kernel_c<KERNEL>(k, ki, eq, px, py, sx[i], sy[i], snx[i], sny[i], snx[i], sny[i],
-                           &kvr, &kvi);
-        else
-          kernel_d<KERNEL>(k, kq, eq, px, py, sx[i], sy[i], snx[i], sny[i], snx[i], sny[i],
-                           &kvr, &kvi);
-        // coefficient * kernel * weight
-        const double2 c = sc[i];
-        const double vr = (c.x * kvr - c.y * kvi) * sw[i],
-                     vi = (c.x * kvi + c.y * kvr) * sw[i];
-        ar += vr;
-        ai += vi;
-      }
-    }
-  }
-  if (p < npts) out[p] = make_double2(ar, ai);
-}
-
-template <bool CK>
-static void launch_potential_k(const DevGeom& g, const NodeTable& t, int ng, int kernel,
-                               double k, double ki, double eta, const double2* coef, int npts,
-                               const double* pts, double2* out, cudaStream_t s) {
-  const int blocks = (npts + 127) / 128;
-  switch (kernel) {
-    case BEM2D_KERNEL_SINGLE:
-      potential_kernel<BEM2D_KERNEL_SINGLE, CK>
-          <<<blocks, 128, 0, s>>>(g.n_unk, t, ng, k, ki, eta, coef, npts, pts, out);
-      break;
-    case BEM2D_KERNEL_DOUBLE:
-      potential_kernel<BEM2D_KERNEL_DOUBLE, CK>
-          <<<blocks, 128, 0, s>>>(g.n_unk, t, ng, k, ki, eta, coef, npts, pts, out);
-      break;
-    case BEM2D_KERNEL_CONJDOUBLE:
-      potential_kernel<BEM2D_KERNEL_CONJDOUBLE, CK>
-          <<<blocks, 128, 0, s>>>(g.n_unk, t, ng, k, ki, eta, coef, npts, pts, out);
-      break;
-    default:
-      potential_kernel<BEM2D_KERNEL_COMBINED, CK>
-          <<<blocks, 128, 0, s>>>(g.n_unk, t, ng, k, ki, eta, coef, npts, pts, out);
-  }
-}
-
-void launch_potential(const DevGeom& g, const NodeTable& t, int ng, int kernel, double k,
-                      double eta, const double2* coef, int npts, const double* pts,
-                      double2* out, cudaStream_t s, double ki) {
-  if (ki != 0.0)
-    launch_potential_k<true>(g, t, ng, kernel, k, ki, eta, coef, npts, pts, out, s);
-  else
-    launch_potential_k<false>(g, t, ng, kernel, k, 0.0, eta, coef, npts, pts, out, s);
 }
 
 }  // namespace bem2d_gpu

@@ -325,6 +325,9 @@ struct Staged {
   bool has_ff = false;
   NearPair* pairs;
   int npairs;
+  // FP64 far field: runs of consecutive unknowns of one element
+  const int2* grp = nullptr;
+  int ngrp = 0, nb = 1;
 };
 
 static int check_quad(bem2d_ctx* c, const bem2d_quad* q) {
@@ -402,6 +405,21 @@ static std::vector<NearPair> near_pairs(const bem2d_geometry* g) {
   return kept;
 }
 
+// Runs of at most 3 consecutive unknowns on one element, in order, as (first
+// unknown, count); *nb: the longest (1: no table needed).
+static std::vector<int2> unknown_groups(const bem2d_geometry* g, int* nb) {
+  std::vector<int2> out;
+  *nb = 1;
+  for (int u = 0; u < g->n_unk;) {
+    int m = 1;
+    while (m < 3 && u + m < g->n_unk && g->unk_elem[u + m] == g->unk_elem[u]) ++m;
+    out.push_back(make_int2(u, m));
+    *nb = std::max(*nb, m);
+    u += m;
+  }
+  return out;
+}
+
 static int stage(bem2d_ctx* c, const bem2d_geometry* g, const bem2d_quad* q, bool nodes,
                  bool pairs, Staged* st, bool ff_nodes = false) {
   int rc = check_geom(c, g);
@@ -454,6 +472,18 @@ static int stage(bem2d_ctx* c, const bem2d_geometry* g, const bem2d_quad* q, boo
       CUDA_TRY(c, cudaMemcpyAsync(st->pairs, np.data(), sizeof(NearPair) * np.size(),
                                   cudaMemcpyHostToDevice, c->stream));
   }
+  std::vector<int2> groups;
+  if (pairs && nodes) {
+    groups = unknown_groups(g, &st->nb);
+    st->ngrp = (int)groups.size();
+    if (st->nb > 1) {
+      int2* dgp = static_cast<int2*>(ws(c, "groups", sizeof(int2) * groups.size(), &rc));
+      if (!dgp) return rc;
+      CUDA_TRY(c, cudaMemcpyAsync(dgp, groups.data(), sizeof(int2) * groups.size(),
+                                  cudaMemcpyHostToDevice, c->stream));
+      st->grp = dgp;
+    }
+  }
   if (nodes) {
     const size_t nn = (size_t)nu * q->N;
     double* t = static_cast<double*>(ws(c, "nodes", sizeof(double) * 5 * nn, &rc));
@@ -498,12 +528,14 @@ static int check_k(bem2d_ctx* c, double k_re, double k_im) {
 static int assemble_dev(bem2d_ctx* c, const Staged& st, int kernel, double k, double eta,
                         double alpha, double beta, double2* A, long long ld, double ki = 0.0) {
   int t = tic(c, BEM2D_PHASE_FAR);
-  if (ki != 0.0)
-    launch_far_fp64_ck(st.g, st.t, st.r.ng, kernel, k, ki, eta, alpha, A, ld, c->stream);
-  else
-    launch_far_fp64(st.g, st.t, st.r.ng, kernel, k, eta, alpha, A, ld, c->stream);
+  int rc = 0;
+  void* ck_tab = ki != 0.0 ? ws(c, "hankel_tab", hankel_tab_bytes(), &rc) : nullptr;
+  if (rc) return rc;
+  if (launch_far_fp64(st.g, st.t, st.grp, st.ngrp, st.nb, st.r.ng, kernel, k, ki, eta, alpha, A,
+                      ld, ck_tab, c->stream) != BEM2D_OK)
+    return fail(c, BEM2D_ERR_NOMEM, "device table for the far-field kernel");
   toc(c, t);
-  ++c->launches;
+  c->launches += ki != 0.0 ? 2 : 1;
   CHECK_LAUNCH(c);
   t = tic(c, BEM2D_PHASE_NEAR);
   if (ki != 0.0)
@@ -2391,8 +2423,15 @@ int bem2d_eval_kernel(bem2d_ctx* c, const bem2d_geometry* geom, const bem2d_quad
   const bool odev = is_device_ptr(out);
   double2* dO = dev_out(c, out, (size_t)npts, "ek_o", &rc);
   if (!dO) return rc;
-  launch_potential(st.g, st.t, st.r.ng, kernel, k_re, eta, dc, npts, dp, dO, c->stream, k_im);
-  ++c->launches;
+  const size_t pb = potential_part_bytes(npts, geom->n_unk * st.r.ng);
+  double2* part = pb ? static_cast<double2*>(ws(c, "ek_part", pb, &rc)) : nullptr;
+  if (rc) return rc;
+  void* ck_tab = k_im != 0.0 ? ws(c, "hankel_tab", hankel_tab_bytes(), &rc) : nullptr;
+  if (rc) return rc;
+  if (launch_potential(st.g, st.t, st.r.ng, kernel, k_re, k_im, eta, dc, npts, dp, dO, part,
+                       ck_tab, c->stream) != BEM2D_OK)
+    return fail(c, BEM2D_ERR_NOMEM, "device table for the potential kernel");
+  c->launches += 1 + (pb ? 1 : 0) + (k_im != 0.0 ? 1 : 0);
   CHECK_LAUNCH(c);
   if (!odev)
     CUDA_TRY(c, cudaMemcpyAsync(out, dO, sizeof(double2) * npts, cudaMemcpyDeviceToHost, c->stream));

@@ -368,14 +368,14 @@ int launch_far_ff(const DevGeom& g, const NodeTable& t, const NodeTableFF& tf, i
 int launch_deferred(const NodeTableFF& tf, int ng, int kernel, double k, double eta,
                     double alpha, const DeferList& dl, double2* out, long long ld,
                     float2* out32, long long ld32, cudaStream_t s);
-void launch_far_fp64(const DevGeom& g, const NodeTable& t, int ng, int kernel,
-                     double k, double eta, double alpha, double2* out,
-                     long long ld, cudaStream_t s);
-// FP64 far field with a complex wavenumber k + i ki (complex-argument Hankel
-// functions).
-void launch_far_fp64_ck(const DevGeom& g, const NodeTable& t, int ng, int kernel, double k,
-                        double ki, double eta, double alpha, double2* out, long long ld,
-                        cudaStream_t s);
+// FP64 far field with wavenumber k + i ki.  grp (first unknown, count): runs of
+// up to nb consecutive unknowns of one element, ngrp of them; unused (null)
+// when nb = 1.  ck_tab: hankel_tab_bytes() of scratch when ki != 0.  Returns
+// BEM2D_ERR_NOMEM if the table of real wavenumbers could not be made.
+int launch_far_fp64(const DevGeom& g, const NodeTable& t, const int2* grp, int ngrp, int nb,
+                    int ng, int kernel, double k, double ki, double eta, double alpha,
+                    double2* out, long long ld, void* ck_tab, cudaStream_t s);
+size_t hankel_tab_bytes();
 // Near field (self and adjacent pairs).  out32 == nullptr: FP64 kernel
 // evaluation into out.  Otherwise the mixed-precision variant (float-float
 // Bessel functions) writes both out and out32.  Returns BEM2D_ERR_NOMEM if
@@ -396,10 +396,12 @@ void launch_rhs(const DevGeom& g, const NodeTable& t, int ng, int fun, double k,
                 double dx, double dy, double eta, double scale, double2* out,
                 cudaStream_t s, double ki = 0.0);
 
-// ki: imaginary part of the wavenumber (0 for a real k).
-void launch_potential(const DevGeom& g, const NodeTable& t, int ng, int kernel, double k,
-                      double eta, const double2* coef, int npts, const double* pts,
-                      double2* out, cudaStream_t s, double ki = 0.0);
+// Potentials at npts points, wavenumber k + i ki; part: potential_part_bytes()
+// of scratch, ck_tab as for launch_far_fp64.
+int launch_potential(const DevGeom& g, const NodeTable& t, int ng, int kernel, double k,
+                     double ki, double eta, const double2* coef, int npts, const double* pts,
+                     double2* out, double2* part, void* ck_tab, cudaStream_t s);
+size_t potential_part_bytes(int npts, int nodes);
 
 // ---- context accessors (capi.cu) ------------------------------------------
 int ctx_device(const bem2d_ctx* c);

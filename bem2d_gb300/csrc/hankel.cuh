@@ -37,6 +37,30 @@ __host__ __device__ __forceinline__ void sincos_d(double x, double* s, double* c
 #endif
 }
 
+// P0, Q0, P1, Q1 of the modulus-phase form at x > 4; returns 1 / x.
+__host__ __device__ __forceinline__ double hankel_pq_d(double x, double* p0, double* q0,
+                                                       double* p1, double* q1) {
+  const double ix = 1.0 / x;
+  if (x <= 8.0) {
+    const double s = 16.0 * ix * ix;                   // (4/x)^2 in [1/4, 1]
+    const double t = fma(s, 8.0 / 3.0, -5.0 / 3.0);    // 2 (s - 1/4)/(3/4) - 1
+    const double q = 4.0 * ix;
+    *p0 = hk_mid_d_0(t);
+    *q0 = hk_mid_d_1(t) * q;
+    *p1 = hk_mid_d_2(t);
+    *q1 = hk_mid_d_3(t) * q;
+  } else {
+    const double s = 64.0 * ix * ix;                   // (8/x)^2 in (0, 1)
+    const double t = fma(s, 2.0, -1.0);
+    const double q = 8.0 * ix;
+    *p0 = hk_far_d_0(t);
+    *q0 = hk_far_d_1(t) * q;
+    *p1 = hk_far_d_2(t);
+    *q1 = hk_far_d_3(t) * q;
+  }
+  return ix;
+}
+
 // J0, Y0, J1, Y1 at x > 0 in FP64.
 __host__ __device__ __forceinline__ void hankel01_d(double x, double* j0,
                                                     double* y0, double* j1,
@@ -53,25 +77,8 @@ __host__ __device__ __forceinline__ void hankel01_d(double x, double* j0,
     *y1 = fma(lx, jj1, fma(x, b1, -kTwoOverPi / x));
     return;
   }
-  const double ix = 1.0 / x;
   double p0, q0, p1, q1;
-  if (x <= 8.0) {
-    const double s = 16.0 * ix * ix;                   // (4/x)^2 in [1/4, 1]
-    const double t = fma(s, 8.0 / 3.0, -5.0 / 3.0);    // 2 (s - 1/4)/(3/4) - 1
-    const double q = 4.0 * ix;
-    p0 = hk_mid_d_0(t);
-    q0 = hk_mid_d_1(t) * q;
-    p1 = hk_mid_d_2(t);
-    q1 = hk_mid_d_3(t) * q;
-  } else {
-    const double s = 64.0 * ix * ix;                   // (8/x)^2 in (0, 1)
-    const double t = fma(s, 2.0, -1.0);
-    const double q = 8.0 * ix;
-    p0 = hk_far_d_0(t);
-    q0 = hk_far_d_1(t) * q;
-    p1 = hk_far_d_2(t);
-    q1 = hk_far_d_3(t) * q;
-  }
+  const double ix = hankel_pq_d(x, &p0, &q0, &p1, &q1);
   const double amp = sqrt(kTwoOverPi * ix);
   double sx, cx;
   sincos_d(x, &sx, &cx);

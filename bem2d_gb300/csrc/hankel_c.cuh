@@ -111,7 +111,7 @@ __host__ __device__ __forceinline__ void hankel01_c_series(cd z, cd* h0, cd* h1)
 //   T0 = h sum e^{-v^2} / s(v),   T1 = h sum e^{-v^2} v^2 s(v)
 //   H0 = (sqrt2/pi) e^{iz} z^{-1/2} e^{-i pi/4} T0
 //   H1 = 2 (sqrt2/pi) e^{iz} z^{-1/2} e^{-3i pi/4} T1
-__host__ __device__ __forceinline__ void hankel01_c_integral(cd z, double r, cd* h0, cd* h1) {
+__host__ __device__ __forceinline__ void hankel01_c_sums(cd z, double r, cd* t0, cd* t1) {
   const double h = r <= 3.0 ? 0.0625 : r <= 7.0 ? 0.125 : r <= 14.0 ? 0.25 : 0.5;
   const int nv = (int)(6.5 / h);
   const double iz2 = 1.0 / fma(z.re, z.re, z.im * z.im);
@@ -132,22 +132,42 @@ __host__ __device__ __forceinline__ void hankel01_c_integral(cd z, double r, cd*
     t1r = fma(et, s.re, t1r);
     t1i = fma(et, s.im, t1i);
   }
-  // p = (sqrt2/pi) e^{iz} / sqrt(z)
+  *t0 = cd{t0r, t0i};
+  *t1 = cd{t1r, t1i};
+}
+
+// f e^{-i pi/4} T0 and 2 f e^{-3i pi/4} T1 with f = (sqrt2/pi) w / sqrt(z):
+// H0(z) and H1(z) for w = e^{iz}, without that factor for w = 1.
+__host__ __device__ __forceinline__ void hankel01_c_apply(cd z, cd w, cd t0, cd t1, cd* h0,
+                                                          cd* h1) {
   const cd sz = cd_sqrt(z);
-  double sn, cs;
-  sincos_d(z.re, &sn, &cs);
-  const double ez = exp_d(-z.im);
-  const cd eiz{ez * cs, ez * sn};
   const double isz = 1.0 / fma(sz.re, sz.re, sz.im * sz.im);
   const cd rz{sz.re * isz, -sz.im * isz};  // 1 / sqrt(z)
-  cd p = cd_mul(eiz, rz);
+  cd p = cd_mul(w, rz);
   p.re *= kSqrt2OverPi;
   p.im *= kSqrt2OverPi;
   // e^{-i pi/4} = (1 - i)/sqrt2, e^{-3i pi/4} = -(1 + i)/sqrt2
   const cd p0{kSqrtHalf * (p.re + p.im), kSqrtHalf * (p.im - p.re)};
   const cd p1{2 * kSqrtHalf * (p.im - p.re), -2 * kSqrtHalf * (p.re + p.im)};
-  *h0 = cd_mul(p0, cd{t0r, t0i});
-  *h1 = cd_mul(p1, cd{t1r, t1i});
+  *h0 = cd_mul(p0, t0);
+  *h1 = cd_mul(p1, t1);
+}
+
+__host__ __device__ __forceinline__ void hankel01_c_integral(cd z, double r, cd* h0, cd* h1) {
+  cd t0, t1;
+  hankel01_c_sums(z, r, &t0, &t1);
+  double sn, cs;
+  sincos_d(z.re, &sn, &cs);
+  const double ez = exp_d(-z.im);
+  hankel01_c_apply(z, cd{ez * cs, ez * sn}, t0, t1, h0, h1);
+}
+
+// H0(z) e^{-iz} and H1(z) e^{-iz}, |z| = r > 1.5.
+__host__ __device__ __forceinline__ void hankel01_c_integral_scaled(cd z, double r, cd* g0,
+                                                                    cd* g1) {
+  cd t0, t1;
+  hankel01_c_sums(z, r, &t0, &t1);
+  hankel01_c_apply(z, cd{1.0, 0.0}, t0, t1, g0, g1);
 }
 
 // H0(z), H1(z) for Re z > 0, -pi/3 <= arg z <= pi/2.
