@@ -2251,6 +2251,13 @@ namespace bem2d_gpu {
 // Eigenvalues of the Hermitian M (N x N, device, overwritten): `count`
 // ascending from the smallest or descending from the largest, into out
 // (host or device, count doubles).
+static int sm_count(const bem2d_ctx* c) {
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess)
+    sms = 0;
+  return std::max(sms, 1);
+}
+
 static int spectra_run(bem2d_ctx* c, double2* M, int N, int count, int descending, double* out) {
   int rc = 0;
   void* work = ws(c, "sp_work", spectra_work_bytes(N), &rc);
@@ -2258,11 +2265,7 @@ static int spectra_run(bem2d_ctx* c, double2* M, int N, int count, int descendin
   const bool odev = is_device_ptr(out);
   double* dout = odev ? out : static_cast<double*>(ws(c, "sp_out", sizeof(double) * count, &rc));
   if (!dout) return rc;
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
-      sms < 1)
-    sms = 1;
-  c->launches += launch_tridiag_eigs(M, N, count, descending, work, dout, sms, c->stream);
+  c->launches += launch_tridiag_eigs(M, N, count, descending, work, dout, sm_count(c), c->stream);
   CHECK_LAUNCH(c);
   if (!odev)
     CUDA_TRY(c, cudaMemcpyAsync(out, dout, sizeof(double) * count, cudaMemcpyDeviceToHost,
@@ -2305,13 +2308,27 @@ int bem2d_singular_values(bem2d_ctx* c, int n, const void* A, int64_t lda, doubl
   long long la = 0;
   const double2* dA = dev_in(c, A, n, n, lda, "sp_A", &la, &rc);
   if (!dA) return rc;
-  const int N = 2 * n;
-  double2* M = static_cast<double2*>(ws(c, "sp_M", sizeof(double2) * (size_t)N * N, &rc));
+  double2* M = static_cast<double2*>(ws(c, "sp_M", sizeof(double2) * (size_t)n * n, &rc));
   if (!M) return rc;
-  launch_jordan_wielandt(dA, la, n, M, c->stream);
-  ++c->launches;
+  CUDA_TRY(c, cudaMemcpy2DAsync(M, sizeof(double2) * n, dA, sizeof(double2) * la,
+                                sizeof(double2) * n, n, cudaMemcpyDeviceToDevice, c->stream));
+  const int sms = sm_count(c);
+  void* work = ws(c, "sp_work", bidiag_work_bytes(n, sms), &rc);
+  if (!work) return rc;
+  const bool odev = is_device_ptr(s);
+  double* dout = odev ? s : static_cast<double*>(ws(c, "sp_out", sizeof(double) * n, &rc));
+  if (!dout) return rc;
+  if ((rc = launch_bidiag_singular(M, n, work, dout, sms, c->stream, &c->launches)))
+    return fail(c, rc, "bidiagonalisation launch: %s", cudaGetErrorString(cudaGetLastError()));
   CHECK_LAUNCH(c);
-  return spectra_run(c, M, N, n, 1, s);
+  int status = 0;
+  CUDA_TRY(c, cudaMemcpyAsync(&status, bidiag_status_ptr(work), sizeof(int),
+                              cudaMemcpyDeviceToHost, c->stream));
+  if (!odev)
+    CUDA_TRY(c, cudaMemcpyAsync(s, dout, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  if (status) return fail(c, BEM2D_ERR_TIMEOUT, "bidiagonalisation barrier timed out");
+  return BEM2D_OK;
 }
 
 int bem2d_eigenvalues(bem2d_ctx* c, int n, const void* A, int64_t lda, void* w) {

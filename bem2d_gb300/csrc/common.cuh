@@ -533,14 +533,26 @@ void launch_nonfinite_scan(const double2* A, long long ld, int rows, int cols, i
 size_t spectra_work_bytes(int N);
 // M (n x n, ld n) = the Hermitian matrix defined by the upper triangle of A.
 void launch_herm_from_upper(const double2* A, long long lda, int n, double2* M, cudaStream_t s);
-// M (2n x 2n, ld 2n) = [0 A; A^H 0].
-void launch_jordan_wielandt(const double2* A, long long lda, int n, double2* M, cudaStream_t s);
 // Householder reduction of the Hermitian M (N x N, ld N, overwritten) to
 // tridiagonal form and bisection for `count` of its eigenvalues: ascending
 // from the smallest, or (descending != 0) descending from the largest, into
 // out (device).  Returns the number of kernels launched.
 long long launch_tridiag_eigs(double2* M, int N, int count, int descending, void* work,
                               double* out, int sms, cudaStream_t s);
+
+// `count` eigenvalues of the symmetric tridiagonal (d[n], e[n - 1]); d null: a
+// zero diagonal, e then holds the squared off-diagonals.
+void launch_bisect(const double* d, const double* e, int n, int count, int descending,
+                   double* out, cudaStream_t s);
+
+// ---- launch interfaces (bidiag.cu) ------------------------------------------
+size_t bidiag_work_bytes(int n, int sms);
+// Singular values of A (n x n, ld n, overwritten), descending, into out
+// (device).  *bidiag_status_ptr(work) is nonzero afterwards if a bounded
+// device wait gave up.
+int launch_bidiag_singular(double2* A, int n, void* work, double* out, int sms, cudaStream_t s,
+                           long long* launches);
+int* bidiag_status_ptr(void* work);
 
 // ---- launch interfaces (eig.cu) --------------------------------------------
 // Work bytes of launch_eigenvalues for order n.

@@ -45,8 +45,8 @@ Matrix operator*(const Matrix& lhs, const Matrix& rhs);
 
 // ||A||_2 and cond_2(A) from the extreme singular values (GPU Lanczos).
 void L2NormCond(const Matrix& stiff, double& norm, double& cond);
-// All singular values, descending (GPU Householder tridiagonalisation of
-// [0 A; A^H 0] and bisection).
+// All singular values, descending (GPU Householder bidiagonalisation and
+// bisection).
 void SingularValues(const Matrix& stiff, pdvector& singvals);
 // x = m^{-1} rhs (GPU LU; precision from BEM2D_PRECISION=fp64|mixed|mixed_tf32).
 pMatrix SolveSystem(Matrix& m, Matrix& rhs);

@@ -267,15 +267,15 @@ int bem2d_l2_norm_cond_prec(bem2d_ctx* ctx, int n, const void* A, int64_t lda, d
  * triangle A holds (the diagonal's real part is used): replaces
  * HermitianEigenvalues (lib/bem2d_mathroutines.cpp:353-433, zheev with
  * jobz 'N', uplo 'U').  Householder reduction to real tridiagonal form on
- * the GPU (four kernels per column), then bisection on Sturm counts, one
- * thread per eigenvalue; absolute accuracy ~ n eps ||A||.  A: host or
+ * the GPU (four kernels per column), then multisection on Sturm counts, one
+ * warp per eigenvalue; absolute accuracy ~ n eps ||A||.  A: host or
  * device; w: host or device. */
 int bem2d_hermitian_eigenvalues(bem2d_ctx* ctx, int n, const void* A, int64_t lda, double* w);
 
 /* s[0..n-1] = singular values of A, descending: replaces SingularValues
- * (lib/bem2d_mathroutines.cpp:268-320, zgesvd without vectors).  They are
- * the n largest eigenvalues of the Hermitian [0 A; A^H 0], computed as in
- * bem2d_hermitian_eigenvalues (absolute accuracy ~ n eps ||A||).
+ * (lib/bem2d_mathroutines.cpp:268-320, zgesvd without vectors).
+ * Householder bidiagonalisation in one persistent kernel, then the Sturm
+ * counts of the Golub-Kahan tridiagonal (absolute accuracy ~ n eps ||A||).
  * n <= BEM2D_SPECTRA_MAX_N / 2. */
 int bem2d_singular_values(bem2d_ctx* ctx, int n, const void* A, int64_t lda, double* s);
 
