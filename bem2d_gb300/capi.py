@@ -35,7 +35,7 @@ EXPORTS = ["bem2d_ctx_create", "bem2d_ctx_destroy", "bem2d_ctx_last_error",
            "bem2d_eval_kernel", "bem2d_solve_system_noalloc",
            "bem2d_sweep_solve", "bem2d_hermitian_eigenvalues", "bem2d_singular_values",
            "bem2d_eigenvalues", "bem2d_debug_panel_timeout", "bem2d_noalloc_scratch_fits",
-           "bem2d_debug_tc_update", "bem2d_matmul", "bem2d_eigenvectors"]
+           "bem2d_debug_tc_update", "bem2d_debug_oz_update", "bem2d_matmul", "bem2d_eigenvectors"]
 
 NOALLOC_MAX_N = 1024  # BEM2D_NOALLOC_MAX_N
 
@@ -115,6 +115,7 @@ def load():
         lib.bem2d_debug_panel_timeout.argtypes = [vp, i32, i32]
         lib.bem2d_noalloc_scratch_fits.argtypes = [ctypes.POINTER(i64), ctypes.POINTER(i64)]
         lib.bem2d_debug_tc_update.argtypes = [vp, i32, i32, i32, vp, i64, vp, i64, vp, i64]
+        lib.bem2d_debug_oz_update.argtypes = [vp, i32, i32, i32, vp, i64, vp, i64, vp, i64]
         lib.bem2d_matmul.argtypes = [vp, i32, i32, i32, vp, i64, vp, i64, vp, i64]
         lib.bem2d_eigenvectors.argtypes = [vp, i32, vp, i64, vp, vp, i64]
         lib.bem2d_ctx_enable_timers.argtypes = [vp, i32]
@@ -353,6 +354,16 @@ class Context:
         M, N = C.shape
         K = A.shape[1]
         self._check(self.lib.bem2d_debug_tc_update(self.h, M, N, K, _ptr(C), _ld(C, M), _ptr(A),
+                                                   _ld(A, M), _ptr(B), _ld(B, K)))
+        return C
+
+    def oz_update(self, C, A, B):
+        """C -= A B in place on complex128 torch CUDA column-major views
+        through bem2d_debug_oz_update."""
+        _sync_producers(C, A, B)
+        M, N = C.shape
+        K = A.shape[1]
+        self._check(self.lib.bem2d_debug_oz_update(self.h, M, N, K, _ptr(C), _ld(C, M), _ptr(A),
                                                    _ld(A, M), _ptr(B), _ld(B, K)))
         return C
 

@@ -1005,7 +1005,7 @@ static int attach_lookahead(bem2d_ctx* c, LuWork& w, int n) {
     CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_far, cudaEventDisableTiming));
   }
   int rc = 0;
-  w.pack2_bytes = lu_pack_bytes(n);
+  w.pack2_bytes = lu_pack_bytes(n, sizeof(float2));
   w.pack2 = ws(c, "lu_pack2", w.pack2_bytes, &rc);
   if (!w.pack2) return rc;
   w.aux = c->stream_aux;
@@ -1054,6 +1054,9 @@ static int solve_dev(bem2d_ctx* c, int n, const double2* A, long long lda, const
     if (!LU) return rc;
     CUDA_TRY(c, cudaMemcpy2DAsync(LU, sizeof(double2) * n, A, sizeof(double2) * lda,
                                   sizeof(double2) * n, n, cudaMemcpyDeviceToDevice, c->stream));
+    w.pack_bytes = lu_pack_bytes(n, sizeof(double2));
+    w.pack = ws(c, "lu_pack", w.pack_bytes, &rc);
+    if (!w.pack) return rc;
     int t = tic(c, BEM2D_PHASE_LU);
     if ((rc = lu_factor<double2>(LU, n, n, w, c->stream, &c->launches)))
       return fail(c, rc, "LU launch failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1083,7 +1086,7 @@ static int solve_dev(bem2d_ctx* c, int n, const double2* A, long long lda, const
   const double accept = std::max(tol, 1e-12);
   float2* LU = static_cast<float2*>(ws(c, "lu32", sizeof(float2) * (size_t)n * n, &rc));
   if (!LU) return rc;
-  w.pack_bytes = lu_pack_bytes(n);
+  w.pack_bytes = lu_pack_bytes(n, sizeof(float2));
   w.pack = ws(c, "lu_pack", w.pack_bytes, &rc);
   if (w.pack && (rc = attach_lookahead(c, w, n))) return rc;
   if (!w.pack) return rc;
@@ -1927,10 +1930,10 @@ int bem2d_l2_norm_cond_prec(bem2d_ctx* c, int n, const void* A, int64_t lda, dou
   w.dinv = aux;
   w.perm = reinterpret_cast<int*>(aux + (lu_aux_bytes(n, esz) - 256 - sizeof(int) * (size_t)n));
   const int tl = tic(c, BEM2D_PHASE_LU);
+  w.pack_bytes = lu_pack_bytes(n, esz);
+  w.pack = ws(c, "lu_pack", w.pack_bytes, &rc);
+  if (!w.pack) return rc;
   if (mixed) {
-    w.pack_bytes = lu_pack_bytes(n);
-    w.pack = ws(c, "lu_pack", w.pack_bytes, &rc);
-    if (!w.pack) return rc;
     if ((rc = attach_lookahead(c, w, n))) return rc;
     launch_to_c64(dA, la, static_cast<float2*>(LU), n, n, n, c->stream);
     ++c->launches;
@@ -2156,6 +2159,31 @@ int bem2d_debug_panel_timeout(bem2d_ctx* c, int n, int polls) {
   if (h[1])
     return fail(c, BEM2D_ERR_TIMEOUT, "panel wait gave up after %d polls on a slot never posted",
                 polls);
+  return BEM2D_OK;
+}
+
+int bem2d_debug_oz_update(bem2d_ctx* c, int M, int N, int K, void* C, int64_t ldc,
+                          const void* A, int64_t lda, const void* B, int64_t ldb) {
+  if (!c) return BEM2D_ERR_ARG;
+  if (M < 1 || N < 1 || K < 1 || !C || !A || !B || ldc < M || lda < M || ldb < K)
+    return fail(c, BEM2D_ERR_ARG, "bad arguments");
+  if (!is_device_ptr(C) || !is_device_ptr(A) || !is_device_ptr(B))
+    return fail(c, BEM2D_ERR_ARG, "the tensor-core update takes device pointers");
+  cudaSetDevice(c->device);
+  int rc = 0;
+  const size_t pb = oz_pack_bytes(M, N);
+  void* pack = ws(c, "dbg_pack", pb, &rc);
+  int* st = static_cast<int*>(ws(c, "dbg_status", 256, &rc));
+  if (!pack || !st) return rc;
+  CUDA_TRY(c, cudaMemsetAsync(st, 0, sizeof(int), c->stream));
+  if ((rc = launch_oz_zgemm(static_cast<double2*>(C), ldc, static_cast<const double2*>(A), lda,
+                            static_cast<const double2*>(B), ldb, M, N, K, 1, -1.0, nullptr, 0,
+                            pack, pb, st, c->stream, &c->launches)))
+    return fail(c, rc, "tensor-core update launch: %s", cudaGetErrorString(cudaGetLastError()));
+  int h = 0;
+  CUDA_TRY(c, cudaMemcpyAsync(&h, st, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  if (h) return fail(c, BEM2D_ERR_TIMEOUT, "tensor-core update wait timed out");
   return BEM2D_OK;
 }
 

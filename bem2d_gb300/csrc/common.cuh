@@ -427,8 +427,8 @@ struct LuWork {
   void* scratch;         // panel exchange slots (lu_scratch_bytes)
   size_t scratch_bytes;
   int* perm;             // [n] row permutation of the pivots (filled by lu_factor)
-  // workspace of the complex64 tensor-core update (lu_pack_bytes(n)); null:
-  // the update runs on the CUDA cores
+  // workspace of the tensor-core updates (lu_pack_bytes()); null: the
+  // updates run on the CUDA cores
   void* pack = nullptr;
   size_t pack_bytes = 0;
   void* dinv;            // inverses of the 64 x 64 diagonal blocks of L and U
@@ -457,10 +457,10 @@ struct LuWork {
 size_t lu_scratch_bytes(int n);
 // Bytes of perm + dinv for n unknowns of `elem` bytes each.
 size_t lu_aux_bytes(int n, size_t elem);
-// Bytes of LuWork::pack for a complex64 factorisation of order n.
-size_t lu_pack_bytes(int n);
+// Bytes of LuWork::pack for a factorisation of order n with `elem`-byte entries.
+size_t lu_pack_bytes(int n, size_t elem);
 // Whether a complex64 factorisation of order n uses the look-ahead (and so
-// LuWork::aux, ev_u12, ev_far, pack2 of lu_pack_bytes(n) bytes), and the
+// LuWork::aux, ev_u12, ev_far, pack2 of lu_pack_bytes() bytes), and the
 // persistent CTAs its far updates get (the rest of the SMs stay free for
 // the next block's panels).
 bool lu_lookahead(int n);
@@ -510,6 +510,16 @@ int launch_tc_cgemm_sub(float2* C, long long ldc, const float2* A, long long lda
                         const float2* B, long long ldb, int M, int N, int K, void* pack,
                         size_t pack_bytes, int* status, cudaStream_t s, int max_ctas = 0,
                         int passes = 3);
+
+// C = beta C + sign A B (complex128, column-major; C is M x N, A M x K, B K x
+// N; beta 0 or 1) on the tensor cores, FP64 accurate (lu_oz.cu).  piv (null:
+// none): entries (k, k) whose exponents scale inner index k.  pack:
+// oz_pack_bytes(M, N) bytes.  Sets *status on a device-side wait timeout.
+size_t oz_pack_bytes(int M, int N);
+int launch_oz_zgemm(double2* C, long long ldc, const double2* A, long long lda, const double2* B,
+                    long long ldb, int M, int N, int K, int beta, double sign,
+                    const double2* piv, long long ldp, void* pack, size_t pack_bytes, int* status,
+                    cudaStream_t s, long long* launches);
 
 void launch_residual(const double2* A, long long lda, int n, const double2* x,
                      const double2* b, double2* r, double2* part, cudaStream_t s);

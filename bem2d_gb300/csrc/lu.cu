@@ -1504,8 +1504,9 @@ __global__ void __launch_bounds__(128) dinv_kernel(const T* __restrict__ LU, lon
   }
 }
 
-size_t lu_pack_bytes(int n) {
-  return tc_pack_bytes(n, n, n >= kOuterMinN ? kOuterNB : kNB);
+size_t lu_pack_bytes(int n, size_t elem) {
+  return elem == sizeof(double2) ? oz_pack_bytes(n, n)
+                                 : tc_pack_bytes(n, n, n >= kOuterMinN ? kOuterNB : kNB);
 }
 
 // SMs left to the panels while a look-ahead update runs beside them
@@ -1534,6 +1535,12 @@ template <typename T>
 static int update_sub(T* C, const T* Am, const T* Bm, long long ld, int M, int N, int K,
                       const LuWork& w, cudaStream_t s, long long* launches) {
   if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
+  if constexpr (sizeof(T) == sizeof(double2)) {
+    // Am holds L: its diagonal block's pivots sit K rows above it in A
+    if (w.pack && oz_pack_bytes(M, N) <= w.pack_bytes)
+      return launch_oz_zgemm(C, ld, Am, ld, Bm, ld, M, N, K, 1, -1.0, Am - K, ld, w.pack,
+                             w.pack_bytes, w.status, s, launches);
+  }
   if constexpr (sizeof(T) == sizeof(float2)) {
     // tall and narrow updates (the columns inside an outer block), and short
     // wide ones (the rows of an outer block right of it) too
@@ -1620,7 +1627,7 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
   // columns only (the update reads block b's L21 and writes the columns
   // beyond), then to the rest
   const bool la = sizeof(T) == sizeof(float2) && lu_lookahead(n) && w.aux && w.ev_u12 &&
-                  w.ev_far && w.pack2 && w.pack2_bytes >= lu_pack_bytes(n);
+                  w.ev_far && w.pack2 && w.pack2_bytes >= lu_pack_bytes(n, sizeof(T));
   LuWork w2 = w;  // the far updates' work: second packing buffer, fewer CTAs
   if (la) {
     w2.pack = w.pack2;

@@ -1,0 +1,508 @@
+// Complex128 products on the 5th-generation tensor cores with FP64 accuracy:
+// C = beta C + sign A B (column-major, any leading dimensions, K in slabs of
+// 64), the trailing update of the complex128 LU.
+//
+// GB300's FP64 pipe issues 2 FMAs per clock and SM (1.06 TFLOP/s measured),
+// its f16 tensor pipe 2 PFLOP/s.  The operands are therefore cut into 8-bit
+// digits, products of digits are summed exactly, and FP64 is left only to add
+// the sum to C (the error-free splitting of Ozaki, Ogita, Oishi and Rump,
+// "Error-free transformations of matrix multiplication by using fast routines
+// of matrix multiplication and its applications", Numer. Algorithms 59, 2012, on tensor cores as
+// in Mukunoki, Ozaki, Ogita and Imamura, ISC 2020).
+//
+// Digits.  Row i of A and column j of B are scaled by powers of two so that
+// every entry is a 63-bit fixed-point integer F and a sign, and F = sum_s a_s
+// 256^(7 - s), s = 0..7, with balanced digits |a_s| <= 128.  f16 holds each
+// digit exactly.  A product of digits is at most 2^14 and one accumulator
+// collects the pairs of one order s + t (at most 8) over K = 64: at most 2^23,
+// exact in the FP32 accumulator.  Kept are the 36 pairs with s + t <= 7; what
+// is dropped is below 2^-52 of (largest entry of the row) x (largest of the
+// column) in the worst case and 2^-59 typically, where an FP64 sum of 64
+// products rounds at about 2^-51.  An entry's 53 bits survive whole while it
+// is within 2^-10 of its row's largest.
+//
+// To keep rows and columns of very different size apart (graded meshes) the
+// LU scales inner index k by the pivot's exponent: A(:, k) 2^p_k, B(k, :)
+// 2^-p_k, so A is read as it was before the division by the pivot.
+//
+// Complex arithmetic as in lu_tc.cu: A' (rows 2i, 2i + 1 = re, im of row i)
+// times [B_r B_i]; re C_i = D1[2i] - D2[2i+1], im C_i = D2[2i] + D1[2i+1].
+//
+// A tile is 64 complex rows by 16 complex columns: 32 accumulator columns for
+// each of the 8 orders, 256 in all, two such sets in tensor memory.  Digit s
+// of A against the digits 0 .. 7 - s of B, which lie one after another as
+// rows of one operand, is one MMA of N = 32 (8 - s) whose result lands on the
+// orders s .. 7: 8 MMAs per 16 of K, A read once for all of them.
+//
+// Persistent CTAs take contiguous runs of tiles (row block major) and keep
+// the row block's A (128 KB) in shared memory:
+//   warp 0     producer (bulk copies; A when the row block changes, B into a
+//              ring of two 32 KB stages)
+//   warp 1     MMA issuer
+//   warps 2-9  epilogue: orders 0-3 and 4-7 of D1 and D2 become two 64-bit
+//              integers each, partners exchange D2, two exact conversions, one
+//              FMA to join them, one to add to C: 4 FP64 instructions per
+//              real number, which bound the kernel (2,600 clocks of MMAs
+//              against 4,100 of FP64 for a tile).
+// Every wait is bounded as in lu_tc.cu.
+//
+// Measured against the FP64-pipe update it replaces: solve n = 3001 111.7 ->
+// 49.7 ms; error of one K = 64 product of Gaussian matrices 8 times smaller
+// (1.4e-13 against 1.2e-12, Frobenius; the same with entries spread over 2^10).
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "tc.cuh"
+
+namespace bem2d_gpu {
+namespace {
+
+using namespace tc;
+
+constexpr int kOzBM = 64;       // complex rows per tile (128 real rows = MMA M)
+constexpr int kOzBN = 16;       // complex columns per tile
+constexpr int kOzS = 8;         // digits
+constexpr int kOzK = 64;        // K of a slab: 4 MMA steps of 16
+constexpr int kOzStages = 2;
+constexpr int kOzThreads = 320;  // producer, MMA, 8 epilogue warps
+constexpr int kOzEpi = 256;
+constexpr int kOzABlk = 128 * 16 * 2;              // one digit, one K-step of A'
+constexpr int kOzBBlk = 2 * kOzBN * 16 * 2;        // the same of B
+constexpr int kOzAStep = kOzS * kOzABlk;           // 32 KB per K-step
+constexpr int kOzBStep = kOzS * kOzBBlk;           // 8 KB per K-step
+constexpr int kOzKSteps = kOzK / 16;
+constexpr int kOzABytes = kOzKSteps * kOzAStep;    // 128 KB
+constexpr int kOzBBytes = kOzKSteps * kOzBStep;    // 32 KB
+constexpr int kOzBarOff = kOzABytes + kOzStages * kOzBBytes;  // 192 KB
+constexpr int kOzSmem = kOzBarOff + 256;
+constexpr unsigned kOzAcc = 2 * kOzBN * kOzS;      // 256 TMEM columns
+
+// scale exponents: zero rows / columns, and rows / columns with a NaN or an
+// infinity
+constexpr int kOzZero = -100000, kOzNaN = 400000;
+
+// K-major, no swizzle: core matrices of 8 rows x 16 bytes, 128 bytes along K,
+// 256 bytes from one group of 8 rows to the next
+__device__ __forceinline__ unsigned long long oz_desc(unsigned addr) {
+  return (unsigned long long)((addr & 0x3FFFF) >> 4) | ((unsigned long long)(128 >> 4) << 16) |
+         ((unsigned long long)(256 >> 4) << 32) | (1ull << 46);
+}
+__device__ __forceinline__ int oz_off(int r, int k8) { return (r >> 3) * 256 + k8 * 128 + (r & 7) * 16; }
+
+__device__ __forceinline__ void oz_mma(unsigned d, unsigned a, unsigned b, unsigned idesc,
+                                       unsigned acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(oz_desc(a)), "l"(oz_desc(b)), "r"(idesc), "r"(acc));
+}
+
+// exponent field of a double (0: zero or subnormal, 2047: not finite)
+__device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 2047; }
+
+__device__ __forceinline__ int scale_of(int emax, bool bad) {
+  return bad ? kOzNaN : emax <= -5000 ? kOzZero : emax;
+}
+
+// x 2^p as a fixed-point integer F (rounded toward zero), |F| < 2^63: x 2^p =
+// F 2^(erow - 1085), erow the largest exponent field plus p of the row, whose
+// largest entry has |F| >= 2^62.  Subnormals count as zero.
+__device__ __forceinline__ long long oz_fixed(double x, int p, int erow) {
+  const int e = expo(x);
+  if (e == 0) return 0;
+  const long long b = __double_as_longlong(x);
+  const long long m = (b & 0xfffffffffffffll) | 0x10000000000000ll;
+  const int d = erow - (e + p);  // >= 0
+  const long long f = d <= 10 ? m << (10 - d) : d < 63 ? m >> (d - 10) : 0;
+  return b < 0 ? -f : f;
+}
+
+// The 8 balanced digits of 8 consecutive k of one real row, as f16.
+struct OzDigits {
+  unsigned w[kOzS][4];
+};
+__device__ __forceinline__ void oz_digits(const long long* f, OzDigits* o) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    long long a = f[2 * q], b = f[2 * q + 1];
+#pragma unroll
+    for (int s = kOzS - 1; s >= 0; --s) {
+      const int da = s ? (int)(signed char)(a & 0xff) : (int)a;
+      const int db = s ? (int)(signed char)(b & 0xff) : (int)b;
+      a = (a - da) >> 8;
+      b = (b - db) >> 8;
+      // (1536 + d) - 1536 in f16: exact for |d| <= 512
+      const unsigned w = 0x66006600u + (unsigned)da + ((unsigned)db << 16);
+      const unsigned base = 0x66006600u;
+      const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&w),
+                                *reinterpret_cast<const __half2*>(&base));
+      o->w[s][q] = *reinterpret_cast<const unsigned*>(&h);
+    }
+  }
+}
+
+// ---- packing -------------------------------------------------------------------
+// Exponent p_k of inner index k: that of the pivot, entry k of column k of
+// the factored block at piv (null: 0).
+__device__ __forceinline__ int oz_shift(const double2* piv, long long ldp, int k, int K) {
+  if (!piv || k >= K) return 0;
+  const double2 p = piv[(size_t)k * ldp + k];
+  const int f = max(expo(p.x), expo(p.y));
+  return f > 0 && f < 2047 ? f - 1023 : 0;
+}
+
+// A (M x K) -> per row block of 64: [K-step][digit][128 x 16]; ea[i]: the
+// row's scale exponent.  Eight threads per complex row, thread c takes k = 8 c
+// .. 8 c + 7.
+__global__ void __launch_bounds__(512)
+oz_pack_a_kernel(const double2* __restrict__ A, long long lda, int M, int K, int ksteps,
+                 const double2* __restrict__ piv, long long ldp, unsigned char* __restrict__ Apk,
+                 int* __restrict__ ea) {
+  __shared__ int pk[kOzK], red[8][kOzBM];
+  const int il = threadIdx.x & 63, c = threadIdx.x >> 6, i = blockIdx.x * kOzBM + il;
+  if (threadIdx.x < kOzK) pk[threadIdx.x] = oz_shift(piv, ldp, threadIdx.x, K);
+  double2 v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int k = 8 * c + q;
+    v[q] = i < M && k < K ? A[(size_t)k * lda + i] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  int emax = -10000;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int e = max(expo(v[q].x), expo(v[q].y));
+    if (e > 0) emax = max(emax, e == 2047 ? kOzNaN : e + pk[8 * c + q]);
+  }
+  red[c][il] = emax;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) emax = max(emax, red[q][il]);
+  const int er = scale_of(emax, emax > 50000);
+  if (c == 0 && i < M) ea[i] = er;
+  if (c >= 2 * ksteps) return;
+  const bool use = er > kOzZero && er < kOzNaN;
+  unsigned char* blk = Apk + ((size_t)blockIdx.x * ksteps + (c >> 1)) * kOzAStep;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    long long f[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      f[q] = oz_fixed(!use ? 0.0 : h ? v[q].y : v[q].x, pk[8 * c + q], er);
+    OzDigits o;
+    oz_digits(f, &o);
+#pragma unroll
+    for (int s = 0; s < kOzS; ++s)
+      *reinterpret_cast<uint4*>(blk + s * kOzABlk + oz_off(2 * il + h, c & 1)) =
+          make_uint4(o.w[s][0], o.w[s][1], o.w[s][2], o.w[s][3]);
+  }
+}
+
+// B (K x N) -> per block of 16 columns: [K-step][digit][32 x 16], rows 0..15
+// re and 16..31 im of the columns.  Eight threads per column, thread c takes
+// k = 8 c .. 8 c + 7.
+__global__ void __launch_bounds__(128)
+oz_pack_b_kernel(const double2* __restrict__ B, long long ldb, int K, int N, int ksteps,
+                 const double2* __restrict__ piv, long long ldp, unsigned char* __restrict__ Bpk,
+                 int* __restrict__ eb) {
+  const int c = threadIdx.x & 7, jl = threadIdx.x >> 3, j = blockIdx.x * kOzBN + jl;
+  double2 v[8];
+  int pk[8];
+  int emax = -10000;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int k = 8 * c + q;
+    v[q] = (j < N && k < K) ? B[(size_t)j * ldb + k] : make_double2(0.0, 0.0);
+    pk[q] = -oz_shift(piv, ldp, k, K);
+    const int e = max(expo(v[q].x), expo(v[q].y));
+    if (e > 0) emax = max(emax, e == 2047 ? kOzNaN : e + pk[q]);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+  const int er = scale_of(emax, emax > 50000);
+  if (c == 0 && j < N) eb[j] = er;
+  if (c >= 2 * ksteps) return;
+  const bool use = er > kOzZero && er < kOzNaN;
+  unsigned char* blk = Bpk + ((size_t)blockIdx.x * ksteps + (c >> 1)) * kOzBStep;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    long long f[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) f[q] = oz_fixed(!use ? 0.0 : h ? v[q].y : v[q].x, pk[q], er);
+    OzDigits o;
+    oz_digits(f, &o);
+#pragma unroll
+    for (int s = 0; s < kOzS; ++s)
+      *reinterpret_cast<uint4*>(blk + s * kOzBBlk + oz_off(h * kOzBN + jl, c & 1)) =
+          make_uint4(o.w[s][0], o.w[s][1], o.w[s][2], o.w[s][3]);
+  }
+}
+
+// ---- the product -----------------------------------------------------------------
+#define OZ_LD8(dst, addr)                                                                   \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"      \
+               : "=r"(dst[0]), "=r"(dst[1]), "=r"(dst[2]), "=r"(dst[3]), "=r"(dst[4]),      \
+                 "=r"(dst[5]), "=r"(dst[6]), "=r"(dst[7])                                   \
+               : "r"(addr))
+
+// (double)v for |v| < 2^51, one FP64 instruction
+__device__ __forceinline__ double oz_to_double(long long v) {
+  return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
+}
+
+// C[M x N] = beta C + sign A B, beta 0 or 1, sign +-1.  grid: min(tiles, SMs).
+__global__ void __launch_bounds__(kOzThreads, 1)
+oz_zgemm_kernel(double2* __restrict__ C, long long ldc, const unsigned char* __restrict__ Apk,
+                const unsigned char* __restrict__ Bpk, const int* __restrict__ ea,
+                const int* __restrict__ eb, int M, int N, int ksteps, int ntiles, int tiles,
+                int beta, double sign, int* status) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  unsigned long long* full = reinterpret_cast<unsigned long long*>(sm + kOzBarOff);
+  unsigned long long* empty = full + kOzStages;
+  unsigned long long* afull = empty + kOzStages;
+  unsigned long long* aempty = afull + 1;
+  unsigned long long* acc_full = aempty + 1;
+  unsigned long long* acc_empty = acc_full + 2;
+  unsigned long long* fin = acc_empty + 2;
+  unsigned* tslot = reinterpret_cast<unsigned*>(fin + 1);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(tslot + 1);
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  const int t0 = (int)((long long)tiles * blockIdx.x / gridDim.x);
+  const int t1 = (int)((long long)tiles * (blockIdx.x + 1) / gridDim.x);
+  if (w == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+        smem_u32(tslot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (t == 32) {
+    for (int s = 0; s < kOzStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(afull, 1);
+    mbar_init(aempty, 1);
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&acc_full[a], 1);
+      mbar_init(&acc_empty[a], kOzEpi);
+    }
+    mbar_init(fin, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;");
+    *s_abort = 0;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const unsigned tmem = *tslot;
+  bool ok = true;
+  const unsigned abytes = (unsigned)ksteps * kOzAStep, bbytes = (unsigned)ksteps * kOzBStep;
+  if (w == 0) {
+    if (lane == 0) {  // ---- producer
+      int it = 0, mt_prev = -1, na = 0;
+      for (int tile = t0; tile < t1 && ok; ++tile, ++it) {
+        const int mt = tile / ntiles, nt = tile - mt * ntiles;
+        if (mt != mt_prev) {
+          if (na > 0 && !mbar_wait(aempty, (unsigned)(na - 1) & 1u, s_abort)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(afull, abytes);
+          for (int k = 0; k < ksteps; ++k)
+            bulk_copy(sm + k * kOzAStep, Apk + (size_t)mt * abytes + (size_t)k * kOzAStep,
+                      kOzAStep, afull);
+          ++na;
+          mt_prev = mt;
+        }
+        const int s = it % kOzStages;
+        if (!mbar_wait(&empty[s], ((unsigned)(it / kOzStages) & 1u) ^ 1u, s_abort)) {
+          ok = false;
+          break;
+        }
+        mbar_expect_tx(&full[s], bbytes);
+        bulk_copy(sm + kOzABytes + s * kOzBBytes, Bpk + (size_t)nt * bbytes, bbytes, &full[s]);
+      }
+      if (!ok) {
+        *s_abort = 1;
+        // let the copies in flight land before the CTA's shared memory goes
+        if (na > 0) mbar_wait(afull, (unsigned)(na - 1) & 1u, nullptr);
+        for (int q = it - 1; q >= 0 && q >= it - kOzStages; --q)
+          mbar_wait(&full[q % kOzStages], (unsigned)(q / kOzStages) & 1u, nullptr);
+      }
+    }
+  } else if (w == 1) {
+    if (lane == 0) {  // ---- MMA issuer
+      int j = 0, mt_prev = -1, na = 0;
+      for (int tile = t0; tile < t1 && ok; ++tile, ++j) {
+        const int mt = tile / ntiles;
+        if (mt != mt_prev) {
+          if (!mbar_wait(afull, (unsigned)na & 1u, s_abort)) {
+            ok = false;
+            break;
+          }
+          ++na;
+          mt_prev = mt;
+        }
+        const int a = j & 1, s = j % kOzStages;
+        if (!mbar_wait(&acc_empty[a], ((unsigned)(j >> 1) & 1u) ^ 1u, s_abort) ||
+            !mbar_wait(&full[s], (unsigned)(j / kOzStages) & 1u, s_abort)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const unsigned d = tmem + (unsigned)a * kOzAcc;
+        const unsigned sa = smem_u32(sm), sb = smem_u32(sm + kOzABytes + s * kOzBBytes);
+        for (int k = 0; k < ksteps; ++k) {
+#pragma unroll
+          for (int i = 0; i < kOzS; ++i) {
+            // kind::f16: D f32 (bits 4-5 = 1), A and B f16 (0), K-major,
+            // N >> 3 at bit 17, M >> 4 at bit 24
+            const unsigned nn = 2 * kOzBN * (kOzS - i);
+            const unsigned idesc = (1u << 4) | ((nn >> 3) << 17) | ((128u >> 4) << 24);
+            oz_mma(d + 2 * kOzBN * i, sa + k * kOzAStep + i * kOzABlk, sb + k * kOzBStep, idesc,
+                   (k == 0 && i == 0) ? 0u : 1u);
+          }
+        }
+        mma_commit(&empty[s]);
+        mma_commit(&acc_full[a]);
+        if (tile + 1 < t1 && (tile + 1) / ntiles != mt) mma_commit(aempty);
+      }
+      if (!ok) *s_abort = 1;
+      // every MMA issued has completed before the tensor memory is released
+      mma_commit(fin);
+      if (!mbar_wait(fin, 0u, nullptr)) ok = false;
+    }
+  } else {  // ---- epilogue, warps 2-9
+    // two warps per TMEM lane quarter (warp w may access lanes 32 (w % 4) ..),
+    // one for each half of the tile's 16 columns
+    const int q = w & 3, part = (w - 2) >> 2;
+    const int tl = q * 32 + lane, cc = tl & 1;  // real row tl = 2 i + cc
+    double* Cf = reinterpret_cast<double*>(C);
+    int j = 0;
+    for (int tile = t0; tile < t1; ++tile, ++j) {
+      const int mt = tile / ntiles, nt = tile - mt * ntiles;
+      const int i = mt * kOzBM + (tl >> 1), n0 = nt * kOzBN + part * 8;
+      const int er = i < M ? __ldg(&ea[i]) : kOzZero;
+      const int nlim = i < M ? min(8, N - n0) : 0;
+      double* pc = Cf + 2 * ((size_t)n0 * ldc + i) + cc;
+      const long long cstep = 2 * ldc;
+      double cv[8];
+      int ec[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        cv[u] = u < nlim && beta ? pc[u * cstep] : 0.0;
+        ec[u] = n0 + u < N ? __ldg(&eb[n0 + u]) : kOzZero;
+      }
+      const int a = j & 1;
+      if (!mbar_wait(&acc_full[a], (unsigned)(j >> 1) & 1u, s_abort)) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const unsigned lanes = tmem + (unsigned)a * kOzAcc + ((unsigned)(q * 32) << 16) +
+                             (unsigned)(part * 8);
+      double hi[8];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        long long d1[8], d2[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) d1[u] = d2[u] = 0;
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+          unsigned x1[8], x2[8];
+          OZ_LD8(x1, lanes + (4 * half + o) * 2 * kOzBN);
+          OZ_LD8(x2, lanes + (4 * half + o) * 2 * kOzBN + kOzBN);
+          asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            d1[u] = (d1[u] << 8) + __float2int_rn(__uint_as_float(x1[u]));
+            d2[u] = (d2[u] << 8) + __float2int_rn(__uint_as_float(x2[u]));
+          }
+        }
+        if (half == 1) {  // the accumulator has been read
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          mbar_arrive(&acc_empty[a]);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const long long p2 = __shfl_xor_sync(0xffffffffu, d2[u], 1);
+          const double v = oz_to_double(d1[u] + (cc ? p2 : -p2));
+          hi[u] = half == 0 ? v : fma(v, 2.3283064365386963e-10, hi[u]);  // 2^-32
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (u >= nlim) break;
+        // digit orders 0-3 weigh 256^11 = 2^88, the operands 2^(er - 1085)
+        const int e = er + ec[u] - 2 * 1085 + 88;
+        double v;
+        if (e > -1000 && e < 960) {
+          v = fma(sign * __hiloint2double((e + 1023) << 20, 0), hi[u], cv[u]);
+        } else if (e > 50000) {
+          v = __longlong_as_double(0x7ff8000000000000ll);
+        } else {
+          v = e < -3000 ? cv[u] : cv[u] + sign * ldexp(hi[u], e);
+        }
+        pc[u * cstep] = v;
+      }
+    }
+    if (!ok) *s_abort = 1;
+  }
+  if (!ok) atomicExch(status, 1);
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (w == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+#undef OZ_LD8
+
+size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
+int oz_sms() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v > 0 ? v : 1;
+  }();
+  return n;
+}
+
+}  // namespace
+
+size_t oz_pack_bytes(int M, int N) {
+  const size_t mt = (size_t)(M + kOzBM - 1) / kOzBM, nt = (size_t)(N + kOzBN - 1) / kOzBN;
+  return up256(mt * kOzABytes) + up256(nt * kOzBBytes) + up256(sizeof(int) * (size_t)M) +
+         up256(sizeof(int) * (size_t)N);
+}
+
+int launch_oz_zgemm(double2* C, long long ldc, const double2* A, long long lda, const double2* B,
+                    long long ldb, int M, int N, int K, int beta, double sign,
+                    const double2* piv, long long ldp, void* pack, size_t pack_bytes, int* status,
+                    cudaStream_t s, long long* launches) {
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      oz_zgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOzSmem);
+  if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
+  if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
+  if (!pack || oz_pack_bytes(M, N) > pack_bytes) return BEM2D_ERR_ARG;
+  const int mt = (M + kOzBM - 1) / kOzBM, nt = (N + kOzBN - 1) / kOzBN;
+  unsigned char* Apk = static_cast<unsigned char*>(pack);
+  unsigned char* Bpk = Apk + up256((size_t)mt * kOzABytes);
+  int* ea = reinterpret_cast<int*>(Bpk + up256((size_t)nt * kOzBBytes));
+  int* eb = reinterpret_cast<int*>(reinterpret_cast<char*>(ea) + up256(sizeof(int) * (size_t)M));
+  const int grid = std::min(mt * nt, oz_sms());
+  for (int k = 0; k < K; k += kOzK) {
+    const int kk = std::min(kOzK, K - k), ksteps = (kk + 15) / 16;
+    const double2* pv = piv ? piv + (size_t)k * ldp + k : nullptr;
+    oz_pack_a_kernel<<<mt, 8 * kOzBM, 0, s>>>(A + (size_t)k * lda, lda, M, kk, ksteps, pv, ldp, Apk,
+                                          ea);
+    oz_pack_b_kernel<<<nt, 128, 0, s>>>(B + k, ldb, kk, N, ksteps, pv, ldp, Bpk, eb);
+    oz_zgemm_kernel<<<grid, kOzThreads, kOzSmem, s>>>(C, ldc, Apk, Bpk, ea, eb, M, N, ksteps, nt,
+                                                      mt * nt, k == 0 ? beta : 1, sign, status);
+    *launches += 3;
+  }
+  return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
+}
+
+}  // namespace bem2d_gpu

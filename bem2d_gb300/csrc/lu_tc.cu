@@ -53,9 +53,12 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "tc.cuh"
 
 namespace bem2d_gpu {
 namespace {
+
+using namespace tc;
 
 constexpr int kTcBM = 64;    // complex rows per tile (128 real rows = MMA M)
 constexpr int kTcBN = 128;   // complex columns per tile (MMA N = 256: re, im)
@@ -73,11 +76,7 @@ constexpr int kTcStage = kTcChunkA + kTcChunkB;   // 48 KB
 constexpr int kTcBarOff = kTcStages * kTcStage;   // 192 KB
 constexpr int kTcSmem = kTcBarOff + 256;
 constexpr unsigned kTcAcc = 2 * kTcBN;            // TMEM columns per accumulator
-constexpr unsigned long long kTcWaitNs = 2000000000ull;  // 2 s
 
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
 // tcgen05 shared-memory matrix descriptor: K-major, no swizzle
 __device__ __forceinline__ unsigned long long smem_desc(unsigned addr) {
   return (unsigned long long)((addr & 0x3FFFF) >> 4) |
@@ -101,61 +100,6 @@ __device__ __forceinline__ void mma_tf32(unsigned d, unsigned a, unsigned b, uns
       " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
       "l"(smem_desc(a)), "l"(smem_desc(b)), "r"(idesc), "r"(acc));
 }
-__device__ __forceinline__ void mma_commit(unsigned long long* m) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(m)));
-}
-
-__device__ __forceinline__ void mbar_init(unsigned long long* m, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(m)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* m, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(m)),
-               "r"(bytes));
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* m) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(m)) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(unsigned long long* m, unsigned parity) {
-  unsigned done;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(done)
-      : "r"(smem_u32(m)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-// Bounded wait for phase `parity` of the mbarrier (try_wait suspends the
-// thread for a short while between polls): false after kTcWaitNs of device
-// time, or, if `abort` is given, as soon as another role has given up.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* m, unsigned parity,
-                                          const volatile int* abort) {
-  if (mbar_test(m, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  for (unsigned it = 1;; ++it) {
-    if (mbar_test(m, parity)) return true;
-    if ((it & 15u) == 0u) {
-      if (abort && *abort) return false;
-      if (global_ns() - t0 > kTcWaitNs) return false;
-    }
-  }
-}
-__device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes,
-                                          unsigned long long* m) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(m))
-      : "memory");
-}
-
 #define TC_LD16(dst, addr)                                                                  \
   asm volatile(                                                                             \
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13," \

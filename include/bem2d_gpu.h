@@ -392,6 +392,12 @@ int bem2d_debug_panel_timeout(bem2d_ctx* ctx, int n, int polls);
 int bem2d_debug_tc_update(bem2d_ctx* ctx, int M, int N, int K, void* C, int64_t ldc,
                           const void* A, int64_t lda, const void* B, int64_t ldb);
 
+/* C -= A B for complex128 column-major device matrices through the complex128
+ * LU's tensor-core trailing update (exact products of 8-bit digits on
+ * tcgen05 kind::f16, FP64 accuracy): exposed for its own parity test. */
+int bem2d_debug_oz_update(bem2d_ctx* ctx, int M, int N, int K, void* C, int64_t ldc,
+                          const void* A, int64_t lda, const void* B, int64_t ldb);
+
 #ifdef __cplusplus
 }
 #endif
