@@ -521,6 +521,12 @@ int launch_oz_zgemm(double2* C, long long ldc, const double2* A, long long lda, 
                     const double2* piv, long long ldp, void* pack, size_t pack_bytes, int* status,
                     cudaStream_t s, long long* launches);
 
+// Complex128 panel of at most 64 columns (lu_zpanel.cu): columns [k0, k0 + nb)
+// of rows k0 .. n, interchanges on these columns only.  1: not possible here
+// (nothing changed).
+int launch_zpanel(double2* A, long long lda, int n, int k0, int nb, const LuWork& w,
+                  cudaStream_t s, long long* launches);
+
 void launch_residual(const double2* A, long long lda, int n, const double2* x,
                      const double2* b, double2* r, double2* part, cudaStream_t s);
 size_t residual_part_bytes(int n);

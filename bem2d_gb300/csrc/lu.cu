@@ -1648,6 +1648,12 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
     // portable) CTAs and kPanelRPT rows per thread.
     const int rows_target = sizeof(T) == sizeof(float2) ? kPanelThreads : 64;
     bool done = false;
+    if constexpr (sizeof(T) == sizeof(double2)) {
+      const int rc = launch_zpanel(A, lda, n, k0, nb, w, s, launches);
+      if (rc < 0) return rc;
+      done = rc == 0;
+      if (done) --*launches;  // counted below
+    }
     if (sizeof(T) == sizeof(float2)) {  // register-window panel
       const int min_rpb = std::min(kWinMaxRows, w.min_rows > 0 ? w.min_rows : kRowsMinRpb);
       for (int cmax : {cluster16 ? kMaxClusterPanel : 8, 8}) {
