@@ -1458,50 +1458,103 @@ __global__ void perm_kernel(int n, const int* __restrict__ ipiv, int* __restrict
   for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = sp[i];
 }
 
+// X = L^{-1} X for a unit lower 64 x 64 L in shared memory (column-major, zero
+// on and above the diagonal) and 8 columns, one CTA of 16 warps: lane (g, c),
+// c = lane % 8, of warp w holds row 4 w + g of column c in x.  Block b of 4
+// rows is solved inside warp b (3 shuffle steps), its rows go to X, and after
+// one barrier every warp below subtracts 4 products.  Bound by the FP64
+// pipe: a warp instruction takes 64 clocks of a scheduler, so the 8-column
+// tiles are there to spread the 2,112 instructions of a tile over all SMs.
+constexpr int kTriThreads = 512;
+template <typename T>
+__device__ __forceinline__ T tri64_solve(const T* L, T* X, T x) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = lane & 7, r = 4 * w + (lane >> 3);
+  for (int b = 0; b < 16; ++b) {
+    if (w == b) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        T xi;
+        xi.x = __shfl_sync(0xffffffffu, x.x, 8 * i + c);
+        xi.y = __shfl_sync(0xffffffffu, x.y, 8 * i + c);
+        x = cfms(x, L[(4 * b + i) * kNB + r], xi);  // zero for rows above
+      }
+      X[r * 8 + c] = x;
+    }
+    __syncthreads();
+    if (w > b) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x = cfms(x, L[(4 * b + i) * kNB + r], X[(4 * b + i) * 8 + c]);
+    }
+  }
+  return x;
+}
+
+template <typename T>
+constexpr size_t tri64_smem() {
+  return sizeof(T) * (kNB * kNB + kNB * 8 + kNB);
+}
+
+// Complex128 U12 = L11^{-1} A12, 8 columns per CTA (kite N =
+// 2048, all panels: 3.4 ms with 32 columns per CTA on at most 64 SMs, 1.1 ms).
+__global__ void __launch_bounds__(kTriThreads)
+trsm8_kernel(double2* __restrict__ A, long long lda, int k0, int nb, int c0, int ncols) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* L = reinterpret_cast<double2*>(smem_raw);
+  double2* X = L + kNB * kNB;
+  for (int v = threadIdx.x; v < kNB * kNB; v += kTriThreads) {
+    const int s = v >> 6, r = v & 63;
+    L[v] = s < r && r < nb ? A[(size_t)(k0 + s) * lda + k0 + r] : make_double2(0.0, 0.0);
+  }
+  const int lane = threadIdx.x & 31, r = 4 * (threadIdx.x >> 5) + (lane >> 3);
+  const int j = blockIdx.x * 8 + (lane & 7);
+  const bool in = j < ncols && r < nb;
+  double2* p = A + (size_t)(c0 + j) * lda + k0 + r;
+  double2 x = in ? *p : make_double2(0.0, 0.0);
+  __syncthreads();
+  x = tri64_solve(L, X, x);
+  if (in) *p = x;
+}
+
 // Inverses of the diagonal blocks: dinv[(2 k) * 64 * 64 ...] = L_kk^{-1}
 // (unit lower), dinv[(2 k + 1) * 64 * 64 ...] = U_kk^{-1}; column-major 64 x 64.
+// blockIdx.y: 8 columns of L^{-1} (0-7) or U^{-1} (8-15) by the same solve on
+// columns of the identity; U read backwards (row and column order reversed,
+// rows divided by their pivots) is unit lower too.  (kite N = 2048, complex128:
+// 420 us with one thread per column, 92 us.)
 template <typename T>
-__global__ void __launch_bounds__(128) dinv_kernel(const T* __restrict__ LU, long long lda, int n,
-                                                   T* __restrict__ dinv) {
+__global__ void __launch_bounds__(kTriThreads)
+dinv_kernel(const T* __restrict__ LU, long long lda, int n, T* __restrict__ dinv) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* D = reinterpret_cast<T*>(smem_raw);  // [kNB][kNB] column-major
+  T* L = reinterpret_cast<T*>(smem_raw);
+  T* X = L + kNB * kNB;
+  T* iv = X + kNB * 8;
   const int k0 = blockIdx.x * kNB, nb = min(kNB, n - k0);
-  for (int v = threadIdx.x; v < nb * nb; v += blockDim.x) {
-    const int c = v / nb, r = v - c * nb;
-    D[c * kNB + r] = LU[(size_t)(k0 + c) * lda + k0 + r];
+  const bool up = blockIdx.y >= 8;
+  const T zero = CTraits<T>::make(0, 0);
+  const T* D = LU + (size_t)k0 * lda + k0;
+  if (threadIdx.x < kNB) {
+    const int d = nb - 1 - (int)threadIdx.x;
+    iv[threadIdx.x] = up && d >= 0 ? crcp(D[(size_t)d * lda + d]) : CTraits<T>::make(1, 0);
   }
   __syncthreads();
-  T* Li = dinv + (size_t)(2 * blockIdx.x) * kNB * kNB;
-  T* Ui = Li + kNB * kNB;
-  const T zero = CTraits<T>::make(0, 0), one = CTraits<T>::make(1, 0);
-  const int j = threadIdx.x & 63;
-  // thread j builds column j of one inverse in place in global memory (its
-  // own column only, so the reads back hit L1)
-  if (threadIdx.x < 64) {
-    // L^{-1}: x_j = 1, x_i = -sum_{m=j}^{i-1} L_im x_m
-    T* x = Li + j * kNB;
-    for (int i = 0; i < kNB; ++i) x[i] = (i == j && j < nb) ? one : zero;
-    if (j < nb) {
-      for (int i = j + 1; i < nb; ++i) {
-        T acc = zero;
-        for (int m = j; m < i; ++m) acc = cfma(D[m * kNB + i], x[m], acc);
-        x[i] = CTraits<T>::make(-acc.x, -acc.y);
-      }
-    }
-  } else {
-    // U^{-1}: x_j = 1/U_jj, x_i = -(sum_{m=i+1}^{j} U_im x_m) / U_ii
-    T* x = Ui + j * kNB;
-    for (int i = 0; i < kNB; ++i) x[i] = zero;
-    if (j < nb) {
-      x[j] = crcp(D[j * kNB + j]);
-      for (int i = j - 1; i >= 0; --i) {
-        T acc = zero;
-        for (int m = i + 1; m <= j; ++m) acc = cfma(D[m * kNB + i], x[m], acc);
-        const T q = cmul(acc, crcp(D[i * kNB + i]));
-        x[i] = CTraits<T>::make(-q.x, -q.y);
-      }
-    }
+  for (int v = threadIdx.x; v < kNB * kNB; v += kTriThreads) {
+    const int s = v >> 6, r = v & 63;
+    T l = zero;
+    if (s < r && r < nb)
+      l = up ? cmul(D[(size_t)(nb - 1 - s) * lda + nb - 1 - r], iv[r]) : D[(size_t)s * lda + r];
+    L[v] = l;
   }
+  const int lane = threadIdx.x & 31, r = 4 * (threadIdx.x >> 5) + (lane >> 3);
+  const int j = (blockIdx.y & 7) * 8 + (lane & 7);
+  T x = zero;
+  if (j < nb && r == (up ? nb - 1 - j : j)) x = iv[r];
+  __syncthreads();
+  x = tri64_solve(L, X, x);
+  T* out = dinv + (size_t)(2 * blockIdx.x + (up ? 1 : 0)) * kNB * kNB + (size_t)j * kNB;
+  if (r < nb)
+    out[up ? nb - 1 - r : r] = x;
+  else
+    out[r] = zero;
 }
 
 size_t lu_pack_bytes(int n, size_t elem) {
@@ -1572,9 +1625,13 @@ template <typename T>
 static void trsm_rows(T* A, long long lda, int k0, int nb, int c0, int nc, cudaStream_t s,
                       long long* launches) {
   if (nc <= 0) return;
-  trsm_kernel<T><<<(nc + 31) / 32, 256, sizeof(T) * (kNB * kNB + kNB * 32), s>>>(A, lda, k0, nb,
-                                                                                c0, nc);
   ++*launches;
+  if constexpr (sizeof(T) == sizeof(double2)) {
+    trsm8_kernel<<<(nc + 7) / 8, kTriThreads, tri64_smem<T>(), s>>>(A, lda, k0, nb, c0, nc);
+  } else {
+    trsm_kernel<T><<<(nc + 31) / 32, 256, sizeof(T) * (kNB * kNB + kNB * 32), s>>>(A, lda, k0, nb,
+                                                                                  c0, nc);
+  }
 }
 
 template <typename T>
@@ -1604,12 +1661,15 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
       cudaGetLastError();
       cluster16 = false;
     }
-    cudaFuncSetAttribute(trsm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(T) * (kNB * kNB + kNB * 32)));
+    if constexpr (sizeof(T) == sizeof(float2))
+      cudaFuncSetAttribute(trsm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(sizeof(T) * (kNB * kNB + kNB * 32)));
     cudaFuncSetAttribute(gemm_sub_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(sizeof(T) * 2 * kNB * kGB));
     cudaFuncSetAttribute(dinv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(T) * kNB * kNB));
+                         (int)tri64_smem<T>());
+    cudaFuncSetAttribute(trsm8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)tri64_smem<double2>());
     cudaFuncSetAttribute(perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(tslu_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(sizeof(int) * 2 * kTsluMaxH));
@@ -1793,7 +1853,8 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
   // solve aids: permutation and diagonal-block inverses
   const int nk = (n + kNB - 1) / kNB;
   perm_kernel<<<1, 1024, sizeof(int) * n, s>>>(n, w.ipiv, w.perm);
-  dinv_kernel<T><<<nk, 128, sizeof(T) * kNB * kNB, s>>>(A, lda, n, reinterpret_cast<T*>(w.dinv));
+  dinv_kernel<T><<<dim3(nk, 16), kTriThreads, tri64_smem<T>(), s>>>(A, lda, n,
+                                                                   reinterpret_cast<T*>(w.dinv));
   *launches += 2;
   return BEM2D_OK;
 }
