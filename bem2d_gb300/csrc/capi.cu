@@ -2382,7 +2382,10 @@ int bem2d_eigenvalues(bem2d_ctx* c, int n, const void* A, int64_t lda, void* w) 
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
       sms < 1)
     sms = 1;
-  c->launches += launch_eigenvalues(H, n, work, dw, sms, c->stream);
+  const long long nl = launch_eigenvalues(H, n, work, dw, sms, c->stream);
+  if (nl < 0)
+    return fail(c, BEM2D_ERR_CUDA, "QR launch: %s", cudaGetErrorString(cudaGetLastError()));
+  c->launches += nl;
   CHECK_LAUNCH(c);
   int status = 0;
   CUDA_TRY(c, cudaMemcpyAsync(&status, eig_status_ptr(work, n), sizeof(int),
@@ -2425,7 +2428,10 @@ int bem2d_eigenvectors(bem2d_ctx* c, int n, const void* A, int64_t lda, void* w,
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
       sms < 1)
     sms = 1;
-  c->launches += launch_eigenvalues(H, n, work, dw, sms, c->stream, Z);
+  const long long nl = launch_eigenvalues(H, n, work, dw, sms, c->stream, Z);
+  if (nl < 0)
+    return fail(c, BEM2D_ERR_CUDA, "QR launch: %s", cudaGetErrorString(cudaGetLastError()));
+  c->launches += nl;
   CHECK_LAUNCH(c);
   int status = 0;
   CUDA_TRY(c, cudaMemcpyAsync(&status, eig_status_ptr(work, n), sizeof(int),

@@ -570,12 +570,18 @@ int launch_bidiag_singular(double2* A, int n, void* work, double* out, int sms, 
                            long long* launches);
 int* bidiag_status_ptr(void* work);
 
-// ---- launch interfaces (eig.cu) --------------------------------------------
+// ---- launch interfaces (eig_qr.cu, eig.cu) -----------------------------------
+// Eigenvalues of the upper Hessenberg H (n x n, ld n, overwritten) into w;
+// *status: 0, or the number not found within the iteration limit.
+size_t hess_eigenvalues_work_bytes();
+int launch_hess_eigenvalues(double2* H, int n, double2* w, int* status, void* work,
+                            cudaStream_t s);
+
 // Work bytes of launch_eigenvalues for order n.
 size_t eig_work_bytes(int n);
 // Eigenvalues of the general A (n x n, ld n, overwritten by its Hessenberg
 // form and the QR iterates) into w (device, n complex128).  Returns the
-// number of kernels launched; eig_status_ptr(work, n) then holds 0 or the
+// number of kernels launched (-1: a launch failed); eig_status_ptr(work, n) then holds 0 or the
 // number of eigenvalues not found within the iteration limit.
 // Z (n x n, optional): if given, receives the Schur vectors (A on exit holds
 // the triangular Schur factor T).

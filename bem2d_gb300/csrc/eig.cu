@@ -10,8 +10,9 @@
 //    six launches per column: reflector, column-split products with a
 //    fixed-order reduction, rank-1 update from the right, one warp per
 //    column for v^H A, rank-1 update from the left.
-// 2. Implicitly shifted single-shift QR on the Hessenberg matrix (Golub &
-//    Van Loan, sec. 7.5), eigenvalues only: deflation where |h(k,k-1)| <=
+// 2. Eigenvalues only: eig_qr.cu.  With eigenvectors, implicitly shifted
+//    single-shift QR on the Hessenberg matrix (Golub & Van Loan, sec. 7.5):
+//    deflation where |h(k,k-1)| <=
 //    eps (|h(k-1,k-1)| + |h(k,k)|) (1-norms of the complex entries),
 //    Wilkinson shift from the trailing 2 x 2 block, an exceptional shift
 //    every tenth iteration on a block, 2 x 2 blocks solved in closed form,
@@ -67,13 +68,26 @@ __global__ void __launch_bounds__(kHessThreads)
 hess_house_kernel(double2* __restrict__ A, long long ld, int n, int j, double2* __restrict__ v,
                   double2* __restrict__ S) {
   __shared__ double red[kHessThreads / 32];
+  __shared__ unsigned rexp[kHessThreads / 32];
   __shared__ double2 sh_scale;
   __shared__ double sh_beta;
   const int m = n - j - 1;
   double2* x = A + (size_t)j * ld + (j + 1);
+  // entries are squared after a scaling by the power of two f that brings the
+  // largest near one
+  unsigned ex = 0;
+  for (int i = threadIdx.x; i < m; i += kHessThreads)
+    ex = max(ex, max((unsigned)__double2hiint(x[i].x) & 0x7ff00000u,
+                     (unsigned)__double2hiint(x[i].y) & 0x7ff00000u));
+  ex = __reduce_max_sync(0xffffffffu, ex);
+  if ((threadIdx.x & 31) == 0) rexp[threadIdx.x >> 5] = ex;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kHessThreads / 32; ++w) ex = max(ex, rexp[w]);
+  const double f = __hiloint2double(max(0x7fd00000 - (int)ex, 0x00100000), 0);
   double s = 0.0;
   for (int i = 1 + threadIdx.x; i < m; i += kHessThreads) {
-    const double2 xi = x[i];
+    const double2 xi = make_double2(x[i].x * f, x[i].y * f);
     s = fma(xi.x, xi.x, fma(xi.y, xi.y, s));
   }
 #pragma unroll
@@ -83,19 +97,20 @@ hess_house_kernel(double2* __restrict__ A, long long ld, int n, int j, double2* 
   if (threadIdx.x == 0) {
     double xn2 = 0.0;
     for (int w = 0; w < kHessThreads / 32; ++w) xn2 += red[w];
-    const double2 a = x[0];
+    const double2 a = make_double2(x[0].x * f, x[0].y * f);
     double2 tau, scale;
     double beta;
     if (xn2 == 0.0 && a.y == 0.0) {
       tau = make_double2(0.0, 0.0);
       scale = make_double2(0.0, 0.0);
-      beta = a.x;
+      beta = x[0].x;
     } else {
       beta = -copysign(sqrt(fma(a.x, a.x, fma(a.y, a.y, xn2))), a.x);
       tau = make_double2((beta - a.x) / beta, -a.y / beta);
       const double2 am = make_double2(a.x - beta, a.y);
-      const double q = fma(am.x, am.x, am.y * am.y);
+      const double q = fma(am.x, am.x, am.y * am.y) / f;
       scale = make_double2(am.x / q, -am.y / q);
+      beta /= f;
     }
     S[0] = tau;
     sh_scale = scale;
@@ -205,16 +220,14 @@ __device__ void eig2(double2 a, double2 b, double2 c, double2 d, double2* l1, do
   *l2 = make_double2(h.x - disc.x, h.y - disc.y);
 }
 
-// Shifted QR on the upper Hessenberg H (n x n, ld); eigenvalues into w as
-// they deflate (bottom up).  status[0] = 0, or the number of eigenvalues
-// not found when the iteration limit was reached.
-// VEC: the Schur form as well (zlahqr with wantt = wantz = true): every
-// rotation is applied to the whole rows (columns to n - 1) and the whole
-// columns (rows from 0) of H and to the columns of Z (n x n, ld, the
-// accumulated Hessenberg reduction on entry), and a deflated 2 x 2 block is
-// made upper triangular by one more rotation, so that on exit H holds the
-// upper triangular T with A = Z T Z^H and w[i] = T(i, i).
-template <bool VEC>
+// Shifted QR on the upper Hessenberg H (n x n, ld) to the Schur form (zlahqr
+// with wantt = wantz = true): every rotation is applied to the whole rows
+// (columns to n - 1) and the whole columns (rows from 0) of H and to the
+// columns of Z (n x n, ld, the accumulated Hessenberg reduction on entry), and
+// a deflated 2 x 2 block is made upper triangular by one more rotation, so
+// that on exit H holds the upper triangular T with A = Z T Z^H and w[i] =
+// T(i, i).  status[0] = 0, or the number of eigenvalues not found when the
+// iteration limit was reached.
 __global__ void __launch_bounds__(kQrThreads)
 hess_qr_kernel(double2* __restrict__ H, long long ld, int n, double2* __restrict__ w,
                int* __restrict__ status, double2* __restrict__ Z) {
@@ -257,7 +270,7 @@ hess_qr_kernel(double2* __restrict__ H, long long ld, int n, double2* __restrict
       } else if (lo == hi - 1) {
         double2 l1, l2;
         eig2(at(hi - 1, hi - 1), at(hi - 1, hi), at(hi, hi - 1), at(hi, hi), &l1, &l2);
-        if (VEC) {
+        {
           // rotation whose first column is the unit eigenvector of the block
           // for l1: (b, l1 - a) or (l1 - d, c), the better scaled one
           const double2 a = at(hi - 1, hi - 1), b = at(hi - 1, hi), cc = at(hi, hi - 1),
@@ -273,11 +286,6 @@ hess_qr_kernel(double2* __restrict__ H, long long ld, int n, double2* __restrict
           s_g0 = r > 0 ? make_double2(x.x / r, x.y / r) : make_double2(1.0, 0.0);
           s_g1 = r > 0 ? make_double2(y.x / r, y.y / r) : make_double2(0.0, 0.0);
           s_mode = 2;
-        } else {
-          w[hi - 1] = l1;
-          w[hi] = l2;
-          s_hi = hi - 2;
-          s_mode = 0;
         }
         its = 0;
       } else if (++total > itmax) {
@@ -308,7 +316,7 @@ hess_qr_kernel(double2* __restrict__ H, long long ld, int n, double2* __restrict
     }
     __syncthreads();
     if (s_mode == 0) continue;  // uniform: every thread read the same flag
-    if (VEC && s_mode == 2) {
+    if (s_mode == 2) {
       // triangularise the deflated 2 x 2 block at rows / columns hi-1, hi
       // with G = [g0 -conj(g1); g1 conj(g0)]: rows (all columns from hi-1)
       // by G^H, columns (rows 0..hi) and Z's columns by G
@@ -380,10 +388,9 @@ hess_qr_kernel(double2* __restrict__ H, long long ld, int n, double2* __restrict
       const double c = s_c;
       const double2 s = s_s;
       const double2 sc = cconjd(s);
-      // rows k, k+1, columns max(lo, k-1)..hi (..n-1 with VEC):
+      // rows k, k+1, columns max(lo, k-1)..n-1:
       // (h1, h2) <- (c h1 + s h2, -conj(s) h1 + c h2)
-      const int jend = VEC ? n - 1 : hi;
-      for (int jc = max(lo, k - 1) + tid; jc <= jend; jc += kQrThreads) {
+      for (int jc = max(lo, k - 1) + tid; jc < n; jc += kQrThreads) {
         const double2 h1 = at(k, jc), h2 = at(k + 1, jc);
         const double2 n1 = cfma(s, h2, make_double2(c * h1.x, c * h1.y));
         const double2 n2 = cfms(make_double2(c * h2.x, c * h2.y), sc, h1);
@@ -392,24 +399,23 @@ hess_qr_kernel(double2* __restrict__ H, long long ld, int n, double2* __restrict
       }
       __syncthreads();
       if (tid == 0 && k > lo) at(k + 1, k - 1) = make_double2(0.0, 0.0);
-      // columns k, k+1, rows lo..min(k+2, hi) (from 0 with VEC):
+      // columns k, k+1, rows 0..min(k+2, hi):
       // (h1, h2) <- (c h1 + conj(s) h2, -s h1 + c h2)
       const int i1 = min(k + 2, hi);
-      for (int i = (VEC ? 0 : lo) + tid; i <= i1; i += kQrThreads) {
+      for (int i = tid; i <= i1; i += kQrThreads) {
         const double2 h1 = at(i, k), h2 = at(i, k + 1);
         const double2 n1 = cfma(sc, h2, make_double2(c * h1.x, c * h1.y));
         const double2 n2 = cfms(make_double2(c * h2.x, c * h2.y), s, h1);
         at(i, k) = n1;
         at(i, k + 1) = n2;
       }
-      if (VEC) {  // the Schur vectors: columns k, k+1 of Z, the same rotation
-        for (int i = tid; i < n; i += kQrThreads) {
-          double2* z1 = Z + (size_t)k * ld + i;
-          double2* z2 = Z + (size_t)(k + 1) * ld + i;
-          const double2 h1 = *z1, h2 = *z2;
-          *z1 = cfma(sc, h2, make_double2(c * h1.x, c * h1.y));
-          *z2 = cfms(make_double2(c * h2.x, c * h2.y), s, h1);
-        }
+      // the Schur vectors: columns k, k+1 of Z, the same rotation
+      for (int i = tid; i < n; i += kQrThreads) {
+        double2* z1 = Z + (size_t)k * ld + i;
+        double2* z2 = Z + (size_t)(k + 1) * ld + i;
+        const double2 h1 = *z1, h2 = *z2;
+        *z1 = cfma(sc, h2, make_double2(c * h1.x, c * h1.y));
+        *z2 = cfms(make_double2(c * h2.x, c * h2.y), s, h1);
       }
       __syncthreads();
     }
@@ -519,7 +525,7 @@ size_t eig_work_bytes(int n) {
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
   // v, u, w (n complex each) | P (kGvSplit * n complex) | S (4 complex) | status
   return 3 * up(sizeof(double2) * n) + up(sizeof(double2) * (size_t)kGvSplit * n) +
-         up(sizeof(double2) * 4) + up(sizeof(int) * 4);
+         up(sizeof(double2) * 4) + 256 + up(hess_eigenvalues_work_bytes());
 }
 
 long long launch_eigenvalues(double2* A, int n, void* work, double2* w, int sms,
@@ -572,9 +578,9 @@ long long launch_eigenvalues(double2* A, int n, void* work, double2* w, int sms,
     }
   }
   if (Z)
-    hess_qr_kernel<true><<<1, kQrThreads, 0, s>>>(A, ld, n, w, status, Z);
-  else
-    hess_qr_kernel<false><<<1, kQrThreads, 0, s>>>(A, ld, n, w, status, nullptr);
+    hess_qr_kernel<<<1, kQrThreads, 0, s>>>(A, ld, n, w, status, Z);
+  else if (launch_hess_eigenvalues(A, n, w, status, status + 64, s) != BEM2D_OK)
+    return -1;
   return launches + 1;
 }
 

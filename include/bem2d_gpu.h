@@ -279,16 +279,17 @@ int bem2d_hermitian_eigenvalues(bem2d_ctx* ctx, int n, const void* A, int64_t ld
  * n <= BEM2D_SPECTRA_MAX_N / 2. */
 int bem2d_singular_values(bem2d_ctx* ctx, int n, const void* A, int64_t lda, double* s);
 
-/* Largest order bem2d_eigenvalues accepts: its QR iteration runs on one
- * CTA, about n^2 dependent rotation steps of a few microseconds each. */
+/* Largest order bem2d_eigenvalues and bem2d_eigenvectors accept: about n^2 /
+ * 10 (eigenvalues alone) or n^2 (with eigenvectors, one CTA) dependent
+ * rotation steps of a few microseconds each. */
 #define BEM2D_EIG_MAX_N 4096
 
 /* w[0..n-1] (complex128) = eigenvalues of the general complex A: replaces
  * Eigenvalues(const Matrix&, pcvector&) (lib/bem2d_mathroutines.cpp:437-466,
  * zgeev without eigenvectors).  Householder reduction to upper Hessenberg
- * form on the GPU (six kernels per column), then implicitly shifted QR
- * (Wilkinson shifts, exceptional shifts, closed-form 2 x 2 blocks) in one
- * CTA; no balancing.  Eigenvalues come in the order they deflate (bottom of
+ * form on the GPU (six kernels per column), then implicitly shifted QR (up
+ * to 16 pipelined sweeps whose shifts are the trailing block's eigenvalues,
+ * exceptional shifts) in one thread-block cluster; no balancing.  Eigenvalues come in the order they deflate (bottom of
  * the matrix first), as in LAPACK's QR.  BEM2D_ERR_NOCONV if the iteration
  * limit 30 max(10, n) is reached.  A: host or device (not modified);
  * w: host or device. */
