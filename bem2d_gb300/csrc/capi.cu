@@ -1383,7 +1383,7 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
                             double* lam_out, T* ritz, bool full_reorth = true,
                             double rtol = 0.0, double etol = 0.0,
                             const double* gap_in = nullptr, double* gap_out = nullptr,
-                            const float2* ffhi = nullptr, const float2* fflo = nullptr) {
+                            int digits = sizeof(T) == sizeof(double2) ? 8 : 4) {
   int rc = 0;
   const long long qs = (long long)n * (mmax + 1);  // per-angle basis stride
   T* Q = static_cast<T*>(ws(c, LzNames<T>::Q, sizeof(T) * (size_t)qs * nang, &rc));
@@ -1418,7 +1418,9 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
   std::vector<std::vector<double>> al(nang), be(nang);
   std::vector<double> lam(nang, 0.0), prev(nang, NAN), dlam(nang, 0.0);
   std::vector<int> stable(nang, 0);
-  std::vector<T> hh((size_t)(mmax + 2) * nang);
+  std::vector<T> hh((size_t)(mmax + 2) * nang), hal(nang);
+  T* dal = static_cast<T*>(ws(c, "nr_al", sizeof(double2) * nang, &rc));
+  if (!dal) return rc;
   const int ldh = mmax + 2;
   int steps = 0;
   // Deflation: an angle whose value has converged leaves the batch (its
@@ -1434,15 +1436,30 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
   int* dmap = static_cast<int*>(ws(c, "nr_map", sizeof(int) * 2 * nang, &rc));
   double* dthc = static_cast<double*>(ws(c, "nr_thc", sizeof(double) * nang, &rc));
   if (!Qalt || !Walt || !dmap || !dthc) return rc;
-  // K-split partials of the products: the most any batch width needs
+  // the products with A and A^H: digits packed once, on the tensor cores;
+  // without room for the two packed copies, on the CUDA cores
   size_t zwork_bytes = 0;
-  for (int m = 1; m <= nang; ++m) zwork_bytes = std::max(zwork_bytes, zgemm_work_bytes(n, m, sizeof(T)));
-  void* zwork = zwork_bytes ? ws(c, LzNames<T>::Z, zwork_bytes, &rc) : nullptr;
-  if (zwork_bytes && !zwork) return rc;
-  float2* ffb = nullptr;  // B's float-float split for the products
-  if (ffhi) {
-    ffb = static_cast<float2*>(ws(c, "nr_ffb", 2 * sizeof(float2) * (size_t)n * nang, &rc));
-    if (!ffb) return rc;
+  for (int m = 1; m <= nang; ++m)
+    zwork_bytes = std::max(zwork_bytes, oz_gemm_work_bytes(n, m, digits, sizeof(T)));
+  const size_t pa = oz_gemm_a_bytes(n, digits);
+  char* oz = static_cast<char*>(ws(c, "nr_oz", 2 * pa + 256, &rc));
+  void* zwork = oz ? ws(c, LzNames<T>::Z, zwork_bytes, &rc) : nullptr;
+  int* oz_status = reinterpret_cast<int*>(oz + 2 * pa);
+  if (oz && zwork) {
+    launch_oz_pack(false, digits, dA, la, n, oz, c->stream);
+    launch_oz_pack(true, digits, dA, la, n, oz + pa, c->stream);
+    CUDA_TRY(c, cudaMemsetAsync(oz_status, 0, sizeof(int), c->stream));
+    c->launches += 4;
+    CHECK_LAUNCH(c);
+  } else {
+    cudaGetLastError();
+    rc = 0;
+    oz = nullptr;
+    zwork_bytes = 0;
+    for (int m = 1; m <= nang; ++m)
+      zwork_bytes = std::max(zwork_bytes, zgemm_work_bytes(n, m, sizeof(T)));
+    zwork = zwork_bytes ? ws(c, LzNames<T>::Z, zwork_bytes, &rc) : nullptr;
+    if (zwork_bytes && !zwork) return rc;
   }
   std::vector<double> th_h(nang);
   CUDA_TRY(c, cudaMemcpyAsync(th_h.data(), dth, sizeof(double) * nang, cudaMemcpyDeviceToHost,
@@ -1485,16 +1502,11 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
   };
   for (int j = 0; j < mmax; ++j) {
     const T* Qj = Q + (size_t)j * n;
-    if constexpr (sizeof(T) == sizeof(double2)) {
-      if (ffhi) {  // the products in float-float on the FP32 pipe
-        launch_zgemm_ff(false, ffhi, fflo, n, Qj, qs, na, Y1, n, zwork, zwork_bytes, ffb,
-                        c->stream);
-        launch_zgemm_ff(true, ffhi, fflo, n, Qj, qs, na, Y2, n, zwork, zwork_bytes, ffb,
-                        c->stream);
-      } else {
-        launch_zgemm(false, dA, la, n, Qj, qs, na, Y1, n, zwork, zwork_bytes, c->stream);
-        launch_zgemm(true, dA, la, n, Qj, qs, na, Y2, n, zwork, zwork_bytes, c->stream);
-      }
+    if (oz) {
+      if ((rc = launch_oz_gemm_pair(digits, oz, oz + pa, n, Qj, qs, na, Y1, Y2, n, zwork,
+                                    oz_status, c->stream)))
+        return fail(c, rc, "product launch: %s", cudaGetErrorString(cudaGetLastError()));
+      c->launches += 2;
     } else {
       launch_zgemm(false, dA, la, n, Qj, qs, na, Y1, n, zwork, zwork_bytes, c->stream);
       launch_zgemm(true, dA, la, n, Qj, qs, na, Y2, n, zwork, zwork_bytes, c->stream);
@@ -1506,18 +1518,21 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
     const int w0 = full_reorth ? 0 : std::max(0, j - 1), nw = j + 1 - w0;
     const T* Qw = Q + (size_t)w0 * n;
     launch_batched_dots(Qw, qs, n, nw, W, n, h, ldh, na, c->stream);
-    CUDA_TRY(c, cudaMemcpyAsync(hh.data(), h, sizeof(T) * (size_t)ldh * na, cudaMemcpyDeviceToHost, c->stream));
+    // alpha_j, one value per angle (the second pass below overwrites h)
+    CUDA_TRY(c, cudaMemcpy2DAsync(dal, sizeof(T), h + (j - w0), sizeof(T) * ldh, sizeof(T), na,
+                                  cudaMemcpyDeviceToDevice, c->stream));
     launch_batched_sub(Qw, qs, n, nw, W, n, h, ldh, na, c->stream);
     launch_batched_dots(Qw, qs, n, nw, W, n, h, ldh, na, c->stream);
     launch_batched_sub(Qw, qs, n, nw, W, n, h, ldh, na, c->stream);
     launch_batched_norm2(n, W, n, sc, na, c->stream);
+    CUDA_TRY(c, cudaMemcpyAsync(hal.data(), dal, sizeof(T) * na, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(nn.data(), sc, sizeof(double) * na, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->launches += 8;
     CHECK_LAUNCH(c);
     steps = j + 1;
     for (int a = 0; a < na; ++a) {
-      al[a].push_back(hh[(size_t)a * ldh + (j - w0)].x);
+      al[a].push_back(hal[a].x);
       const double b = std::sqrt(nn[a]);
       inv[a] = b > 1e-300 ? 1.0 / b : 0.0;
       // Ritz values interlace: the previous value bounds the new one below.
@@ -1627,6 +1642,12 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
     rest.push_back(a);
   }
   if ((rc = emit_ritz(rest, steps))) return rc;
+  if (oz) {
+    int st = 0;
+    CUDA_TRY(c, cudaMemcpyAsync(&st, oz_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    if (st) return fail(c, BEM2D_ERR_TIMEOUT, "tensor-core product wait timed out");
+  }
   return BEM2D_OK;
 }
 
@@ -1879,22 +1900,17 @@ int bem2d_l2_norm_cond_prec(bem2d_ctx* c, int n, const void* A, int64_t lda, dou
   // A split once, 16 n^2 bytes)
   float2* Ahi = nullptr;
   float2* Alo = nullptr;
-  float2* ffb = nullptr;
-  void* ffw = nullptr;
-  const size_t ffw_bytes = zgemm_work_bytes(n, 1, sizeof(double2));
   if (mixed) {
     Ahi = static_cast<float2*>(ws(c, "nc_Ahi", sizeof(float2) * (size_t)n * n, &rc));
     Alo = static_cast<float2*>(ws(c, "nc_Alo", sizeof(float2) * (size_t)n * n, &rc));
-    ffb = static_cast<float2*>(ws(c, "nc_ffb", 2 * sizeof(float2) * (size_t)n, &rc));
-    ffw = ws(c, "nc_ffw", ffw_bytes + 256, &rc);
-    if (!Ahi || !Alo || !ffb || !ffw) return rc;
+    if (!Ahi || !Alo) return rc;
     launch_split_ff(dA, la, n, Ahi, Alo, c->stream);
     ++c->launches;
   }
   auto op = [&](const double2* x, double2* y) -> int {
     if (mixed) {
-      launch_zgemm_ff(false, Ahi, Alo, n, x, n, 1, y, n, ffw, ffw_bytes, ffb, c->stream);
-      c->launches += 3;
+      launch_mv_ff(false, Ahi, Alo, n, x, y, part, c->stream);
+      c->launches += 2;
     } else {
       launch_mv(dA, la, n, x, y, part, c->stream);
       c->launches += 2;
@@ -1903,8 +1919,8 @@ int bem2d_l2_norm_cond_prec(bem2d_ctx* c, int n, const void* A, int64_t lda, dou
   };
   auto oph = [&](const double2* x, double2* y) -> int {
     if (mixed) {
-      launch_zgemm_ff(true, Ahi, Alo, n, x, n, 1, y, n, ffw, ffw_bytes, ffb, c->stream);
-      c->launches += 3;
+      launch_mv_ff(true, Ahi, Alo, n, x, y, part, c->stream);
+      c->launches += 1;
     } else {
       launch_mvh(dA, la, n, x, y, c->stream);
       c->launches += 1;
@@ -2260,16 +2276,10 @@ int bem2d_num_range(bem2d_ctx* c, int n, const void* A, int64_t lda, int nang,
   for (int a = 0; a < nang; ++a) gap[a] = std::max(0.0, 0.25 * gap[a] - 1e-6 * hs);
   launch_widen(n, R32, n, S64, n, nang, c->stream);
   ++c->launches;
-  // the complex128 phase's products in float-float (~1e-13 relative to
-  // |A| |x|, a hundred times below tol): A split once into fl32(A) and the
-  // rest, 16 N^2 bytes
-  float2* Ahi = static_cast<float2*>(ws(c, "nr_Ahi", sizeof(float2) * (size_t)n * n, &rc));
-  float2* Alo = static_cast<float2*>(ws(c, "nr_Alo", sizeof(float2) * (size_t)n * n, &rc));
-  if (!Ahi || !Alo) return rc;
-  launch_split_ff(dA, la, n, Ahi, Alo, c->stream);
-  ++c->launches;
+  // the complex128 phase's products with 7 digits (2^-51 of row maximum x
+  // column maximum, a thousand times below tol)
   return numrange_lanczos<double2>(c, n, dA, la, nang, dth, tol, mmax, S64, lmax, nullptr, true,
-                                   0.0, tol, gap.data(), nullptr, Ahi, Alo);
+                                   0.0, tol, gap.data(), nullptr, 7);
 }
 
 }  // extern "C"

@@ -305,17 +305,19 @@ static void zgemm_t(bool herm, const T* A, long long lda, int n, const T* B, lon
   else
     zgemm_bn_t<T, 64>(herm, A, lda, n, B, ldb, m, C, ldc, P, z, s);
 }
-// ---- complex GEMM in float-float on the FP32 pipe ----------------------------
-// C = op(A) B for complex128 data whose products are wanted to ~1e-13
-// relative (the second, FP64-accurate phase of the numerical range), on the
-// FP32 pipe, which issues 64x the FP64 pipe's FMAs on GB300.  A is given
-// split once into A_hi = fl32(A), A_lo = fl32(A - A_hi) (float2 each); B is
-// split while it is staged.  Per complex multiply-add the four hi*hi real
-// products are exact as two-products (p + e) and accumulated with two-sum
-// into a float-float sum; the hi*lo and lo*hi terms (2^-24 of the main ones)
-// and the two-product errors go into a plain FP32 companion sum; lo*lo
-// (2^-48) is dropped.  Result: hi + lo + companion, in FP64.  Partial sums
-// of a K split are reduced in FP64.
+
+// Matrix-vector products in float-float arithmetic, accurate to ~1e-13
+// relative to |A| |x| (sigma_max of the mixed norm / condition number), on the
+// FP32 pipe, which issues 64x the FP64 pipe's FMAs on GB300.  A is given split
+// once into A_hi = fl32(A), A_lo = fl32(A - A_hi) (float2 each).  Per complex
+// multiply-add the four hi*hi real products are exact as two-products (p + e)
+// and accumulated with two-sum into a float-float sum; the hi*lo and lo*hi
+// terms (2^-24 of the main ones) and the two-product errors go into a plain
+// FP32 companion sum; lo*lo (2^-48) is dropped.  Result: hi + lo + companion,
+// in FP64; partial sums are added in FP64.  About 44 FP32 instructions per
+// entry: bound by the one pass over the split matrix (16 n^2 bytes).  n =
+// 8192: 0.20 ms for A x, 0.27 for A^H x (a 64 x 4 tile of a matrix product took 0.62 and 0.94 ms, three
+// quarters of it for columns that are not there).
 struct FfAcc {
   float hi, lo, x;  // value = hi + lo + x
 };
@@ -327,127 +329,97 @@ __device__ __forceinline__ void ffacc_add(FfAcc& a, float p) {
   a.hi = s;
 }
 
-template <bool HERM, int BN>
+// re += ar br - ai bi, im += ar bi + ai br
+__device__ __forceinline__ void ffacc_cmul(FfAcc& re, FfAcc& im, float2 ah, float2 al, float2 bh,
+                                           float2 bl) {
+  const float p1 = __fmul_rn(ah.x, bh.x), p2 = __fmul_rn(ah.y, bh.y);
+  const float p3 = __fmul_rn(ah.x, bh.y), p4 = __fmul_rn(ah.y, bh.x);
+  float xr = fmaf(ah.x, bh.x, -p1) - fmaf(ah.y, bh.y, -p2);
+  float xi = fmaf(ah.x, bh.y, -p3) + fmaf(ah.y, bh.x, -p4);
+  xr = fmaf(ah.x, bl.x, xr);
+  xr = fmaf(al.x, bh.x, xr);
+  xr = fmaf(-ah.y, bl.y, xr);
+  xr = fmaf(-al.y, bh.y, xr);
+  xi = fmaf(ah.x, bl.y, xi);
+  xi = fmaf(al.x, bh.y, xi);
+  xi = fmaf(ah.y, bl.x, xi);
+  xi = fmaf(al.y, bh.x, xi);
+  ffacc_add(re, p1);
+  ffacc_add(re, -p2);
+  ffacc_add(im, p3);
+  ffacc_add(im, p4);
+  re.x += xr;
+  im.x += xi;
+}
+__device__ __forceinline__ double ffacc_value(const FfAcc& a) {
+  return (double)a.hi + ((double)a.lo + (double)a.x);
+}
+__device__ __forceinline__ void ff_split(double2 d, float2* h, float2* l) {
+  *h = make_float2((float)d.x, (float)d.y);
+  *l = make_float2((float)(d.x - (double)h->x), (float)(d.y - (double)h->y));
+}
+
+// part[c][r]: chunk c of kMvChunk columns of A x, one thread per row.
+__global__ void __launch_bounds__(128)
+mv_ff_partial_kernel(const float2* __restrict__ Ahi, const float2* __restrict__ Alo, int n,
+                     const double2* __restrict__ x, double2* __restrict__ part) {
+  __shared__ float2 xh[kMvChunk], xl[kMvChunk];
+  const int c0 = blockIdx.y * kMvChunk, nc = min(kMvChunk, n - c0);
+  for (int v = threadIdx.x; v < nc; v += blockDim.x) ff_split(x[c0 + v], &xh[v], &xl[v]);
+  __syncthreads();
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  FfAcc re{0.f, 0.f, 0.f}, im{0.f, 0.f, 0.f};
+  const size_t o = (size_t)c0 * n + r;
+#pragma unroll 8
+  for (int c = 0; c < nc; ++c)
+    ffacc_cmul(re, im, Ahi[o + (size_t)c * n], Alo[o + (size_t)c * n], xh[c], xl[c]);
+  part[(size_t)blockIdx.y * n + r] = make_double2(ffacc_value(re), ffacc_value(im));
+}
+
+// y = A^H x: a warp per column, lanes over rows, x split once per CTA in
+// chunks.
 __global__ void __launch_bounds__(256)
-zgemm_ff_kernel(const float2* __restrict__ Ahi, const float2* __restrict__ Alo, long long lda,
-                int n, const float2* __restrict__ Bhi, const float2* __restrict__ Blo, long long ldb,
-                int m, double2* __restrict__ C, long long ldc, int kchunk, long long cz,
-                int rows) {
-  constexpr int TY = BN >= 16 ? 16 : BN, TX = 256 / TY, RA = 64 / TX, RB = BN / TY;
-  constexpr int LA = 16 * 64 / 256, LB = (16 * BN + 255) / 256;  // staged entries per thread
-  __shared__ float2 Ah[16][64 + 1], Al[16][64 + 1];
-  __shared__ float2 Bh[16][BN + 1], Bl[16][BN + 1];
-  const int i0 = blockIdx.x * 64, j0 = blockIdx.y * BN;
-  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-  const int kb = blockIdx.z * kchunk, ke = min(n, kb + kchunk);
-  double2* Cz = C + (size_t)blockIdx.z * cz;
-  FfAcc re[RA][RB], im[RA][RB];
-#pragma unroll
-  for (int a = 0; a < RA; ++a)
-#pragma unroll
-    for (int b = 0; b < RB; ++b) re[a][b] = im[a][b] = FfAcc{0.f, 0.f, 0.f};
-  // the next chunk's entries, loaded while the current chunk is computed
-  float2 nah[LA], nal[LA], nbh[LB], nbl[LB];
-  auto load = [&](int k0) {
-#pragma unroll
-    for (int u = 0; u < LA; ++u) {
-      const int v = threadIdx.x + 256 * u, kk = v / 64, ii = v - kk * 64;
-      const int i = i0 + ii, k = k0 + kk;
-      float2 h = make_float2(0.f, 0.f), l = h;
-      if (i < rows && k < ke) {
-        const size_t o = HERM ? (size_t)i * lda + k : (size_t)k * lda + i;
-        h = Ahi[o];
-        l = Alo[o];
-        if (HERM) {  // (A^H)_{ik} = conj(A_{ki})
-          h.y = -h.y;
-          l.y = -l.y;
-        }
-      }
-      nah[u] = h;
-      nal[u] = l;
-    }
-#pragma unroll
-    for (int u = 0; u < LB; ++u) {
-      const int v = threadIdx.x + 256 * u, jj = v / 16, kk = v - jj * 16;
-      const int j = j0 + jj, k = k0 + kk;
-      const bool ok = v < 16 * BN && j < m && k < ke;
-      nbh[u] = ok ? Bhi[(size_t)j * ldb + k] : make_float2(0.f, 0.f);
-      nbl[u] = ok ? Blo[(size_t)j * ldb + k] : make_float2(0.f, 0.f);
-    }
-  };
-  load(kb);
-  for (int k0 = kb; k0 < ke; k0 += 16) {
-#pragma unroll
-    for (int u = 0; u < LA; ++u) {
-      const int v = threadIdx.x + 256 * u, kk = v / 64, ii = v - kk * 64;
-      Ah[kk][ii] = nah[u];
-      Al[kk][ii] = nal[u];
-    }
-#pragma unroll
-    for (int u = 0; u < LB; ++u) {
-      const int v = threadIdx.x + 256 * u, jj = v / 16, kk = v - jj * 16;
-      if (v < 16 * BN) {
-        Bh[kk][jj] = nbh[u];
-        Bl[kk][jj] = nbl[u];
-      }
-    }
+mvh_ff_kernel(const float2* __restrict__ Ahi, const float2* __restrict__ Alo, int n,
+              const double2* __restrict__ x, double2* __restrict__ y) {
+  constexpr int kChunk = 1024;
+  __shared__ float2 xh[kChunk], xl[kChunk];
+  const int j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  FfAcc re{0.f, 0.f, 0.f}, im{0.f, 0.f, 0.f};
+  const size_t o = (size_t)j * n;
+  for (int r0 = 0; r0 < n; r0 += kChunk) {
+    const int nr = min(kChunk, n - r0);
     __syncthreads();
-    if (k0 + 16 < ke) load(k0 + 16);
-#pragma unroll 2
-    for (int kk = 0; kk < 16; ++kk) {
-      float2 ah[RA], al[RA], bh[RB], bl[RB];
-#pragma unroll
-      for (int a = 0; a < RA; ++a) {
-        ah[a] = Ah[kk][tx + TX * a];
-        al[a] = Al[kk][tx + TX * a];
-      }
-#pragma unroll
-      for (int b = 0; b < RB; ++b) {
-        bh[b] = Bh[kk][ty + TY * b];
-        bl[b] = Bl[kk][ty + TY * b];
-      }
-#pragma unroll
-      for (int a = 0; a < RA; ++a)
-#pragma unroll
-        for (int b = 0; b < RB; ++b) {
-          // re += ar br - ai bi,  im += ar bi + ai br
-          const float p1 = __fmul_rn(ah[a].x, bh[b].x), p2 = __fmul_rn(ah[a].y, bh[b].y);
-          const float p3 = __fmul_rn(ah[a].x, bh[b].y), p4 = __fmul_rn(ah[a].y, bh[b].x);
-          float xr = fmaf(ah[a].x, bh[b].x, -p1) - fmaf(ah[a].y, bh[b].y, -p2);
-          float xi = fmaf(ah[a].x, bh[b].y, -p3) + fmaf(ah[a].y, bh[b].x, -p4);
-          xr = fmaf(ah[a].x, bl[b].x, xr);
-          xr = fmaf(al[a].x, bh[b].x, xr);
-          xr = fmaf(-ah[a].y, bl[b].y, xr);
-          xr = fmaf(-al[a].y, bh[b].y, xr);
-          xi = fmaf(ah[a].x, bl[b].y, xi);
-          xi = fmaf(al[a].x, bh[b].y, xi);
-          xi = fmaf(ah[a].y, bl[b].x, xi);
-          xi = fmaf(al[a].y, bh[b].x, xi);
-          ffacc_add(re[a][b], p1);
-          ffacc_add(re[a][b], -p2);
-          ffacc_add(im[a][b], p3);
-          ffacc_add(im[a][b], p4);
-          re[a][b].x += xr;
-          im[a][b].x += xi;
-        }
-    }
+    for (int v = threadIdx.x; v < nr; v += blockDim.x) ff_split(x[r0 + v], &xh[v], &xl[v]);
     __syncthreads();
-  }
-#pragma unroll
-  for (int b = 0; b < RB; ++b) {
-    const int j = j0 + ty + TY * b;
-    if (j >= m) continue;
-#pragma unroll
-    for (int a = 0; a < RA; ++a) {
-      const int i = i0 + tx + TX * a;
-      if (i < rows) {
-        const FfAcc& r = re[a][b];
-        const FfAcc& q = im[a][b];
-        Cz[(size_t)j * ldc + i] = make_double2((double)r.hi + ((double)r.lo + (double)r.x),
-                                               (double)q.hi + ((double)q.lo + (double)q.x));
+    if (j < n) {
+#pragma unroll 4
+      for (int r = lane; r < nr; r += 32) {
+        float2 h = Ahi[o + r0 + r], l = Alo[o + r0 + r];
+        h.y = -h.y;
+        l.y = -l.y;
+        ffacc_cmul(re, im, h, l, xh[r], xl[r]);
       }
     }
   }
+  double sr = ffacc_value(re), si = ffacc_value(im);
+#pragma unroll
+  for (int q = 16; q > 0; q >>= 1) {
+    sr += __shfl_xor_sync(0xffffffffu, sr, q);
+    si += __shfl_xor_sync(0xffffffffu, si, q);
+  }
+  if (lane == 0 && j < n) y[j] = make_double2(sr, si);
+}
+
+void launch_mv_ff(bool herm, const float2* Ahi, const float2* Alo, int n, const double2* x,
+                  double2* y, double2* part, cudaStream_t s) {
+  if (herm) {
+    mvh_ff_kernel<<<(n + 7) / 8, 256, 0, s>>>(Ahi, Alo, n, x, y);
+    return;
+  }
+  const int nchunk = (n + kMvChunk - 1) / kMvChunk;
+  mv_ff_partial_kernel<<<dim3((n + 127) / 128, nchunk), 128, 0, s>>>(Ahi, Alo, n, x, part);
+  mv_final_kernel<double2><<<(n + 255) / 256, 256, 0, s>>>(n, nchunk, part, y);
 }
 
 // hi / lo (rows x cols, ld rows) = the float-float split of S (complex128,
@@ -468,45 +440,6 @@ __global__ void split_ff_kernel(const double2* __restrict__ S, long long lds, in
 void launch_split_ff(const double2* A, long long lda, int n, float2* hi, float2* lo,
                      cudaStream_t s) {
   split_ff_kernel<<<1024, 256, 0, s>>>(A, lda, n, n, hi, lo);
-}
-
-template <int BN>
-static void zgemm_ff_bn(bool herm, const float2* Ahi, const float2* Alo, int n, const float2* Bhi,
-                        const float2* Blo, int m, double2* C, long long ldc, double2* P, int z,
-                        cudaStream_t s) {
-  const int kchunk = ((n + z - 1) / z + 15) / 16 * 16;
-  dim3 g((n + 63) / 64, (m + BN - 1) / BN, z);
-  double2* out = z > 1 ? P : C;
-  const long long lo = z > 1 ? n : ldc, cz = z > 1 ? (long long)n * m : 0;
-  if (herm)
-    zgemm_ff_kernel<true, BN><<<g, 256, 0, s>>>(Ahi, Alo, n, n, Bhi, Blo, n, m, out, lo, kchunk,
-                                                cz, n);
-  else
-    zgemm_ff_kernel<false, BN><<<g, 256, 0, s>>>(Ahi, Alo, n, n, Bhi, Blo, n, m, out, lo, kchunk,
-                                                 cz, n);
-  if (z > 1)
-    zgemm_reduce_kernel<double2><<<dim3((n + 255) / 256, m), 256, 0, s>>>(P, cz, z, n, m, C, ldc);
-}
-
-void launch_zgemm_ff(bool herm, const float2* Ahi, const float2* Alo, int n, const double2* B,
-                     long long ldb, int m, double2* C, long long ldc, void* work,
-                     size_t work_bytes, float2* bsplit, cudaStream_t s) {
-  if (m <= 0 || n <= 0) return;
-  // B split once here, not once per row tile of the product
-  float2* Bhi = bsplit;
-  float2* Blo = bsplit + (size_t)n * m;
-  split_ff_kernel<<<std::min(1024, (int)(((long long)n * m + 255) / 256)), 256, 0, s>>>(
-      B, ldb, n, m, Bhi, Blo);
-  const int bn = zgemm_bn(m);
-  int z = zgemm_splits(n, m, bn);
-  if (z > 1 && work_bytes < sizeof(double2) * (size_t)z * n * m) z = 1;
-  double2* P = static_cast<double2*>(work);
-  if (bn == 4)
-    zgemm_ff_bn<4>(herm, Ahi, Alo, n, Bhi, Blo, m, C, ldc, P, z, s);
-  else if (bn == 16)
-    zgemm_ff_bn<16>(herm, Ahi, Alo, n, Bhi, Blo, m, C, ldc, P, z, s);
-  else
-    zgemm_ff_bn<64>(herm, Ahi, Alo, n, Bhi, Blo, m, C, ldc, P, z, s);
 }
 
 void launch_zgemm(bool herm, const double2* A, long long lda, int n, const double2* B,

@@ -30,16 +30,28 @@ void launch_zgemm(bool herm, const float2* A, long long lda, int n, const float2
                   long long ldb, int m, float2* C, long long ldc, void* work,
                   size_t work_bytes, cudaStream_t s);
 size_t zgemm_work_bytes(int n, int m, size_t elem);
-// C (n x m, ldc) = op(A) B in float-float on the FP32 pipe (~1e-13 relative
-// to |A| |B|): A (n x n) given as hi = fl32(A), lo = fl32(A - hi), ld n;
-// B, C complex128.  work: zgemm_work_bytes(n, m, sizeof(double2));
-// bsplit: 2 n m float2 of scratch for B's split.
-void launch_zgemm_ff(bool herm, const float2* Ahi, const float2* Alo, int n, const double2* B,
-                     long long ldb, int m, double2* C, long long ldc, void* work,
-                     size_t work_bytes, float2* bsplit, cudaStream_t s);
-// hi / lo (n x n, ld n) = the float-float split of A (complex128, ld lda)
+// y = A x or A^H x (herm) in float-float on the FP32 pipe (~1e-13 relative to
+// |A| |x|): A (n x n) given as hi = fl32(A), lo = fl32(A - hi), ld n; part:
+// mv_part_bytes(n) bytes.  launch_split_ff makes the split.
+void launch_mv_ff(bool herm, const float2* Ahi, const float2* Alo, int n, const double2* x,
+                  double2* y, double2* part, cudaStream_t s);
 void launch_split_ff(const double2* A, long long lda, int n, float2* hi, float2* lo,
                      cudaStream_t s);
+
+// Products with an n x n matrix through exact digit products on the tensor
+// cores (oz_gemm.cu): S digits, 8 or 7 for complex128 (FP64 and better than
+// float-float accuracy), 4 for complex64 (FP32).  launch_oz_pack packs A or
+// A^H (herm) once into oz_gemm_a_bytes(n, S); launch_oz_gemm_pair forms C1 = A
+// B and C2 = A^H B (B n x m, ldb) with oz_gemm_work_bytes(n, m, S, sizeof(T)) of
+// work.  Sets *status on a device-side wait timeout.
+size_t oz_gemm_a_bytes(int n, int S);
+size_t oz_gemm_work_bytes(int n, int m, int S, size_t elem);
+template <typename T>
+void launch_oz_pack(bool herm, int S, const T* A, long long lda, int n, void* dst, cudaStream_t s);
+template <typename T>
+int launch_oz_gemm_pair(int S, const void* Apk, const void* Ahpk, int n, const T* B, long long ldb,
+                        int m, T* C1, T* C2, long long ldc, void* work, int* status,
+                        cudaStream_t s);
 // C (rows x m, ldc) = A (rows x k, lda) B (k x m, ldb), complex128
 void launch_zgemm_rect(const double2* A, long long lda, int rows, int k, const double2* B,
                        long long ldb, int m, double2* C, long long ldc, cudaStream_t s);

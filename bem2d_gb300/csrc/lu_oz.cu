@@ -49,18 +49,18 @@
 // Measured against the FP64-pipe update it replaces: solve n = 3001 111.7 ->
 // 49.7 ms; error of one K = 64 product of Gaussian matrices 8 times smaller
 // (1.4e-13 against 1.2e-12, Frobenius; the same with entries spread over 2^10).
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
 #include "common.cuh"
-#include "tc.cuh"
+#include "oz.cuh"
 
 namespace bem2d_gpu {
 namespace {
 
 using namespace tc;
+using namespace oz;
 
 constexpr int kOzBM = 64;       // complex rows per tile (128 real rows = MMA M)
 constexpr int kOzBN = 16;       // complex columns per tile
@@ -79,70 +79,6 @@ constexpr int kOzBBytes = kOzKSteps * kOzBStep;    // 32 KB
 constexpr int kOzBarOff = kOzABytes + kOzStages * kOzBBytes;  // 192 KB
 constexpr int kOzSmem = kOzBarOff + 256;
 constexpr unsigned kOzAcc = 2 * kOzBN * kOzS;      // 256 TMEM columns
-
-// scale exponents: zero rows / columns, and rows / columns with a NaN or an
-// infinity
-constexpr int kOzZero = -100000, kOzNaN = 400000;
-
-// K-major, no swizzle: core matrices of 8 rows x 16 bytes, 128 bytes along K,
-// 256 bytes from one group of 8 rows to the next
-__device__ __forceinline__ unsigned long long oz_desc(unsigned addr) {
-  return (unsigned long long)((addr & 0x3FFFF) >> 4) | ((unsigned long long)(128 >> 4) << 16) |
-         ((unsigned long long)(256 >> 4) << 32) | (1ull << 46);
-}
-__device__ __forceinline__ int oz_off(int r, int k8) { return (r >> 3) * 256 + k8 * 128 + (r & 7) * 16; }
-
-__device__ __forceinline__ void oz_mma(unsigned d, unsigned a, unsigned b, unsigned idesc,
-                                       unsigned acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-      "l"(oz_desc(a)), "l"(oz_desc(b)), "r"(idesc), "r"(acc));
-}
-
-// exponent field of a double (0: zero or subnormal, 2047: not finite)
-__device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 2047; }
-
-__device__ __forceinline__ int scale_of(int emax, bool bad) {
-  return bad ? kOzNaN : emax <= -5000 ? kOzZero : emax;
-}
-
-// x 2^p as a fixed-point integer F (rounded toward zero), |F| < 2^63: x 2^p =
-// F 2^(erow - 1085), erow the largest exponent field plus p of the row, whose
-// largest entry has |F| >= 2^62.  Subnormals count as zero.
-__device__ __forceinline__ long long oz_fixed(double x, int p, int erow) {
-  const int e = expo(x);
-  if (e == 0) return 0;
-  const long long b = __double_as_longlong(x);
-  const long long m = (b & 0xfffffffffffffll) | 0x10000000000000ll;
-  const int d = erow - (e + p);  // >= 0
-  const long long f = d <= 10 ? m << (10 - d) : d < 63 ? m >> (d - 10) : 0;
-  return b < 0 ? -f : f;
-}
-
-// The 8 balanced digits of 8 consecutive k of one real row, as f16.
-struct OzDigits {
-  unsigned w[kOzS][4];
-};
-__device__ __forceinline__ void oz_digits(const long long* f, OzDigits* o) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    long long a = f[2 * q], b = f[2 * q + 1];
-#pragma unroll
-    for (int s = kOzS - 1; s >= 0; --s) {
-      const int da = s ? (int)(signed char)(a & 0xff) : (int)a;
-      const int db = s ? (int)(signed char)(b & 0xff) : (int)b;
-      a = (a - da) >> 8;
-      b = (b - db) >> 8;
-      // (1536 + d) - 1536 in f16: exact for |d| <= 512
-      const unsigned w = 0x66006600u + (unsigned)da + ((unsigned)db << 16);
-      const unsigned base = 0x66006600u;
-      const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&w),
-                                *reinterpret_cast<const __half2*>(&base));
-      o->w[s][q] = *reinterpret_cast<const unsigned*>(&h);
-    }
-  }
-}
 
 // ---- packing -------------------------------------------------------------------
 // Exponent p_k of inner index k: that of the pivot, entry k of column k of
@@ -175,28 +111,28 @@ oz_pack_a_kernel(const double2* __restrict__ A, long long lda, int M, int K, int
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int e = max(expo(v[q].x), expo(v[q].y));
-    if (e > 0) emax = max(emax, e == 2047 ? kOzNaN : e + pk[8 * c + q]);
+    if (e > 0) emax = max(emax, e == 2047 ? kNaN : e + pk[8 * c + q]);
   }
   red[c][il] = emax;
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < 8; ++q) emax = max(emax, red[q][il]);
-  const int er = scale_of(emax, emax > 50000);
+  const int er = scale_of(emax);
   if (c == 0 && i < M) ea[i] = er;
   if (c >= 2 * ksteps) return;
-  const bool use = er > kOzZero && er < kOzNaN;
+  const bool use = er > kZero && er < kNaN;
   unsigned char* blk = Apk + ((size_t)blockIdx.x * ksteps + (c >> 1)) * kOzAStep;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     long long f[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q)
-      f[q] = oz_fixed(!use ? 0.0 : h ? v[q].y : v[q].x, pk[8 * c + q], er);
-    OzDigits o;
-    oz_digits(f, &o);
+      f[q] = fixed<kOzS>(!use ? 0.0 : h ? v[q].y : v[q].x, pk[8 * c + q], er);
+    Digits<kOzS> o;
+    digits<kOzS>(f, &o);
 #pragma unroll
     for (int s = 0; s < kOzS; ++s)
-      *reinterpret_cast<uint4*>(blk + s * kOzABlk + oz_off(2 * il + h, c & 1)) =
+      *reinterpret_cast<uint4*>(blk + s * kOzABlk + off(2 * il + h, c & 1)) =
           make_uint4(o.w[s][0], o.w[s][1], o.w[s][2], o.w[s][3]);
   }
 }
@@ -218,25 +154,25 @@ oz_pack_b_kernel(const double2* __restrict__ B, long long ldb, int K, int N, int
     v[q] = (j < N && k < K) ? B[(size_t)j * ldb + k] : make_double2(0.0, 0.0);
     pk[q] = -oz_shift(piv, ldp, k, K);
     const int e = max(expo(v[q].x), expo(v[q].y));
-    if (e > 0) emax = max(emax, e == 2047 ? kOzNaN : e + pk[q]);
+    if (e > 0) emax = max(emax, e == 2047 ? kNaN : e + pk[q]);
   }
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
-  const int er = scale_of(emax, emax > 50000);
+  const int er = scale_of(emax);
   if (c == 0 && j < N) eb[j] = er;
   if (c >= 2 * ksteps) return;
-  const bool use = er > kOzZero && er < kOzNaN;
+  const bool use = er > kZero && er < kNaN;
   unsigned char* blk = Bpk + ((size_t)blockIdx.x * ksteps + (c >> 1)) * kOzBStep;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     long long f[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) f[q] = oz_fixed(!use ? 0.0 : h ? v[q].y : v[q].x, pk[q], er);
-    OzDigits o;
-    oz_digits(f, &o);
+    for (int q = 0; q < 8; ++q) f[q] = fixed<kOzS>(!use ? 0.0 : h ? v[q].y : v[q].x, pk[q], er);
+    Digits<kOzS> o;
+    digits<kOzS>(f, &o);
 #pragma unroll
     for (int s = 0; s < kOzS; ++s)
-      *reinterpret_cast<uint4*>(blk + s * kOzBBlk + oz_off(h * kOzBN + jl, c & 1)) =
+      *reinterpret_cast<uint4*>(blk + s * kOzBBlk + off(h * kOzBN + jl, c & 1)) =
           make_uint4(o.w[s][0], o.w[s][1], o.w[s][2], o.w[s][3]);
   }
 }
@@ -356,12 +292,8 @@ oz_zgemm_kernel(double2* __restrict__ C, long long ldc, const unsigned char* __r
         for (int k = 0; k < ksteps; ++k) {
 #pragma unroll
           for (int i = 0; i < kOzS; ++i) {
-            // kind::f16: D f32 (bits 4-5 = 1), A and B f16 (0), K-major,
-            // N >> 3 at bit 17, M >> 4 at bit 24
-            const unsigned nn = 2 * kOzBN * (kOzS - i);
-            const unsigned idesc = (1u << 4) | ((nn >> 3) << 17) | ((128u >> 4) << 24);
-            oz_mma(d + 2 * kOzBN * i, sa + k * kOzAStep + i * kOzABlk, sb + k * kOzBStep, idesc,
-                   (k == 0 && i == 0) ? 0u : 1u);
+            mma(d + 2 * kOzBN * i, sa + k * kOzAStep + i * kOzABlk, sb + k * kOzBStep,
+                2 * kOzBN * (kOzS - i), (k == 0 && i == 0) ? 0u : 1u);
           }
         }
         mma_commit(&empty[s]);
@@ -383,7 +315,7 @@ oz_zgemm_kernel(double2* __restrict__ C, long long ldc, const unsigned char* __r
     for (int tile = t0; tile < t1; ++tile, ++j) {
       const int mt = tile / ntiles, nt = tile - mt * ntiles;
       const int i = mt * kOzBM + (tl >> 1), n0 = nt * kOzBN + part * 8;
-      const int er = i < M ? __ldg(&ea[i]) : kOzZero;
+      const int er = i < M ? __ldg(&ea[i]) : kZero;
       const int nlim = i < M ? min(8, N - n0) : 0;
       double* pc = Cf + 2 * ((size_t)n0 * ldc + i) + cc;
       const long long cstep = 2 * ldc;
@@ -392,7 +324,7 @@ oz_zgemm_kernel(double2* __restrict__ C, long long ldc, const unsigned char* __r
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         cv[u] = u < nlim && beta ? pc[u * cstep] : 0.0;
-        ec[u] = n0 + u < N ? __ldg(&eb[n0 + u]) : kOzZero;
+        ec[u] = n0 + u < N ? __ldg(&eb[n0 + u]) : kZero;
       }
       const int a = j & 1;
       if (!mbar_wait(&acc_full[a], (unsigned)(j >> 1) & 1u, s_abort)) {
