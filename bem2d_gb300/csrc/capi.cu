@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "dense.cuh"
+#include "host_pool.h"
 
 namespace bem2d_gpu {
 
@@ -1431,6 +1432,10 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
   std::vector<int> slot_angle(nang);
   for (int a = 0; a < nang; ++a) slot_angle[a] = a;
   int na = nang;
+  // between two GPU steps the host resolves one tridiagonal per angle: 0.3 ms
+  // a step for 360 angles on one core, shared by up to 8 here
+  HostPool pool(std::min(7, std::max(0, std::min(nang / 16 - 1,
+                                                 (int)std::thread::hardware_concurrency() - 1))));
   T* Qalt = static_cast<T*>(ws(c, LzNames<T>::Q2, sizeof(T) * (size_t)qs * nang, &rc));
   T* Walt = static_cast<T*>(ws(c, LzNames<T>::W2, sizeof(T) * (size_t)n * nang, &rc));
   int* dmap = static_cast<int*>(ws(c, "nr_map", sizeof(int) * 2 * nang, &rc));
@@ -1475,7 +1480,7 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
     const int m = (int)sl.size();
     if (!ritz || m == 0) return BEM2D_OK;
     std::vector<int> ang(m);
-    for (int i = 0; i < m; ++i) {
+    const bool made = pool.run(m, [&](int i) {
       const int a = sl[i];
       std::vector<double> e(be[a].begin(), be[a].begin() + (st - 1));
       const std::vector<double> sv = tridiag_eigenvector(al[a], e, lam[a]);
@@ -1485,7 +1490,8 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
       for (int r = 0; r < st; ++r)
         hh[(size_t)i * ldh + r] = {(decltype(hh[0].x))(-sv[r]), (decltype(hh[0].x))0};
       ang[i] = slot_angle[a];
-    }
+    });
+    if (!made) return fail(c, BEM2D_ERR_NOMEM, "host memory of the numerical range");
     CUDA_TRY(c, cudaMemcpyAsync(h, hh.data(), sizeof(T) * (size_t)ldh * m, cudaMemcpyHostToDevice,
                                 c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(dmap, sl.data(), sizeof(int) * m, cudaMemcpyHostToDevice, c->stream));
@@ -1531,7 +1537,7 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
     c->launches += 8;
     CHECK_LAUNCH(c);
     steps = j + 1;
-    for (int a = 0; a < na; ++a) {
+    const bool analysed = pool.run(na, [&](int a) {
       al[a].push_back(hal[a].x);
       const double b = std::sqrt(nn[a]);
       inv[a] = b > 1e-300 ? 1.0 / b : 0.0;
@@ -1581,13 +1587,15 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
       }
       prev[a] = lam[a];
       be[a].push_back(b);
-    }
+      if (stable[a] >= 2 && (j >= 3 || gap_in))
+        lam[a] = tridiag_lmax_from(al[a], be[a], lam[a], 0.0, 0.0);  // to roundoff
+    });
+    if (!analysed) return fail(c, BEM2D_ERR_NOMEM, "host memory of the numerical range");
     {
       std::vector<int> keep, done;
       keep.reserve(na);
       for (int a = 0; a < na; ++a) {
         if (stable[a] >= 2 && (j >= 3 || gap_in)) {
-          lam[a] = tridiag_lmax_from(al[a], be[a], lam[a], 0.0, 0.0);  // to roundoff
           lam_out[slot_angle[a]] = lam[a];
           done.push_back(a);
         } else {
