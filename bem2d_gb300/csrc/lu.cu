@@ -29,6 +29,7 @@ namespace cg = cooperative_groups;
 
 #include "common.cuh"
 #include "cplx.cuh"
+#include "tc.cuh"
 
 namespace bem2d_gpu {
 
@@ -828,16 +829,21 @@ panel_rows_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, 
 // Reductions use the warp reduce instructions: the maximum of (bits of
 // |re|+|im|) + 1 (0 = no candidate; non-negative floats order like their
 // bits), then the minimum label among the lanes holding that maximum.
-// Per column: one __syncthreads for the warp maxima, one for the CTA
-// candidate, whose two threads stage its row (columns c..63) in shared
-// memory; one cluster barrier; the threads pull every CTA's key and staged
-// row (one DSMEM round trip); a third __syncthreads; every warp picks the
-// pivot and each thread updates its registers.
+// Per column: one __syncthreads for the warp maxima, from which every warp
+// forms the CTA candidate; the candidate's warp sends the row (columns c..63)
+// and its key to every CTA with asynchronous stores that count their bytes on
+// the receiver's mbarrier; every warp waits there (bounded), picks the pivot
+// and updates its registers.  No cluster barrier: a CTA sends its candidate of
+// column c + 1 after it has used the ones of column c, so with two buffers
+// (column parity) whoever holds all candidates of c + 1 may overwrite those of
+// c.  Bound by the latency of that one-way exchange: 64 columns of 2048 rows
+// 70 us; with a cluster barrier and a pull of every candidate over DSMEM 109
+// us, with asynchronous stores from the candidate's warp alone 102 us.
 constexpr int kWinMaxRows = 256;
 constexpr int kWinMaxThreads = 2 * kWinMaxRows;
 
 __host__ __device__ constexpr size_t panel_win_smem(int rpb) {
-  return sizeof(float2) * ((size_t)rpb * kRowsLd + (size_t)(2 + kMaxClusterPanel) * kNB);
+  return sizeof(float2) * ((size_t)rpb * kRowsLd + (size_t)(2 + 2 * kMaxClusterPanel) * kNB);
 }
 
 __device__ __forceinline__ float2 crcp_fast(float2 a) {
@@ -857,7 +863,7 @@ __device__ __forceinline__ float4 cfms2(float4 w, float2 l, float4 q) {
 
 __global__ void __launch_bounds__(kWinMaxThreads, 1)
 panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, int rpb,
-                 int* __restrict__ ipiv, int* info) {
+                 int* __restrict__ ipiv, int* info, int* status) {
   constexpr int kW = kNB / 4;  // pairs per thread
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -865,10 +871,13 @@ panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, i
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* Fin = reinterpret_cast<float2*>(smem_raw);    // [rpb][kRowsLd] finished pairs
   float4* cand4 = reinterpret_cast<float4*>(Fin + (size_t)rpb * kRowsLd);  // [2][32]
-  float4* stage4 = cand4 + 2 * (kNB / 2);                // [kMaxClusterPanel][32]
-  __shared__ unsigned ckv[2], ckl[2];
-  __shared__ unsigned skv[kMaxClusterPanel], skl[kMaxClusterPanel];
-  __shared__ unsigned wkv[kWinMaxThreads / 32], wkl[kWinMaxThreads / 32];
+  float4* stage2 = cand4 + 2 * (kNB / 2);                // [2][kMaxClusterPanel][32]
+  // by column parity: candidates' keys {value, label}, the warps' maxima, and
+  // the mbarrier that counts the bytes of a column's candidates
+  __shared__ __align__(16) uint4 skey[2][kMaxClusterPanel];
+  __shared__ unsigned wkv2[2][kWinMaxThreads / 32], wkl2[2][kWinMaxThreads / 32];
+  __shared__ __align__(8) unsigned long long mb[2];
+  __shared__ int s_abort;
   __shared__ int s_ipiv[kNB];
   __shared__ int s_info;
   const int lw = threadIdx.x >> 5, ln = threadIdx.x & 31;
@@ -886,7 +895,13 @@ panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, i
     if (active && c0 + 1 < nb) b = A[(size_t)(k0 + c0 + 1) * lda + label];
     r[i] = make_float4(a.x, a.y, b.x, b.y);
   }
-  if (threadIdx.x == 0) s_info = 0;
+  if (threadIdx.x == 0) {
+    s_info = 0;
+    s_abort = 0;
+    tc::mbar_init(&mb[0], 1);
+    tc::mbar_init(&mb[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
   __syncthreads();
   cl.sync();  // every CTA of the cluster is running before any DSMEM access
   for (int b = 0; 4 * b < nb; ++b) {
@@ -898,6 +913,12 @@ panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, i
         const bool hi = (cc & 1) != 0;  // static
         const unsigned kc = (unsigned)(k0 + c);
         const int par = c & 1;
+        unsigned* wkv = wkv2[par];
+        unsigned* wkl = wkl2[par];
+        float4* stage4 = stage2 + par * kMaxClusterPanel * (kNB / 2);
+        // bytes of the C candidates: pairs c/2 .. 31 and a key each
+        if (threadIdx.x == 0)
+          tc::mbar_expect_tx(&mb[par], (unsigned)C * 16u * (unsigned)(kNB / 2 - (c >> 1) + 1));
         // 1. warp and CTA candidates
         const float2 vv = hi ? make_float2(r[0].z, r[0].w) : make_float2(r[0].x, r[0].y);
         const float a = cabs1(vv);
@@ -910,9 +931,7 @@ panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, i
           wkl[lw] = lab;
         }
         __syncthreads();
-        // every warp forms the CTA candidate from the warp maxima (no second
-        // barrier: the next column rewrites them only after the cluster
-        // barrier below, which every thread reaches after reading them)
+        // every warp forms the CTA candidate from the warp maxima
         unsigned cand;
         {
           const unsigned wv = ln < nw ? wkv[ln] : 0u;
@@ -920,75 +939,36 @@ panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, i
           m = __reduce_max_sync(0xffffffffu, wv);
           lab = __reduce_min_sync(0xffffffffu, (wv == m && m) ? wl : 0xffffffffu);
           cand = m ? lab : 0xfffffffeu;
-          if (lw == 0 && ln == 0) {
-            ckv[par] = m;
-            ckl[par] = lab;
-          }
         }
-        if (label == cand) {  // this row is the CTA candidate: stage pairs >= c/2
+        // 2. the candidate's threads stage its row; the warps share the sends
+        //    of the row, pairs >= c/2, and its key to every CTA (one warp
+        //    sending to 16 CTAs took 960 clocks)
+        if (label == cand) {
           float4* dst = cand4 + par * (kNB / 2) + 2 * b + h;
 #pragma unroll
           for (int i = 0; i < kW; ++i)
             if (i < kW - b && (i > 0 || h >= hc)) dst[2 * i] = r[i];
         }
-        // 2. every CTA's candidate visible
-        cl.sync();
-        // 3. pull all keys and staged rows: loads first, then stores, so
-        //    that a thread's DSMEM loads (up to four ranks) are in flight at
-        //    once; with no more ranks than warps, warp q pulls rank q
-        if (C <= nw) {
-          if (lw < C) {
-            const int j = ln;
-            float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            unsigned tv = 0u, tl = 0u;
-            if (j >= (c >> 1)) t4 = cl.map_shared_rank(cand4, lw)[par * (kNB / 2) + j];
-            if (j == 0) {
-              tv = *cl.map_shared_rank(&ckv[par], lw);
-              tl = *cl.map_shared_rank(&ckl[par], lw);
-            }
-            if (j >= (c >> 1)) stage4[lw * (kNB / 2) + j] = t4;
-            if (j == 0) {
-              skv[lw] = tv;
-              skl[lw] = tl;
-            }
-          }
-        } else {
-        for (int q0 = 0; q0 < C; q0 += 4 * nw) {
-          constexpr int kPer = 4;
-          const int j = ln;  // absolute pair index
-          float4 t4[kPer];
-          unsigned tv[kPer], tl[kPer];
-#pragma unroll
-          for (int u = 0; u < kPer; ++u) {
-            const int q = q0 + lw + u * nw;
-            if (q < C) {
-              if (j >= (c >> 1)) t4[u] = cl.map_shared_rank(cand4, q)[par * (kNB / 2) + j];
-              if (j == 0) {
-                tv[u] = *cl.map_shared_rank(&ckv[par], q);
-                tl[u] = *cl.map_shared_rank(&ckl[par], q);
-              }
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < kPer; ++u) {
-            const int q = q0 + lw + u * nw;
-            if (q < C) {
-              if (j >= (c >> 1)) stage4[q * (kNB / 2) + j] = t4[u];
-              if (j == 0) {
-                skv[q] = tv[u];
-                skl[q] = tl[u];
-              }
-            }
-          }
-        }
-        }
         __syncthreads();
+        {
+          const uint4 v = *reinterpret_cast<const uint4*>(&cand4[par * (kNB / 2) + ln]);
+          for (int q = lw; q < C; q += nw) {
+            const unsigned bar = tc::map_rank(&mb[par], q);
+            if (ln >= (c >> 1))
+              tc::store_async(tc::map_rank(&stage4[rank * (kNB / 2) + ln], q), v, bar);
+            if (ln == 0)
+              tc::store_async(tc::map_rank(&skey[par][rank], q), make_uint4(m, lab, 0u, 0u), bar);
+          }
+        }
+        // 3. every candidate has arrived
+        const bool live = tc::mbar_wait_cluster(&mb[par], (unsigned)(c >> 1) & 1u, &s_abort);
         // 4. the pivot, from the local keys (every warp)
-        const unsigned kv = ln < C ? skv[ln] : 0u;
-        const unsigned kl = ln < C ? skl[ln] : 0xffffffffu;
+        const unsigned kv = ln < C ? skey[par][ln].x : 0u;
+        const unsigned kl = ln < C ? skey[par][ln].y : 0xffffffffu;
         const unsigned bm = __reduce_max_sync(0xffffffffu, kv);
         const unsigned p = __reduce_min_sync(0xffffffffu, (kv == bm && bm) ? kl : 0xffffffffu);
-        const bool zero = bm <= 1u || p < kc || p >= (unsigned)n;  // bm == 1: |pivot| = 0
+        // bm == 1: |pivot| = 0; after a wait that gave up nothing is used
+        const bool zero = !__all_sync(0xffffffffu, live) || bm <= 1u || p < kc || p >= (unsigned)n;
         if (threadIdx.x == 0) {
           s_ipiv[c] = zero ? (int)kc : (int)p;
           if (zero && s_info == 0) s_info = (int)kc + 1;
@@ -1032,7 +1012,8 @@ panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, i
     for (int i = 0; i < kW - 1; ++i) r[i] = r[i + 1];
     r[kW - 1] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  cl.sync();  // no CTA leaves while another may still read its shared memory
+  cl.sync();  // no CTA leaves while another may still write its shared memory
+  if (threadIdx.x == 0 && s_abort) atomicExch(status, 1);
   if (rank == 0) {
     for (int c = threadIdx.x; c < nb; c += T) ipiv[k0 + c] = s_ipiv[c];
     if (threadIdx.x == 0 && s_info && *info == 0) *info = s_info;
@@ -1419,7 +1400,7 @@ static bool tslu_panel(float2* A, long long lda, int n, int k0, int nb, const Lu
   const int threads = std::max(64, (2 * rpb + 31) / 32 * 32);
   cudaMemsetAsync(ts.infc, 0, sizeof(int), s);
   if (launch_cluster(panel_win_kernel, C, threads, panel_win_smem(rpb), s, Cf, (long long)ld, Gf,
-                     0, nb, rpb, ts.ipc, ts.infc) != cudaSuccess) {
+                     0, nb, rpb, ts.ipc, ts.infc, w.status) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -1724,7 +1705,7 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
         const int threads = std::max(64, (2 * rpb + 31) / 32 * 32);
         cudaError_t e = launch_cluster(panel_win_kernel, C, threads, panel_win_smem(rpb), s,
                                        reinterpret_cast<float2*>(A), lda, n, k0, nb, rpb,
-                                       w.ipiv, w.info);
+                                       w.ipiv, w.info, w.status);
         if (e == cudaSuccess) {
           done = true;
           break;

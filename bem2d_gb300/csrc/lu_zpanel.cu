@@ -9,8 +9,8 @@
 //                     the block (36 FP64 instructions a column on average
 //                     instead of 128 for 64 columns); pivot search on the
 //                     integer pipe (|re| + |im| as 64-bit keys, warp reduce
-//                     instructions); one reciprocal, formed by the candidate's
-//                     warp before it pushes the row to the other CTAs
+//                     instructions); candidates travel by asynchronous
+//                     stores, no cluster barrier per column
 //   panel_side_kernel row swaps on the panel's other columns and, right of the
 //                     block, U = L11^{-1} A (a warp per column)
 //   panel_update_kernel  A -= L U on the panel's columns right of the block,
@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "cplx.cuh"
+#include "tc.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -35,24 +36,28 @@ namespace {
 constexpr int kZW = 16;            // block width
 constexpr int kZMaxC = 16;         // CTAs of a cluster
 constexpr int kZThreads = 256;
-constexpr int kZSlot = kZW + 1;    // candidate row and the pivot's reciprocal
 
 __device__ __forceinline__ int zexpo(double x) { return (__double2hiint(x) >> 20) & 2047; }
 
-// 1/a: |a|^2 scaled by a power of two, its reciprocal by a third-order
-// correction of the hardware's 2^-20 seed (subnormal a: the general routine).
+// 1/a: the reciprocal of |a|^2 by a third-order correction of the hardware's
+// 2^-20 seed; a scaled by a power of two first unless |a|^2 is far from the
+// ends of the range (subnormal or infinite a: the general routine).
 __device__ __forceinline__ double2 zrcp(double2 a) {
   const int e = max(zexpo(a.x), zexpo(a.y));
   if (e == 0 || e == 2047) return crcp(a);
-  // s = 2^(1023 - e): scaled parts below 2
-  const double s = e < 2046 ? __hiloint2double((2046 - e) << 20, 0) : 1.1125369292536007e-308;
-  const double x = a.x * s, y = a.y * s;
-  const double q = fma(x, x, y * y);
+  double s = 1.0;
+  if (e < 600 || e > 1400) {  // scaled parts below 2
+    s = e < 2046 ? __hiloint2double((2046 - e) << 20, 0) : 1.1125369292536007e-308;
+    a.x *= s;
+    a.y *= s;
+  }
+  const double q = fma(a.x, a.x, a.y * a.y);
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(q));
   const double t = fma(-q, r, 1.0);
-  r = fma(r, fma(t, t, t), r) * s;
-  return make_double2(x * r, -y * r);
+  r = fma(r, fma(t, t, t), r);
+  a = make_double2(a.x * r, -a.y * r);
+  return s == 1.0 ? a : make_double2(a.x * s, a.y * s);
 }
 
 struct ZKey {
@@ -75,14 +80,17 @@ __device__ __forceinline__ ZKey zkey_max(ZKey k) {
 template <int R>
 __global__ void __launch_bounds__(kZThreads, 1)
 panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int rpb,
-               int* __restrict__ ipiv, int* info) {
+               int* __restrict__ ipiv, int* info, int* status) {
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-  __shared__ double2 slot[2][kZMaxC][kZSlot];
-  __shared__ ZKey key[2][kZMaxC];
-  __shared__ ZKey wkey[kZThreads / 32];
-  __shared__ double2 srow[kZW];
-  __shared__ int s_ipiv[kZW], s_info;
+  // by column parity: the candidates' rows and keys, the warps' candidates,
+  // the staged own row, the mbarrier that counts a column's bytes
+  __shared__ __align__(16) double2 slot[2][kZMaxC][kZW];
+  __shared__ __align__(16) uint4 key[2][kZMaxC];
+  __shared__ ZKey wkey[2][kZThreads / 32];
+  __shared__ __align__(16) double2 srow[2][kZW];
+  __shared__ __align__(8) unsigned long long mb[2];
+  __shared__ int s_ipiv[kZW], s_info, s_abort;
   const int T = (int)blockDim.x, tid = threadIdx.x, ln = tid & 31, lw = tid >> 5, nw = T >> 5;
   unsigned label[R];
   double2 a[R][kZW];
@@ -95,13 +103,21 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
       a[r][c] = label[r] != 0xffffffffu && c < w ? A[(size_t)(kb + c) * lda + gr]
                                                  : make_double2(0.0, 0.0);
   }
-  if (tid == 0) s_info = 0;
+  if (tid == 0) {
+    s_info = 0;
+    s_abort = 0;
+    tc::mbar_init(&mb[0], 1);
+    tc::mbar_init(&mb[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
   cl.sync();  // every CTA of the cluster is running before any DSMEM access
 #pragma unroll
   for (int c = 0; c < kZW; ++c) {
     if (c >= w) break;
     const unsigned kc = (unsigned)(kb + c);
     const int par = c & 1;
+    // bytes of the C candidates: entries c .. 15 and a key each
+    if (tid == 0) tc::mbar_expect_tx(&mb[par], (unsigned)C * 16u * (unsigned)(kZW - c + 1));
     // 1. the CTA's candidate
     ZKey k{0u, 0u, 0xffffffffu};
 #pragma unroll
@@ -114,41 +130,43 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
         k = ZKey{h, l, label[r]};
     }
     k = zkey_max(k);
-    if (ln == 0) wkey[lw] = k;
+    if (ln == 0) wkey[par][lw] = k;
     __syncthreads();
-    // every warp forms the CTA's candidate; the maxima are rewritten only
-    // after the cluster barrier below
-    k = zkey_max(ln < nw ? wkey[ln] : ZKey{0u, 0u, 0xffffffffu});
-    bool mine = false;
+    // every warp forms the CTA's candidate, whose thread stages its row; the
+    // warps share the sends to the other CTAs, asynchronous stores that count
+    // their bytes on the receiver's mbarrier.  A CTA sends its candidate of
+    // column c + 1 after it has used the ones of column c, so two buffers do.
+    k = zkey_max(ln < nw ? wkey[par][ln] : ZKey{0u, 0u, 0xffffffffu});
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (k.label != 0xffffffffu && label[r] == k.label) {
-        mine = true;
 #pragma unroll
         for (int e = 0; e < kZW; ++e)
-          if (e >= c) srow[e] = a[r][e];
+          if (e >= c) srow[par][e] = a[r][e];
       }
     }
-    const bool any = (k.hi | k.lo) != 0u;
-    if (any ? __any_sync(0xffffffffu, mine) : lw == 0) {
-      __syncwarp();
-      if (any) {
-        const double2 inv = zrcp(srow[c]);
-        const int e = ln & 15;
-        for (int q = ln >> 4; q < C; q += 2) {
-          double2* dst = cl.map_shared_rank(&slot[par][rank][0], q);
-          if (e >= c) dst[e] = srow[e];
-          if (e == 0) dst[kZW] = inv;
-        }
+    __syncthreads();
+    {
+      // lanes 0-15: entry ln to rank q, lanes 16-31 to rank q + 1
+      const int e = ln & 15;
+      const uint4 v = *reinterpret_cast<const uint4*>(&srow[par][e]);
+      for (int q = 2 * lw + (ln >> 4); q < C; q += 2 * nw) {
+        const unsigned bar = tc::map_rank(&mb[par], q);
+        if (e >= c) tc::store_async(tc::map_rank(&slot[par][rank][e], q), v, bar);
+        if (e == 0)
+          tc::store_async(tc::map_rank(&key[par][rank], q), make_uint4(k.hi, k.lo, k.label, 0u),
+                          bar);
       }
-      if (ln < C) *cl.map_shared_rank(&key[par][rank], ln) = k;
     }
-    // 2. every candidate local to every CTA
-    cl.sync();
+    // 2. every candidate has arrived
+    const bool live = tc::mbar_wait_cluster(&mb[par], (unsigned)(c >> 1) & 1u, &s_abort);
     // 3. the pivot, from the local slots (every warp)
-    const ZKey mk = ln < C ? key[par][ln] : ZKey{0u, 0u, 0xffffffffu};
+    const uint4 kv = ln < C ? key[par][ln] : make_uint4(0u, 0u, 0xffffffffu, 0u);
+    const ZKey mk{kv.x, kv.y, kv.z};
     k = zkey_max(mk);
-    const bool zero = (k.hi | k.lo) == 0u;
+    // after a wait that gave up nothing is used
+    const bool zero = !__all_sync(0xffffffffu, live) || (k.hi | k.lo) == 0u || k.label < kc ||
+                      k.label >= (unsigned)n;
     if (tid == 0) {
       s_ipiv[c] = zero ? (int)kc : (int)k.label;
       if (zero && s_info == 0) s_info = (int)kc + 1;
@@ -156,7 +174,7 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
     if (zero) continue;  // LAPACK: no swap and no elimination for a zero pivot
     const int win = __ffs(__ballot_sync(0xffffffffu, ln < C && mk.label == k.label)) - 1;
     const double2* p = slot[par][win];
-    const double2 inv = p[kZW];
+    const double2 inv = zrcp(p[c]);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (label[r] == k.label)
@@ -173,6 +191,7 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
     }
   }
   cl.sync();  // no CTA leaves while another may still write its shared memory
+  if (tid == 0 && s_abort) atomicExch(status, 1);
   if (rank == 0) {
     if (tid < w) ipiv[kb + tid] = s_ipiv[tid];
     if (tid == 0 && s_info && *info == 0) *info = s_info;
@@ -292,8 +311,8 @@ int launch_zpanel(double2* A, long long lda, int n, int k0, int nb, const LuWork
       cfg.attrs = at;
       cfg.numAttrs = 1;
       const cudaError_t e =
-          R == 1 ? cudaLaunchKernelEx(&cfg, panel16_kernel<1>, A, lda, n, kb, bw, rpb, w.ipiv, w.info)
-                 : cudaLaunchKernelEx(&cfg, panel16_kernel<2>, A, lda, n, kb, bw, rpb, w.ipiv, w.info);
+          R == 1 ? cudaLaunchKernelEx(&cfg, panel16_kernel<1>, A, lda, n, kb, bw, rpb, w.ipiv, w.info, w.status)
+                 : cudaLaunchKernelEx(&cfg, panel16_kernel<2>, A, lda, n, kb, bw, rpb, w.ipiv, w.info, w.status);
       if (e == cudaSuccess) break;
       cudaGetLastError();
       if (cmax <= 8) return kb == k0 ? 1 : BEM2D_ERR_CUDA;

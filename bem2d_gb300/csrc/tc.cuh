@@ -65,5 +65,49 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned b
       : "memory");
 }
 
+// ---- cluster exchange through asynchronous remote stores ----------------------
+// Address of shared-memory variable p in the CTA of rank `rank`.
+__device__ __forceinline__ unsigned map_rank(const void* p, unsigned rank) {
+  unsigned a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+// 16 bytes to a mapped address; they count 16 on the mbarrier (same CTA).
+__device__ __forceinline__ void store_async(unsigned dst, uint4 v, unsigned mbar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, "
+      "[%5];" ::"r"(dst),
+      "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(mbar)
+      : "memory");
+}
+__device__ __forceinline__ bool mbar_test_cluster(unsigned long long* m, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(smem_u32(m)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// As mbar_wait, for data that other CTAs of the cluster have stored; a thread
+// that gives up sets *abort, and nobody waits again after that.
+__device__ __forceinline__ bool mbar_wait_cluster(unsigned long long* m, unsigned parity,
+                                                  volatile int* abort) {
+  if (mbar_test_cluster(m, parity)) return *abort == 0;
+  const unsigned long long t0 = global_ns();
+  for (unsigned it = 1;; ++it) {
+    if (mbar_test_cluster(m, parity)) return *abort == 0;
+    if ((it & 15u) == 0u) {
+      if (*abort) return false;
+      if (global_ns() - t0 > kWaitNs) {
+        *abort = 1;
+        return false;
+      }
+    }
+  }
+}
+
 }  // namespace tc
 }  // namespace bem2d_gpu
