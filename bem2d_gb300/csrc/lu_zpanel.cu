@@ -39,26 +39,28 @@ constexpr int kZThreads = 256;
 
 __device__ __forceinline__ int zexpo(double x) { return (__double2hiint(x) >> 20) & 2047; }
 
-// 1/a: the reciprocal of |a|^2 by a third-order correction of the hardware's
-// 2^-20 seed; a scaled by a power of two first unless |a|^2 is far from the
-// ends of the range (subnormal or infinite a: the general routine).
-__device__ __forceinline__ double2 zrcp(double2 a) {
-  const int e = max(zexpo(a.x), zexpo(a.y));
-  if (e == 0 || e == 2047) return crcp(a);
-  double s = 1.0;
+// The factor r of a / p = a conj(p) r, r = 1 / |p|^2 by a third-order correction
+// of the hardware's 2^-20 seed.  p is scaled by the power of two *s first where
+// |p|^2 would leave the range (then a / p = a s conj(p) r).  Forming a conj(p)
+// beside r keeps the chain of dependent FP64 instructions at seven.
+// False for subnormal and non-finite p: use zdiv_general.
+__device__ __forceinline__ bool zrcp(double2* p, double* s, double* r) {
+  const int e = max(zexpo(p->x), zexpo(p->y));
+  *s = 1.0;
+  if (e == 0 || e == 2047) return false;
   if (e < 600 || e > 1400) {  // scaled parts below 2
-    s = e < 2046 ? __hiloint2double((2046 - e) << 20, 0) : 1.1125369292536007e-308;
-    a.x *= s;
-    a.y *= s;
+    *s = e < 2046 ? __hiloint2double((2046 - e) << 20, 0) : 1.1125369292536007e-308;
+    p->x *= *s;
+    p->y *= *s;
   }
-  const double q = fma(a.x, a.x, a.y * a.y);
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(q));
-  const double t = fma(-q, r, 1.0);
-  r = fma(r, fma(t, t, t), r);
-  a = make_double2(a.x * r, -a.y * r);
-  return s == 1.0 ? a : make_double2(a.x * s, a.y * s);
+  const double q = fma(p->x, p->x, p->y * p->y);
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
+  const double t = fma(-q, y, 1.0);
+  *r = fma(y, fma(t, t, t), y);
+  return true;
 }
+__device__ __noinline__ double2 zdiv_general(double2 a, double2 p) { return cmul(a, crcp(p)); }
 
 struct ZKey {
   unsigned hi, lo, label;  // bits of |re| + |im| (0: none), row
@@ -77,7 +79,10 @@ __device__ __forceinline__ ZKey zkey_max(ZKey k) {
 // Columns kb .. kb + w of rows kb .. n.  Row exchanges by renaming: a row
 // carries the matrix row it stands for; the pivot row takes kc, the row that
 // held kc takes the pivot's, and rows are written to their names at the end.
-template <int R>
+// R rows per thread, or TPR threads (neighbouring lanes) per row, thread t
+// holding columns t, t + TPR, ...: a CTA of 32 or 64 rows then spreads its
+// updates over all four schedulers.
+template <int R, int TPR>
 __global__ void __launch_bounds__(kZThreads, 1)
 panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int rpb,
                int* __restrict__ ipiv, int* info, int* status) {
@@ -91,17 +96,21 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
   __shared__ __align__(16) double2 srow[2][kZW];
   __shared__ __align__(8) unsigned long long mb[2];
   __shared__ int s_ipiv[kZW], s_info, s_abort;
+  constexpr int kL = kZW / TPR;  // columns per thread
   const int T = (int)blockDim.x, tid = threadIdx.x, ln = tid & 31, lw = tid >> 5, nw = T >> 5;
+  const int t = tid % TPR;
   unsigned label[R];
-  double2 a[R][kZW];
+  double2 a[R][kL];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int lr = tid + r * T, gr = kb + rank * rpb + lr;
+    const int lr = tid / TPR + r * T, gr = kb + rank * rpb + lr;
     label[r] = lr < rpb && gr < n ? (unsigned)gr : 0xffffffffu;
 #pragma unroll
-    for (int c = 0; c < kZW; ++c)
-      a[r][c] = label[r] != 0xffffffffu && c < w ? A[(size_t)(kb + c) * lda + gr]
+    for (int i = 0; i < kL; ++i) {
+      const int c = i * TPR + t;
+      a[r][i] = label[r] != 0xffffffffu && c < w ? A[(size_t)(kb + c) * lda + gr]
                                                  : make_double2(0.0, 0.0);
+    }
   }
   if (tid == 0) {
     s_info = 0;
@@ -122,8 +131,8 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
     ZKey k{0u, 0u, 0xffffffffu};
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      if (label[r] == 0xffffffffu || label[r] < kc) continue;
-      const long long b = __double_as_longlong(cabs1(a[r][c]));
+      if (label[r] == 0xffffffffu || label[r] < kc || t != c % TPR) continue;
+      const long long b = __double_as_longlong(cabs1(a[r][c / TPR]));
       if (b > 0x7ff0000000000000ll) continue;  // NaN
       const unsigned h = (unsigned)(b >> 32), l = (unsigned)b;
       if (h > k.hi || (h == k.hi && (l > k.lo || (l == k.lo && label[r] < k.label))))
@@ -141,8 +150,8 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
     for (int r = 0; r < R; ++r) {
       if (k.label != 0xffffffffu && label[r] == k.label) {
 #pragma unroll
-        for (int e = 0; e < kZW; ++e)
-          if (e >= c) srow[par][e] = a[r][e];
+        for (int i = 0; i < kL; ++i)
+          if (i >= c / TPR) srow[par][i * TPR + t] = a[r][i];
       }
     }
     __syncthreads();
@@ -174,19 +183,38 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
     if (zero) continue;  // LAPACK: no swap and no elimination for a zero pivot
     const int win = __ffs(__ballot_sync(0xffffffffu, ln < C && mk.label == k.label)) - 1;
     const double2* p = slot[par][win];
-    const double2 inv = zrcp(p[c]);
+    double2 ps = p[c];
+    double sc, rc;
+    const bool fast = zrcp(&ps, &sc, &rc);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (label[r] == k.label)
         label[r] = kc;
       else if (label[r] == kc)
         label[r] = k.label;
+      // the row's column-c value, from the thread that holds it
+      double2 v = a[r][c / TPR];
+      if (TPR > 1) {
+        v.x = __shfl_sync(0xffffffffu, v.x, (ln & ~(TPR - 1)) | (c % TPR));
+        v.y = __shfl_sync(0xffffffffu, v.y, (ln & ~(TPR - 1)) | (c % TPR));
+      }
       if (label[r] != 0xffffffffu && label[r] > kc) {
-        const double2 l = cmul(a[r][c], inv);
-        a[r][c] = l;
+        double2 l;
+        if (fast) {
+          if (sc != 1.0) v = make_double2(v.x * sc, v.y * sc);
+          l = make_double2(fma(v.x, ps.x, v.y * ps.y) * rc, fma(v.y, ps.x, -v.x * ps.y) * rc);
+        } else {
+          l = zdiv_general(v, p[c]);
+        }
+        if (TPR == 1) {
+          a[r][c] = l;
+        } else if (t >= c % TPR) {  // the slot of column c: l, or an update right of c
+          const int i = c / TPR;
+          a[r][i] = t == c % TPR ? l : cfms(a[r][i], l, p[i * TPR + t]);
+        }
 #pragma unroll
-        for (int e = 0; e < kZW; ++e)
-          if (e > c) a[r][e] = cfms(a[r][e], l, p[e]);
+        for (int i = 0; i < kL; ++i)
+          if (i > c / TPR) a[r][i] = cfms(a[r][i], l, p[i * TPR + t]);
       }
     }
   }
@@ -200,8 +228,8 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
   for (int r = 0; r < R; ++r)
     if (label[r] != 0xffffffffu)
 #pragma unroll
-      for (int c = 0; c < kZW; ++c)
-        if (c < w) A[(size_t)(kb + c) * lda + label[r]] = a[r][c];
+      for (int i = 0; i < kL; ++i)
+        if (i * TPR + t < w) A[(size_t)(kb + i * TPR + t) * lda + label[r]] = a[r][i];
 }
 
 // The interchanges ipiv[kb .. kb + w) on the panel columns [k0, kb) and
@@ -281,10 +309,12 @@ int launch_zpanel(double2* A, long long lda, int n, int k0, int nb, const LuWork
   static std::atomic<int> max_cluster{kZMaxC};
   static std::once_flag attr;
   std::call_once(attr, [] {
-    if (cudaFuncSetAttribute(panel16_kernel<1>, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                             1) != cudaSuccess ||
-        cudaFuncSetAttribute(panel16_kernel<2>, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                             1) != cudaSuccess) {
+    bool ok = true;
+    for (auto k : {panel16_kernel<1, 1>, panel16_kernel<1, 2>, panel16_kernel<1, 4>,
+                   panel16_kernel<2, 1>})
+      ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                     cudaSuccess;
+    if (!ok) {
       cudaGetLastError();
       max_cluster = 8;
     }
@@ -296,9 +326,16 @@ int launch_zpanel(double2* A, long long lda, int n, int k0, int nb, const LuWork
     for (;;) {
       const int cmax = max_cluster;
       const int rpb = std::max(32, ((H + cmax - 1) / cmax + 31) / 32 * 32);
-      const int R = rpb <= kZThreads ? 1 : 2;
       if (rpb > 2 * kZThreads) return kb == k0 ? 1 : BEM2D_ERR_CUDA;
-      const int C = (H + rpb - 1) / rpb, threads = (rpb / R + 31) / 32 * 32;
+      const int C = (H + rpb - 1) / rpb;
+      const int threads = rpb <= 32    ? 4 * rpb
+                          : rpb <= 64  ? 2 * rpb
+                          : rpb <= kZThreads ? rpb
+                                             : (rpb / 2 + 31) / 32 * 32;
+      auto kern = rpb <= 32          ? panel16_kernel<1, 4>
+                  : rpb <= 64        ? panel16_kernel<1, 2>
+                  : rpb <= kZThreads ? panel16_kernel<1, 1>
+                                     : panel16_kernel<2, 1>;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(C);
       cfg.blockDim = dim3(threads);
@@ -311,8 +348,7 @@ int launch_zpanel(double2* A, long long lda, int n, int k0, int nb, const LuWork
       cfg.attrs = at;
       cfg.numAttrs = 1;
       const cudaError_t e =
-          R == 1 ? cudaLaunchKernelEx(&cfg, panel16_kernel<1>, A, lda, n, kb, bw, rpb, w.ipiv, w.info, w.status)
-                 : cudaLaunchKernelEx(&cfg, panel16_kernel<2>, A, lda, n, kb, bw, rpb, w.ipiv, w.info, w.status);
+          cudaLaunchKernelEx(&cfg, kern, A, lda, n, kb, bw, rpb, w.ipiv, w.info, w.status);
       if (e == cudaSuccess) break;
       cudaGetLastError();
       if (cmax <= 8) return kb == k0 ? 1 : BEM2D_ERR_CUDA;
