@@ -1,8 +1,8 @@
 // Mixed-precision far-field assembly (sm_103a): the bulk of the Galerkin
 // matrix evaluated in float-float arithmetic on the FP32 pipe.
 //
-// Same tiling as the FP64 far kernel (32 x 32 tiles, one lane per test
-// unknown, node data staged in shared memory).  Pair geometry: the centre
+// 32 x 32 tiles, one lane per test unknown, node data staged in shared
+// memory; H0 and H1 from the table of hankel_tab_ff.cuh.  Pair geometry: the centre
 // difference of the two elements in FP64, node offsets from the centres in
 // float-float, so |x - y| keeps ~48 bits relative to itself even for
 // neighbouring elements.  Entries whose element pair admits k|x - y| <= 4
@@ -12,43 +12,37 @@
 // loop keeps its warps on one branch.  Adjacent and identical pairs belong to
 // the near-field kernel as in the FP64 path.  Each entry is stored twice:
 // complex128 (refinement residual) and complex64 (the LU).
+#include <algorithm>
 #include <mutex>
+#include <vector>
 
 #include "common.cuh"
 #include "ff.cuh"
-#include "hankel_ff.cuh"
+#include "hankel_tab_ff.cuh"
 #include "kernel_ff.cuh"
 
 namespace bem2d_gpu {
 
-// The distance-dependent part of the kernel at one node pair: 1/d, the
-// asymptotic P/Q factors of H0 and H1, 1/sqrt(x) (the amplitude
-// sqrt(2/(pi x)) without its constant) and e^{i(x - pi/4)}.  Shared by entry
-// (i, j) and entry (j, i).
-struct HankelTermsFF {
-  ff y, p0, q0, p1, q1, rx;
-  ffc e;
-};
-
-__device__ __forceinline__ HankelTermsFF hankel_terms_ff(ff dx, ff dy, const KConstFF& kc,
-                                                        const float* tab) {
-  HankelTermsFF h;
-  const ff d2 = ff_dot2(dx, dx, dy, dy);
-  h.y = ff_rsqrt(d2);  // 1/d
-  const ff d = ff_mul(d2, h.y);
-  const ff x = ff_mul(d, kc.k);
-  const ff ix = ff_mul(h.y, kc.invk);
-  pq_ff(x.hi, ix, &h.p0, &h.q0, &h.p1, &h.q1);
-  h.rx = ff_rsqrt(x);
-  h.e = expi_ff(x, tab);
-  return h;
+// amp P0, amp Q0, (amp/x) P1, (amp/x) Q1 (amp = sqrt(2/(pi x))) and
+// e^{i(x - pi/4)} by the general evaluator: arguments outside the table's octaves.
+__device__ __noinline__ void hankel_direct_ff(ff x, const float* etab, ff* p0, ff* q0, ff* p1,
+                                              ff* q1, ffc* e) {
+  const ff ix = ff_rcp(x);
+  const ff amp = ff_mul(ff_make(0.7978845834732056f, -2.2670340271702116e-08f), ff_rsqrt(x));
+  const ff ampx = ff_mul(amp, ix);
+  pq_ff(x.hi, ix, p0, q0, p1, q1);
+  *p0 = ff_mul(amp, *p0);
+  *q0 = ff_mul(amp, *q0);
+  *p1 = ff_mul(ampx, *p1);
+  *q1 = ff_mul(ampx, *q1);
+  *e = expi_ff(x, etab);
 }
 
-// E (P + i Q) and a complex value times a real one (ff).
-__device__ __forceinline__ ffc ffc_mul_pq(const ffc& e, ff p, ff q) {
+// E (P + i Q)
+__device__ __forceinline__ ffc ffcu_mul_pq(const ffc& e, ff p, ff q) {
   ffc r;
-  r.re = ff_dot2(e.re, p, ff_neg(e.im), q);
-  r.im = ff_dot2(e.re, q, e.im, p);
+  r.re = ffu_dot2(e.re, p, ff_neg(e.im), q);
+  r.im = ffu_dot2(e.re, q, e.im, p);
   return r;
 }
 
@@ -61,13 +55,6 @@ __device__ __forceinline__ void ff_acc(ff& acc, ff v) {
   acc.lo += s.lo + v.lo;
 }
 __device__ __forceinline__ void ff_acc_norm(ff& acc) { acc = fast_two_sum(acc.hi, acc.lo); }
-
-__device__ __forceinline__ ffc ffc_scale(const ffc& z, ff a) {
-  ffc r;
-  r.re = ff_mul(z.re, a);
-  r.im = ff_mul(z.im, a);
-  return r;
-}
 
 // One entry in FP64 from the FP64 node table (deferred entries).
 template <int KERNEL>
@@ -97,6 +84,8 @@ constexpr int kDeferCR = 1 << 29;  // deferred item: entry (col, row) wanted
 constexpr int kDeferIdx = kDeferCR - 1;
 constexpr int kFarFFThreads = 256;
 constexpr float kDeferX = 4.001f;
+// table intervals in shared memory (27 KB: with rules of 64 nodes a CTA takes 214 KB)
+constexpr int kFtCap = 192;
 
 // Tiles are processed in symmetric pairs: CTA b owns tile (I, J), I <= J,
 // and computes both (I, J) and (J, I).  The distance-dependent work at a node
@@ -116,45 +105,62 @@ __device__ __forceinline__ void tile_of(unsigned b, int* I, int* J) {
   *I = (int)((long long)b - (long long)j * (j + 1) / 2);
 }
 
+// Bound by FP32 issue (76 % of the issue slots, 65 % of the FMA pipe): 704
+// thread instructions per node pair with pq_ff (1/d, 1/sqrt(x), four
+// polynomials of degree 9-12 and e^{ix} each), 472 with the table; 1.24 ->
+// 0.85 ms at kite N = 2048, 69 -> 51 ms at L-shape N = 16384, with about half
+// the error against FP64.  More warps (3 CTAs at 80 registers, 22 warps at 80,
+// 20 at 96) measured no faster.  All coordinates are scaled by k first, so that x = |k (x - y)| is
+// one square root and H1 comes as H1/x, the factor the normal product needs;
+// k, eta and alpha enter once per entry.  The CTA's arguments lie between two
+// bounds from its 1024 centre distances; when the table intervals between them
+// fit (kFtCap of 144 bytes: stride 9 x 16 bytes, so that neighbouring
+// intervals fall into different banks), they are copied to shared memory,
+// otherwise they are read from the global table.
 template <int KERNEL, int NG>
 __global__ void __launch_bounds__(kFarFFThreads, 2)
 far_ff_kernel(DevGeom g, NodeTable t, NodeTableFF tf, int ng_rt, KConstFF kc, double k,
               double eta, double alpha, double2* __restrict__ out, long long ld,
-              float2* __restrict__ out32, long long ld32, DeferList dl, const float* gtab) {
+              float2* __restrict__ out32, long long ld32, DeferList dl,
+              const float4* __restrict__ ftab, const float* __restrict__ etab) {
+  constexpr bool kH0 = KERNEL == BEM2D_KERNEL_SINGLE || KERNEL == BEM2D_KERNEL_COMBINED;
+  constexpr bool kH1 = KERNEL != BEM2D_KERNEL_SINGLE;
   const int ng = NG > 0 ? NG : ng_rt;
+  const int SZ = ng * kTileF;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* tT = reinterpret_cast<double2*>(smem_raw);          // [32][33] tile (J, I)
-  unsigned* vT = reinterpret_cast<unsigned*>(tT + kTileF * (kTileF + 1));  // [32] masks
-  float* tab = reinterpret_cast<float*>(vT + kTileF);          // 256
-  double2* cen = reinterpret_cast<double2*>(tab + 256);        // rows 32, cols 32
-  float2* rs = reinterpret_cast<float2*>(cen + 2 * kTileF);    // [5][ng][32]
-  float2* cs = rs + 5 * ng * kTileF;                           // [5][ng][32]
-  float* rad = reinterpret_cast<float*>(cs + 5 * ng * kTileF); // rows 32, cols 32
-  long long* links = reinterpret_cast<long long*>(rad + 2 * kTileF);  // 6 x 32
+  double2* cen = tT + kTileF * (kTileF + 1);                   // rows 32, cols 32
+  float4* rxy = reinterpret_cast<float4*>(cen + 2 * kTileF);   // [ng][32] k (x, y) offsets
+  float4* rnn = rxy + SZ;                                      // [ng][32] normals
+  float4* cxy = rnn + SZ;
+  float4* cnn = cxy + SZ;
+  float4* bins = cnn + SZ;                                     // [kFtCap][9]
+  float4* trig = bins + kFtCap * (kFtWords / 4);               // [512]
+  float2* rw = reinterpret_cast<float2*>(trig + kFtTrig);      // [ng][32] weights
+  float2* cw = rw + SZ;
+  long long* links = reinterpret_cast<long long*>(cw + SZ);    // 6 x 32
+  float* rad = reinterpret_cast<float*>(links + 6 * kTileF);   // rows 32, cols 32
+  unsigned* vT = reinterpret_cast<unsigned*>(rad + 2 * kTileF);  // [32] masks
+  float* red = reinterpret_cast<float*>(vT + kTileF);          // 2 x 8
 
   int I, J;
   tile_of(blockIdx.x, &I, &J);
   const int row0 = I * kTileF, col0 = J * kTileF;
   const bool diag = I == J;
   const int n = g.n_unk;
-  for (int v = threadIdx.x; v < 256; v += blockDim.x) tab[v] = gtab[v];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int v = threadIdx.x; v < kFtTrig; v += blockDim.x)
+    trig[v] = ftab[kFtBins * (kFtWords / 4) + v];
   if (threadIdx.x < kTileF) vT[threadIdx.x] = 0u;
-  const int SZ = ng * kTileF;
-  for (int v = threadIdx.x; v < SZ; v += blockDim.x) {
-    const int q = v / kTileF, l = v - q * kTileF;
-    const int ur = min(row0 + l, n - 1), uc = min(col0 + l, n - 1);
-    const size_t ir = (size_t)ur * ng + q, ic = (size_t)uc * ng + q;
-    const int o = q * kTileF + l;
-    rs[o] = tf.ox[ir];
-    rs[SZ + o] = tf.oy[ir];
-    rs[2 * SZ + o] = tf.nx[ir];
-    rs[3 * SZ + o] = tf.ny[ir];
-    rs[4 * SZ + o] = tf.w[ir];
-    cs[o] = tf.ox[ic];
-    cs[SZ + o] = tf.oy[ic];
-    cs[2 * SZ + o] = tf.nx[ic];
-    cs[3 * SZ + o] = tf.ny[ic];
-    cs[4 * SZ + o] = tf.w[ic];
+  for (int v = threadIdx.x; v < 2 * SZ; v += blockDim.x) {
+    const bool isc = v >= SZ;
+    const int o = isc ? v - SZ : v, q = o / kTileF, l = o - q * kTileF;
+    const size_t i = (size_t)min((isc ? col0 : row0) + l, n - 1) * ng + q;
+    const float2 ox = tf.ox[i], oy = tf.oy[i], nx = tf.nx[i], ny = tf.ny[i];
+    const ff X = ff_mul(ff_make(ox.x, ox.y), kc.k), Y = ff_mul(ff_make(oy.x, oy.y), kc.k);
+    (isc ? cxy : rxy)[o] = make_float4(X.hi, X.lo, Y.hi, Y.lo);
+    (isc ? cnn : rnn)[o] = make_float4(nx.x, nx.y, ny.x, ny.y);
+    (isc ? cw : rw)[o] = tf.w[i];
   }
   if (threadIdx.x < kTileF) {
     const int l = threadIdx.x;
@@ -173,16 +179,52 @@ far_ff_kernel(DevGeom g, NodeTable t, NodeTableFF tf, int ng_rt, KConstFF kc, do
   }
   __syncthreads();
 
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = row0 + lane;
-  const long long ri = links[lane], rn = links[kTileF + lane], rp = links[2 * kTileF + lane];
-  const double2 crow = cen[lane];
-  const float rrow = rad[lane];
   const float kf = (float)k;
+
+  // the table intervals between the smallest and the largest argument
+  float xlo = INFINITY, xhi = 0.0f;
+  for (int cc = warp; cc < kTileF; cc += kFarFFThreads / 32) {
+    const float dx = (float)(cen[lane].x - cen[kTileF + cc].x),
+                dy = (float)(cen[lane].y - cen[kTileF + cc].y);
+    const float dist = sqrtf(dx * dx + dy * dy), rr = rad[lane] + rad[kTileF + cc];
+    xlo = fminf(xlo, kf * (dist * (1.0f - 1e-6f) - rr));
+    xhi = fmaxf(xhi, kf * (dist * (1.0f + 1e-6f) + rr));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    xlo = fminf(xlo, __shfl_xor_sync(0xffffffffu, xlo, o));
+    xhi = fmaxf(xhi, __shfl_xor_sync(0xffffffffu, xhi, o));
+  }
+  if (lane == 0) {
+    red[warp] = xlo;
+    red[kFarFFThreads / 32 + warp] = xhi;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int v = 0; v < kFarFFThreads / 32; ++v) {
+    xlo = fminf(xlo, red[v]);
+    xhi = fmaxf(xhi, red[kFarFFThreads / 32 + v]);
+  }
+  // one interval to spare on each side; a pair outside them takes the general
+  // evaluator
+  int bin0 = max(ft_bin(fmaxf(xlo, 4.0f)) - 1, 0);
+  int nbin = max(min(ft_bin(xhi) + 1, kFtBins - 1) - bin0 + 1, 0);
+  const float4* fb = bins;
+  if (nbin <= kFtCap) {
+    for (int v = threadIdx.x; v < nbin * (kFtWords / 4); v += blockDim.x)
+      bins[v] = ftab[bin0 * (kFtWords / 4) + v];
+  } else {
+    bin0 = 0;
+    nbin = kFtBins;
+    fb = ftab;
+  }
+  __syncthreads();
 
 #pragma unroll 1
   for (int cc = warp; cc < kTileF; cc += kFarFFThreads / 32) {
     const int col = col0 + cc;
+    const long long ri = links[lane], rn = links[kTileF + lane], rp = links[2 * kTileF + lane];
     const long long ci = links[3 * kTileF + cc], cn = links[4 * kTileF + cc],
                     cp = links[5 * kTileF + cc];
     // rc: entry (row, col); cr: entry (col, row)
@@ -190,9 +232,10 @@ far_ff_kernel(DevGeom g, NodeTable t, NodeTableFF tf, int ng_rt, KConstFF kc, do
     bool cr = row < n && col < n && !((ci == ri) || (cn == ri) || (cp == ri));
     if (diag && lane >= cc) rc = cr = false;
     if (!rc && !cr) continue;
-    const double dxc = crow.x - cen[kTileF + cc].x, dyc = crow.y - cen[kTileF + cc].y;
-    const float dist = sqrtf((float)(dxc * dxc + dyc * dyc));
-    if (kf * (dist * (1.0f - 1e-6f) - rrow - rad[kTileF + cc]) <= kDeferX) {
+    const ff dxc = ff_from_double(cen[lane].x - cen[kTileF + cc].x),
+             dyc = ff_from_double(cen[lane].y - cen[kTileF + cc].y);
+    const float dist = sqrtf(dxc.hi * dxc.hi + dyc.hi * dyc.hi);
+    if (kf * (dist * (1.0f - 1e-6f) - rad[lane] - rad[kTileF + cc]) <= kDeferX) {
       // small arguments somewhere on this pair: second pass (or here, in
       // FP64, if the list is full).  One list item per pair: (row, col) with the flags
       // kDeferRC / kDeferCR in the top bits of .x for the directions needed.
@@ -211,80 +254,95 @@ far_ff_kernel(DevGeom g, NodeTable t, NodeTableFF tf, int ng_rt, KConstFF kc, do
       }
       continue;
     }
-    const ff Dx = ff_from_double(dxc), Dy = ff_from_double(dyc);
-    // s0: the terms both orientations share (the single-layer part), t_rc /
-    // t_cr: the normal-factor terms of entry (row, col) / (col, row)
-    ffc s0, trc, tcr;
-    s0.re = s0.im = trc.re = trc.im = tcr.re = tcr.im = ff_make(0.0f, 0.0f);
+    const ff Dx = ff_mul(dxc, kc.k), Dy = ff_mul(dyc, kc.k);
+    // With X = k (x - y), Z0 = w_x w_y amp E (P0 + i Q0) and
+    // Z1 = w_x w_y (amp/x) E (P1 + i Q1):
+    //   single layer  (i/4) sum Z0
+    //   combined      (eta/4) sum Z0 - (k/4) sum (n . X) Z1 (double layers
+    //                 without the Z0 term), n . X = n_y . (y - x) k for the
+    //                 double layer at (x, y), n_x . (x - y) k otherwise
+    // s0 = sum Z0, t1 = sum (n_x . X) Z1, t2 = sum (n_y . X) Z1 (x on the row
+    // element) serve both entries of the pair.
+    ffc s0, t1, t2;
+    s0.re = s0.im = t1.re = t1.im = t2.re = t2.im = ff_make(0.0f, 0.0f);
 #pragma unroll 1
     for (int q1 = 0; q1 < ng; ++q1) {
       const int o1 = q1 * kTileF + lane;
-      const float2 a0 = rs[o1], a1 = rs[SZ + o1], a2 = rs[2 * SZ + o1], a3 = rs[3 * SZ + o1],
-                   a4 = rs[4 * SZ + o1];
-      // the row node's position relative to the column element's centre,
-      // once per row node: (c_row - c_col) + o_row
+      const float4 a0 = rxy[o1], a1 = rnn[o1];
+      const float2 a2 = rw[o1];
+      // the row node's position relative to the column element's centre
       const ff Px = ff_add_fast(Dx, ff_make(a0.x, a0.y));
-      const ff Py = ff_add_fast(Dy, ff_make(a1.x, a1.y));
-      const ff n1x = ff_make(a2.x, a2.y), n1y = ff_make(a3.x, a3.y);
-      // the row node's constant factors: amp0 w_x with k/4 (double-layer
-      // part) and eta/4 or 1/4 (single-layer part)
-      const ff aw1 = ff_mul(kc.amp0, ff_make(a4.x, a4.y));
-      const ff c1 = ff_mul(aw1, kc.kq);
-      const ff c0 = KERNEL == BEM2D_KERNEL_SINGLE ? ff_scale2(aw1, 0.25f) : ff_mul(aw1, kc.eq);
+      const ff Py = ff_add_fast(Dy, ff_make(a0.z, a0.w));
 #pragma unroll 1
       for (int q2 = 0; q2 < ng; ++q2) {
         const int o2 = q2 * kTileF + cc;
-        const float2 b0 = cs[o2], b1 = cs[SZ + o2], b2 = cs[2 * SZ + o2], b3 = cs[3 * SZ + o2],
-                     b4 = cs[4 * SZ + o2];
-        // w = x - y, x a node of the row element, y of the column element
-        const ff dx = ff_add_fast(Px, ff_make(-b0.x, -b0.y));
-        const ff dy = ff_add_fast(Py, ff_make(-b1.x, -b1.y));
-        const HankelTermsFF h = hankel_terms_ff(dx, dy, kc, tab);
-        const ff g = ff_mul(h.rx, ff_make(b4.x, b4.y));  // w_y / sqrt(x)
-        if (KERNEL == BEM2D_KERNEL_SINGLE) {
-          // K w_x w_y = (i/4) amp w_x w_y E (P0 + i Q0), the same in both
-          // orientations
-          const ffc Z = ffc_scale(ffc_mul_pq(h.e, h.p0, h.q0), ff_mul(g, c0));
-          ff_acc(s0.re, ff_neg(Z.im));
-          ff_acc(s0.im, Z.re);
+        const float4 b0 = cxy[o2], b1 = cnn[o2];
+        const float2 b2 = cw[o2];
+        const ff dx = ffu_add(Px, ff_make(-b0.x, -b0.y));
+        const ff dy = ffu_add(Py, ff_make(-b0.z, -b0.w));
+        const ff x = ff_sqrt(ffu_dot2(dx, dx, dy, dy));
+        ff p0, q0, p1, q1v;
+        ffc E;
+        const int bin = ft_bin(x.hi) - bin0;
+        if ((unsigned)bin < (unsigned)nbin) {
+          ft_pq<kH0, kH1>(fb + bin * (kFtWords / 4), x, &p0, &q0, &p1, &q1v);
+          E = ft_expi(x, trig);
         } else {
-          // K w_x w_y = Z0 - dot Z1 with Z1 = amp w_x w_y (k/4)/d E (P1 + i Q1)
-          // and, for the combined operator, Z0 = amp w_x w_y (eta/4) E (P0 +
-          // i Q0); dot is the orientation's normal factor (n_y . (y - x) for
-          // the double layer at (x, y), n_x . (x - y) otherwise)
-          const ffc Z1 = ffc_scale(ffc_mul_pq(h.e, h.p1, h.q1), ff_mul(ff_mul(g, h.y), c1));
-          if (KERNEL == BEM2D_KERNEL_COMBINED) {
-            const ffc Z0 = ffc_scale(ffc_mul_pq(h.e, h.p0, h.q0), ff_mul(g, c0));
-            ff_acc(s0.re, Z0.re);
-            ff_acc(s0.im, Z0.im);
-          }
-          const ff n1w = ff_dot2(n1x, dx, n1y, dy);                                // n_x . (x - y)
-          const ff n2w = ff_dot2(ff_make(b2.x, b2.y), dx, ff_make(b3.x, b3.y), dy);  // n_y . (x - y)
-          // (row, col): -dot = n2w (double layer) or -n1w; (col, row): the reverse
-          const ff m_rc = KERNEL == BEM2D_KERNEL_DOUBLE ? n2w : ff_neg(n1w);
-          const ff m_cr = KERNEL == BEM2D_KERNEL_DOUBLE ? ff_neg(n1w) : n2w;
-          if (rc) {
-            ff_acc(trc.re, ff_mul(m_rc, Z1.re));
-            ff_acc(trc.im, ff_mul(m_rc, Z1.im));
-          }
-          if (cr) {
-            ff_acc(tcr.re, ff_mul(m_cr, Z1.re));
-            ff_acc(tcr.im, ff_mul(m_cr, Z1.im));
-          }
+          hankel_direct_ff(x, etab, &p0, &q0, &p1, &q1v, &E);
+        }
+        const ff ww = ffu_mul(ff_make(a2.x, a2.y), ff_make(b2.x, b2.y));
+        E.re = ffu_mul(E.re, ww);
+        E.im = ffu_mul(E.im, ww);
+        if (kH0) {
+          const ffc Z0 = ffcu_mul_pq(E, p0, q0);
+          ff_acc(s0.re, Z0.re);
+          ff_acc(s0.im, Z0.im);
+        }
+        if (kH1) {
+          const ffc Z1 = ffcu_mul_pq(E, p1, q1v);
+          const ff n1 = ffu_dot2(ff_make(a1.x, a1.y), dx, ff_make(a1.z, a1.w), dy);
+          const ff n2 = ffu_dot2(ff_make(b1.x, b1.y), dx, ff_make(b1.z, b1.w), dy);
+          ff_acc(t1.re, ffu_mul(n1, Z1.re));
+          ff_acc(t1.im, ffu_mul(n1, Z1.im));
+          ff_acc(t2.re, ffu_mul(n2, Z1.re));
+          ff_acc(t2.im, ffu_mul(n2, Z1.im));
         }
       }
-      ff_acc_norm(s0.re);
-      ff_acc_norm(s0.im);
-      ff_acc_norm(trc.re);
-      ff_acc_norm(trc.im);
-      ff_acc_norm(tcr.re);
-      ff_acc_norm(tcr.im);
+      if (kH0) {
+        ff_acc_norm(s0.re);
+        ff_acc_norm(s0.im);
+      }
+      if (kH1) {
+        ff_acc_norm(t1.re);
+        ff_acc_norm(t1.im);
+        ff_acc_norm(t2.re);
+        ff_acc_norm(t2.im);
+      }
     }
     ffc arc, acr;
-    arc.re = ff_add(s0.re, trc.re);
-    arc.im = ff_add(s0.im, trc.im);
-    acr.re = ff_add(s0.re, tcr.re);
-    acr.im = ff_add(s0.im, tcr.im);
+    if (KERNEL == BEM2D_KERNEL_SINGLE) {
+      arc.re = ff_scale2(ff_neg(s0.im), 0.25f);
+      arc.im = ff_scale2(s0.re, 0.25f);
+      acr = arc;
+    } else {
+      // -n . X of entry (row, col): n2 (double layer) or -n1; (col, row): the reverse
+      const ff kq = kc.kq, mkq = ff_neg(kc.kq);
+      const ffc& trc = KERNEL == BEM2D_KERNEL_DOUBLE ? t2 : t1;
+      const ffc& tcr = KERNEL == BEM2D_KERNEL_DOUBLE ? t1 : t2;
+      const ff frc = KERNEL == BEM2D_KERNEL_DOUBLE ? kq : mkq;
+      const ff fcr = KERNEL == BEM2D_KERNEL_DOUBLE ? mkq : kq;
+      arc.re = ff_mul(frc, trc.re);
+      arc.im = ff_mul(frc, trc.im);
+      acr.re = ff_mul(fcr, tcr.re);
+      acr.im = ff_mul(fcr, tcr.im);
+      if (KERNEL == BEM2D_KERNEL_COMBINED) {
+        const ff er = ff_mul(kc.eq, s0.re), ei = ff_mul(kc.eq, s0.im);
+        arc.re = ff_add(arc.re, er);
+        arc.im = ff_add(arc.im, ei);
+        acr.re = ff_add(acr.re, er);
+        acr.im = ff_add(acr.im, ei);
+      }
+    }
     if (rc) {
       const double re = alpha * ff_to_double(arc.re), im = alpha * ff_to_double(arc.im);
       out[(size_t)col * ld + row] = make_double2(re, im);
@@ -383,23 +441,39 @@ deferred_ff_kernel(NodeTableFF tf, int ng, KConstFF kc, double alpha, const int2
   }
 }
 
-const float* expi_table_dev() {
-  constexpr int kMaxDev = 64;
-  static std::mutex mu;
-  static float* tab[kMaxDev] = {};
+// A table of `count` floats made by `build` on the host and kept on the current
+// device.
+template <typename B>
+static const float* device_table(float* (&tab)[64], std::mutex& mu, size_t count, B build) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= kMaxDev) return nullptr;
+  if (dev < 0 || dev >= 64) return nullptr;
   std::lock_guard<std::mutex> lock(mu);
   if (!tab[dev]) {
-    float h[256];
-    expi_table(h);
+    std::vector<float> h(count);
+    build(h.data());
     float* d = nullptr;
-    if (cudaMalloc(&d, sizeof h) != cudaSuccess) return nullptr;
-    cudaMemcpy(d, h, sizeof h, cudaMemcpyHostToDevice);
+    if (cudaMalloc(&d, sizeof(float) * count) != cudaSuccess) return nullptr;
+    if (cudaMemcpy(d, h.data(), sizeof(float) * count, cudaMemcpyHostToDevice) != cudaSuccess) {
+      cudaFree(d);
+      return nullptr;
+    }
     tab[dev] = d;
   }
   return tab[dev];
+}
+
+const float* expi_table_dev() {
+  static std::mutex mu;
+  static float* tab[64] = {};
+  return device_table(tab, mu, 256, expi_table);
+}
+
+// The far field's table (see hankel_tab_ff.cuh).
+static const float* ft_table_dev() {
+  static std::mutex mu;
+  static float* tab[64] = {};
+  return device_table(tab, mu, kFtFloats, ft_build);
 }
 
 template <int KERNEL>
@@ -407,24 +481,20 @@ static int launch_far_ff_k(const DevGeom& g, const NodeTable& t, const NodeTable
                             double k, double eta, double alpha, double2* out, long long ld,
                             float2* out32, long long ld32, DeferList dl, cudaStream_t s) {
   const KConstFF kc = make_kconst(k, eta);
-  const size_t smem = sizeof(double2) * kTileF * (kTileF + 1) + sizeof(unsigned) * kTileF +
-                      sizeof(float) * 256 + sizeof(double2) * 2 * kTileF +
-                      sizeof(float2) * 10 * ng * kTileF + sizeof(float) * 2 * kTileF +
-                      sizeof(long long) * 6 * kTileF;
+  const size_t smem = sizeof(double2) * (kTileF * (kTileF + 1) + 2 * kTileF) +
+                      (4 * sizeof(float4) + 2 * sizeof(float2)) * (size_t)ng * kTileF +
+                      sizeof(float) * kFtWords * kFtCap + sizeof(float4) * kFtTrig +
+                      sizeof(long long) * 6 * kTileF + sizeof(float) * (3 * kTileF + 16);
   const unsigned nt = (unsigned)((g.n_unk + kTileF - 1) / kTileF);
   dim3 grid(nt * (nt + 1) / 2);  // tile pairs (I, J), I <= J
-  const float* tab = expi_table_dev();
-  if (!tab) return BEM2D_ERR_NOMEM;
-  if (ng == 5) {
-    far_ff_kernel<KERNEL, 5><<<grid, kFarFFThreads, smem, s>>>(g, t, tf, ng, kc, k, eta, alpha, out,
-                                                               ld, out32, ld32, dl, tab);
-  } else {
-    auto fn = far_ff_kernel<KERNEL, 0>;
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    fn<<<grid, kFarFFThreads, smem, s>>>(g, t, tf, ng, kc, k, eta, alpha, out, ld, out32, ld32, dl,
-                                         tab);
-  }
+  const float* ftab = ft_table_dev();
+  const float* etab = expi_table_dev();
+  if (!ftab || !etab) return BEM2D_ERR_NOMEM;
+  auto fn = ng == 5 ? far_ff_kernel<KERNEL, 5> : far_ff_kernel<KERNEL, 0>;
+  // one value for all rules: calls of several threads must not undo each other
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  fn<<<grid, kFarFFThreads, smem, s>>>(g, t, tf, ng, kc, k, eta, alpha, out, ld, out32, ld32, dl,
+                                       reinterpret_cast<const float4*>(ftab), etab);
   return BEM2D_OK;
 }
 

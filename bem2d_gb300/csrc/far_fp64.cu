@@ -423,8 +423,9 @@ static void launch_far_nb(const DevGeom& g, const NodeTable& t, const FarGroups&
   const size_t smem = fixed + per_col * cols;
   const dim3 grid((fg.n + cols - 1) / cols, rows);
   auto fn = far_fp64_kernel<KERNEL, NB, CK>;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // one value for all rules: calls of several threads must not undo each other
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)std::max<size_t>(smem, 208 * 1024));
   fn<<<grid, 32 * nw, smem, s>>>(g, t, fg, ng, cols, tb, k, ki, ka, eta, alpha, out, ld);
 }
 

@@ -9,7 +9,7 @@
 namespace bem2d_gpu {
 
 struct KConstFF {
-  ff k, invk, kq, eq, amp0;
+  ff k, invk, kq, eq;
 };
 
 inline KConstFF make_kconst(double k, double eta) {
@@ -18,7 +18,6 @@ inline KConstFF make_kconst(double k, double eta) {
   kc.invk = ff_from_double(1.0 / k);
   kc.kq = ff_from_double(0.25 * k);
   kc.eq = ff_from_double(0.25 * eta);
-  kc.amp0 = ff_from_double(0.79788456080286535588);  // sqrt(2/pi)
   return kc;
 }
 
