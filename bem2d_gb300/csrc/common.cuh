@@ -440,7 +440,7 @@ struct LuWork {
   // persistent CTAs of the tensor-core update (0: one per SM); fewer leave
   // SMs to concurrent factorisations
   int tc_ctas = 0;
-  // products per term of the tensor-core update: 3 (3xTF32) or 1 (1xTF32)
+  // products per term of the tensor-core update: 3 (hi and lo halves) or 1 (hi only)
   int tc_passes = 3;
   // look-ahead of the blocked complex64 factorisation (all set, or none):
   // the trailing update of the columns beyond the next block runs on `aux`
@@ -500,9 +500,9 @@ void launch_gather_to_c64(int n, const double2* src, const int* perm, double sca
 void launch_scatter_c64(int n, const float2* src, const int* perm, float2* dst, cudaStream_t s);
 
 // C -= A B for complex64 column-major operands on the tensor cores
-// (tcgen05 kind::tf32; lu_tc.cu).  C is M x N, A M x K, B K x N.
-// passes = 3: 3xTF32 split (FP32-accurate products); 1: 1xTF32 (operands
-// rounded to TF32, a third of the tensor work).
+// (tcgen05 kind::f16; lu_tc.cu).  C is M x N, A M x K, B K x N.
+// passes = 3: scaled entries split into two f16 (FP32-accurate products); 1:
+// the first of them only (10 mantissa bits, a third of the tensor work).
 // Sets *status on a device-side wait timeout.
 // `pack` (tc_pack_bytes(M, N, K) bytes) holds the split, re-laid-out operands.
 size_t tc_pack_bytes(int M, int N, int K);

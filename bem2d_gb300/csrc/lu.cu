@@ -1582,7 +1582,7 @@ static int update_sub(T* C, const T* Am, const T* Bm, long long ld, int M, int N
         (N >= 4 * kTensorMinN && M >= kNB)) {
       ++*launches;
       if (w.pack && tc_pack_bytes(M, N, K) <= w.pack_bytes) {
-        *launches += 2;  // + the two packing kernels
+        ++*launches;  // + the packing kernel
         return launch_tc_cgemm_sub(reinterpret_cast<float2*>(C), ld,
                                    reinterpret_cast<const float2*>(Am), ld,
                                    reinterpret_cast<const float2*>(Bm), ld, M, N, K, w.pack,
@@ -2467,7 +2467,7 @@ int lu_inverse_c64(const float2* LU, long long lda, int n, const LuWork& w, floa
     if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
     if (launch_tc_cgemm_sub(C, ldw, Am, lda, Bm, ldw, M, N, K, w.pack, w.pack_bytes, w.status, s))
       return BEM2D_ERR_CUDA;
-    *launches += 3;
+    *launches += 2;
     return BEM2D_OK;
   };
   if (cudaMemset2DAsync(W, sizeof(float2) * ldw, 0, sizeof(float2) * n, n, s) != cudaSuccess)

@@ -1,6 +1,6 @@
 // Trailing update of the complex64 LU on the 5th-generation tensor cores:
 // C -= A B (complex64, column-major, arbitrary leading dimensions), as
-// tcgen05.mma kind::tf32 with FP32 accumulators in tensor memory.
+// tcgen05.mma kind::f16 with FP32 accumulators in tensor memory.
 //
 // Complex arithmetic as one real product.  The complex M x K operand A is
 // read as a real (2M) x K matrix A' whose rows 2i and 2i + 1 hold re and im
@@ -13,29 +13,38 @@
 // A tile is 64 complex rows (128 real rows = the MMA's M) by 128 complex
 // columns: 256 tensor-memory columns per accumulator.
 //
-// Accuracy (3xTF32): every FP32 operand x is split into hi = x rounded to
-// the nearest TF32 value (10 mantissa bits) and lo = x - hi (exact); each
-// product is accumulated as hi*hi + hi*lo + lo*hi, which keeps about 21 bits
-// per product - the accuracy of the FP32 update it replaces, so the LU keeps
-// the quality the FP64 refinement expects.  With passes = 1 (1xTF32) only
-// hi*hi is issued: a third of the tensor work, products to about 2^-11
-// relative, for systems whose condition number the refinement tolerates at
-// that precision.
+// Accuracy: row i of A and column j of B are scaled by powers of two so that
+// their largest entry lies in [2^14, 2^15), and every scaled FP32 entry x is
+// split into hi = x rounded to f16 and lo = x - hi rounded to f16 (11 bits
+// each); a product is accumulated as hi*hi + hi*lo + lo*hi.  That keeps 22 bits
+// of every entry within 2^-16 of its row's (column's) largest and an absolute
+// error of 2^-40 of the largest below - no less than the 3xTF32 split it
+// replaces (TF32 has the same 10 mantissa bits), at twice its rate: f16
+// operands are half the bytes and an MMA covers 16 of K instead of 8.  With
+// passes = 1 only hi*hi is issued: a third of the tensor work, products to
+// about 2^-11 relative, for systems whose condition number the refinement
+// tolerates at that precision.  Error against complex128 over (|A| |B|)_ij,
+// rank-256 update of random 3000 x 3000: 7.8e-8 rms, 3.7e-7 at most (3xTF32:
+// 1.5e-7, 7.1e-7); smaller too for rows, columns or entries over many decades.
+// All updates of the L-shape's LU, N = 16384: 51.4 -> 30.1 ms, their packing
+// (one kernel instead of two) 8.7 -> 3.9 ms; norm and condition number's, N =
+// 8192: 19 -> 12.4 ms.
 //
-// Operands are packed once per update (pack_a_kernel, pack_b_kernel): split
-// into hi/lo and laid out, per tile and per chunk of 16 along K, exactly as
+// Operands are packed once per update (pack_kernel): scaled, split into hi/lo
+// and laid out, per tile and per chunk of 32 along K, exactly as
 // the MMA reads them from shared memory - the K-major, non-swizzled
 // canonical layout (core matrices of 8 rows x 16 bytes, 128 bytes from one
 // core matrix to the next along K, 512 bytes from one group of 8 rows to the
 // next).  A chunk is then one contiguous block per operand: 16 KB of A'
-// (hi, lo) and 32 KB of B (hi, lo).
+// (hi, lo) and 32 KB of B (hi, lo).  The inverse scales (a byte each, the
+// exponent field) are applied in the epilogue.
 //
 // The update kernel is persistent (one CTA per SM, tiles in a static
 // round-robin) and warp-specialised:
 //   warp 0      producer: two bulk copies (cp.async.bulk, completion counted
 //               in bytes on the stage's `full` mbarrier) per chunk into a
 //               ring of four 48 KB shared-memory stages;
-//   warp 1      MMA issuer: six MMAs per chunk (two K-steps of 8, 3xTF32);
+//   warp 1      MMA issuer: six MMAs per chunk (two K-steps of 16, three products);
 //               tcgen05.commit frees the stage (`empty`) once its MMAs have
 //               read it, and marks the tile's accumulator complete (`acc_full`);
 //   warps 2-17  epilogue: tcgen05.ld of the accumulator (warp w reads TMEM
@@ -50,6 +59,7 @@
 // (2 s of device time): on timeout the status flag is set, every role stops,
 // the producer waits (bounded) for its copies in flight and the MMA thread
 // for its MMAs, and the tensor memory is released before the kernel returns.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -62,14 +72,14 @@ using namespace tc;
 
 constexpr int kTcBM = 64;    // complex rows per tile (128 real rows = MMA M)
 constexpr int kTcBN = 128;   // complex columns per tile (MMA N = 256: re, im)
-constexpr int kTcBK = 16;    // K per chunk (two MMAs of K = 8)
+constexpr int kTcBK = 32;    // K per chunk (two MMAs of K = 16)
 constexpr int kTcStages = 4;
 constexpr int kTcThreads = 576;  // producer warp, MMA warp, 16 epilogue warps
 constexpr int kTcEpiThreads = 512;
 constexpr int kCoreBytes = 128;                   // 8 rows x 16 bytes
-constexpr int kTcSBO = (kTcBK / 4) * kCoreBytes;  // 512
-constexpr int kTcApart = 2 * kTcBM * kTcBK * 4;   // 8 KB: 128 real rows x 16
-constexpr int kTcBpart = 2 * kTcBN * kTcBK * 4;   // 16 KB: 256 rows x 16
+constexpr int kTcSBO = (kTcBK / 8) * kCoreBytes;  // 512
+constexpr int kTcApart = 2 * kTcBM * kTcBK * 2;   // 8 KB: 128 real rows x 32
+constexpr int kTcBpart = 2 * kTcBN * kTcBK * 2;   // 16 KB: 256 rows x 32
 constexpr int kTcChunkA = 2 * kTcApart;           // hi, lo
 constexpr int kTcChunkB = 2 * kTcBpart;           // hi, lo
 constexpr int kTcStage = kTcChunkA + kTcChunkB;   // 48 KB
@@ -83,78 +93,112 @@ __device__ __forceinline__ unsigned long long smem_desc(unsigned addr) {
          ((unsigned long long)(kCoreBytes >> 4) << 16) |
          ((unsigned long long)(kTcSBO >> 4) << 32) | (1ull << 46);
 }
-// byte offset of (row r, k) inside one packed chunk
-__host__ __device__ __forceinline__ int kmajor_off(int r, int k) {
-  return (r >> 3) * kTcSBO + (k >> 2) * kCoreBytes + (r & 7) * 16 + (k & 3) * 4;
-}
-// hi = x rounded to 10 mantissa bits (ties away from zero), lo = x - hi
-__device__ __forceinline__ void tf32_split(float x, float& hi, float& lo) {
-  hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
-  lo = x - hi;
+// byte offset of (row r, 8 consecutive k from 8 o) inside one packed chunk
+__device__ __forceinline__ int kmajor_off(int r, int o) {
+  return (r >> 3) * kTcSBO + o * kCoreBytes + (r & 7) * 16;
 }
 
-__device__ __forceinline__ void mma_tf32(unsigned d, unsigned a, unsigned b, unsigned idesc,
-                                         unsigned acc) {
+__device__ __forceinline__ void mma_f16(unsigned d, unsigned a, unsigned b, unsigned idesc,
+                                        unsigned acc) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
       "l"(smem_desc(a)), "l"(smem_desc(b)), "r"(idesc), "r"(acc));
 }
-#define TC_LD16(dst, addr)                                                                  \
-  asm volatile(                                                                             \
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13," \
-      "%14,%15}, [%16];"                                                                     \
-      : "=r"(dst[0]), "=r"(dst[1]), "=r"(dst[2]), "=r"(dst[3]), "=r"(dst[4]), "=r"(dst[5]), \
-        "=r"(dst[6]), "=r"(dst[7]), "=r"(dst[8]), "=r"(dst[9]), "=r"(dst[10]), "=r"(dst[11]), \
-        "=r"(dst[12]), "=r"(dst[13]), "=r"(dst[14]), "=r"(dst[15])                          \
-      : "r"(addr))
+#define TC_LD8(dst, addr)                                                                 \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"   \
+               : "=r"(dst[0]), "=r"(dst[1]), "=r"(dst[2]), "=r"(dst[3]), "=r"(dst[4]),    \
+                 "=r"(dst[5]), "=r"(dst[6]), "=r"(dst[7])                                 \
+               : "r"(addr))
 
 // ---- packing ---------------------------------------------------------------
-// A (M x K complex) -> Apk[mt][kc] = {hi, lo} chunks of kTcApart bytes each.
-// grid: (ceil(M / 64) * 64 / 128 x nkc * 16), 128 threads
-__global__ void pack_a_kernel(const float2* __restrict__ A, long long lda, int M, int K, int nkc,
-                              int passes, unsigned char* __restrict__ Apk) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // complex row
-  const int k = blockIdx.y;                             // 0 .. nkc * 16 - 1
-  const int mt = i / kTcBM, il = i - mt * kTcBM;
-  const int kc = k / kTcBK, kl = k - kc * kTcBK;
-  if (i >= ((M + kTcBM - 1) / kTcBM) * kTcBM) return;
-  const float2 v = (i < M && k < K) ? A[(size_t)k * lda + i] : make_float2(0.f, 0.f);
-  unsigned char* chunk = Apk + ((size_t)mt * nkc + kc) * kTcChunkA;
-  float h, l;
-  float h2, l2;
-  tf32_split(v.x, h, l);
-  tf32_split(v.y, h2, l2);
-  *reinterpret_cast<float*>(chunk + kmajor_off(2 * il, kl)) = h;
-  *reinterpret_cast<float*>(chunk + kmajor_off(2 * il + 1, kl)) = h2;
-  if (passes > 1) {
-    *reinterpret_cast<float*>(chunk + kTcApart + kmajor_off(2 * il, kl)) = l;
-    *reinterpret_cast<float*>(chunk + kTcApart + kmajor_off(2 * il + 1, kl)) = l2;
+// Exponent field of the power of two that brings a largest absolute value of m
+// to [2^14, 2^15), within what a float holds on both sides (m = 0, infinite or
+// below 2^-110 included), and of its inverse.
+__device__ __forceinline__ int scale_exp(float m) {
+  const int e = min(max((__float_as_int(m) >> 23) & 0xff, 17), 254);
+  return 254 + 14 - e;
+}
+__device__ __forceinline__ float exp_float(int e) { return __int_as_float(e << 23); }
+
+// 8 values times sc, split into f16 hi and lo, 16 bytes each
+__device__ __forceinline__ void split8(const float (&v)[8], float sc, int passes,
+                                       unsigned char* hi, unsigned char* lo) {
+  unsigned h[4], l[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float x = v[2 * j] * sc, y = v[2 * j + 1] * sc;
+    const __half2 p = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(p);
+    const __half2 r = __floats2half2_rn(x - f.x, y - f.y);
+    h[j] = *reinterpret_cast<const unsigned*>(&p);
+    l[j] = *reinterpret_cast<const unsigned*>(&r);
   }
+  *reinterpret_cast<uint4*>(hi) = make_uint4(h[0], h[1], h[2], h[3]);
+  if (passes > 1) *reinterpret_cast<uint4*>(lo) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// A (M x K complex) -> Apk[mt][kc] = {hi, lo} chunks of kTcApart bytes each;
 // B (K x N complex) -> Bpk[nt][kc] = {hi, lo} chunks of kTcBpart bytes, each
-// with rows 0..127 = re and rows 128..255 = im of the tile's 128 columns.
-// grid: (ceil(N / 128) * 128 x ceil(nkc * 16 / 64)), 64 threads
-__global__ void pack_b_kernel(const float2* __restrict__ B, long long ldb, int K, int N, int nkc,
-                              int passes, unsigned char* __restrict__ Bpk) {
-  const int n = blockIdx.x;                             // complex column
-  const int k = blockIdx.y * blockDim.x + threadIdx.x;  // 0 .. nkc * 16 - 1
-  if (k >= nkc * kTcBK) return;
-  const int nt = n / kTcBN, nl = n - nt * kTcBN;
-  const int kc = k / kTcBK, kl = k - kc * kTcBK;
-  const float2 v = (k < K && n < N) ? B[(size_t)n * ldb + k] : make_float2(0.f, 0.f);
-  unsigned char* chunk = Bpk + ((size_t)nt * nkc + kc) * kTcChunkB;
-  const int ore = kmajor_off(nl, kl), oim = kmajor_off(kTcBN + nl, kl);
-  float h, l;
-  float h2, l2;
-  tf32_split(v.x, h, l);
-  tf32_split(v.y, h2, l2);
-  *reinterpret_cast<float*>(chunk + ore) = h;
-  *reinterpret_cast<float*>(chunk + oim) = h2;
-  if (passes > 1) {
-    *reinterpret_cast<float*>(chunk + kTcBpart + ore) = l;
-    *reinterpret_cast<float*>(chunk + kTcBpart + oim) = l2;
+// with rows 0..127 = re and rows 128..255 = im of the tile's 128 columns;
+// isa, isb: exponent fields of the inverse scales.  One launch for both
+// operands: the first ab CTAs take 32 rows of A each (a warp 32 rows x 8 k at a
+// time), the others 8 columns of B (a warp 8 columns x 32 k).  Each operand is
+// read twice, for the largest entry and for the split (the second time from
+// L1).  256 threads.
+__global__ void __launch_bounds__(256)
+pack_kernel(const float2* __restrict__ A, long long lda, const float2* __restrict__ B,
+            long long ldb, int M, int N, int K, int nkc, int ab, int passes,
+            unsigned char* __restrict__ Apk, unsigned char* __restrict__ Bpk,
+            unsigned char* __restrict__ isa, unsigned char* __restrict__ isb) {
+  __shared__ float red[8][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool is_a = (int)blockIdx.x < ab;
+  // row of A, or column of B; first octet of k and octet step of this thread
+  const int r = is_a ? blockIdx.x * 32 + lane : (blockIdx.x - ab) * 8 + (lane & 7);
+  const int o0 = is_a ? w : 4 * w + (lane >> 3), os = is_a ? 8 : 32;
+  const bool ok = r < (is_a ? M : N);
+  const float2* src = is_a ? A + r : B + (size_t)r * ldb;
+  const long long st = is_a ? lda : 1;
+  float mx = 0.f;
+  for (int o = o0; o < 4 * nkc; o += os) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = 8 * o + j;
+      const float2 v = ok && k < K ? src[k * st] : make_float2(0.f, 0.f);
+      mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+    }
+  }
+  if (!is_a) {
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+  }
+  red[w][lane] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) mx = fmaxf(mx, red[j][lane]);
+  const int se = scale_exp(mx);
+  const float sc = exp_float(se);
+  const int T = is_a ? kTcBM : kTcBN;
+  const int tl = r / T, il = r - tl * T;
+  if (w == 0 && (is_a || lane < 8)) (is_a ? isa : isb)[r] = (unsigned char)(254 - se);
+  const int part = is_a ? kTcApart : kTcBpart, chunk_bytes = 2 * part;
+  unsigned char* dst = (is_a ? Apk : Bpk) + (size_t)tl * nkc * chunk_bytes;
+  const int rre = is_a ? 2 * il : il, rim = is_a ? 2 * il + 1 : kTcBN + il;
+  for (int o = o0; o < 4 * nkc; o += os) {
+    float re[8], im[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = 8 * o + j;
+      const float2 v = ok && k < K ? src[k * st] : make_float2(0.f, 0.f);
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    unsigned char* c = dst + (size_t)(o >> 2) * chunk_bytes;
+    unsigned char* cre = c + kmajor_off(rre, o & 3);
+    unsigned char* cim = c + kmajor_off(rim, o & 3);
+    split8(re, sc, passes, cre, cre + part);
+    split8(im, sc, passes, cim, cim + part);
   }
 }
 
@@ -163,7 +207,8 @@ __global__ void pack_b_kernel(const float2* __restrict__ B, long long ldb, int K
 // of shared memory (one CTA per SM).  Tile t: mt = t % mtiles, nt = t / mtiles.
 __global__ void __launch_bounds__(kTcThreads, 1)
 tc_cgemm_sub_kernel(float2* __restrict__ C, long long ldc, const unsigned char* __restrict__ Apk,
-                    const unsigned char* __restrict__ Bpk, int M, int N, int nkc, int mtiles,
+                    const unsigned char* __restrict__ Bpk, const unsigned char* __restrict__ isa,
+                    const unsigned char* __restrict__ isb, int M, int N, int nkc, int mtiles,
                     int ntiles, int passes, int* status) {
   extern __shared__ __align__(1024) unsigned char sm[];
   unsigned long long* full = reinterpret_cast<unsigned long long*>(sm + kTcBarOff);
@@ -197,10 +242,9 @@ tc_cgemm_sub_kernel(float2* __restrict__ C, long long ldc, const unsigned char* 
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const unsigned tmem = *tslot;
-  // kind::tf32: D f32 (bits 4-5 = 1), A/B tf32 (bits 7-9, 10-12 = 2), both
-  // K-major, N >> 3 at bit 17, M >> 4 at bit 24
-  const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((kTcAcc >> 3) << 17) |
-                         ((128u >> 4) << 24);
+  // kind::f16: D f32 (bits 4-5 = 1), A and B f16 (0), both K-major, N >> 3 at
+  // bit 17, M >> 4 at bit 24
+  const unsigned idesc = (1u << 4) | ((kTcAcc >> 3) << 17) | ((128u >> 4) << 24);
   bool ok = true;
   if (w == 0) {
     if (lane == 0) {  // ---- producer
@@ -217,7 +261,7 @@ tc_cgemm_sub_kernel(float2* __restrict__ C, long long ldc, const unsigned char* 
             break;
           }
           unsigned char* st = sm + s * kTcStage;
-          // 1xTF32: the hi halves only (the first half of each packed chunk)
+          // one product: the hi halves only (the first half of each packed chunk)
           const unsigned abytes = passes > 1 ? kTcChunkA : kTcApart;
           const unsigned bbytes = passes > 1 ? kTcChunkB : kTcBpart;
           mbar_expect_tx(&full[s], abytes + bbytes);
@@ -256,12 +300,12 @@ tc_cgemm_sub_kernel(float2* __restrict__ C, long long ldc, const unsigned char* 
           const unsigned ah = base, al = base + kTcApart;
           const unsigned bh = base + kTcChunkA, bl = bh + kTcBpart;
 #pragma unroll
-          for (int ks = 0; ks < kTcBK / 8; ++ks) {
-            const unsigned o = 256u * ks;  // K = 8 tf32 = two core matrices
-            mma_tf32(d, ah + o, bh + o, idesc, (c == 0 && ks == 0) ? 0u : 1u);
+          for (int ks = 0; ks < kTcBK / 16; ++ks) {
+            const unsigned o = 256u * ks;  // K = 16 f16 = two core matrices
+            mma_f16(d, ah + o, bh + o, idesc, (c == 0 && ks == 0) ? 0u : 1u);
             if (passes > 1) {
-              mma_tf32(d, ah + o, bl + o, idesc, 1u);
-              mma_tf32(d, al + o, bh + o, idesc, 1u);
+              mma_f16(d, ah + o, bl + o, idesc, 1u);
+              mma_f16(d, al + o, bh + o, idesc, 1u);
             }
           }
           mma_commit(&empty[s]);  // the stage may be refilled once these MMAs read it
@@ -313,6 +357,7 @@ tc_cgemm_sub_kernel(float2* __restrict__ C, long long ldc, const unsigned char* 
           for (int u = 0; u < kTcBN / 4; ++u, pc += cstep) cv[u] = u < nlim ? *pc : 0.f;
         }
       }
+      const float isr = exp_float(isa[i0 + i]);  // the row's inverse scale
       const int a = j & 1;
       const unsigned aph = (unsigned)(j >> 1) & 1u;
       if (!mbar_wait(&acc_full[a], aph, s_abort)) {
@@ -324,23 +369,26 @@ tc_cgemm_sub_kernel(float2* __restrict__ C, long long ldc, const unsigned char* 
                              (unsigned)(part * (kTcBN / 4));
       float* pw = crow + (size_t)n0 * cstep;
 #pragma unroll
-      for (int h = 0; h < kTcBN / 4; h += 16) {
-        unsigned d1[16], d2[16];
-        TC_LD16(d1, lanes + h);
-        TC_LD16(d2, lanes + kTcBN + h);
+      for (int h = 0; h < kTcBN / 4; h += 8) {
+        unsigned d1[8], d2[8];
+        TC_LD8(d1, lanes + h);
+        TC_LD8(d2, lanes + kTcBN + h);
+        // exponent fields of the 8 columns' inverse scales
+        const uint2 iv = *reinterpret_cast<const uint2*>(isb + n0 + h);
         asm volatile("tcgen05.wait::ld.sync.aligned;");
-        float o[16];
+        float o[8];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
+        for (int u = 0; u < 8; ++u) {
           const float p2 = __shfl_xor_sync(0xffffffffu, __uint_as_float(d2[u]), 1);
-          o[u] = cv[h + u] - (__uint_as_float(d1[u]) + (cc ? p2 : -p2));
+          const float isc = exp_float(((u < 4 ? iv.x : iv.y) >> (8 * (u & 3))) & 0xff);
+          o[u] = cv[h + u] - (__uint_as_float(d1[u]) + (cc ? p2 : -p2)) * isr * isc;
         }
         if (nlim == kTcBN / 4) {
 #pragma unroll
-          for (int u = 0; u < 16; ++u, pw += cstep) *pw = o[u];
+          for (int u = 0; u < 8; ++u, pw += cstep) *pw = o[u];
         } else {
 #pragma unroll
-          for (int u = 0; u < 16; ++u, pw += cstep)
+          for (int u = 0; u < 8; ++u, pw += cstep)
             if (h + u < nlim) *pw = o[u];
         }
       }
@@ -356,7 +404,7 @@ tc_cgemm_sub_kernel(float2* __restrict__ C, long long ldc, const unsigned char* 
   if (w == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }
 
-#undef TC_LD16
+#undef TC_LD8
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
@@ -375,7 +423,8 @@ int num_sms() {
 size_t tc_pack_bytes(int M, int N, int K) {
   const size_t nkc = (size_t)(K + kTcBK - 1) / kTcBK;
   const size_t mt = (size_t)(M + kTcBM - 1) / kTcBM, nt = (size_t)(N + kTcBN - 1) / kTcBN;
-  return align256(mt * nkc * kTcChunkA) + align256(nt * nkc * kTcChunkB);
+  return align256(mt * nkc * kTcChunkA) + align256(nt * nkc * kTcChunkB) +
+         align256(mt * kTcBM) + align256(nt * kTcBN);
 }
 
 int launch_tc_cgemm_sub(float2* C, long long ldc, const float2* A, long long lda,
@@ -392,13 +441,14 @@ int launch_tc_cgemm_sub(float2* C, long long ldc, const float2* A, long long lda
   const int mt = (M + kTcBM - 1) / kTcBM, nt = (N + kTcBN - 1) / kTcBN;
   unsigned char* Apk = static_cast<unsigned char*>(pack);
   unsigned char* Bpk = Apk + align256((size_t)mt * nkc * kTcChunkA);
-  pack_a_kernel<<<dim3((mt * kTcBM + 127) / 128, nkc * kTcBK), 128, 0, s>>>(A, lda, M, K, nkc,
-                                                                            passes, Apk);
-  pack_b_kernel<<<dim3(nt * kTcBN, (nkc * kTcBK + 63) / 64), 64, 0, s>>>(B, ldb, K, N, nkc,
-                                                                        passes, Bpk);
+  unsigned char* isa = Bpk + align256((size_t)nt * nkc * kTcChunkB);
+  unsigned char* isb = isa + align256((size_t)mt * kTcBM);
+  const int ab = mt * (kTcBM / 32);
+  pack_kernel<<<ab + nt * (kTcBN / 8), 256, 0, s>>>(A, lda, B, ldb, M, N, K, nkc, ab, passes, Apk,
+                                                    Bpk, isa, isb);
   const int grid = std::min(mt * nt, max_ctas > 0 ? max_ctas : num_sms());
-  tc_cgemm_sub_kernel<<<grid, kTcThreads, kTcSmem, s>>>(C, ldc, Apk, Bpk, M, N, nkc, mt, nt,
-                                                        passes, status);
+  tc_cgemm_sub_kernel<<<grid, kTcThreads, kTcSmem, s>>>(C, ldc, Apk, Bpk, isa, isb, M, N, nkc, mt,
+                                                        nt, passes, status);
   return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
 }
 

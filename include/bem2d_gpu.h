@@ -79,8 +79,8 @@ extern "C" {
 #define BEM2D_PREC_FP64 0  /* complex128 LU, FP64 throughout                 */
 #define BEM2D_PREC_MIXED 1 /* complex64 LU + FP64 iterative refinement      */
 /* As BEM2D_PREC_MIXED, with the LU's tensor-core trailing updates as one
- * TF32 product per term (1xTF32: operands rounded to 10 mantissa bits, a
- * third of the 3xTF32 tensor work).  The factor is then accurate to about
+ * product per term (operands rounded to 10 mantissa bits, as TF32 holds; a
+ * third of the tensor work).  The factor is then accurate to about
  * 1e-3 relative instead of 1e-6, so refinement contracts the error by about
  * cond(A) 1e-3 per step: for systems with cond(A) up to ~100; beyond that
  * GMRES-IR takes over (see bem2d_solve_system).  Accepted by
@@ -388,7 +388,7 @@ int bem2d_debug_panel_timeout(bem2d_ctx* ctx, int n, int polls);
 
 /* C -= A B for complex64 column-major device matrices (C M x N, A M x K,
  * B K x N) through the complex64 LU's tensor-core trailing update
- * (tcgen05 kind::tf32, 3xTF32 split): the update of zgetrf's right-looking
+ * (tcgen05 kind::f16, scaled two-way split): the update of zgetrf's right-looking
  * step (lib/bem2d_mathroutines.cpp:345) exposed for its own parity test. */
 int bem2d_debug_tc_update(bem2d_ctx* ctx, int M, int N, int K, void* C, int64_t ldc,
                           const void* A, int64_t lda, const void* B, int64_t ldb);
