@@ -817,212 +817,303 @@ panel_rows_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, 
 }
 
 // ---- register-window complex64 panel ----------------------------------------
-// Complex64 panels of up to 16 x 256 rows.  Two threads per row, each
-// holding every other column pair of it in registers (thread h of a row holds
-// pairs 2i + h, i = 0..15, as float4 r[16]).  Columns are processed in
-// blocks of four (two pairs, one per thread of the row): inside a block the
-// column index is a compile-time constant (the loop is unrolled), so every
-// register index is static; after a block its finished pairs go to shared
-// memory (Fin) and each thread's window shifts by one, so r[i] holds pair
-// 2(b + i) + h in block b.  Rows are exchanged by renaming, as in the
-// shared-memory panels (same ipiv).
-// Reductions use the warp reduce instructions: the maximum of (bits of
-// |re|+|im|) + 1 (0 = no candidate; non-negative floats order like their
-// bits), then the minimum label among the lanes holding that maximum.
-// Per column: one __syncthreads for the warp maxima, from which every warp
-// forms the CTA candidate; the candidate's warp sends the row (columns c..63)
-// and its key to every CTA with asynchronous stores that count their bytes on
-// the receiver's mbarrier; every warp waits there (bounded), picks the pivot
-// and updates its registers.  No cluster barrier: a CTA sends its candidate of
-// column c + 1 after it has used the ones of column c, so with two buffers
-// (column parity) whoever holds all candidates of c + 1 may overwrite those of
-// c.  Bound by the latency of that one-way exchange: 64 columns of 2048 rows
-// 70 us; with a cluster barrier and a pull of every candidate over DSMEM 109
-// us, with asynchronous stores from the candidate's warp alone 102 us.
+// Complex64 panels of up to 16 x 256 rows, one thread per row, the row in
+// registers.  Columns are processed in sub-blocks of 8: the rank-1 updates of a
+// column touch its sub-block only (w, shifted by one per column so that the
+// current column is always w[0]), and the columns right of it (R) take the 8
+// pivots at once.  Finished columns go to shared memory (Fin).  Rows are
+// exchanged by renaming, as in the shared-memory panels (same ipiv).
+// Candidates are compared by (bits of |re|+|im|) + 1 (0 = no candidate;
+// non-negative floats order like their bits); the lowest label wins a tie.
+// Per column: every warp's candidate stages its key, reciprocal and row; after
+// one __syncthreads every warp finds the CTA's candidate and sends its share of
+// it to the other CTAs with asynchronous stores that count their bytes on the
+// receiver's mbarrier; every warp waits there (bounded), picks the pivot and
+// updates w.  No cluster barrier: a CTA sends its candidate of column c + 1
+// after it has used the ones of column c, so with two buffers (column parity)
+// whoever holds all candidates of c + 1 may overwrite those of c.
+// Per sub-block: the CTAs that own its pivot rows send them (multipliers and
+// right part) to every CTA with bulk copies, one per run of consecutive
+// pivots; every CTA solves L11 U = right part for itself and applies U to its
+// rows.  Every entry still takes its updates in the order of the columns.
+// Bound by the latency of a column's chain: about 330 instructions at two
+// clocks each and a one-way exchange of 600.  64 columns of 2048 rows take 66
+// us; with rank-1 updates and exchanges of all 64 columns 70 us, with cluster
+// barriers instead of asynchronous stores 109 us; in sub-blocks of 16 as long
+// for one panel, 2 % longer for many at once.
 constexpr int kWinMaxRows = 256;
-constexpr int kWinMaxThreads = 2 * kWinMaxRows;
+constexpr int kSub = 8;          // columns of a sub-block
+constexpr int kSubP = kSub / 2;   // 16-byte words of a candidate
 
+__host__ __device__ constexpr int win_threads(int rpb) {
+  return rpb <= 64 ? 64 : (rpb + 31) / 32 * 32;
+}
 __host__ __device__ constexpr size_t panel_win_smem(int rpb) {
-  return sizeof(float2) * ((size_t)rpb * kRowsLd + (size_t)(2 + 2 * kMaxClusterPanel) * kNB);
+  return sizeof(float2) * (size_t)win_threads(rpb) * kNB +
+         sizeof(float4) * (2 * (kWinMaxRows / 32) * (kSubP + 1) + 2 * kMaxClusterPanel * kSubP +
+                           2 * kSub * (kNB / 2 + 1));
 }
 
+// 1/a = conj(a) / |a|^2 with the components scaled by a power of two near
+// 1/max(|re|,|im|): |a|^2 in [1, 8), its reciprocal by Newton's iteration from
+// the hardware's approximation.
 __device__ __forceinline__ float2 crcp_fast(float2 a) {
-  // 1/a = conj(a) / |a|^2 with the components scaled by 1/max(|re|,|im|)
-  const float sc = fmaxf(fabsf(a.x), fabsf(a.y));
-  const float rs = __frcp_rn(sc);
-  const float ar = a.x * rs, ai = a.y * rs;
-  const float rd = __frcp_rn(fmaf(ar, ar, ai * ai)) * rs;
-  return make_float2(ar * rd, -ai * rd);
+  const int e = (__float_as_int(fmaxf(fabsf(a.x), fabsf(a.y))) >> 23) & 0xff;
+  const float sc = __int_as_float((254 - min(max(e, 1), 253)) << 23);
+  const float ar = a.x * sc, ai = a.y * sc;
+  const float d = fmaf(ar, ar, ai * ai);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(r, fmaf(-d, r, 1.f), r) * sc;
+  return make_float2(ar * r, -ai * r);
 }
 
-__device__ __forceinline__ float4 cfms2(float4 w, float2 l, float4 q) {
-  const float2 a = cfms(make_float2(w.x, w.y), l, make_float2(q.x, q.y));
-  const float2 b = cfms(make_float2(w.z, w.w), l, make_float2(q.z, q.w));
-  return make_float4(a.x, a.y, b.x, b.y);
-}
-
-__global__ void __launch_bounds__(kWinMaxThreads, 1)
+__global__ void __launch_bounds__(kWinMaxRows, 1)
 panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, int rpb,
                  int* __restrict__ ipiv, int* info, int* status) {
-  constexpr int kW = kNB / 4;  // pairs per thread
+  constexpr int kR = kNB - kSub;
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-  const int T = (int)blockDim.x, nw = T >> 5;
+  const int T = (int)blockDim.x, nw = T >> 5, lr = (int)threadIdx.x;
+  const int lw = lr >> 5, ln = lr & 31;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* Fin = reinterpret_cast<float2*>(smem_raw);    // [rpb][kRowsLd] finished pairs
-  float4* cand4 = reinterpret_cast<float4*>(Fin + (size_t)rpb * kRowsLd);  // [2][32]
-  float4* stage2 = cand4 + 2 * (kNB / 2);                // [2][kMaxClusterPanel][32]
-  // by column parity: candidates' keys {value, label}, the warps' maxima, and
-  // the mbarrier that counts the bytes of a column's candidates
+  float2* Fin = reinterpret_cast<float2*>(smem_raw);     // [kNB][T] finished columns
+  float4* cand2 = reinterpret_cast<float4*>(Fin + (size_t)kNB * T);  // [2][warps][key, row]
+  float4* stage2 = cand2 + 2 * (kWinMaxRows / 32) * (kSubP + 1);     // [2][kMaxClusterPanel][kSubP]
+  float4* prow = stage2 + 2 * kMaxClusterPanel * kSubP;  // [kSub][<= kNB/2 + 1] own pivot rows
+  float4* pin = prow + kSub * (kNB / 2 + 1);             // [kSub][<= kNB/2 + 1] all pivot rows
+  // by column parity: candidates' keys {value, label, 1/pivot}, the warps'
+  // maxima, and the mbarrier that counts the bytes of a column's candidates;
+  // mb[2]: the bytes of a sub-block's pivot rows
   __shared__ __align__(16) uint4 skey[2][kMaxClusterPanel];
-  __shared__ unsigned wkv2[2][kWinMaxThreads / 32], wkl2[2][kWinMaxThreads / 32];
-  __shared__ __align__(8) unsigned long long mb[2];
+  __shared__ unsigned wk[2][kWinMaxRows / 32];
+  __shared__ float4 s_zero[kSubP];
+  __shared__ __align__(8) unsigned long long mb[3];
   __shared__ int s_abort;
+  __shared__ unsigned s_own[kNB / kSub];  // pivots of the sub-block held by this CTA
   __shared__ int s_ipiv[kNB];
   __shared__ int s_info;
-  const int lw = threadIdx.x >> 5, ln = threadIdx.x & 31;
-  const int lr = threadIdx.x >> 1, h = threadIdx.x & 1;
   const int r0 = k0 + rank * rpb;
-  const int nr = max(min(rpb, n - r0), 0);
-  const bool active = lr < nr;
+  const bool active = lr < max(min(rpb, n - r0), 0);
   unsigned label = active ? (unsigned)(r0 + lr) : 0xffffffffu;
-  float4 r[kW];
+  float2 w[kSub], R[kR];
 #pragma unroll
-  for (int i = 0; i < kW; ++i) {
-    const int c0 = 4 * i + 2 * h;
-    float2 a = make_float2(0.f, 0.f), b = make_float2(0.f, 0.f);
-    if (active && c0 < nb) a = A[(size_t)(k0 + c0) * lda + label];
-    if (active && c0 + 1 < nb) b = A[(size_t)(k0 + c0 + 1) * lda + label];
-    r[i] = make_float4(a.x, a.y, b.x, b.y);
+  for (int i = 0; i < kNB; ++i) {
+    const float2 a = active && i < nb ? A[(size_t)(k0 + i) * lda + label] : make_float2(0.f, 0.f);
+    if (i < kSub)
+      w[i < kSub ? i : 0] = a;
+    else
+      R[i < kSub ? 0 : i - kSub] = a;
   }
-  if (threadIdx.x == 0) {
+  if (lr < kNB / kSub) s_own[lr] = 0u;
+  if (lr < kSubP) s_zero[lr] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (lr == 0) {
     s_info = 0;
     s_abort = 0;
-    tc::mbar_init(&mb[0], 1);
-    tc::mbar_init(&mb[1], 1);
+    for (int i = 0; i < 3; ++i) tc::mbar_init(&mb[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   __syncthreads();
   cl.sync();  // every CTA of the cluster is running before any DSMEM access
-  for (int b = 0; 4 * b < nb; ++b) {
+  // a warp sends word pr of the row to CTAs q0, q0 + kTgt nw (two at most: T >= 64)
+  constexpr int kTgt = 32 / kSubP;
+  const int pr = ln & (kSubP - 1), q0 = kTgt * lw + ln / kSubP, q1 = q0 + kTgt * nw;
+  const int qa = min(q0, C - 1), qb = min(q1, C - 1);
+  const unsigned ra = tc::map_rank(&stage2[rank * kSubP + pr], qa),
+                 ka = tc::map_rank(&skey[0][rank], qa), ba = tc::map_rank(&mb[0], qa),
+                 rb = tc::map_rank(&stage2[rank * kSubP + pr], qb),
+                 kb = tc::map_rank(&skey[0][rank], qb), bb = tc::map_rank(&mb[0], qb);
+  for (int sb = 0; kSub * sb < nb; ++sb) {
+    unsigned zmask = 0u;  // columns of the sub-block without a pivot
+    const int cend = min(kSub, nb - kSub * sb);
+    // the row's key for the current column, and the warp's largest
+    auto key_of = [&](unsigned kc) {
+      const float a = cabs1(w[0]);
+      return (active && label >= kc && a >= 0.f) ? __float_as_uint(a) + 1u : 0u;
+    };
+    unsigned vb = key_of((unsigned)(k0 + kSub * sb));
+    unsigned m = __reduce_max_sync(0xffffffffu, vb);
+#pragma unroll 1
+    for (int cs = 0; cs < cend; ++cs) {
+      const int c = kSub * sb + cs, par = c & 1;
+      const unsigned kc = (unsigned)(k0 + c);
+      // 1. the warp's candidate (the lowest label where several rows share the
+      //    largest key) stages its key and row; without one lane 0 a key of 0
+      float4* slots = cand2 + par * (kWinMaxRows / 32) * (kSubP + 1);
+      {
+        unsigned at = __ballot_sync(0xffffffffu, vb == m);
+        if (m && (at & (at - 1))) {
+          const unsigned lo = __reduce_min_sync(0xffffffffu, vb == m ? label : 0xffffffffu);
+          at = __ballot_sync(0xffffffffu, vb == m && label == lo);
+        }
+        const float2 rcp = crcp_fast(w[0]);
+        if (ln == (m ? __ffs(at) - 1 : 0)) {
+          wk[par][lw] = m;
+          float4* d = slots + lw * (kSubP + 1);
+          *reinterpret_cast<uint4*>(d) =
+              make_uint4(m, label, __float_as_uint(rcp.x), __float_as_uint(rcp.y));
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {
-      const int c = 4 * b + cc;
-      if (c < nb) {
-        const int hc = cc >> 1;         // the thread of a row holding column c (static)
-        const bool hi = (cc & 1) != 0;  // static
-        const unsigned kc = (unsigned)(k0 + c);
-        const int par = c & 1;
-        unsigned* wkv = wkv2[par];
-        unsigned* wkl = wkl2[par];
-        float4* stage4 = stage2 + par * kMaxClusterPanel * (kNB / 2);
-        // bytes of the C candidates: pairs c/2 .. 31 and a key each
-        if (threadIdx.x == 0)
-          tc::mbar_expect_tx(&mb[par], (unsigned)C * 16u * (unsigned)(kNB / 2 - (c >> 1) + 1));
-        // 1. warp and CTA candidates
-        const float2 vv = hi ? make_float2(r[0].z, r[0].w) : make_float2(r[0].x, r[0].y);
-        const float a = cabs1(vv);
-        const unsigned vb =
-            (active && h == hc && label >= kc && a >= 0.f) ? __float_as_uint(a) + 1u : 0u;
-        unsigned m = __reduce_max_sync(0xffffffffu, vb);
-        unsigned lab = __reduce_min_sync(0xffffffffu, (vb == m && m) ? label : 0xffffffffu);
-        if (ln == 0) {
-          wkv[lw] = m;
-          wkl[lw] = lab;
+          for (int i = 0; i < kSubP; ++i)
+            d[1 + i] = make_float4(w[2 * i].x, w[2 * i].y, w[2 * i + 1].x, w[2 * i + 1].y);
         }
-        __syncthreads();
-        // every warp forms the CTA candidate from the warp maxima
-        unsigned cand;
-        {
-          const unsigned wv = ln < nw ? wkv[ln] : 0u;
-          const unsigned wl = ln < nw ? wkl[ln] : 0xffffffffu;
-          m = __reduce_max_sync(0xffffffffu, wv);
-          lab = __reduce_min_sync(0xffffffffu, (wv == m && m) ? wl : 0xffffffffu);
-          cand = m ? lab : 0xfffffffeu;
+      }
+      __syncthreads();
+      // 2. every warp finds the CTA's candidate and sends its share of it
+      {
+        const unsigned x = ln < nw ? wk[par][ln] : 0u;
+        const unsigned xm = __reduce_max_sync(0xffffffffu, x);
+        unsigned at = __ballot_sync(0xffffffffu, ln < nw && x == xm);
+        if (xm && (at & (at - 1))) {
+          const unsigned xl = ((at >> ln) & 1u)
+                                  ? reinterpret_cast<const uint4*>(slots + ln * (kSubP + 1))->y
+                                  : 0xffffffffu;
+          const unsigned lo = __reduce_min_sync(0xffffffffu, xl);
+          at = __ballot_sync(0xffffffffu, xl == lo);
         }
-        // 2. the candidate's threads stage its row; the warps share the sends
-        //    of the row, pairs >= c/2, and its key to every CTA (one warp
-        //    sending to 16 CTAs took 960 clocks)
-        if (label == cand) {
-          float4* dst = cand4 + par * (kNB / 2) + 2 * b + h;
+        const uint4* d = reinterpret_cast<const uint4*>(slots + (__ffs(at) - 1) * (kSubP + 1));
+        const uint4 key = d[0], v = d[1 + pr];
+        const unsigned ro = par * kMaxClusterPanel * kSubP * 16u, ko = par * kMaxClusterPanel * 16u,
+                       bo = par * 8u;
+        if (q0 < C) {
+          tc::store_async(ra + ro, v, ba + bo);
+          if (pr == 0) tc::store_async(ka + ko, key, ba + bo);
+        }
+        if (q1 < C) {
+          tc::store_async(rb + ro, v, bb + bo);
+          if (pr == 0) tc::store_async(kb + ko, key, bb + bo);
+        }
+      }
+      // bytes of the C candidates: the row's part and a key each
+      if (lr == 0) tc::mbar_expect_tx(&mb[par], (unsigned)C * 16u * (kSubP + 1));
+      // 3. every candidate has arrived
+      const bool live = tc::mbar_wait_cluster(&mb[par], (unsigned)(c >> 1) & 1u, &s_abort);
+      // 4. the pivot, from the local keys (every warp)
+      const unsigned kv = ln < C && live ? skey[par][ln].x : 0u;
+      const unsigned bm = __reduce_max_sync(0xffffffffu, kv);
+      unsigned at = __ballot_sync(0xffffffffu, ln < C && kv == bm);
+      if (bm && (at & (at - 1))) {
+        const unsigned kl = ((at >> ln) & 1u) ? skey[par][ln].y : 0xffffffffu;
+        const unsigned lo = __reduce_min_sync(0xffffffffu, kl);
+        at = __ballot_sync(0xffffffffu, kl == lo);
+      }
+      const int q = __ffs(at) - 1;
+      const uint4 pk = skey[par][q];
+      const unsigned p = pk.y;
+      // bm == 1: |pivot| = 0; after a wait that gave up nothing is used
+      const bool zero = bm <= 1u || p < kc || p >= (unsigned)n;
+      if (!zero) label = label == p ? kc : label == kc ? p : label;
+      // 5. the update: l = 0 for the rows that are done; the next column's key
+      //    as soon as it is there
+      const float4* u4 = zero ? s_zero : stage2 + (par * kMaxClusterPanel + q) * kSubP;
+      const bool upd = !zero && active && label > kc;
+      float2 l = cmul(w[0], make_float2(__uint_as_float(pk.z), __uint_as_float(pk.w)));
+      Fin[(size_t)c * T + lr] = upd ? l : w[0];
+      l.x = upd ? l.x : 0.f;
+      l.y = upd ? l.y : 0.f;
+      const float4 u0 = u4[0];
+      w[0] = cfms(w[1], l, make_float2(u0.z, u0.w));
+      vb = key_of(kc + 1);
+      m = __reduce_max_sync(0xffffffffu, vb);
 #pragma unroll
-          for (int i = 0; i < kW; ++i)
-            if (i < kW - b && (i > 0 || h >= hc)) dst[2 * i] = r[i];
-        }
-        __syncthreads();
-        {
-          const uint4 v = *reinterpret_cast<const uint4*>(&cand4[par * (kNB / 2) + ln]);
-          for (int q = lw; q < C; q += nw) {
-            const unsigned bar = tc::map_rank(&mb[par], q);
-            if (ln >= (c >> 1))
-              tc::store_async(tc::map_rank(&stage4[rank * (kNB / 2) + ln], q), v, bar);
-            if (ln == 0)
-              tc::store_async(tc::map_rank(&skey[par][rank], q), make_uint4(m, lab, 0u, 0u), bar);
-          }
-        }
-        // 3. every candidate has arrived
-        const bool live = tc::mbar_wait_cluster(&mb[par], (unsigned)(c >> 1) & 1u, &s_abort);
-        // 4. the pivot, from the local keys (every warp)
-        const unsigned kv = ln < C ? skey[par][ln].x : 0u;
-        const unsigned kl = ln < C ? skey[par][ln].y : 0xffffffffu;
-        const unsigned bm = __reduce_max_sync(0xffffffffu, kv);
-        const unsigned p = __reduce_min_sync(0xffffffffu, (kv == bm && bm) ? kl : 0xffffffffu);
-        // bm == 1: |pivot| = 0; after a wait that gave up nothing is used
-        const bool zero = !__all_sync(0xffffffffu, live) || bm <= 1u || p < kc || p >= (unsigned)n;
-        if (threadIdx.x == 0) {
-          s_ipiv[c] = zero ? (int)kc : (int)p;
-          if (zero && s_info == 0) s_info = (int)kc + 1;
-        }
-        // the row's column-c value, from the thread holding it
-        const float2 v = make_float2(__shfl_sync(0xffffffffu, vv.x, (ln & ~1) | hc),
-                                     __shfl_sync(0xffffffffu, vv.y, (ln & ~1) | hc));
-        if (!zero) {
-          const int q = __ffs(__ballot_sync(0xffffffffu, kv == bm && kl == p)) - 1;
-          const float4* pr = stage4 + q * (kNB / 2) + 2 * b + h;  // pr[2i]: this thread's pair i
-          if (label == p)
-            label = kc;
-          else if (label == kc)
-            label = p;
-          if (active && label > kc) {
-            const float4 pc = stage4[q * (kNB / 2) + (c >> 1)];
-            const float2 piv = hi ? make_float2(pc.z, pc.w) : make_float2(pc.x, pc.y);
-            const float2 l = cmul(v, crcp_fast(piv));
-            // window position 0 without divergence between the two threads
-            // of a row: the update of the whole pair (pr[0] is the pivot
-            // row's pair of this thread; for h == hc it is pc, for h < hc a
-            // stale slot whose result is discarded), then a select: the
-            // pair holding column c keeps its finished column c - 1 (hi) and
-            // takes the multiplier l at column c; pair 2b + 1 right of column
-            // c takes the update; a finished pair left of c stays
-            const float4 x = cfms2(r[0], l, pr[0]);
-            if (h == hc)
-              r[0] = hi ? make_float4(r[0].x, r[0].y, l.x, l.y) : make_float4(l.x, l.y, x.z, x.w);
-            else if (h > hc)
-              r[0] = x;
+      for (int i = 1; i < kSubP; ++i) {
+        const float4 u = u4[i];
+        w[2 * i - 1] = cfms(w[2 * i], l, make_float2(u.x, u.y));
+        w[2 * i] = cfms(w[2 * i + 1], l, make_float2(u.z, u.w));
+      }
+      zmask |= zero ? 1u << cs : 0u;
+      if (lr == 0) {
+        s_ipiv[c] = zero ? (int)kc : (int)p;
+        if (zero && s_info == 0) s_info = (int)kc + 1;
+      }
+    }
+    const int cr = kSub * (sb + 1);  // first column right of the sub-block
+    if (cr >= nb) break;
+    // 5. pivot rows to every CTA: the sub-block's columns and those right of it
+    const int np = (kNB - kSub * sb) / 2 + 1;                // 16-byte words of a row (odd)
+    const int ng = kNB / kSub - 1 - sb;                      // groups of 16 columns right
+    const unsigned pj = label - (unsigned)(k0 + kSub * sb);  // pivot of the sub-block if < 16
+    if (lr == 0) tc::mbar_expect_tx(&mb[2], (unsigned)(kSub * np * 16));
+    if (active && pj < (unsigned)kSub) {
+      float4* d = prow + pj * np;
 #pragma unroll
-            for (int i = 1; i < kW; ++i)
-              if (i < kW - b) r[i] = cfms2(r[i], l, pr[2 * i]);
+      for (int i = 0; i < kSubP; ++i) {
+        const float2 x = Fin[(size_t)(kSub * sb + 2 * i) * T + lr],
+                     y = Fin[(size_t)(kSub * sb + 2 * i + 1) * T + lr];
+        d[i] = make_float4(x.x, x.y, y.x, y.y);
+      }
+#pragma unroll
+      for (int i = 0; i < kR / 2; ++i)
+        if (i < ng * kSubP)
+          d[kSubP + i] = make_float4(R[2 * i].x, R[2 * i].y, R[2 * i + 1].x, R[2 * i + 1].y);
+      atomicOr(&s_own[sb], 1u << pj);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+    if (lw == 0 && ln < C && !*reinterpret_cast<volatile int*>(&s_abort)) {
+      unsigned own = s_own[sb];
+      while (own) {
+        const int j0 = __ffs(own) - 1, len = __ffs(~(own >> j0)) - 1;
+        tc::copy_to_rank(tc::map_rank(pin + j0 * np, ln), prow + j0 * np,
+                         (unsigned)(len * np * 16), tc::map_rank(&mb[2], ln));
+        own &= ~(((1u << len) - 1u) << j0);
+      }
+    }
+    const bool live =
+        __all_sync(0xffffffffu, tc::mbar_wait_cluster(&mb[2], (unsigned)sb & 1u, &s_abort));
+    // 6. U = L11^{-1} (right part): a thread per column
+    if (live && lr < kNB - cr) {
+      float2* pf = reinterpret_cast<float2*>(pin) + kSub + lr;
+      float2 u[kSub];
+#pragma unroll
+      for (int i = 0; i < kSub; ++i) u[i] = pf[i * 2 * np];
+      const float2* L = reinterpret_cast<const float2*>(pin);
+#pragma unroll
+      for (int q = 0; q < kSub - 1; ++q)
+        if (!((zmask >> q) & 1u)) {
+#pragma unroll
+          for (int i = q + 1; i < kSub; ++i) u[i] = cfms(u[i], L[i * 2 * np + q], u[q]);
+        }
+#pragma unroll
+      for (int i = 1; i < kSub; ++i) pf[i * 2 * np] = u[i];
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next copies land here
+    }
+    __syncthreads();
+    // 7. the rows below take U, the pivot rows become U
+    if (live && active && label >= (unsigned)(k0 + kSub * sb)) {
+      const bool piv = pj < (unsigned)kSub;
+      const int q0 = piv ? (int)pj : 0, q1 = piv ? q0 + 1 : kSub;
+#pragma unroll 1
+      for (int q = q0; q < q1; ++q) {
+        if (!piv && ((zmask >> q) & 1u)) continue;
+        const float2 l = Fin[(size_t)(kSub * sb + q) * T + lr];
+        const float4* u4 = pin + q * np + kSubP;
+#pragma unroll
+        for (int g = 0; g < kR / kSub; ++g) {
+          if (g >= ng) break;
+#pragma unroll
+          for (int i = 0; i < kSubP; ++i) {
+            const float4 u = u4[g * kSubP + i];
+            float2& x = R[g * kSub + 2 * i];
+            float2& y = R[g * kSub + 2 * i + 1];
+            x = piv ? make_float2(u.x, u.y) : cfms(x, l, make_float2(u.x, u.y));
+            y = piv ? make_float2(u.z, u.w) : cfms(y, l, make_float2(u.z, u.w));
           }
         }
       }
     }
-    // block b done: pair 2b + h is final; shift the window by one
-    if (active) reinterpret_cast<float4*>(Fin + (size_t)lr * kRowsLd)[2 * b + h] = r[0];
 #pragma unroll
-    for (int i = 0; i < kW - 1; ++i) r[i] = r[i + 1];
-    r[kW - 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < kSub; ++i) w[i] = R[i];
+#pragma unroll
+    for (int i = 0; i < kR - kSub; ++i) R[i] = R[i + kSub];
   }
   cl.sync();  // no CTA leaves while another may still write its shared memory
-  if (threadIdx.x == 0 && s_abort) atomicExch(status, 1);
+  if (lr == 0 && s_abort) atomicExch(status, 1);
   if (rank == 0) {
-    for (int c = threadIdx.x; c < nb; c += T) ipiv[k0 + c] = s_ipiv[c];
-    if (threadIdx.x == 0 && s_info && *info == 0) *info = s_info;
+    for (int c = lr; c < nb; c += T) ipiv[k0 + c] = s_ipiv[c];
+    if (lr == 0 && s_info && *info == 0) *info = s_info;
   }
-  __syncthreads();  // Fin complete
-  if (active) {
-    const float2* fr = Fin + (size_t)lr * kRowsLd;
-    for (int c = h; c < nb; c += 2) A[(size_t)(k0 + c) * lda + label] = fr[c];
-  }
+  if (active)
+    for (int c = 0; c < nb; ++c) A[(size_t)(k0 + c) * lda + label] = Fin[(size_t)c * T + lr];
 }
 
 template <typename K, typename... Args>
@@ -1119,92 +1210,146 @@ size_t lu_scratch_bytes(int n) { return slots_region() + tslu_bytes(n); }
 // 32, at most kTsluMaxRows).  Block b runs partial pivoting on rows r0 ..
 // r0 + R - 1 (r0 = k0 + b R) of columns k0 .. k0 + nb - 1 and writes the
 // rows it pivoted on (absolute indices) to cand[b nb + c], -1 for steps not
-// taken.  Each thread holds its row in registers as a window over the
-// columns: in block q of four columns, a[i] is column 4 q + i, so every
-// register index is static while the loop over blocks stays a loop (the
-// window shifts by four after each block).  Per column: the warp's best row
-// (reduce by shuffles) stages itself in shared memory, one barrier, every
-// warp picks the block's best from the warp bests and updates its rows from
-// the staged row.  The staging area alternates between two buffers, so one
-// barrier per column suffices.
+// taken.  Columns in sub-blocks of 8 as in the register-window panel: per
+// column the warps' candidates stage their key and row, one barrier, every
+// warp picks the block's best and updates the sub-block's columns; after a
+// sub-block the columns right of it take its pivots at once.  64 columns of 256
+// rows take 42 us; with rank-1 updates of all 64 columns 67 us.
 __global__ void __launch_bounds__(kTsluMaxRows, 1)
 tslu_select_kernel(const float2* __restrict__ A, long long lda, int n, int k0, int nb, int R,
                    int* __restrict__ cand) {
-  constexpr int kW = kTsluMaxRows / 32;
-  __shared__ __align__(16) float2 stage[2][kW][kNB];
-  __shared__ unsigned wv[2][kW], wi[2][kW];
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = (int)blockDim.x >> 5;
+  constexpr int kW = kTsluMaxRows / 32, kR = kNB - kSub;
+  __shared__ __align__(16) float4 slots[2][kW][kSubP + 1];  // by column parity: key, row
+  __shared__ unsigned wk[2][kW];
+  __shared__ float2 Ls[kSub][kTsluMaxRows];                 // the sub-block's multipliers
+  __shared__ __align__(16) float4 pin[kSub][kNB / 2 + 1];   // its pivot rows
+  const int t = threadIdx.x, ln = t & 31, lw = t >> 5, nw = (int)blockDim.x >> 5;
   const int r0 = k0 + blockIdx.x * R;
   const int nr = max(0, min(R, n - r0));
   bool active = t < nr;
-  float2 a[kNB];
+  float2 w[kSub], Rt[kR];
 #pragma unroll
-  for (int c = 0; c < kNB; ++c)
-    a[c] = (active && c < nb) ? A[(size_t)(k0 + c) * lda + r0 + t] : make_float2(0.f, 0.f);
+  for (int i = 0; i < kNB; ++i) {
+    const float2 a =
+        active && i < nb ? A[(size_t)(k0 + i) * lda + r0 + t] : make_float2(0.f, 0.f);
+    if (i < kSub)
+      w[i < kSub ? i : 0] = a;
+    else
+      Rt[i < kSub ? 0 : i - kSub] = a;
+  }
   int* out = cand + (size_t)blockIdx.x * nb;
-  const int npiv = min(nb, nr);
-  int taken = 0;
-  for (int q = 0; 4 * q < npiv && taken == 4 * q; ++q) {
+  const int npiv = min(nb, nr);  // a row is left at each of these steps
+  // bits of |re| + |im| plus one (non-negative floats order like their bits; 0
+  // = not a candidate, NaN counts as zero); among equals the smallest row,
+  // which is the lowest lane of the lowest warp (LAPACK's izamax)
+  auto key_of = [&]() {
+    float v = cabs1(w[0]);
+    if (!(v >= 0.f)) v = 0.f;
+    return active ? __float_as_uint(v) + 1u : 0u;
+  };
+  for (int sb = 0; kSub * sb < npiv; ++sb) {
+    unsigned zmask = 0u;
+    int pj = -1;  // step of the sub-block that picked this row
+    const int cend = min(kSub, npiv - kSub * sb);
+    unsigned vb = key_of();
+    unsigned m = __reduce_max_sync(0xffffffffu, vb);
+#pragma unroll 1
+    for (int cs = 0; cs < cend; ++cs) {
+      const int par = cs & 1;
+      const unsigned at = __ballot_sync(0xffffffffu, vb == m);
+      const float2 rcp = crcp_fast(w[0]);
+      if (ln == __ffs(at) - 1) {  // the warp's candidate stages its key and row
+        wk[par][lw] = m;
+        float4* d = slots[par][lw];
+        d[0] = make_float4(__uint_as_float(m), __int_as_float(t), rcp.x, rcp.y);
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {
-      const int col = 4 * q + cc, par = cc & 1;
-      if (col < npiv && taken == col) {  // uniform over the block
-        // keys: bits of |re| + |im| plus one (non-negative floats order like
-        // their bits; 0 = not a candidate, NaN counts as zero); the warp's
-        // best key, then the smallest row holding it (LAPACK's izamax)
-        float v = cabs1(a[cc]);
-        if (!(v >= 0.f)) v = 0.f;
-        const unsigned key = active ? __float_as_uint(v) + 1u : 0u;
-        const unsigned m = __reduce_max_sync(0xffffffffu, key);
-        const unsigned lab = __reduce_min_sync(0xffffffffu, (key == m && m) ? (unsigned)t : 0xffffffffu);
-        if (lane == 0) {
-          wv[par][wid] = m;
-          wi[par][wid] = lab;
-        }
-        const int lim = kNB - 4 * q;  // window positions still holding columns
-        if (m && (unsigned)t == lab) {  // the warp's best row: stage columns col ..
-          float4* st4 = reinterpret_cast<float4*>(stage[par][wid]);
+        for (int i = 0; i < kSubP; ++i)
+          d[1 + i] = make_float4(w[2 * i].x, w[2 * i].y, w[2 * i + 1].x, w[2 * i + 1].y);
+      }
+      __syncthreads();
+      const unsigned x = ln < nw ? wk[par][ln] : 0u;
+      const unsigned bm = __reduce_max_sync(0xffffffffu, x);
+      const unsigned aw = __ballot_sync(0xffffffffu, ln < nw && x == bm);
+      const float4* u4 = slots[par][__ffs(aw) - 1];
+      const float4 key = u4[0];
+      if (t == __float_as_int(key.y)) {
+        out[kSub * sb + cs] = r0 + t;
+        active = false;  // the pivot row is not updated from here on
+        pj = cs;
+      }
+      const bool upd = active && bm > 1u;  // bm == 1: a zero column
+      float2 l = cmul(w[0], make_float2(key.z, key.w));
+      l.x = upd ? l.x : 0.f;
+      l.y = upd ? l.y : 0.f;
+      Ls[cs][t] = l;
+      const float4 u0 = u4[1];
+      w[0] = cfms(w[1], l, make_float2(u0.z, u0.w));
+      vb = key_of();
+      m = __reduce_max_sync(0xffffffffu, vb);
 #pragma unroll
-          for (int j = cc & ~1; j < kNB; j += 2) {
-            if (j >= lim) break;
-            st4[j >> 1] = make_float4(a[j].x, a[j].y, a[j + 1].x, a[j + 1].y);
+      for (int i = 1; i < kSubP; ++i) {
+        const float4 u = u4[1 + i];
+        w[2 * i - 1] = cfms(w[2 * i], l, make_float2(u.x, u.y));
+        w[2 * i] = cfms(w[2 * i + 1], l, make_float2(u.z, u.w));
+      }
+      zmask |= bm > 1u ? 0u : 1u << cs;
+    }
+    if (kSub * (sb + 1) >= npiv) break;
+    // the pivot rows' multipliers and right parts, U = L11^{-1} (right parts),
+    // then the rows left take U
+    const int np = (kNB - kSub * (sb + 1)) / 2;  // 16-byte words right of the sub-block
+    if (pj >= 0) {
+      float4* d = pin[pj];
+#pragma unroll
+      for (int i = 0; i < kSubP; ++i) {
+        const float2 x = Ls[2 * i][t], y = Ls[2 * i + 1][t];
+        d[i] = make_float4(x.x, x.y, y.x, y.y);
+      }
+#pragma unroll
+      for (int i = 0; i < kR / 2; ++i)
+        if (i < np)
+          d[kSubP + i] = make_float4(Rt[2 * i].x, Rt[2 * i].y, Rt[2 * i + 1].x, Rt[2 * i + 1].y);
+    }
+    __syncthreads();
+    for (int c = t; c < 2 * np; c += blockDim.x) {
+      float2 u[kSub];
+#pragma unroll
+      for (int i = 0; i < kSub; ++i) u[i] = reinterpret_cast<const float2*>(pin[i])[kSub + c];
+#pragma unroll
+      for (int q = 0; q < kSub - 1; ++q)
+#pragma unroll
+        for (int i = q + 1; i < kSub; ++i)
+          u[i] = cfms(u[i], reinterpret_cast<const float2*>(pin[i])[q], u[q]);
+#pragma unroll
+      for (int i = 1; i < kSub; ++i) reinterpret_cast<float2*>(pin[i])[kSub + c] = u[i];
+    }
+    __syncthreads();
+    if (active) {
+#pragma unroll 1
+      for (int q = 0; q < kSub; ++q) {
+        if ((zmask >> q) & 1u) continue;
+        const float2 l = Ls[q][t];
+        const float4* u4 = pin[q] + kSubP;
+#pragma unroll
+        for (int g = 0; g < kR / kSub; ++g) {
+          if (g * kSubP >= np) break;
+#pragma unroll
+          for (int i = 0; i < kSubP; ++i) {
+            const float4 u = u4[g * kSubP + i];
+            float2& x = Rt[g * kSub + 2 * i];
+            float2& y = Rt[g * kSub + 2 * i + 1];
+            x = cfms(x, l, make_float2(u.x, u.y));
+            y = cfms(y, l, make_float2(u.z, u.w));
           }
-        }
-        __syncthreads();
-        const unsigned kv = lane < nw ? wv[par][lane] : 0u;
-        const unsigned bm = __reduce_max_sync(0xffffffffu, kv);
-        const unsigned bl = __reduce_min_sync(0xffffffffu,
-                                              (kv == bm && bm) ? wi[par][lane] : 0xffffffffu);
-        const int p = bm ? (int)bl : -1;  // an active row (one is left while col < nr)
-        if (p >= 0 && p < nr) {
-          if (t == 0) out[col] = r0 + p;
-          if (t == p) active = false;  // the pivot row is not updated from here on
-          if (active) {
-            const float4* pr4 = reinterpret_cast<const float4*>(stage[par][p >> 5]);
-            const float4 pc = pr4[cc >> 1];
-            const float2 pv = (cc & 1) ? make_float2(pc.z, pc.w) : make_float2(pc.x, pc.y);
-            if (pv.x != 0.f || pv.y != 0.f) {
-              const float2 l = cmul(a[cc], crcp_fast(pv));
-              if (!(cc & 1)) a[cc + 1] = cfms(a[cc + 1], l, make_float2(pc.z, pc.w));
-#pragma unroll
-              for (int j = (cc & ~1) + 2; j < kNB; j += 2) {
-                if (j >= lim) break;
-                const float4 u = pr4[j >> 1];
-                a[j] = cfms(a[j], l, make_float2(u.x, u.y));
-                a[j + 1] = cfms(a[j + 1], l, make_float2(u.z, u.w));
-              }
-            }
-          }
-          taken = col + 1;
         }
       }
     }
 #pragma unroll
-    for (int i = 0; i < kNB - 4; ++i) a[i] = a[i + 4];
+    for (int i = 0; i < kSub; ++i) w[i] = Rt[i];
 #pragma unroll
-    for (int i = kNB - 4; i < kNB; ++i) a[i] = make_float2(0.f, 0.f);
+    for (int i = 0; i < kR - kSub; ++i) Rt[i] = Rt[i + kSub];
   }
-  for (int j = taken + t; j < nb; j += blockDim.x) out[j] = -1;  // steps not taken
+  for (int j = npiv + t; j < nb; j += blockDim.x) out[j] = -1;  // steps not taken
 }
 
 // Cb (Gc x nb, column-major, ld Gc) = rows src[j] of S (column-major, ld
@@ -1397,7 +1542,7 @@ static bool tslu_panel(float2* A, long long lda, int n, int k0, int nb, const Lu
   int C = std::max(1, (Gf + kWinMaxRows - 1) / kWinMaxRows);
   if (C > cmax) return false;
   const int rpb = (Gf + C - 1) / C;
-  const int threads = std::max(64, (2 * rpb + 31) / 32 * 32);
+  const int threads = win_threads(rpb);
   cudaMemsetAsync(ts.infc, 0, sizeof(int), s);
   if (launch_cluster(panel_win_kernel, C, threads, panel_win_smem(rpb), s, Cf, (long long)ld, Gf,
                      0, nb, rpb, ts.ipc, ts.infc, w.status) != cudaSuccess) {
@@ -1702,7 +1847,7 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
         while ((H + C - 1) / C > kWinMaxRows) ++C;
         if (C > cmax) continue;
         const int rpb = (H + C - 1) / C;
-        const int threads = std::max(64, (2 * rpb + 31) / 32 * 32);
+        const int threads = win_threads(rpb);
         cudaError_t e = launch_cluster(panel_win_kernel, C, threads, panel_win_smem(rpb), s,
                                        reinterpret_cast<float2*>(A), lda, n, k0, nb, rpb,
                                        w.ipiv, w.info, w.status);
@@ -1735,7 +1880,7 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
     if (!done && sizeof(T) == sizeof(float2)) {
       // taller still: tournament pivoting (measured against the shared-memory
       // rows panel above: ~200 us per 64 columns for it up to 16 x 416 rows,
-      // ~260 us for the tournament there; beyond, the grid panel: ~370 us)
+      // about as much for the tournament there; beyond, the grid panel: ~370 us)
       done = tslu_panel(reinterpret_cast<float2*>(A), lda, n, k0, nb, w,
                         cluster16 ? kMaxClusterPanel : 8, s, launches);
     }

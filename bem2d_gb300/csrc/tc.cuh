@@ -80,6 +80,16 @@ __device__ __forceinline__ void store_async(unsigned dst, uint4 v, unsigned mbar
       "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(mbar)
       : "memory");
 }
+// Bulk copy from this CTA's shared memory to a mapped address (multiples of 16
+// bytes); the bytes count on the mbarrier (same CTA as the destination).
+__device__ __forceinline__ void copy_to_rank(unsigned dst, const void* src, unsigned bytes,
+                                             unsigned mbar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+      "[%3];" ::"r"(dst),
+      "r"(smem_u32(src)), "r"(bytes), "r"(mbar)
+      : "memory");
+}
 __device__ __forceinline__ bool mbar_test_cluster(unsigned long long* m, unsigned parity) {
   unsigned done;
   asm volatile(
