@@ -1688,8 +1688,10 @@ size_t lu_pack_bytes(int n, size_t elem) {
                                  : tc_pack_bytes(n, n, n >= kOuterMinN ? kOuterNB : kNB);
 }
 
-// SMs left to the panels while a look-ahead update runs beside them
-constexpr int kLookaheadFreeSMs = 40;
+// SMs left to the panels while a look-ahead update runs beside them: one for each
+// CTA of the tournament's first round (L-shape N = 16384: 141.4 ms with 40, 138.7
+// with 64, 139.5 with 80; N = 8192 the same with all three)
+constexpr int kLookaheadFreeSMs = 64;
 #ifndef BEM2D_LOOKAHEAD_MIN_N
 #define BEM2D_LOOKAHEAD_MIN_N 8192
 #endif

@@ -80,6 +80,14 @@ __device__ __forceinline__ void store_async(unsigned dst, uint4 v, unsigned mbar
       "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(mbar)
       : "memory");
 }
+// 8 bytes, counted the same way.
+__device__ __forceinline__ void store_async8(unsigned dst, float2 v, unsigned mbar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::
+          "r"(dst),
+      "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(mbar)
+      : "memory");
+}
 // Bulk copy from this CTA's shared memory to a mapped address (multiples of 16
 // bytes); the bytes count on the mbarrier (same CTA as the destination).
 __device__ __forceinline__ void copy_to_rank(unsigned dst, const void* src, unsigned bytes,
