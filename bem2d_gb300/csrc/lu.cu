@@ -17,7 +17,8 @@
 //   gemm_kernel    A22 -= L21 U12  (register-tiled, 64 x 64 CTA tiles)
 // After the factorisation: perm (the row permutation of the pivots) and the
 // inverses of the 64 x 64 diagonal blocks of L and U, so that a solve is a
-// chain of small matrix-vector products (trisolve_cluster_kernel).
+// chain of small matrix-vector products (trisolve64_kernel,
+// trisolve_cluster_kernel, trisolve_wave_kernel).
 #include <cooperative_groups.h>
 
 namespace cg = cooperative_groups;
@@ -1995,7 +1996,7 @@ template <typename T, typename TS>
 __device__ __forceinline__ T cvt(TS v) {
   return CTraits<T>::make(v.x, v.y);
 }
-// x = U^{-1} L^{-1} P b in one cluster launch.  CTA r owns rows
+// x = U^{-1} L^{-1} P b in one cluster launch, arithmetic in complex128.  CTA r owns rows
 // [r rpb, (r+1) rpb) of b in shared memory (rpb a multiple of 64).  Step k of
 // the forward sweep: the owner of block k forms y_k = L_kk^{-1} b_k from the
 // stored inverse; one cluster barrier; every CTA reads y_k over DSMEM and
@@ -2080,6 +2081,202 @@ trisolve_cluster_kernel(const TS* __restrict__ LU, long long lda, int n,
   }
   cl.sync();
   for (int i = threadIdx.x; i < nr; i += blockDim.x) xout[r0 + i] = bc[i];
+}
+
+// ---- complex64 triangular solves in one cluster --------------------------------
+// x = U^{-1} L^{-1} P b.  Block b of 64 rows belongs to CTA b % C.  Whoever
+// holds y_k subtracts L[m, k] y_k from its blocks m > k; the owner of block k +
+// 1 takes that block first, forms y_{k+1} = L_{k+1,k+1}^{-1} b_{k+1} from the
+// stored inverse and sends it to every CTA before it turns to its other blocks.
+// Going back the same with U.  A step of the chain is then one 512-byte
+// message (asynchronous stores counted on the receiver's mbarrier; every block
+// has its own slot and mbarrier, used once in each direction: y_k has no reader
+// left when x_k is sent, since all later y depend on its readers), and two
+// products of 64 x 64, whose matrices are loaded a step ahead.  Thread (row r,
+// quarter g) = lane 4 (r % 8) + g of warp r / 8 takes the columns 8 u + 2 g, + 1.
+// Bound by that chain: 2048 rows take 100 us; with contiguous rows per CTA and a
+// cluster barrier in every step 270 us.  The FP64 solve keeps that scheme: there
+// a 64 x 64 product costs 4 us of one SM's FP64 pipe, not the exchange.
+constexpr int kSolveThreads = 256;
+
+__host__ __device__ constexpr size_t solve64_smem(int nk, int C) {
+  // y slots, own blocks' right-hand sides, mbarriers
+  return sizeof(float2) * ((size_t)nk + (nk + C - 1) / C) * kNB + sizeof(long long) * nk;
+}
+
+__global__ void __launch_bounds__(kSolveThreads, 1)
+trisolve64_kernel(const float2* __restrict__ LU, long long lda, int n,
+                  const int* __restrict__ perm, const float2* __restrict__ dinv,
+                  const float2* bin, float2* xout, int* status) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int nk = (n + kNB - 1) / kNB, own = (nk + C - 1) / C;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* ys = reinterpret_cast<float2*>(smem_raw);  // [nk][64] solution blocks
+  float2* bl = ys + (size_t)nk * kNB;                // [own][64] own blocks, i = b / C
+  unsigned long long* mb = reinterpret_cast<unsigned long long*>(bl + (size_t)own * kNB);  // [nk]
+  __shared__ int s_abort;
+  const int t = threadIdx.x, ln = t & 31, lw = t >> 5;
+  const int r = 8 * lw + (ln >> 2), g = ln & 3;
+  constexpr unsigned kBytes = kNB * sizeof(float2);
+  for (int i = t; i < own * kNB; i += kSolveThreads) {
+    const int row = ((i >> 6) * C + rank) * kNB + (i & 63);
+    bl[i] = row < n ? bin[perm[row]] : make_float2(0.f, 0.f);
+  }
+  if (t == 0) {
+    s_abort = 0;
+    for (int k = 0; k < nk; ++k) tc::mbar_init(&mb[k], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  __syncthreads();
+  if (t == 0)
+    for (int k = 0; k < nk; ++k)
+      if (k % C != rank) tc::mbar_expect_tx(&mb[k], kBytes);
+  cl.sync();  // every mbarrier is set, every read of bin done (xout may be bin)
+  // the CTAs this thread sends its row's value to: lane quarters g take ranks
+  // rank + 1 + g, + 4, ..; the next block's owner (either direction) is among
+  // the first
+  unsigned ya[4], ma[4];
+  bool to[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int d = (i & 1) ? C - 1 - (g + 4 * (i >> 1)) : 1 + g + 4 * (i >> 1);
+    // forward distances 1..8 (i = 0, 2), backward ones C-1..C-8 (i = 1, 3), each rank once
+    to[i] = d >= 1 && d < C && ((i & 1) ? d > 8 : d <= 8);
+    const int q = (rank + (to[i] ? d : 0)) % C;
+    ya[i] = tc::map_rank(ys + r, q);
+    ma[i] = tc::map_rank(mb, q);
+  }
+  auto load = [&](float2 (&m)[16], const float2* base, long long ld, int rows, int cols) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int c = 8 * (u >> 1) + 2 * g + (u & 1);
+      m[u] = r < rows && c < cols ? base[(size_t)c * ld + r] : make_float2(0.f, 0.f);
+    }
+  };
+  // sum over a row's 64 columns of m times v, in all four lanes of the row
+  auto dot = [&](const float2 (&m)[16], const float2* v) {
+    float2 a = make_float2(0.f, 0.f), b = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float4 x = *reinterpret_cast<const float4*>(v + 8 * u + 2 * g);
+      a = cfma(m[2 * u], make_float2(x.x, x.y), a);
+      b = cfma(m[2 * u + 1], make_float2(x.z, x.w), b);
+    }
+    a.x += b.x;
+    a.y += b.y;
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+      a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+    }
+    return a;
+  };
+  bool ok = true;
+  for (int dir = 0; dir < 2; ++dir) {
+    // step s of the direction is block k(s); L or U block (m, k); D_k^{-1}
+    const int st = dir ? -1 : 1, kfirst = dir ? nk - 1 : 0;
+    auto lblock = [&](float2 (&m)[16], int mr, int k) {
+      load(m, LU + (size_t)k * kNB * lda + (size_t)mr * kNB, lda, min(kNB, n - mr * kNB),
+           min(kNB, n - k * kNB));
+    };
+    auto dblock = [&](float2 (&m)[16], int k) {
+      const int nb = min(kNB, n - k * kNB);
+      load(m, dinv + (size_t)(2 * k + dir) * kNB * kNB, kNB, nb, nb);
+    };
+    // solves block k (held here) and sends the result
+    auto solve = [&](const float2 (&d)[16], int k) {
+      const float2 y = dot(d, bl + (size_t)(k / C) * kNB);
+      const unsigned yo = (unsigned)k * kBytes, mo = (unsigned)k * 8u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (to[i]) tc::store_async8(ya[i] + yo, y, ma[i] + mo);
+      if (g == 0) {
+        ys[(size_t)k * kNB + r] = y;
+        if (dir && k * kNB + r < n) xout[(size_t)k * kNB + r] = y;
+      }
+    };
+    // the first own block after k, in the order of this direction
+    auto next_own = [&](int k) {
+      int m = k + st;
+      const int dlt = dir ? ((m - rank) % C + C) % C : ((rank - m) % C + C) % C;
+      return m + st * dlt;
+    };
+    auto inside = [&](int m) { return m >= 0 && m < nk; };
+    float2 d[16], p[16], o[16];
+    int mn = kfirst % C == rank ? kfirst : next_own(kfirst);  // whose D is in d
+    if (inside(mn)) dblock(d, mn);
+    if (dir) {  // the own blocks' right-hand side is y
+      __syncthreads();
+      for (int i = t; i < own * kNB; i += kSolveThreads) {
+        const int b = (i >> 6) * C + rank;
+        if (b < nk) bl[i] = ys[(size_t)b * kNB + (i & 63)];
+      }
+      __syncthreads();
+    }
+    if (kfirst % C == rank) {
+      solve(d, kfirst);
+      mn = next_own(kfirst);
+      if (inside(mn)) dblock(d, mn);
+    }
+    if (inside(mn)) lblock(p, mn, kfirst);
+    if (inside(mn + st * C)) lblock(o, mn + st * C, kfirst);
+    for (int s = 0; s < nk - 1; ++s) {
+      const int k = kfirst + st * s;
+      if (k % C == rank) {
+        __syncthreads();  // this CTA's y_k
+      } else {
+        ok = tc::mbar_wait_cluster(&mb[k], (unsigned)dir, &s_abort) && ok;
+        if (!dir && t == 0) tc::mbar_expect_tx(&mb[k], kBytes);  // x_k, on the way back
+      }
+      const float2* yk = ys + (size_t)k * kNB;
+      const int m0 = next_own(k);
+      if (!inside(m0)) continue;
+      // the first own block (p holds its factor block), then its solution if it is next
+      {
+        const float2 v = dot(p, yk);
+        if (g == 0) {
+          float2& x = bl[(size_t)(m0 / C) * kNB + r];
+          x.x -= v.x;
+          x.y -= v.y;
+        }
+      }
+      if (m0 == k + st) {
+        __syncthreads();
+        solve(d, m0);
+        mn = next_own(m0);
+        if (inside(mn)) dblock(d, mn);
+      }
+      const bool more = s + 1 < nk - 1;
+      if (more && inside(mn)) lblock(p, mn, k + st);
+      // the others, the second own block from o
+      auto sub = [&](const float2 (&l)[16], int m) {
+        const float2 v = dot(l, yk);
+        if (g == 0) {
+          float2& x = bl[(size_t)(m / C) * kNB + r];
+          x.x -= v.x;
+          x.y -= v.y;
+        }
+      };
+      int m = m0 + st * C;
+      if (inside(m)) sub(o, m);
+      if (more && inside(mn + st * C)) lblock(o, mn + st * C, k + st);
+      for (m += st * C; inside(m); m += st * C) {
+        float2 l[16];
+        lblock(l, m, k);
+        sub(l, m);
+      }
+    }
+    // the last block of the direction has no readers there, but its message
+    // completes the phase before the barrier's next use
+    const int kl = dir ? 0 : nk - 1;
+    if (kl % C != rank) {
+      ok = tc::mbar_wait_cluster(&mb[kl], (unsigned)dir, &s_abort) && ok;
+      if (!dir && t == 0) tc::mbar_expect_tx(&mb[kl], kBytes);
+    }
+  }
+  if (!ok) atomicExch(status, 1);
+  cl.sync();  // no CTA leaves while another may still write its shared memory
 }
 
 // ---- wavefront triangular solves (large n) -----------------------------------
@@ -2257,9 +2454,8 @@ static int lu_solve_wave(const TS* LU, long long lda, int n, const LuWork& w, co
 }
 
 template <typename T>
-int lu_solve(const T* LU, long long lda, int n, const LuWork& w, const T* b, T* x,
-             cudaStream_t s, long long* launches) {
-  if (n >= kWaveMinN) return lu_solve_wave(LU, lda, n, w, b, x, s, launches);
+static int lu_solve_cluster(const T* LU, long long lda, int n, const LuWork& w, const T* b, T* x,
+                            cudaStream_t s, long long* launches) {
   static std::atomic<int> cmax{kMaxCluster};
   static std::once_flag attr;
   std::call_once(attr, [] {
@@ -2286,6 +2482,44 @@ int lu_solve(const T* LU, long long lda, int n, const LuWork& w, const T* b, T* 
   }
   ++*launches;
   return BEM2D_OK;
+}
+
+static int lu_solve64(const float2* LU, long long lda, int n, const LuWork& w, const float2* b,
+                      float2* x, cudaStream_t s, long long* launches) {
+  static std::atomic<int> cmax{kMaxCluster};
+  static std::once_flag attr;
+  std::call_once(attr, [] {
+    cudaFuncSetAttribute(trisolve64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kClusterSmem);
+    if (cudaFuncSetAttribute(trisolve64_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                             1) != cudaSuccess) {
+      cudaGetLastError();
+      cmax = 8;
+    }
+  });
+  const int nk = (n + kNB - 1) / kNB;
+  for (;;) {
+    const int C = std::max(1, std::min(cmax.load(), nk));
+    const cudaError_t e =
+        launch_cluster(trisolve64_kernel, C, kSolveThreads, solve64_smem(nk, C), s, LU, lda, n,
+                       (const int*)w.perm, (const float2*)w.dinv, b, x, w.status);
+    if (e == cudaSuccess) break;
+    cudaGetLastError();
+    if (cmax == 8) return BEM2D_ERR_CUDA;
+    cmax = 8;
+  }
+  ++*launches;
+  return BEM2D_OK;
+}
+
+template <typename T>
+int lu_solve(const T* LU, long long lda, int n, const LuWork& w, const T* b, T* x,
+             cudaStream_t s, long long* launches) {
+  if (n >= kWaveMinN) return lu_solve_wave(LU, lda, n, w, b, x, s, launches);
+  if constexpr (sizeof(T) == sizeof(float2))
+    return lu_solve64(LU, lda, n, w, b, x, s, launches);
+  else
+    return lu_solve_cluster(LU, lda, n, w, b, x, s, launches);
 }
 
 // x = A^{-1} b with a complex64 factor, the arithmetic in complex128.
