@@ -13,7 +13,8 @@
 //                  sequence flags (bounded waits) across a cooperative grid,
 //                  for taller panels.
 //   laswp_kernel   the panel's row swaps on all other columns (LAPACK order)
-//   trsm_kernel    U12 = L11^{-1} A12
+//   trsm_kernel    U12 = L11^{-1} A12 (complex64 below kOuterMinN: both, and the
+//                  update, in launch_tc_step)
 //   gemm_kernel    A22 -= L21 U12  (register-tiled, 64 x 64 CTA tiles)
 // After the factorisation: perm (the row permutation of the pivots) and the
 // inverses of the 64 x 64 diagonal blocks of L and U, so that a solve is a
@@ -1569,20 +1570,31 @@ static size_t panel_cluster_smem(int rpb) {
 }
 
 // Row permutation of the pivots: perm[i] = the original row that ends at i.
-__global__ void perm_kernel(int n, const int* __restrict__ ipiv, int* __restrict__ perm) {
-  extern __shared__ int sp[];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) sp[i] = i;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < n; ++i) {
-      const int p = ipiv[i];
-      const int t = sp[i];
-      sp[i] = sp[p];
-      sp[p] = t;
+// A thread per i follows its position back through the swaps; swap s moves the
+// positions s and ipiv[s] >= s only, so it starts at s = i.  2048 rows: 76 us as
+// n swaps in a row by one thread, 24 us.
+constexpr int kPermThreads = 64, kPermTile = 1024;
+__global__ void __launch_bounds__(kPermThreads)
+perm_kernel(int n, const int* __restrict__ ipiv, int* __restrict__ perm) {
+  __shared__ __align__(16) int ip[kPermTile];
+  const int i = blockIdx.x * kPermThreads + threadIdx.x;
+  const int last = min(n, (int)(blockIdx.x + 1) * kPermThreads) - 1;
+  int x = i;
+  for (int t0 = last / kPermTile * kPermTile; t0 >= 0; t0 -= kPermTile) {
+    __syncthreads();
+    for (int v = threadIdx.x; v < kPermTile; v += kPermThreads)
+      ip[v] = t0 + v <= last ? ipiv[t0 + v] : t0 + v;
+    __syncthreads();
+    for (int v = min(kPermTile, last - t0 + 4) / 4 * 4 - 4; v >= 0; v -= 4) {
+      const int4 p = *reinterpret_cast<const int4*>(ip + v);
+      const int s = t0 + v;
+      x = x == s + 3 ? p.w : x == p.w ? s + 3 : x;
+      x = x == s + 2 ? p.z : x == p.z ? s + 2 : x;
+      x = x == s + 1 ? p.y : x == p.y ? s + 1 : x;
+      x = x == s ? p.x : x == p.x ? s : x;
     }
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = sp[i];
+  if (i < n) perm[i] = x;
 }
 
 // X = L^{-1} X for a unit lower 64 x 64 L in shared memory (column-major, zero
@@ -1799,7 +1811,6 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
                          (int)tri64_smem<T>());
     cudaFuncSetAttribute(trsm8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)tri64_smem<double2>());
-    cudaFuncSetAttribute(perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(tslu_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(sizeof(int) * 2 * kTsluMaxH));
   });
@@ -1921,6 +1932,23 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
     if (la) {  // the block's own columns; the rest after the far update
       laswp_cols(A, lda, w.ipiv, k0, nb, K0, k0, s, launches);
       laswp_cols(A, lda, w.ipiv, k0, nb, k0 + nb, bend, s, launches);
+    } else if (sizeof(T) == sizeof(float2) && outer == kNB) {
+      // swaps, U12 and the update of everything right of the panel
+      const int M = n - k0 - nb;
+      const bool tc = M > 0 && w.pack && tc_pack_bytes(M, M, nb) <= w.pack_bytes;
+      if (n > nb) {
+        if (launch_tc_step(reinterpret_cast<float2*>(A), lda, n, k0, nb, w.ipiv, tc, w.pack,
+                           w.status, s, w.tc_ctas, w.tc_passes))
+          return BEM2D_ERR_CUDA;
+        *launches += tc ? 2 : 1;
+      }
+      if (!tc) {
+        const size_t c1 = (size_t)(k0 + nb);
+        const int rc = update_sub(A + c1 * lda + c1, A + (size_t)k0 * lda + c1, A + c1 * lda + k0,
+                                  lda, M, M, nb, w, s, launches);
+        if (rc) return rc;
+      }
+      continue;  // a panel is its own block
     } else if (n > nb) {
       laswp_kernel<T><<<(n - nb + 127) / 128, 128, 0, s>>>(A, lda, n, w.ipiv, k0, nb);
       ++*launches;
@@ -1943,7 +1971,8 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
   // columns right of the block: U12 = L11^{-1} A12 block row by block row,
   // then A22 -= L21 U12 with K = the block width
   const int nc = n - bend;
-  if (nc > 0) {
+  const bool stepped = sizeof(T) == sizeof(float2) && outer == kNB && !la;
+  if (nc > 0 && !stepped) {
     for (int j0 = K0; j0 < bend; j0 += kNB) {
       trsm_rows(A, lda, j0, kNB, bend, nc, s, launches);
       const int r1 = j0 + kNB;
@@ -1981,7 +2010,7 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
   if (far_pending && cudaStreamWaitEvent(s, w.ev_far, 0) != cudaSuccess) return BEM2D_ERR_CUDA;
   // solve aids: permutation and diagonal-block inverses
   const int nk = (n + kNB - 1) / kNB;
-  perm_kernel<<<1, 1024, sizeof(int) * n, s>>>(n, w.ipiv, w.perm);
+  perm_kernel<<<(n + kPermThreads - 1) / kPermThreads, kPermThreads, 0, s>>>(n, w.ipiv, w.perm);
   dinv_kernel<T><<<dim3(nk, 16), kTriThreads, tri64_smem<T>(), s>>>(A, lda, n,
                                                                    reinterpret_cast<T*>(w.dinv));
   *launches += 2;

@@ -63,6 +63,7 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "cplx.cuh"
 #include "tc.cuh"
 
 namespace bem2d_gpu {
@@ -138,30 +139,41 @@ __device__ __forceinline__ void split8(const float (&v)[8], float sc, int passes
   if (passes > 1) *reinterpret_cast<uint4*>(lo) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// Rows / columns r of an operand with their k octets, as the MMA reads them:
 // A (M x K complex) -> Apk[mt][kc] = {hi, lo} chunks of kTcApart bytes each;
 // B (K x N complex) -> Bpk[nt][kc] = {hi, lo} chunks of kTcBpart bytes, each
 // with rows 0..127 = re and rows 128..255 = im of the tile's 128 columns;
-// isa, isb: exponent fields of the inverse scales.  One launch for both
-// operands: the first ab CTAs take 32 rows of A each (a warp 32 rows x 8 k at a
-// time), the others 8 columns of B (a warp 8 columns x 32 k).  Each operand is
-// read twice, for the largest entry and for the split (the second time from
-// L1).  256 threads.
-__global__ void __launch_bounds__(256)
-pack_kernel(const float2* __restrict__ A, long long lda, const float2* __restrict__ B,
-            long long ldb, int M, int N, int K, int nkc, int ab, int passes,
-            unsigned char* __restrict__ Apk, unsigned char* __restrict__ Bpk,
-            unsigned char* __restrict__ isa, unsigned char* __restrict__ isb) {
-  __shared__ float red[8][32];
+// isa, isb: exponent fields of the inverse scales.
+struct TcPack {
+  unsigned char *A, *B, *isa, *isb;
+  int nkc, passes;
+};
+template <bool IS_A>
+__device__ __forceinline__ void pack_octet(const TcPack& pk, int r, int o, const float (&re)[8],
+                                           const float (&im)[8], float sc) {
+  constexpr int T = IS_A ? kTcBM : kTcBN, part = IS_A ? kTcApart : kTcBpart;
+  const int tl = r / T, il = r - tl * T;
+  unsigned char* c = (IS_A ? pk.A : pk.B) + ((size_t)tl * pk.nkc + (o >> 2)) * (2 * part);
+  unsigned char* cre = c + kmajor_off(IS_A ? 2 * il : il, o & 3);
+  unsigned char* cim = c + kmajor_off(IS_A ? 2 * il + 1 : kTcBN + il, o & 3);
+  split8(re, sc, pk.passes, cre, cre + part);
+  split8(im, sc, pk.passes, cim, cim + part);
+}
+// 32 rows of A from row 32 blk (a warp 32 rows x 8 k at a time) or 8 columns of
+// B from column 8 blk (a warp 8 columns x 32 k).  Each entry is read twice, for
+// the largest and for the split (the second time from L1).  256 threads.
+template <bool IS_A>
+__device__ __forceinline__ void pack_block(const float2* __restrict__ P, long long ld, int lim,
+                                           int K, int blk, const TcPack& pk, float (*red)[32]) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool is_a = (int)blockIdx.x < ab;
   // row of A, or column of B; first octet of k and octet step of this thread
-  const int r = is_a ? blockIdx.x * 32 + lane : (blockIdx.x - ab) * 8 + (lane & 7);
-  const int o0 = is_a ? w : 4 * w + (lane >> 3), os = is_a ? 8 : 32;
-  const bool ok = r < (is_a ? M : N);
-  const float2* src = is_a ? A + r : B + (size_t)r * ldb;
-  const long long st = is_a ? lda : 1;
+  const int r = IS_A ? blk * 32 + lane : blk * 8 + (lane & 7);
+  const int o0 = IS_A ? w : 4 * w + (lane >> 3), os = IS_A ? 8 : 32;
+  const bool ok = r < lim;
+  const float2* src = IS_A ? P + r : P + (size_t)r * ld;
+  const long long st = IS_A ? ld : 1;
   float mx = 0.f;
-  for (int o = o0; o < 4 * nkc; o += os) {
+  for (int o = o0; o < 4 * pk.nkc; o += os) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int k = 8 * o + j;
@@ -169,7 +181,7 @@ pack_kernel(const float2* __restrict__ A, long long lda, const float2* __restric
       mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
     }
   }
-  if (!is_a) {
+  if (!IS_A) {
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
   }
@@ -179,13 +191,8 @@ pack_kernel(const float2* __restrict__ A, long long lda, const float2* __restric
   for (int j = 0; j < 8; ++j) mx = fmaxf(mx, red[j][lane]);
   const int se = scale_exp(mx);
   const float sc = exp_float(se);
-  const int T = is_a ? kTcBM : kTcBN;
-  const int tl = r / T, il = r - tl * T;
-  if (w == 0 && (is_a || lane < 8)) (is_a ? isa : isb)[r] = (unsigned char)(254 - se);
-  const int part = is_a ? kTcApart : kTcBpart, chunk_bytes = 2 * part;
-  unsigned char* dst = (is_a ? Apk : Bpk) + (size_t)tl * nkc * chunk_bytes;
-  const int rre = is_a ? 2 * il : il, rim = is_a ? 2 * il + 1 : kTcBN + il;
-  for (int o = o0; o < 4 * nkc; o += os) {
+  if (w == 0 && (IS_A || lane < 8)) (IS_A ? pk.isa : pk.isb)[r] = (unsigned char)(254 - se);
+  for (int o = o0; o < 4 * pk.nkc; o += os) {
     float re[8], im[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -194,12 +201,154 @@ pack_kernel(const float2* __restrict__ A, long long lda, const float2* __restric
       re[j] = v.x;
       im[j] = v.y;
     }
-    unsigned char* c = dst + (size_t)(o >> 2) * chunk_bytes;
-    unsigned char* cre = c + kmajor_off(rre, o & 3);
-    unsigned char* cim = c + kmajor_off(rim, o & 3);
-    split8(re, sc, passes, cre, cre + part);
-    split8(im, sc, passes, cim, cim + part);
+    pack_octet<IS_A>(pk, r, o, re, im, sc);
   }
+}
+
+// One launch for both operands: the first ab CTAs take A, the others B.
+__global__ void __launch_bounds__(256)
+pack_kernel(const float2* __restrict__ A, long long lda, const float2* __restrict__ B,
+            long long ldb, int M, int N, int K, int ab, TcPack pk) {
+  __shared__ float red[8][32];
+  if ((int)blockIdx.x < ab)
+    pack_block<true>(A, lda, M, K, blockIdx.x, pk, red);
+  else
+    pack_block<false>(B, ldb, N, K, blockIdx.x - ab, pk, red);
+}
+
+// ---- between a panel and its update ----------------------------------------
+// Row swaps of the panel at k0 on all other columns, U12 = L11^{-1} A12 and
+// (packing) the operands of A22 -= L21 U12, in one launch.  CTAs:
+//   [0, nright)  32 columns right of the panel each: swaps, U12, its pack;
+//   then nleft   32 columns left of it: swaps;
+//   then         32 rows of L21 each: their pack.
+// The swaps are applied as the permutation they amount to: 128 threads each
+// follow one position (the panel's 64 rows; the other row of each swap) back
+// through them, then every column is gathered and written once.  U12: warp w
+// holds rows 8w .. 8w + 7 of its lane's column; block b of 8 rows is solved by
+// warp b, then the warps below subtract L[w, b] x_b.
+// Bound by latency (launch, loads, eight steps of the solve): 10.5 us per panel
+// of the LU at N = 2048.  As three kernels - swaps by a thread per column in 64
+// dependent steps, solve, packing - it took 21 us and two launches more.
+constexpr int kStepCols = 32;
+constexpr int kNBs = 64;  // panel width
+constexpr size_t kStepSmem = sizeof(float2) * (kNBs * kNBs + kNBs * kStepCols);
+
+__global__ void __launch_bounds__(256)
+tc_step_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb,
+               const int* __restrict__ ipiv, int nright, int nleft, bool packing, TcPack pk) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int s_ip[kNBs], s_src[kNBs], s_pos[kNBs], s_from[kNBs];
+  __shared__ float red[8][32];
+  const int t = threadIdx.x, c = t & 31, w = t >> 5;
+  const int b = blockIdx.x;
+  if (b >= nright + nleft) {
+    pack_block<true>(A + (size_t)k0 * lda + k0 + nb, lda, n - k0 - nb, nb, b - nright - nleft, pk,
+                     red);
+    return;
+  }
+  const bool right = b < nright;
+  const int cb = right ? k0 + nb + kStepCols * b : kStepCols * (b - nright);
+  const int nc = min(kStepCols, (right ? n : k0) - cb);
+  float2* L = reinterpret_cast<float2*>(smem);  // [kNBs][kNBs] column-major
+  float2* X = L + kNBs * kNBs;                  // [kNBs][kStepCols]
+  if (t < kNBs) s_ip[t] = t < nb ? ipiv[k0 + t] : k0 + t;
+  if (right) {  // nb = 64
+#pragma unroll
+    for (int v = 0; v < kNBs * kNBs / 256; ++v) {
+      const int s = (v * 256 + t) >> 6, r = t & 63;
+      L[s * kNBs + r] = A[(size_t)(k0 + s) * lda + k0 + r];
+    }
+  }
+  __syncthreads();
+  if (t < 2 * kNBs) {  // the row that ends at position x
+    const int x0 = t < kNBs ? k0 + t : s_ip[t - kNBs];
+    int x = x0;
+    for (int s = kNBs - 1; s >= 0; --s) {
+      const int p = s_ip[s], q = k0 + s;
+      x = x == q ? p : x == p ? q : x;
+    }
+    if (t < kNBs) {
+      s_src[t] = x;
+    } else {
+      s_pos[t - kNBs] = x0 >= k0 + nb && x0 != x ? x0 : -1;
+      s_from[t - kNBs] = x;
+    }
+  }
+  __syncthreads();
+  // gather: thread row t & 63, columns t >> 6, + 4, ..; the displaced rows wait
+  // in registers until every column has been read
+  const int r = t & 63, pos = s_pos[r], from = s_from[r], src = s_src[r];
+  float2 top[kStepCols / 4], out[kStepCols / 4];
+#pragma unroll
+  for (int i = 0; i < kStepCols / 4; ++i) {
+    const int cc = (t >> 6) + 4 * i;
+    const float2* col = A + (size_t)(cb + cc) * lda;
+    top[i] = cc < nc && r < nb ? col[src] : make_float2(0.f, 0.f);
+    if (cc < nc && pos >= 0) out[i] = col[from];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kStepCols / 4; ++i) {
+    const int cc = (t >> 6) + 4 * i;
+    float2* col = A + (size_t)(cb + cc) * lda;
+    if (cc < nc && pos >= 0) col[pos] = out[i];
+    if (right)
+      X[r * kStepCols + cc] = top[i];
+    else if (cc < nc && r < nb && src != k0 + r)
+      col[k0 + r] = top[i];
+  }
+  if (!right) return;
+  __syncthreads();
+  float2 x[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) x[i] = X[(8 * w + i) * kStepCols + c];
+  for (int q = 0; q < 8; ++q) {
+    if (w == q) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = i + 1; j < 8; ++j) x[j] = cfms(x[j], L[(8 * q + i) * kNBs + 8 * q + j], x[i]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) X[(8 * q + i) * kStepCols + c] = x[i];
+    }
+    __syncthreads();
+    if (w > q) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 xb = X[(8 * q + j) * kStepCols + c];
+        const float4* l4 = reinterpret_cast<const float4*>(L + (8 * q + j) * kNBs + 8 * w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 l = l4[i];
+          x[2 * i] = cfms(x[2 * i], make_float2(l.x, l.y), xb);
+          x[2 * i + 1] = cfms(x[2 * i + 1], make_float2(l.z, l.w), xb);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kStepCols / 4; ++i) {
+    const int cc = (t >> 6) + 4 * i;
+    if (cc < nc) A[(size_t)(cb + cc) * lda + k0 + r] = X[r * kStepCols + cc];
+  }
+  if (!packing) return;
+  // pack: thread (column c, octet w)
+  float re[8], im[8], mx = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float2 v = X[(8 * w + j) * kStepCols + c];
+    re[j] = v.x;
+    im[j] = v.y;
+    mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+  }
+  red[w][c] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) mx = fmaxf(mx, red[j][c]);
+  const int se = scale_exp(mx), col = kStepCols * b + c;
+  if (w == 0) pk.isb[col] = (unsigned char)(254 - se);
+  pack_octet<false>(pk, col, w, re, im, exp_float(se));
 }
 
 // ---- the update --------------------------------------------------------------
@@ -427,28 +576,60 @@ size_t tc_pack_bytes(int M, int N, int K) {
          align256(mt * kTcBM) + align256(nt * kTcBN);
 }
 
+// The pack buffer's parts for an M x N x K update.
+static TcPack pack_parts(void* pack, int M, int N, int K, int passes) {
+  const int nkc = (K + kTcBK - 1) / kTcBK;
+  const int mt = (M + kTcBM - 1) / kTcBM, nt = (N + kTcBN - 1) / kTcBN;
+  TcPack pk;
+  pk.A = static_cast<unsigned char*>(pack);
+  pk.B = pk.A + align256((size_t)mt * nkc * kTcChunkA);
+  pk.isa = pk.B + align256((size_t)nt * nkc * kTcChunkB);
+  pk.isb = pk.isa + align256((size_t)mt * kTcBM);
+  pk.nkc = nkc;
+  pk.passes = passes;
+  return pk;
+}
+
+// The update of packed operands.
+static int update_packed(float2* C, long long ldc, int M, int N, const TcPack& pk, int* status,
+                         cudaStream_t s, int max_ctas) {
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      tc_cgemm_sub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+  if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
+  const int mt = (M + kTcBM - 1) / kTcBM, nt = (N + kTcBN - 1) / kTcBN;
+  const int grid = std::min(mt * nt, max_ctas > 0 ? max_ctas : num_sms());
+  tc_cgemm_sub_kernel<<<grid, kTcThreads, kTcSmem, s>>>(C, ldc, pk.A, pk.B, pk.isa, pk.isb, M, N,
+                                                        pk.nkc, mt, nt, pk.passes, status);
+  return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
+}
+
 int launch_tc_cgemm_sub(float2* C, long long ldc, const float2* A, long long lda,
                         const float2* B, long long ldb, int M, int N, int K, void* pack,
                         size_t pack_bytes, int* status, cudaStream_t s, int max_ctas,
                         int passes) {
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      tc_cgemm_sub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-  if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
   if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
   if (!pack || tc_pack_bytes(M, N, K) > pack_bytes) return BEM2D_ERR_ARG;
   if (passes != 1 && passes != 3) return BEM2D_ERR_ARG;
-  const int nkc = (K + kTcBK - 1) / kTcBK;
-  const int mt = (M + kTcBM - 1) / kTcBM, nt = (N + kTcBN - 1) / kTcBN;
-  unsigned char* Apk = static_cast<unsigned char*>(pack);
-  unsigned char* Bpk = Apk + align256((size_t)mt * nkc * kTcChunkA);
-  unsigned char* isa = Bpk + align256((size_t)nt * nkc * kTcChunkB);
-  unsigned char* isb = isa + align256((size_t)mt * kTcBM);
-  const int ab = mt * (kTcBM / 32);
-  pack_kernel<<<ab + nt * (kTcBN / 8), 256, 0, s>>>(A, lda, B, ldb, M, N, K, nkc, ab, passes, Apk,
-                                                    Bpk, isa, isb);
-  const int grid = std::min(mt * nt, max_ctas > 0 ? max_ctas : num_sms());
-  tc_cgemm_sub_kernel<<<grid, kTcThreads, kTcSmem, s>>>(C, ldc, Apk, Bpk, isa, isb, M, N, nkc, mt,
-                                                        nt, passes, status);
+  const TcPack pk = pack_parts(pack, M, N, K, passes);
+  const int ab = (M + kTcBM - 1) / kTcBM * (kTcBM / 32), bb = (N + kTcBN - 1) / kTcBN * (kTcBN / 8);
+  pack_kernel<<<ab + bb, 256, 0, s>>>(A, lda, B, ldb, M, N, K, ab, pk);
+  return update_packed(C, ldc, M, N, pk, status, s, max_ctas);
+}
+
+int launch_tc_step(float2* A, long long lda, int n, int k0, int nb, const int* ipiv, bool update,
+                   void* pack, int* status, cudaStream_t s, int max_ctas, int passes) {
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      tc_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepSmem);
+  if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
+  const int M = n - k0 - nb;  // rows and columns right of the panel (then nb = 64)
+  const int nright = (M + kStepCols - 1) / kStepCols, nleft = (k0 + kStepCols - 1) / kStepCols;
+  TcPack pk{};
+  if (update) pk = pack_parts(pack, M, M, nb, passes);
+  const int grid = nright + nleft + (update ? (M + 31) / 32 : 0);
+  if (grid == 0) return BEM2D_OK;
+  tc_step_kernel<<<grid, 256, kStepSmem, s>>>(A, lda, n, k0, nb, ipiv, nright, nleft, update, pk);
+  if (update)
+    return update_packed(A + (size_t)(k0 + nb) * lda + k0 + nb, lda, M, M, pk, status, s, max_ctas);
   return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
 }
 
