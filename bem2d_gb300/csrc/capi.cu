@@ -900,10 +900,8 @@ static int gmres_ir(bem2d_ctx* c, int n, const double2* A, long long lda, const 
   int stall = 0;
   for (int outer = 0; outer < 20; ++outer) {
     // residual and backward error
-    launch_residual(A, lda, n, x, b, r, part, c->stream);
-    launch_sumsq(r, n, n, 1, red, scal + 2, c->stream);
-    launch_sumsq(x, n, n, 1, red, scal + 3, c->stream);
-    c->launches += 6;
+    launch_residual(A, lda, n, x, b, r, part, red, scal + 2, c->stream);
+    c->launches += 3;
     double hs[2];
     CUDA_TRY(c, cudaMemcpyAsync(hs, scal + 2, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
@@ -1167,11 +1165,9 @@ static int solve_dev(bem2d_ctx* c, int n, const double2* A, long long lda, const
     if ((rc = lu_solve<float2>(LU, n, n, w, d, d, c->stream, &c->launches)))
       return fail(c, rc, "triangular solve launch: %s", cudaGetErrorString(cudaGetLastError()));
     launch_axpy_c64(n, rnorm, d, x, c->stream);
-    launch_residual(A, lda, n, x, b, r, part, c->stream);
-    launch_sumsq(r, n, n, 1, red, scal + 2, c->stream);
-    launch_sumsq(x, n, n, 1, red, scal + 3, c->stream);
+    launch_residual(A, lda, n, x, b, r, part, red, scal + 2, c->stream);
     toc(c, ts);
-    c->launches += 8;
+    c->launches += 5;
     CHECK_LAUNCH(c);
     CUDA_TRY(c, cudaMemcpyAsync(hs, scal, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(hinfo, w.info, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -2084,12 +2080,11 @@ int bem2d_l2_norm_cond_prec(bem2d_ctx* c, int n, const void* A, int64_t lda, dou
         CUDA_TRY(c, cudaMemcpyAsync(r, x, sizeof(double2) * n, cudaMemcpyDeviceToDevice,
                                     c->stream));
         launch_axpy_real(n, 1.0, tmp, r, c->stream);
+        launch_norms(n, r, y, red, scal + 2, c->stream);
       } else {
-        launch_residual(dA, la, n, y, x, r, rpart, c->stream);
+        launch_residual(dA, la, n, y, x, r, rpart, red, scal + 2, c->stream);
       }
-      launch_sumsq(r, n, n, 1, red, scal + 2, c->stream);
-      launch_sumsq(y, n, n, 1, red, scal + 3, c->stream);
-      c->launches += 8;
+      c->launches += herm ? 5 : 4;
       CUDA_TRY(c, cudaMemcpyAsync(hs + 2, scal + 2, 2 * sizeof(double), cudaMemcpyDeviceToHost,
                                   c->stream));
       CUDA_TRY(c, cudaMemcpyAsync(hinfo, w.info, 2 * sizeof(int), cudaMemcpyDeviceToHost,

@@ -533,8 +533,13 @@ int launch_oz_zgemm(double2* C, long long ldc, const double2* A, long long lda, 
 int launch_zpanel(double2* A, long long lda, int n, int k0, int nb, const LuWork& w,
                   cudaStream_t s, long long* launches);
 
+// r = b - A x; out[0] = |r|^2, out[1] = |x|^2 (part: residual_part_bytes(n), red:
+// sumsq_part_bytes() of scratch)
 void launch_residual(const double2* A, long long lda, int n, const double2* x,
-                     const double2* b, double2* r, double2* part, cudaStream_t s);
+                     const double2* b, double2* r, double2* part, double* red, double* out,
+                     cudaStream_t s);
+// out[0] = |r|^2, out[1] = |x|^2
+void launch_norms(int n, double2* r, const double2* x, double* red, double* out, cudaStream_t s);
 size_t residual_part_bytes(int n);
 void launch_to_c64(const double2* src, long long lds, float2* dst, long long ldd,
                    int rows, int cols, cudaStream_t s);

@@ -2739,46 +2739,105 @@ template int lu_solve<float2>(const float2*, long long, int, const LuWork&, cons
                               cudaStream_t, long long*);
 
 // ---- refinement helpers -----------------------------------------------------
-// r = b - A x in FP64; column chunks of 256 give partial sums per row.
+// r = b - A x in FP64: column chunks give partial sums per row; the kernel that
+// adds them also forms the partial sums of |r|^2 and |x|^2.  FP64 pipe: 4 n^2
+// FMAs.  Chunks of 64 columns below 4096 rows, so that every SM has several
+// blocks (n = 2048: 39 us, with chunks of 256 72 us; 28 us is the pipe's time);
+// above, longer chunks fill the GPU too and write fewer partial sums.
 constexpr int kResChunk = 256;
-__global__ void residual_partial_kernel(const double2* __restrict__ A, long long lda, int n,
-                                        const double2* __restrict__ x, double2* part) {
+static int res_chunk(int n) { return n < 4096 ? kResChunk / 4 : n < 8192 ? kResChunk / 2 : kResChunk; }
+__global__ void __launch_bounds__(128)
+residual_partial_kernel(const double2* __restrict__ A, long long lda, int n, int chunk,
+                        const double2* __restrict__ x, double2* part) {
   __shared__ double2 xs[kResChunk];
-  const int c0 = blockIdx.y * kResChunk;
-  const int nc = min(kResChunk, n - c0);
+  const int c0 = blockIdx.y * chunk;
+  const int nc = min(chunk, n - c0);
   for (int v = threadIdx.x; v < nc; v += blockDim.x) xs[v] = x[c0 + v];
   __syncthreads();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   double2 acc = make_double2(0, 0);
   const double2* col = A + (size_t)c0 * lda + r;
+#pragma unroll 8
   for (int c = 0; c < nc; ++c) acc = cfma(col[(size_t)c * lda], xs[c], acc);
   part[(size_t)blockIdx.y * n + r] = acc;
 }
 
-__global__ void residual_final_kernel(int n, int nchunk, const double2* __restrict__ part,
-                                      const double2* __restrict__ b, double2* r) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double2 acc = b[i];
-  for (int c = 0; c < nchunk; ++c) {
-    const double2 p = part[(size_t)c * n + i];
-    acc.x -= p.x;
-    acc.y -= p.y;
+// With nchunk > 0: r = b - the partial sums.  red[2 block], + 1: the block's sums
+// of |r|^2 and |x|^2.
+__global__ void __launch_bounds__(256)
+residual_final_kernel(int n, int nchunk, const double2* __restrict__ part,
+                      const double2* __restrict__ b, double2* r, const double2* __restrict__ x,
+                      double* __restrict__ red) {
+  double s[2] = {0.0, 0.0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double2 acc;
+    if (nchunk > 0) {
+      acc = b[i];
+#pragma unroll 8
+      for (int c = 0; c < nchunk; ++c) {
+        const double2 p = part[(size_t)c * n + i];
+        acc.x -= p.x;
+        acc.y -= p.y;
+      }
+      r[i] = acc;
+    } else {
+      acc = r[i];
+    }
+    const double2 v = x[i];
+    s[0] = fma(acc.x, acc.x, fma(acc.y, acc.y, s[0]));
+    s[1] = fma(v.x, v.x, fma(v.y, v.y, s[1]));
   }
-  r[i] = acc;
+  __shared__ double w[2][8];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+    if ((threadIdx.x & 31) == 0) w[j][threadIdx.x >> 5] = s[j];
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double a = 0.0;
+    for (int k = 0; k < 8; ++k) a += w[threadIdx.x][k];
+    red[2 * blockIdx.x + threadIdx.x] = a;
+  }
+}
+
+// out[j] = sum of red[2 i + j], i < nb: a warp for each j
+__global__ void __launch_bounds__(64)
+sum2_kernel(int nb, const double* __restrict__ red, double* out) {
+  const int j = threadIdx.x >> 5;
+  double s = 0.0;
+  for (int i = threadIdx.x & 31; i < nb; i += 32) s += red[2 * i + j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) out[j] = s;
+}
+
+constexpr int kSumsqBlocks = 304;
+static void final_norms(int n, int nchunk, const double2* part, const double2* b, double2* r,
+                        const double2* x, double* red, double* out, cudaStream_t s) {
+  const int nb = std::min((n + 255) / 256, kSumsqBlocks / 2);
+  residual_final_kernel<<<nb, 256, 0, s>>>(n, nchunk, part, b, r, x, red);
+  sum2_kernel<<<1, 64, 0, s>>>(nb, red, out);
 }
 
 void launch_residual(const double2* A, long long lda, int n, const double2* x,
-                     const double2* b, double2* r, double2* part, cudaStream_t s) {
-  const int nchunk = (n + kResChunk - 1) / kResChunk;
+                     const double2* b, double2* r, double2* part, double* red, double* out,
+                     cudaStream_t s) {
+  const int chunk = res_chunk(n), nchunk = (n + chunk - 1) / chunk;
   dim3 g((n + 127) / 128, nchunk);
-  residual_partial_kernel<<<g, 128, 0, s>>>(A, lda, n, x, part);
-  residual_final_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, nchunk, part, b, r);
+  residual_partial_kernel<<<g, 128, 0, s>>>(A, lda, n, chunk, x, part);
+  final_norms(n, nchunk, part, b, r, x, red, out, s);
+}
+
+void launch_norms(int n, double2* r, const double2* x, double* red, double* out, cudaStream_t s) {
+  final_norms(n, 0, nullptr, nullptr, r, x, red, out, s);
 }
 
 size_t residual_part_bytes(int n) {
-  return sizeof(double2) * (size_t)n * ((n + kResChunk - 1) / kResChunk);
+  const int chunk = res_chunk(n);
+  return sizeof(double2) * (size_t)n * ((n + chunk - 1) / chunk);
 }
 
 __global__ void to_c64_kernel(const double2* __restrict__ src, long long lds,
@@ -2946,24 +3005,32 @@ void launch_axpy_c64(int n, double scale, const float2* d, double2* x, cudaStrea
 
 // Sum of |a_ij|^2 over a rows x cols column-major block: per-block partial
 // sums, then one block adds them (deterministic order).
-__global__ void sumsq_partial_kernel(const double2* __restrict__ A, long long ld, int rows,
-                                     int cols, double* part) {
-  __shared__ double red[256];
+__global__ void __launch_bounds__(256)
+sumsq_partial_kernel(const double2* __restrict__ A, long long ld, long long rows, int cols,
+                     double* part) {
+  __shared__ double red[8];
+  // blocks of 1024 consecutive rows of a column
+  const long long per = (rows + 1023) / 1024, tot = per * cols;
   double acc = 0.0;
-  const long long tot = (long long)rows * cols;
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < tot;
-       v += (long long)gridDim.x * blockDim.x) {
-    const int j = (int)(v / rows), i = (int)(v - (long long)j * rows);
-    const double2 a = A[(size_t)j * ld + i];
-    acc = fma(a.x, a.x, fma(a.y, a.y, acc));
+  for (long long v = blockIdx.x; v < tot; v += gridDim.x) {
+    const long long j = cols == 1 ? 0 : v / per, i0 = (v - j * per) * 1024;
+    const double2* col = A + j * ld;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * 256 + threadIdx.x;
+      const double2 a = i < rows ? col[i] : make_double2(0.0, 0.0);
+      acc = fma(a.x, a.x, fma(a.y, a.y, acc));
+    }
   }
-  red[threadIdx.x] = acc;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int k = 0; k < 8; ++k) s += red[k];
+    part[blockIdx.x] = s;
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
 __global__ void sum_kernel(int n, const double* __restrict__ part, double* out) {
@@ -2979,10 +3046,12 @@ __global__ void sum_kernel(int n, const double* __restrict__ part, double* out) 
   if (threadIdx.x == 0) *out = red[0];
 }
 
-constexpr int kSumsqBlocks = 304;
 void launch_sumsq(const double2* A, long long ld, int rows, int cols, double* part,
                   double* out, cudaStream_t s) {
-  sumsq_partial_kernel<<<kSumsqBlocks, 256, 0, s>>>(A, ld, rows, cols, part);
+  // a contiguous matrix is one column
+  const bool one = ld == rows;
+  const long long r = one ? (long long)rows * cols : rows;
+  sumsq_partial_kernel<<<kSumsqBlocks, 256, 0, s>>>(A, ld, r, one ? 1 : cols, part);
   sum_kernel<<<1, 256, 0, s>>>(kSumsqBlocks, part, out);
 }
 size_t sumsq_part_bytes() { return sizeof(double) * kSumsqBlocks; }
