@@ -1432,63 +1432,86 @@ tslu_perm_kernel(int n, int k0, int nb, const int* __restrict__ candF, int Gc,
 // row order.  Positions k0 .. k0 + nb - 1: rows 0 .. nb - 1 of the
 // candidates' factor (L11 \ U11, Cf: ld Gc); position i beyond: the row r
 // there (i itself unless listed in `moved`), x U11 = A(r, :) solved for x =
-// L21(i).  A warp per position (lane j holds columns j and j + 32), each CTA
-// looping over positions with stride.
-__global__ void __launch_bounds__(256)
+// L21(i).  A thread per position, the row in registers; columns in sub-blocks of
+// 8 as in the panels: the sub-block's triangle, then the columns right of it.
+// FP32 issue bounds it (2016 complex multiply-subtracts per row); 16384 x 64 take
+// 22 us, as a warp per row with lanes on columns (a shuffle per column, strided
+// loads) 41 us.
+constexpr int kRowsCta = 128, kULd = kNB + 2;
+__global__ void __launch_bounds__(kRowsCta)
 tslu_rows_kernel(const float2* __restrict__ A, long long lda, int n, int k0, int nb,
                  const float2* __restrict__ Cf, int Gc, const int* __restrict__ moved,
                  float2* __restrict__ P) {
-  __shared__ float2 U[kNB * (kNB + 1)];  // U[c (kNB + 1) + r] = U11(c, r): row c of U11
+  constexpr int kR = kNB - kSub;
+  __shared__ __align__(16) float2 U[kNB][kULd];  // row c of U11
   __shared__ float2 dv[kNB];
-  __shared__ int mv[2 * kNB + 1];
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int c = e / nb, r = e - c * nb;  // coalesced: consecutive rows of column c
-    U[r * (kNB + 1) + c] = Cf[(size_t)c * Gc + r];
+  __shared__ float2 Xs[kSub][kRowsCta];
+  __shared__ int src[kRowsCta];
+  const int t = threadIdx.x, H = n - k0, i = blockIdx.x * kRowsCta + t;
+  src[t] = k0 + i;
+  for (int e = t; e < kNB * kNB; e += kRowsCta) {
+    const int c = e / kNB, r = e - c * kNB;  // coalesced: consecutive rows of column c
+    U[r][c] = c < nb && r < nb ? Cf[(size_t)c * Gc + r] : make_float2(0.f, 0.f);
   }
-  for (int e = threadIdx.x; e < 2 * kNB + 1; e += blockDim.x) mv[e] = moved[e];
   __syncthreads();
-  for (int c = threadIdx.x; c < nb; c += blockDim.x) {
-    const float2 d = U[c * (kNB + 1) + c];
+  for (int c = t; c < kNB; c += kRowsCta) {
+    const float2 d = U[c][c];
     dv[c] = (d.x != 0.f || d.y != 0.f) ? crcp(d) : make_float2(0.f, 0.f);
   }
-  __syncthreads();
-  const int H = n - k0, lane = threadIdx.x & 31, m = mv[0];
-  const int j0 = lane, j1 = lane + 32;
-  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < H; i += gridDim.x * 8) {
-    if (i < nb) {
-      for (int c = lane; c < nb; c += 32) P[(size_t)c * H + i] = Cf[(size_t)c * Gc + i];
-      continue;
-    }
-    int f = -1;  // the row moved to position k0 + i, if any
-    for (int u = lane; u < m; u += 32)
-      if (mv[1 + 2 * u] == k0 + i) f = mv[2 + 2 * u];
-    f = __reduce_max_sync(0xffffffffu, f);
-    const int r = f >= 0 ? f : k0 + i;
-    float2 a0 = j0 < nb ? A[(size_t)(k0 + j0) * lda + r] : make_float2(0.f, 0.f);
-    float2 a1 = j1 < nb ? A[(size_t)(k0 + j1) * lda + r] : make_float2(0.f, 0.f);
-    for (int c = 0; c < nb; ++c) {
-      const float2 src = c < 32 ? a0 : a1;
-      const float2 ac = make_float2(__shfl_sync(0xffffffffu, src.x, c & 31),
-                                    __shfl_sync(0xffffffffu, src.y, c & 31));
-      const float2 x = cmul(ac, dv[c]);
-      if (j0 == c) a0 = x;
-      if (j1 == c) a1 = x;
-      if (j0 > c && j0 < nb) a0 = cfms(a0, x, U[c * (kNB + 1) + j0]);
-      if (j1 > c && j1 < nb) a1 = cfms(a1, x, U[c * (kNB + 1) + j1]);
-    }
-    if (j0 < nb) P[(size_t)j0 * H + i] = a0;
-    if (j1 < nb) P[(size_t)j1 * H + i] = a1;
+  for (int u = t; u < moved[0]; u += kRowsCta) {  // the rows moved to positions of this CTA
+    const int q = moved[1 + 2 * u] - k0 - blockIdx.x * kRowsCta;
+    if (q >= 0 && q < kRowsCta) src[q] = moved[2 + 2 * u];
   }
-}
-
-static int num_sms_lu() {
-  static const int v = [] {
-    int dev = 0, c = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-    return c > 0 ? c : 1;
-  }();
-  return v;
+  __syncthreads();
+  if (i >= H) return;
+  if (i < nb) {
+    for (int c = 0; c < nb; ++c) P[(size_t)c * H + i] = Cf[(size_t)c * Gc + i];
+    return;
+  }
+  const float2* row = A + (size_t)k0 * lda + src[t];
+  float2 w[kSub], R[kR];
+#pragma unroll
+  for (int c = 0; c < kNB; ++c) {
+    const float2 a = c < nb ? row[(size_t)c * lda] : make_float2(0.f, 0.f);
+    if (c < kSub)
+      w[c < kSub ? c : 0] = a;
+    else
+      R[c < kSub ? 0 : c - kSub] = a;
+  }
+#pragma unroll 1
+  for (int c0 = 0; c0 < nb; c0 += kSub) {
+#pragma unroll
+    for (int q = 0; q < kSub; ++q) {
+      const float2 x = cmul(w[q], dv[c0 + q]);
+      w[q] = x;
+      Xs[q][t] = x;
+#pragma unroll
+      for (int j = q + 1; j < kSub; ++j) w[j] = cfms(w[j], x, U[c0 + q][c0 + j]);
+    }
+#pragma unroll
+    for (int q = 0; q < kSub; ++q)
+      if (c0 + q < nb) P[(size_t)(c0 + q) * H + i] = w[q];
+    const int ng = (kNB - c0) / kSub - 1;  // groups of 8 columns right
+#pragma unroll 1
+    for (int q = 0; q < kSub; ++q) {
+      const float2 x = Xs[q][t];
+      const float4* u4 = reinterpret_cast<const float4*>(&U[c0 + q][c0 + kSub]);
+#pragma unroll
+      for (int g = 0; g < kR / kSub; ++g) {
+        if (g >= ng) break;
+#pragma unroll
+        for (int j = 0; j < kSubP; ++j) {
+          const float4 u = u4[g * kSubP + j];
+          R[g * kSub + 2 * j] = cfms(R[g * kSub + 2 * j], x, make_float2(u.x, u.y));
+          R[g * kSub + 2 * j + 1] = cfms(R[g * kSub + 2 * j + 1], x, make_float2(u.z, u.w));
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kSub; ++j) w[j] = R[j];
+#pragma unroll
+    for (int j = 0; j < kR - kSub; ++j) R[j] = R[j + kSub];
+  }
 }
 
 // Tournament-pivoted panel of columns k0 .. k0 + nb - 1 (rows k0 .. n - 1).
@@ -1553,8 +1576,8 @@ static bool tslu_panel(float2* A, long long lda, int n, int k0, int nb, const Lu
   }
   tslu_perm_kernel<<<1, 1024, sizeof(int) * 2 * (size_t)H, s>>>(n, k0, nb, candF, Gf, ts.ipc,
                                                                 ts.infc, w.ipiv, w.info, ts.moved);
-  const int rgrid = std::min((H + 7) / 8, 4 * num_sms_lu());
-  tslu_rows_kernel<<<rgrid, 256, 0, s>>>(A, lda, n, k0, nb, Cf, ld, ts.moved, ts.P);
+  tslu_rows_kernel<<<(H + kRowsCta - 1) / kRowsCta, kRowsCta, 0, s>>>(A, lda, n, k0, nb, Cf, ld,
+                                                                      ts.moved, ts.P);
   cudaMemcpy2DAsync(A + (size_t)k0 * lda + k0, sizeof(float2) * lda, ts.P, sizeof(float2) * H,
                     sizeof(float2) * H, nb, cudaMemcpyDeviceToDevice, s);
   *launches += 2;  // + the cluster launch the caller counts
