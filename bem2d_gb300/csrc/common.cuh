@@ -510,12 +510,14 @@ int launch_tc_cgemm_sub(float2* C, long long ldc, const float2* A, long long lda
                         const float2* B, long long ldb, int M, int N, int K, void* pack,
                         size_t pack_bytes, int* status, cudaStream_t s, int max_ctas = 0,
                         int passes = 3);
-// What follows a complex64 panel of nb columns at k0 (ipiv[k0 ..]: its pivots):
-// the row swaps on all other columns, U12 = L11^{-1} A12 and, with `update`, A22
-// -= L21 U12 (pack: tc_pack_bytes(M, M, nb) bytes, M = n - k0 - nb).  nb = 64
-// unless the panel is the last.
-int launch_tc_step(float2* A, long long lda, int n, int k0, int nb, const int* ipiv, bool update,
-                   void* pack, int* status, cudaStream_t s, int max_ctas, int passes);
+// What follows a complex64 panel of nb columns at k0 (ipiv[k0 ..]: its pivots;
+// null: no swaps): the row swaps on the columns [cl, k0) and [rs, cr), U12 =
+// L11^{-1} A12 on the latter and, with `update`, A22 -= L21 U12 there for the M
+// rows below the panel (pack: tc_pack_bytes(M, cr - rs, nb) bytes).  nb = 64
+// unless cr = rs.
+int launch_tc_step(float2* A, long long lda, int M, int k0, int nb, int cl, int rs, int cr,
+                   const int* ipiv, bool update, void* pack, int* status, cudaStream_t s,
+                   int max_ctas, int passes);
 
 // C = beta C + sign A B (complex128, column-major; C is M x N, A M x K, B K x
 // N; beta 0 or 1) on the tensor cores, FP64 accurate (lu_oz.cu).  piv (null:

@@ -1952,26 +1952,24 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
       if (e != cudaSuccess) return BEM2D_ERR_CUDA;
     }
     ++*launches;
-    if (la) {  // the block's own columns; the rest after the far update
-      laswp_cols(A, lda, w.ipiv, k0, nb, K0, k0, s, launches);
-      laswp_cols(A, lda, w.ipiv, k0, nb, k0 + nb, bend, s, launches);
-    } else if (sizeof(T) == sizeof(float2) && outer == kNB) {
-      // swaps, U12 and the update of everything right of the panel
-      const int M = n - k0 - nb;
-      const bool tc = M > 0 && w.pack && tc_pack_bytes(M, M, nb) <= w.pack_bytes;
-      if (n > nb) {
-        if (launch_tc_step(reinterpret_cast<float2*>(A), lda, n, k0, nb, w.ipiv, tc, w.pack,
+    if (sizeof(T) == sizeof(float2) && (la || outer == kNB)) {
+      // swaps, U12 and the update of the block's own columns with la (the rest
+      // after the far update), of all others without (a panel is its own
+      // block)
+      const int cl = la ? K0 : 0, cr = la ? bend : n, c1 = k0 + nb, M = n - c1, N = cr - c1;
+      const bool tc = N > 0 && w.pack && tc_pack_bytes(M, N, nb) <= w.pack_bytes;
+      if (N > 0 || k0 > cl) {
+        if (launch_tc_step(reinterpret_cast<float2*>(A), lda, M, k0, nb, cl, c1, cr, w.ipiv, tc, w.pack,
                            w.status, s, w.tc_ctas, w.tc_passes))
           return BEM2D_ERR_CUDA;
         *launches += tc ? 2 : 1;
       }
       if (!tc) {
-        const size_t c1 = (size_t)(k0 + nb);
-        const int rc = update_sub(A + c1 * lda + c1, A + (size_t)k0 * lda + c1, A + c1 * lda + k0,
-                                  lda, M, M, nb, w, s, launches);
+        const int rc = update_sub(A + (size_t)c1 * lda + c1, A + (size_t)k0 * lda + c1,
+                                  A + (size_t)c1 * lda + k0, lda, M, N, nb, w, s, launches);
         if (rc) return rc;
       }
-      continue;  // a panel is its own block
+      continue;
     } else if (n > nb) {
       laswp_kernel<T><<<(n - nb + 127) / 128, 128, 0, s>>>(A, lda, n, w.ipiv, k0, nb);
       ++*launches;
@@ -1997,8 +1995,15 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
   const bool stepped = sizeof(T) == sizeof(float2) && outer == kNB && !la;
   if (nc > 0 && !stepped) {
     for (int j0 = K0; j0 < bend; j0 += kNB) {
-      trsm_rows(A, lda, j0, kNB, bend, nc, s, launches);
       const int r1 = j0 + kNB;
+      if (la && w.pack && tc_pack_bytes(bend - r1, nc, kNB) <= w.pack_bytes) {
+        if (launch_tc_step(reinterpret_cast<float2*>(A), lda, bend - r1, j0, kNB, j0, bend, n,
+                           nullptr, r1 < bend, w.pack, w.status, s, w.tc_ctas, w.tc_passes))
+          return BEM2D_ERR_CUDA;
+        *launches += r1 < bend ? 2 : 1;
+        continue;
+      }
+      trsm_rows(A, lda, j0, kNB, bend, nc, s, launches);
       if (r1 < bend) {
         int rc = update_sub(A + (size_t)bend * lda + r1, A + (size_t)j0 * lda + r1,
                             A + (size_t)bend * lda + j0, lda, bend - r1, nc, kNB, w, s, launches);

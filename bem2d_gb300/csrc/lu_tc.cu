@@ -217,8 +217,9 @@ pack_kernel(const float2* __restrict__ A, long long lda, const float2* __restric
 }
 
 // ---- between a panel and its update ----------------------------------------
-// Row swaps of the panel at k0 on all other columns, U12 = L11^{-1} A12 and
-// (packing) the operands of A22 -= L21 U12, in one launch.  CTAs:
+// Row swaps of the panel at k0 (ipiv, null: none) on the columns [cl, k0) and
+// [rs, cr), U12 = L11^{-1} A12 on the latter and (packing) the operands of A22 -=
+// L21 U12 for the M rows below the panel, in one launch.  CTAs:
 //   [0, nright)  32 columns right of the panel each: swaps, U12, its pack;
 //   then nleft   32 columns left of it: swaps;
 //   then         32 rows of L21 each: their pack.
@@ -235,24 +236,27 @@ constexpr int kNBs = 64;  // panel width
 constexpr size_t kStepSmem = sizeof(float2) * (kNBs * kNBs + kNBs * kStepCols);
 
 __global__ void __launch_bounds__(256)
-tc_step_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb,
-               const int* __restrict__ ipiv, int nright, int nleft, bool packing, TcPack pk) {
+tc_step_kernel(float2* __restrict__ A, long long lda, int M, int k0, int nb, int cl, int rs,
+               int cr, const int* __restrict__ ipiv, int nright, int nleft, bool packing, TcPack pk) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_ip[kNBs], s_src[kNBs], s_pos[kNBs], s_from[kNBs];
   __shared__ float red[8][32];
   const int t = threadIdx.x, c = t & 31, w = t >> 5;
   const int b = blockIdx.x;
   if (b >= nright + nleft) {
-    pack_block<true>(A + (size_t)k0 * lda + k0 + nb, lda, n - k0 - nb, nb, b - nright - nleft, pk,
-                     red);
+    pack_block<true>(A + (size_t)k0 * lda + k0 + nb, lda, M, nb, b - nright - nleft, pk, red);
     return;
   }
   const bool right = b < nright;
-  const int cb = right ? k0 + nb + kStepCols * b : kStepCols * (b - nright);
-  const int nc = min(kStepCols, (right ? n : k0) - cb);
+  const int cb = right ? rs + kStepCols * b : cl + kStepCols * (b - nright);
+  const int nc = min(kStepCols, (right ? cr : k0) - cb);
   float2* L = reinterpret_cast<float2*>(smem);  // [kNBs][kNBs] column-major
   float2* X = L + kNBs * kNBs;                  // [kNBs][kStepCols]
-  if (t < kNBs) s_ip[t] = t < nb ? ipiv[k0 + t] : k0 + t;
+  if (t < kNBs) {
+    s_ip[t] = ipiv && t < nb ? ipiv[k0 + t] : k0 + t;
+    s_src[t] = k0 + t;
+    s_pos[t] = -1;
+  }
   if (right) {  // nb = 64
 #pragma unroll
     for (int v = 0; v < kNBs * kNBs / 256; ++v) {
@@ -261,7 +265,7 @@ tc_step_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb,
     }
   }
   __syncthreads();
-  if (t < 2 * kNBs) {  // the row that ends at position x
+  if (ipiv && t < 2 * kNBs) {  // the row that ends at position x
     const int x0 = t < kNBs ? k0 + t : s_ip[t - kNBs];
     int x = x0;
     for (int s = kNBs - 1; s >= 0; --s) {
@@ -616,20 +620,22 @@ int launch_tc_cgemm_sub(float2* C, long long ldc, const float2* A, long long lda
   return update_packed(C, ldc, M, N, pk, status, s, max_ctas);
 }
 
-int launch_tc_step(float2* A, long long lda, int n, int k0, int nb, const int* ipiv, bool update,
-                   void* pack, int* status, cudaStream_t s, int max_ctas, int passes) {
+int launch_tc_step(float2* A, long long lda, int M, int k0, int nb, int cl, int rs, int cr,
+                   const int* ipiv, bool update, void* pack, int* status, cudaStream_t s,
+                   int max_ctas, int passes) {
   static const cudaError_t attr = cudaFuncSetAttribute(
       tc_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepSmem);
   if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
-  const int M = n - k0 - nb;  // rows and columns right of the panel (then nb = 64)
-  const int nright = (M + kStepCols - 1) / kStepCols, nleft = (k0 + kStepCols - 1) / kStepCols;
+  const int N = cr - rs;  // N > 0: nb = 64
+  const int nright = (N + kStepCols - 1) / kStepCols, nleft = (k0 - cl + kStepCols - 1) / kStepCols;
   TcPack pk{};
-  if (update) pk = pack_parts(pack, M, M, nb, passes);
+  if (update) pk = pack_parts(pack, M, N, nb, passes);
   const int grid = nright + nleft + (update ? (M + 31) / 32 : 0);
   if (grid == 0) return BEM2D_OK;
-  tc_step_kernel<<<grid, 256, kStepSmem, s>>>(A, lda, n, k0, nb, ipiv, nright, nleft, update, pk);
+  tc_step_kernel<<<grid, 256, kStepSmem, s>>>(A, lda, M, k0, nb, cl, rs, cr, ipiv, nright, nleft,
+                                              update, pk);
   if (update)
-    return update_packed(A + (size_t)(k0 + nb) * lda + k0 + nb, lda, M, M, pk, status, s, max_ctas);
+    return update_packed(A + (size_t)rs * lda + k0 + nb, lda, M, N, pk, status, s, max_ctas);
   return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
 }
 
