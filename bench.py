@@ -245,19 +245,19 @@ def far_roofline(n, far_ms, fp32_peak, key=None):
 
 
 def lu_roofline(n, lu_ms, peaks):
-    """The complex64 LU against the TF32 tensor peak (half the measured bf16
-    rate): 8N^3/3 real flops per factorisation (zgetrf's count).  The
-    trailing update issues each product as three TF32 MMAs (hi*hi, hi*lo,
-    lo*hi), so the tensor pipe executes about 3x the algorithmic flops."""
+    """The complex64 LU against the f16 tensor peak (the measured bf16 rate):
+    8N^3/3 real flops per factorisation (zgetrf's count).  The trailing
+    update issues each product as three f16 MMAs (hi*hi, hi*lo, lo*hi), so
+    the tensor pipe executes about 3x the algorithmic flops."""
     flops = 8.0 * n ** 3 / 3.0
     ach = flops / (lu_ms * 1e-3) / 1e12
-    peak = peaks["bf16_tflops"] / 2.0
+    peak = peaks["bf16_tflops"]
     return {"bound": "tensor", "kernel": "complex64 LU (panels, trsm, tcgen05 trailing update)",
             "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
-            "peak_source": "TF32 dense = bf16 burst / 2, bf16 %s (MEASURED_PEAKS.json)"
+            "peak_source": "f16 dense = bf16 burst, %s (MEASURED_PEAKS.json)"
                            % peaks["source"],
             "traffic": None,
-            "note": "N=%d; 8N^3/3 flops per factorisation; 3xTF32 split issues 3x" % n}
+            "note": "N=%d; 8N^3/3 flops per factorisation; the two-way f16 split issues 3x" % n}
 
 
 class Stepper:
@@ -599,7 +599,7 @@ def solve_record(ctx, args, wname, steps, warmup, ws=1, rank=0, sub=False):
         "data": "synthetic",
         "config": {"workload": w["desc"], "problems_per_step": P,
                    "n_unknowns": ns[0] if P == 1 else [min(ns), max(ns)],
-                   "precision": "mixed", "lu_update": "3xTF32 (tcgen05 kind::tf32)",
+                   "precision": "mixed", "lu_update": "3 products of scaled f16 halves (tcgen05 kind::f16)",
                    "sweep_workers": args.workers if P > 1 else None,
                    "l2": "256 MB write between timed steps, outside the step events",
                    "parallelism": "replicas" if ws > 1 else "single GPU"},
@@ -641,8 +641,8 @@ def solve_record(ctx, args, wname, steps, warmup, ws=1, rank=0, sub=False):
         res["backward_error"] = {"mixed": berr(x_dev[0]), "fp64": berr(x_fp64[0]),
                                  "measure": "|b - A x| / (|A|_F |x| + |b|), FP64 A"}
         # the LU's trailing-update precision options on the same system: the
-        # value above runs 3xTF32; 1xTF32 issues a third of the tensor work
-        # and leaves more to the refinement
+        # value above runs three products per term; one product issues a third
+        # of the tensor work and leaves more to the refinement
         x_t = torch.zeros(nb, dtype=torch.complex128, device="cuda")
         ms_t = st.run(lambda: ctx.scattering_solve(holds[0].arrays, k, w["d"], eta, QUAD,
                                                    precision="mixed_tf32", out=x_t),
@@ -651,12 +651,12 @@ def solve_record(ctx, args, wname, steps, warmup, ws=1, rank=0, sub=False):
         ph_t = phases("mixed_tf32")
         t_t = max_over_ranks([sum(ms_t) / len(ms_t)], ws, "cuda")[0]
         res["update_options"] = {
-            "ran": "3xTF32 (value, e2e)",
-            "3xTF32": {"ms_per_step": t_mixed, "lu_ms": ph_mixed["lu"],
+            "ran": "3xf16 (value, e2e)",
+            "3xf16": {"ms_per_step": t_mixed, "lu_ms": ph_mixed["lu"],
                        "solve_ms": ph_mixed["solve"], "iterations": infos[0][1],
                        "backward_error": res["backward_error"]["mixed"],
                        "rel_err_vs_fp64": errs[0]},
-            "1xTF32": {"ms_per_step": t_t, "lu_ms": ph_t["lu"], "solve_ms": ph_t["solve"],
+            "1xf16": {"ms_per_step": t_t, "lu_ms": ph_t["lu"], "solve_ms": ph_t["solve"],
                        "iterations": info_t[1], "backward_error": berr(x_t),
                        "rel_err_vs_fp64": float(torch.linalg.vector_norm(x_t - x_fp64[0]) /
                                                 torch.linalg.vector_norm(x_fp64[0]))}}

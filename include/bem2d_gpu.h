@@ -176,7 +176,7 @@ int bem2d_dot_prod_basfuns(bem2d_ctx* ctx, const bem2d_geometry* geom,
  * LAPACK zgetrf + zgetrs).  A (n x n, lda) and b are not modified.
  * BEM2D_PREC_FP64: blocked complex128 LU with partial pivoting.
  * BEM2D_PREC_MIXED: complex64 LU with partial pivoting (tournament
- *   pivoting for panels taller than 4096 rows), then FP64 iterative
+ *   pivoting for panels taller than 6656 rows), then FP64 iterative
  *   refinement with the complex128 A until the backward error
  *   ||b - A x|| / (||A||_F ||x|| + ||b||) <= tol (tol <= 0 selects 1e-14);
  *   at most 30 steps.  If plain refinement stalls or diverges above
