@@ -118,7 +118,7 @@ static const void* hankel_tab_real() {
 size_t hankel_tab_bytes() { return kHtBytes; }
 
 // ---- far field ---------------------------------------------------------------
-// Bound by the FP64 pipe (81 % of its rate by ncu at kite N = 2048).  Per node
+// Bound by the FP64 pipe (90 % of its rate by ncu at kite N = 2048).  Per node
 // pair 70 FP64 instructions serve entry (i, j) and entry (j, i) of every
 // basis-function pair of the two elements: the distance, 1/d, H0 and H1 are
 // shared, an orientation adds its normal factor n . (x - y), a basis function
