@@ -1381,6 +1381,9 @@ tslu_perm_kernel(int n, int k0, int nb, const int* __restrict__ candF, int Gc,
   int* pos = sh;       // [H] position of row k0 + i
   int* at = sh + H;    // [H] row at position k0 + i
   __shared__ int cw[kTsluMaxCand];
+  __shared__ int sp[kNB], ic[kNB], m;  // the panel's pivots, the candidates' pivots, moved rows
+  if (threadIdx.x < nb) ic[threadIdx.x] = ipc[threadIdx.x];
+  if (threadIdx.x == 0) m = 0;
   for (int i = threadIdx.x; i < H; i += blockDim.x) {
     pos[i] = i;
     at[i] = i;
@@ -1390,7 +1393,7 @@ tslu_perm_kernel(int n, int k0, int nb, const int* __restrict__ candF, int Gc,
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int c = 0; c < nb; ++c) {  // the candidates' interchanges: cw[c] = pivot row c
-      const int q = ipc[c];
+      const int q = ic[c];
       if (q != c && q >= 0 && q < Gc) {
         const int tmp = cw[c];
         cw[c] = cw[q];
@@ -1400,32 +1403,34 @@ tslu_perm_kernel(int n, int k0, int nb, const int* __restrict__ candF, int Gc,
     for (int c = 0; c < nb; ++c) {
       const int r = cw[c] - k0;
       if (r < 0 || r >= H) {  // a zero column: no interchange (info is set)
-        ipiv[k0 + c] = k0 + c;
+        sp[c] = c;
         continue;
       }
       const int p = pos[r], rt = at[c];
-      ipiv[k0 + c] = k0 + p;
+      sp[c] = p;
       at[p] = rt;
       pos[rt] = p;
       at[c] = r;
       pos[r] = c;
     }
-    int m = 0;
-    for (int c = 0; c < nb; ++c) {
-      const int p = ipiv[k0 + c] - k0;
-      if (p >= nb && at[p] != p) {
-        bool seen = false;
-        for (int u = 0; u < m; ++u) seen |= moved[1 + 2 * u] == k0 + p;
-        if (!seen) {
-          moved[1 + 2 * m] = k0 + p;
-          moved[2 + 2 * m] = k0 + at[p];
-          ++m;
-        }
-      }
-    }
-    moved[0] = m;
     if (*infc && *info == 0) *info = k0 + *infc;
   }
+  __syncthreads();
+  // a thread per step: its pivot, and the row that an interchange left at the
+  // pivot's position (listed once, by the first step that names it)
+  if (threadIdx.x < nb) {
+    const int c = threadIdx.x, p = sp[c];
+    ipiv[k0 + c] = k0 + p;
+    bool first = p >= nb && at[p] != p;
+    for (int u = 0; u < c; ++u) first &= sp[u] != p;
+    if (first) {
+      const int j = atomicAdd(&m, 1);
+      moved[1 + 2 * j] = k0 + p;
+      moved[2 + 2 * j] = k0 + at[p];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) moved[0] = m;
 }
 
 // P (H x nb, column-major, ld H = n - k0): the factored panel in its final
