@@ -12,6 +12,7 @@
 //  ident_kernel       EvalIdent (lib/bem2d_quadrature.cpp:79-127)
 //  rhs_kernel         DotProdBasFuns (lib/bem2d_quadrature.h:111-156)
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "ff.cuh"
@@ -92,17 +93,21 @@ __device__ __forceinline__ double mass_entry(const DevGeom& g, const DevRules& r
 
 // Element geometry at the distinct coordinates of a rule, per warp in shared
 // memory (structure of arrays): Map, Normal and |J| phi, phi the basis
-// function of the pair's unknown on that element.
+// functions of the pair's unknowns on that element (basis b at f + b cap).
 struct GeoTab {
   double* x;
   double* y;
   double* nx;
   double* ny;
   double* f;
+  int cap;
 };
 
-__device__ __forceinline__ void geo_fill(const DevGeom& g, int e, int u, const double* vals, int n,
-                                         bool mirror, const GeoTab& tb, int off, int lane) {
+// Geometry of element e and the basis functions of its unknowns u .. u + nu - 1.
+template <int NB>
+__device__ __forceinline__ void geo_fill(const DevGeom& g, int e, int u, int nu,
+                                         const double* vals, int n, bool mirror, const GeoTab& tb,
+                                         int off, int lane) {
   const double* prm = g.param + 8 * (size_t)e;
   for (int v = lane; v < n; v += 32) {
     const double s = mirror ? 1 - vals[v] : vals[v];
@@ -113,7 +118,11 @@ __device__ __forceinline__ void geo_fill(const DevGeom& g, int e, int u, const d
     tb.y[off + v] = p.my;
     tb.nx[off + v] = nx;
     tb.ny[off + v] = ny;
-    tb.f[off + v] = elem_jac(p) * basis_eval(g.unk_kind[u], g.unk_param[u], s);
+    const double jac = elem_jac(p);
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+      if (NB == 1 || b < nu)
+        tb.f[b * tb.cap + off + v] = jac * basis_eval(g.unk_kind[u + b], g.unk_param[u + b], s);
   }
 }
 
@@ -170,7 +179,51 @@ __device__ __forceinline__ void near_point(double k, double ki, double kq, doubl
   }
 }
 
-template <int KERNEL, bool MIXED, bool CK>
+// Sums over a rule's points of K f_i f_j w for the NB x NB basis functions of a
+// pair: f_i at stride sa from fa, f_j w in gb.
+template <int NB>
+struct NearSums {
+  double re[NB][NB], im[NB][NB];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+#pragma unroll
+      for (int j = 0; j < NB; ++j) re[i][j] = im[i][j] = 0.0;
+  }
+  __device__ __forceinline__ void add(double r, double m, const double (&fa)[NB],
+                                      const double (&gb)[NB]) {
+    if (NB == 1) {
+      const double f = fa[0] * gb[0];
+      re[0][0] = fma(r, f, re[0][0]);
+      im[0][0] = fma(m, f, im[0][0]);
+      return;
+    }
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const double rj = r * gb[j], mj = m * gb[j];
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        re[i][j] = fma(rj, fa[i], re[i][j]);
+        im[i][j] = fma(mj, fa[i], im[i][j]);
+      }
+    }
+  }
+  __device__ __forceinline__ void reduce() {
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        re[i][j] = warp_sum(re[i][j]);
+        im[i][j] = warp_sum(im[i][j]);
+      }
+  }
+};
+
+// One pair of groups: runs of up to NB consecutive unknowns of one element (NB
+// = 1: of unknowns).  Every point's kernel value, the work that counts, serves
+// all NB x NB entries: 801 elements of PolBasis(2), N = 2403, double layer,
+// 1.46 ms with a warp per entry, 0.27 so.
+template <int KERNEL, bool MIXED, bool CK, int NB>
 __global__ void __launch_bounds__(256)
 near_kernel(DevGeom g, DevRules r, const NearPair* __restrict__ pairs, int npairs, double k,
             double ki, double eta, double alpha, double beta, KConstFF kc, const float* gtab, int cap_s,
@@ -180,8 +233,8 @@ near_kernel(DevGeom g, DevRules r, const NearPair* __restrict__ pairs, int npair
   float* tab = reinterpret_cast<float*>(smem_raw);  // e^{ix} table (MIXED)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cap = cap_s + cap_t;
-  double* base = reinterpret_cast<double*>(smem_raw + 1024) + (size_t)warp * 5 * cap;
-  const GeoTab S{base, base + cap, base + 2 * cap, base + 3 * cap, base + 4 * cap};
+  double* base = reinterpret_cast<double*>(smem_raw + 1024) + (size_t)warp * (4 + NB) * cap;
+  const GeoTab S{base, base + cap, base + 2 * cap, base + 3 * cap, base + 4 * cap, cap};
   if (MIXED) {
     for (int v = threadIdx.x; v < 256; v += blockDim.x) tab[v] = gtab[v];
     __syncthreads();
@@ -191,14 +244,15 @@ near_kernel(DevGeom g, DevRules r, const NearPair* __restrict__ pairs, int npair
   const NearPair pr = pairs[wid];
   const int e1 = g.unk_elem[pr.i], e2 = g.unk_elem[pr.j];
   const double kq = 0.25 * k, eq = 0.25 * eta;
-  double acc_re = 0.0, acc_im = 0.0;
+  NearSums<NB> acc, acc2;  // acc2: the second orientation of RULE_G3_PAIR
+  acc.clear();
   double u1, u2;  // unused second orientation
   if (pr.rule == RULE_SELF) {
     // IntegrateIdent: Duffy split, points (x, (1-y)x) and (1-x, 1-x+yx),
     // both weighted by x * w.  Test-side geometry from the table (x values,
     // then 1 - x); trial-side evaluated per point.
-    geo_fill(g, e1, pr.i, r.u1, r.nu1, false, S, 0, lane);
-    geo_fill(g, e1, pr.i, r.u1, r.nu1, true, S, r.nu1, lane);
+    geo_fill<NB>(g, e1, pr.i, pr.ni, r.u1, r.nu1, false, S, 0, lane);
+    geo_fill<NB>(g, e1, pr.i, pr.ni, r.u1, r.nu1, true, S, r.nu1, lane);
     __syncwarp();
     const double* p2 = g.param + 8 * (size_t)e2;
     for (int p = lane; p < r.n1; p += 32) {
@@ -214,10 +268,16 @@ near_kernel(DevGeom g, DevRules r, const NearPair* __restrict__ pairs, int npair
         near_point<KERNEL, MIXED, false, CK>(k, ki, kq, eq, kc, tab, S.x[a], S.y[a], S.nx[a],
                                              S.ny[a], b.mx, b.my, n2x, n2y, &re, &im, &u1,
                                              &u2);
-        const double f =
-            S.f[a] * (elem_jac(b) * basis_eval(g.unk_kind[pr.j], g.unk_param[pr.j], t));
-        acc_re = fma(re * f, x * w, acc_re);
-        acc_im = fma(im * f, x * w, acc_im);
+        const double jw = elem_jac(b) * (x * w);
+        double fa[NB], gb[NB];
+#pragma unroll
+        for (int v = 0; v < NB; ++v) {
+          fa[v] = NB == 1 || v < pr.ni ? S.f[v * cap + a] : 0.0;
+          gb[v] = NB == 1 || v < pr.nj
+                      ? jw * basis_eval(g.unk_kind[pr.j + v], g.unk_param[pr.j + v], t)
+                      : 0.0;
+        }
+        acc.add(re, im, fa, gb);
       }
     }
   } else {
@@ -229,53 +289,67 @@ near_kernel(DevGeom g, DevRules r, const NearPair* __restrict__ pairs, int npair
     const double* rule = g2 ? r.r2 : r.r3;
     const int* key = g2 ? r.k2 : r.k3;
     const int np = g2 ? r.n2 : r.n3;
-    geo_fill(g, e1, pr.i, g2 ? r.u2 : r.u3, g2 ? r.nu2 : r.nu3, false, S, 0, lane);
-    geo_fill(g, e2, pr.j, g2 ? r.v2 : r.v3, g2 ? r.nv2 : r.nv3, false, S, cap_s, lane);
+    geo_fill<NB>(g, e1, pr.i, pr.ni, g2 ? r.u2 : r.u3, g2 ? r.nu2 : r.nu3, false, S, 0, lane);
+    geo_fill<NB>(g, e2, pr.j, pr.nj, g2 ? r.v2 : r.v3, g2 ? r.nv2 : r.nv3, false, S, cap_s, lane);
     __syncwarp();
+    auto weights = [&](int p, int* a, int* b, double (&fa)[NB], double (&gb)[NB]) {
+      const int kk = key[p];
+      *a = kk & 0xffff;
+      *b = cap_s + (kk >> 16);
+      const double w = rule[3 * p + 2];
+#pragma unroll
+      for (int v = 0; v < NB; ++v) {
+        fa[v] = NB == 1 || v < pr.ni ? S.f[v * cap + *a] : 0.0;
+        gb[v] = NB == 1 || v < pr.nj ? S.f[v * cap + *b] * w : 0.0;
+      }
+    };
     if (pr.rule == RULE_G3_PAIR) {
-      double acc2_re = 0.0, acc2_im = 0.0;
+      acc2.clear();
       for (int p = lane; p < np; p += 32) {
-        const int kk = key[p];
-        const int a = kk & 0xffff, b = cap_s + (kk >> 16);
-        double r1, i1, r2, i2;
+        int a, b;
+        double fa[NB], gb[NB], r1, i1, r2, i2;
+        weights(p, &a, &b, fa, gb);
         near_point<KERNEL, MIXED, true, CK>(k, ki, kq, eq, kc, tab, S.x[a], S.y[a], S.nx[a],
                                             S.ny[a], S.x[b], S.y[b], S.nx[b], S.ny[b], &r1,
                                             &i1, &r2, &i2);
-        const double f = S.f[a] * S.f[b] * rule[3 * p + 2];
-        acc_re = fma(r1, f, acc_re);
-        acc_im = fma(i1, f, acc_im);
-        acc2_re = fma(r2, f, acc2_re);
-        acc2_im = fma(i2, f, acc2_im);
+        acc.add(r1, i1, fa, gb);
+        acc2.add(r2, i2, fa, gb);
       }
-      acc2_re = warp_sum(acc2_re);
-      acc2_im = warp_sum(acc2_im);
-      if (lane == 0) {
-        const double re = alpha * acc2_re, im = alpha * acc2_im;
-        out[(size_t)pr.i * ld + pr.j] = make_double2(re, im);
-        if (MIXED) out32[(size_t)pr.i * ld32 + pr.j] = make_float2((float)re, (float)im);
-      }
+      acc2.reduce();
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+#pragma unroll
+        for (int j = 0; j < NB; ++j)
+          if (lane == i * NB + j && (NB == 1 || (i < pr.ni && j < pr.nj))) {
+            const double re = alpha * acc2.re[i][j], im = alpha * acc2.im[i][j];
+            const size_t row = pr.j + j, col = pr.i + i;
+            out[col * ld + row] = make_double2(re, im);
+            if (MIXED) out32[col * ld32 + row] = make_float2((float)re, (float)im);
+          }
     } else {
       for (int p = lane; p < np; p += 32) {
-        const int kk = key[p];
-        const int a = kk & 0xffff, b = cap_s + (kk >> 16);
-        double re, im;
+        int a, b;
+        double fa[NB], gb[NB], re, im;
+        weights(p, &a, &b, fa, gb);
         near_point<KERNEL, MIXED, false, CK>(k, ki, kq, eq, kc, tab, S.x[a], S.y[a], S.nx[a],
                                              S.ny[a], S.x[b], S.y[b], S.nx[b], S.ny[b], &re,
                                              &im, &u1, &u2);
-        const double f = S.f[a] * S.f[b] * rule[3 * p + 2];
-        acc_re = fma(re, f, acc_re);
-        acc_im = fma(im, f, acc_im);
+        acc.add(re, im, fa, gb);
       }
     }
   }
-  acc_re = warp_sum(acc_re);
-  acc_im = warp_sum(acc_im);
-  if (lane == 0) {
-    double re = alpha * acc_re, im = alpha * acc_im;
-    if (pr.same && beta != 0.0) re = fma(beta, mass_entry(g, r, pr.i, pr.j), re);
-    out[(size_t)pr.j * ld + pr.i] = make_double2(re, im);
-    if (MIXED) out32[(size_t)pr.j * ld32 + pr.i] = make_float2((float)re, (float)im);
-  }
+  acc.reduce();
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (lane == i * NB + j && (NB == 1 || (i < pr.ni && j < pr.nj))) {
+        const int row = pr.i + i, col = pr.j + j;
+        double re = alpha * acc.re[i][j], im = alpha * acc.im[i][j];
+        if (pr.same && beta != 0.0) re = fma(beta, mass_entry(g, r, row, col), re);
+        out[(size_t)col * ld + row] = make_double2(re, im);
+        if (MIXED) out32[(size_t)col * ld32 + row] = make_float2((float)re, (float)im);
+      }
 }
 
 // Table capacities (entries per warp) of the near-field kernel for rules r.
@@ -284,13 +358,23 @@ static void near_caps(const DevRules& r, int* cap_s, int* cap_t) {
   *cap_t = std::max(r.nv2, r.nv3);
 }
 
-size_t near_table_bytes(const DevRules& r) {
+static size_t near_table_bytes(const DevRules& r, int nb) {
   int cs, ct;
   near_caps(r, &cs, &ct);
-  return sizeof(double) * 5 * (size_t)(cs + ct);
+  return sizeof(double) * (size_t)(nb > 1 ? 4 + kNearBasis : 5) * (cs + ct);
 }
 
-template <int KERNEL, bool MIXED, bool CK>
+static int near_sms() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v > 0 ? v : 1;
+  }();
+  return n;
+}
+
+template <int KERNEL, bool MIXED, bool CK, int NB>
 static void launch_near_k(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs,
                           double k, double ki, double eta, double alpha, double beta,
                           const float* tab,
@@ -298,64 +382,77 @@ static void launch_near_k(const DevGeom& g, const DevRules& r, const NearPair* p
                           cudaStream_t s) {
   int cs, ct;
   near_caps(r, &cs, &ct);
-  const size_t per_warp = std::max<size_t>(near_table_bytes(r), 8);  // L = 0: empty rules
-  // warps per block: up to 8, within 96 KB of shared memory
-  const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (96 * 1024 - 1024) / per_warp));
+  const size_t per_warp = std::max<size_t>(near_table_bytes(r, NB), 8);  // L = 0: empty rules
+  // warps per block: up to 8, within 96 KB of shared memory; fewer while the
+  // blocks would not give every SM eight of them (self and neighbour pairs
+  // differ in cost; kite N = 2048, FP64: 20.25 -> 19.9 ms of the whole solve).
+  // Two are enough in the mixed path, where every block copies the e^{ix} table
+  // (kite N = 2048: 414 us with 8 warps, 427 with 2).
+  int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (96 * 1024 - 1024) / per_warp));
+  while (wpb > 1 && (npairs + wpb - 1) / wpb < (MIXED ? 2 : 8) * near_sms()) wpb /= 2;
   const size_t smem = 1024 + per_warp * wpb;
   const int blocks = (npairs + wpb - 1) / wpb;
-  auto fn = near_kernel<KERNEL, MIXED, CK>;
+  auto fn = near_kernel<KERNEL, MIXED, CK, NB>;
+  // (one value for all rules: calls of several threads must not undo each other)
   if (smem > 48 * 1024)
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   fn<<<blocks, 32 * wpb, smem, s>>>(g, r, pairs, npairs, k, ki, eta, alpha, beta,
                                      make_kconst(k, eta), tab, cs, ct, out, ld, out32, ld32);
 }
 
-template <bool MIXED, bool CK>
+template <bool MIXED, bool CK, int NB>
 static void launch_near_m(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs,
                           int kernel, double k, double ki, double eta, double alpha, double beta,
                           const float* tab, double2* out, long long ld, float2* out32,
                           long long ld32, cudaStream_t s) {
   switch (kernel) {
     case BEM2D_KERNEL_SINGLE:
-      launch_near_k<BEM2D_KERNEL_SINGLE, MIXED, CK>(g, r, pairs, npairs, k, ki, eta, alpha,
+      launch_near_k<BEM2D_KERNEL_SINGLE, MIXED, CK, NB>(g, r, pairs, npairs, k, ki, eta, alpha,
                                                     beta, tab, out, ld, out32, ld32, s);
       break;
     case BEM2D_KERNEL_DOUBLE:
-      launch_near_k<BEM2D_KERNEL_DOUBLE, MIXED, CK>(g, r, pairs, npairs, k, ki, eta, alpha,
+      launch_near_k<BEM2D_KERNEL_DOUBLE, MIXED, CK, NB>(g, r, pairs, npairs, k, ki, eta, alpha,
                                                     beta, tab, out, ld, out32, ld32, s);
       break;
     case BEM2D_KERNEL_CONJDOUBLE:
-      launch_near_k<BEM2D_KERNEL_CONJDOUBLE, MIXED, CK>(g, r, pairs, npairs, k, ki, eta, alpha,
+      launch_near_k<BEM2D_KERNEL_CONJDOUBLE, MIXED, CK, NB>(g, r, pairs, npairs, k, ki, eta, alpha,
                                                         beta, tab, out, ld, out32, ld32, s);
       break;
     default:
-      launch_near_k<BEM2D_KERNEL_COMBINED, MIXED, CK>(g, r, pairs, npairs, k, ki, eta, alpha,
+      launch_near_k<BEM2D_KERNEL_COMBINED, MIXED, CK, NB>(g, r, pairs, npairs, k, ki, eta, alpha,
                                                       beta, tab, out, ld, out32, ld32, s);
   }
 }
 
-int launch_near(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs,
+int launch_near(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs, int nb,
                 int kernel, double k, double eta, double alpha, double beta, double2* out,
                 long long ld, cudaStream_t s, float2* out32, long long ld32) {
   if (npairs == 0) return BEM2D_OK;
-  if (out32) {
-    const float* tab = expi_table_dev();
-    if (!tab) return BEM2D_ERR_NOMEM;
-    launch_near_m<true, false>(g, r, pairs, npairs, kernel, k, 0.0, eta, alpha, beta, tab, out,
-                               ld, out32, ld32, s);
-  } else {
-    launch_near_m<false, false>(g, r, pairs, npairs, kernel, k, 0.0, eta, alpha, beta, nullptr,
-                                out, ld, nullptr, 0, s);
-  }
+  const float* tab = out32 ? expi_table_dev() : nullptr;
+  if (out32 && !tab) return BEM2D_ERR_NOMEM;
+  auto go = [&](auto mixed, auto n) {
+    launch_near_m<decltype(mixed)::value, false, decltype(n)::value>(
+        g, r, pairs, npairs, kernel, k, 0.0, eta, alpha, beta, tab, out, ld, out32, ld32, s);
+  };
+  using One = std::integral_constant<int, 1>;
+  using Run = std::integral_constant<int, kNearBasis>;
+  if (out32)
+    nb > 1 ? go(std::true_type{}, Run{}) : go(std::true_type{}, One{});
+  else
+    nb > 1 ? go(std::false_type{}, Run{}) : go(std::false_type{}, One{});
   return BEM2D_OK;
 }
 
-int launch_near_ck(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs,
+int launch_near_ck(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs, int nb,
                    int kernel, double k, double ki, double eta, double alpha, double beta,
                    double2* out, long long ld, cudaStream_t s) {
   if (npairs == 0) return BEM2D_OK;
-  launch_near_m<false, true>(g, r, pairs, npairs, kernel, k, ki, eta, alpha, beta, nullptr, out,
-                             ld, nullptr, 0, s);
+  if (nb > 1)
+    launch_near_m<false, true, kNearBasis>(g, r, pairs, npairs, kernel, k, ki, eta, alpha, beta,
+                                           nullptr, out, ld, nullptr, 0, s);
+  else
+    launch_near_m<false, true, 1>(g, r, pairs, npairs, kernel, k, ki, eta, alpha, beta, nullptr,
+                                  out, ld, nullptr, 0, s);
   return BEM2D_OK;
 }
 

@@ -367,13 +367,15 @@ static int check_geom(bem2d_ctx* c, const bem2d_geometry* g) {
 // Pairs that DiscreteKernel integrates with the graded rules
 // (lib/bem2d_quadrature.h:271-282): same element index -> IntegrateIdent,
 // else test next() == trial index -> AdaptedGauss3, else prev() -> AdaptedGauss2.
-static std::vector<NearPair> near_pairs(const bem2d_geometry* g) {
+// The items are runs of unknowns of one element: (first, count).
+static std::vector<NearPair> near_pairs(const bem2d_geometry* g, const std::vector<int2>& items) {
   std::unordered_map<long long, std::vector<int>> by_index;
-  for (int u = 0; u < g->n_unk; ++u) by_index[g->index[g->unk_elem[u]]].push_back(u);
+  const int n = (int)items.size();
+  for (int u = 0; u < n; ++u) by_index[g->index[g->unk_elem[items[u].x]]].push_back(u);
   std::vector<NearPair> out;
-  out.reserve((size_t)g->n_unk * 3);
-  for (int i = 0; i < g->n_unk; ++i) {
-    const int e = g->unk_elem[i];
+  out.reserve((size_t)n * 3);
+  for (int i = 0; i < n; ++i) {
+    const int e = g->unk_elem[items[i].x];
     const long long keys[3] = {g->index[e], g->next[e], g->prev[e]};
     const int rules[3] = {RULE_SELF, RULE_G3, RULE_G2};
     for (int k = 0; k < 3; ++k) {
@@ -381,7 +383,9 @@ static std::vector<NearPair> near_pairs(const bem2d_geometry* g) {
       if (k == 2 && keys[2] == keys[1]) continue;
       auto it = by_index.find(keys[k]);
       if (it == by_index.end()) continue;
-      for (int j : it->second) out.push_back(NearPair{i, j, rules[k], k == 0 ? 1 : 0});
+      for (int j : it->second)
+        out.push_back(NearPair{items[i].x, items[j].x, (short)items[i].y, (short)items[j].y,
+                               (short)rules[k], (short)(k == 0)});
     }
   }
   // Pair each (i, j, G3) with its reverse (j, i, G2) when that exists: one
@@ -410,10 +414,11 @@ static std::vector<NearPair> near_pairs(const bem2d_geometry* g) {
 // unknown, count); *nb: the longest (1: no table needed).
 static std::vector<int2> unknown_groups(const bem2d_geometry* g, int* nb) {
   std::vector<int2> out;
+  out.reserve(g->n_unk);
   *nb = 1;
   for (int u = 0; u < g->n_unk;) {
     int m = 1;
-    while (m < 3 && u + m < g->n_unk && g->unk_elem[u + m] == g->unk_elem[u]) ++m;
+    while (m < kNearBasis && u + m < g->n_unk && g->unk_elem[u + m] == g->unk_elem[u]) ++m;
     out.push_back(make_int2(u, m));
     *nb = std::max(*nb, m);
     u += m;
@@ -464,8 +469,17 @@ static int stage(bem2d_ctx* c, const bem2d_geometry* g, const bem2d_quad* q, boo
   dg.unk_kind = di + ne + nu;
   st->pairs = nullptr;
   st->npairs = 0;
+  // assembly takes runs of unknowns, the mass matrix single ones
+  std::vector<int2> groups;
+  if (pairs && nodes) {
+    groups = unknown_groups(g, &st->nb);
+    st->ngrp = (int)groups.size();
+  } else if (pairs) {
+    groups.reserve(nu);
+    for (int u = 0; u < nu; ++u) groups.push_back(make_int2(u, 1));
+  }
   if (pairs) {
-    const std::vector<NearPair> np = near_pairs(g);
+    const std::vector<NearPair> np = near_pairs(g, groups);
     st->npairs = (int)np.size();
     st->pairs = static_cast<NearPair*>(ws(c, "pairs", sizeof(NearPair) * np.size(), &rc));
     if (!st->pairs) return rc;
@@ -473,10 +487,7 @@ static int stage(bem2d_ctx* c, const bem2d_geometry* g, const bem2d_quad* q, boo
       CUDA_TRY(c, cudaMemcpyAsync(st->pairs, np.data(), sizeof(NearPair) * np.size(),
                                   cudaMemcpyHostToDevice, c->stream));
   }
-  std::vector<int2> groups;
   if (pairs && nodes) {
-    groups = unknown_groups(g, &st->nb);
-    st->ngrp = (int)groups.size();
     if (st->nb > 1) {
       int2* dgp = static_cast<int2*>(ws(c, "groups", sizeof(int2) * groups.size(), &rc));
       if (!dgp) return rc;
@@ -540,10 +551,10 @@ static int assemble_dev(bem2d_ctx* c, const Staged& st, int kernel, double k, do
   CHECK_LAUNCH(c);
   t = tic(c, BEM2D_PHASE_NEAR);
   if (ki != 0.0)
-    launch_near_ck(st.g, st.r, st.pairs, st.npairs, kernel, k, ki, eta, alpha, beta, A, ld,
+    launch_near_ck(st.g, st.r, st.pairs, st.npairs, st.nb, kernel, k, ki, eta, alpha, beta, A, ld,
                    c->stream);
   else
-    launch_near(st.g, st.r, st.pairs, st.npairs, kernel, k, eta, alpha, beta, A, ld, c->stream);
+    launch_near(st.g, st.r, st.pairs, st.npairs, st.nb, kernel, k, eta, alpha, beta, A, ld, c->stream);
   toc(c, t);
   if (st.npairs) ++c->launches;
   CHECK_LAUNCH(c);
@@ -579,7 +590,7 @@ static int assemble_mixed_dev(bem2d_ctx* c, const Staged& st, int kernel, double
   c->launches += 2;
   CHECK_LAUNCH(c);
   t = tic(c, BEM2D_PHASE_NEAR);
-  if (launch_near(st.g, st.r, st.pairs, st.npairs, kernel, k, eta, alpha, beta, A, ld,
+  if (launch_near(st.g, st.r, st.pairs, st.npairs, st.nb, kernel, k, eta, alpha, beta, A, ld,
                   c->stream, A32, ld32) != BEM2D_OK)
     return fail(c, BEM2D_ERR_NOMEM, "device table for the near-field kernel");
   toc(c, t);

@@ -288,10 +288,12 @@ __device__ __forceinline__ void kernel_c_pair(double kr, double ki, double eq, d
 enum NearRule : int { RULE_SELF = 0, RULE_G2 = 1, RULE_G3 = 2, RULE_G3_PAIR = 3 };
 
 struct NearPair {
-  int i;     // test unknown (row)
-  int j;     // trial unknown (column)
-  int rule;  // NearRule
-  int same;  // element indices equal (mass-matrix term applies)
+  int i;       // first test unknown (row)
+  int j;       // first trial unknown (column)
+  short ni;    // their counts: runs of unknowns of one element (up to kNearBasis)
+  short nj;
+  short rule;  // NearRule
+  short same;  // element indices equal (mass-matrix term applies)
 };
 
 // Quadrature rules on the device: Gauss nodes on [0,1] and the three
@@ -378,17 +380,17 @@ int launch_far_fp64(const DevGeom& g, const NodeTable& t, const int2* grp, int n
 size_t hankel_tab_bytes();
 // Near field (self and adjacent pairs).  out32 == nullptr: FP64 kernel
 // evaluation into out.  Otherwise the mixed-precision variant (float-float
-// Bessel functions) writes both out and out32.  Returns BEM2D_ERR_NOMEM if
+// Bessel functions) writes both out and out32.  nb: the largest count in the
+// pairs.  Returns BEM2D_ERR_NOMEM if
 // the device reduction table could not be made.
-int launch_near(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs,
+constexpr int kNearBasis = 3;
+int launch_near(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs, int nb,
                 int kernel, double k, double eta, double alpha, double beta, double2* out,
                 long long ld, cudaStream_t s, float2* out32 = nullptr, long long ld32 = 0);
 // FP64 near field with a complex wavenumber k + i ki.
-int launch_near_ck(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs,
+int launch_near_ck(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs, int nb,
                    int kernel, double k, double ki, double eta, double alpha, double beta,
                    double2* out, long long ld, cudaStream_t s);
-// Shared-memory bytes per warp of the near-field geometry tables for rules r.
-size_t near_table_bytes(const DevRules& r);
 void launch_ident(const DevGeom& g, const DevRules& r, const NearPair* pairs,
                   int npairs, double2* out, long long ld, cudaStream_t s);
 // ki: imaginary part of the wavenumber (0 for a real k).
