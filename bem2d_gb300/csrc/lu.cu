@@ -2149,12 +2149,15 @@ trisolve_cluster_kernel(const TS* __restrict__ LU, long long lda, int n,
 // x = U^{-1} L^{-1} P b.  Block b of 64 rows belongs to CTA b % C.  Whoever
 // holds y_k subtracts L[m, k] y_k from its blocks m > k; the owner of block k +
 // 1 takes that block first, forms y_{k+1} = L_{k+1,k+1}^{-1} b_{k+1} from the
-// stored inverse and sends it to every CTA before it turns to its other blocks.
-// Going back the same with U.  A step of the chain is then one 512-byte
-// message (asynchronous stores counted on the receiver's mbarrier; every block
-// has its own slot and mbarrier, used once in each direction: y_k has no reader
-// left when x_k is sent, since all later y depend on its readers), and two
-// products of 64 x 64, whose matrices are loaded a step ahead.  Thread (row r,
+// stored inverse and sends it to the CTAs with a block after it before it turns
+// to its other blocks.  Going back the same with U, to every CTA.  A step of the
+// chain is then one 512-byte message (asynchronous stores counted on the
+// receiver's mbarrier; every block has its own slot and mbarrier) and two
+// products of 64 x 64, whose matrices are loaded a step ahead.  x_k takes the
+// slot and the next phase of y_k: whoever was sent y_k has a block m > k, x_k
+// depends on y_m, and that left only after all of y_k had arrived and been
+// read.  A CTA without a later block is not sent y_k (nothing would order that
+// message before x_k); x_k is the first phase of its mbarrier.  Thread (row r,
 // quarter g) = lane 4 (r % 8) + g of warp r / 8 takes the columns 8 u + 2 g, + 1.
 // Bound by that chain: 2048 rows take 100 us; with contiguous rows per CTA and a
 // cluster barrier in every step 270 us.  The FP64 solve keeps that scheme: there
@@ -2200,12 +2203,16 @@ trisolve64_kernel(const float2* __restrict__ LU, long long lda, int n,
   // the first
   unsigned ya[4], ma[4];
   bool to[4];
+  int lastq[4];
+  auto last_own = [&](int q) { return nk - 1 - (nk - 1 - q) % C; };  // last block of CTA q
+  const int last = last_own(rank);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int d = (i & 1) ? C - 1 - (g + 4 * (i >> 1)) : 1 + g + 4 * (i >> 1);
     // forward distances 1..8 (i = 0, 2), backward ones C-1..C-8 (i = 1, 3), each rank once
     to[i] = d >= 1 && d < C && ((i & 1) ? d > 8 : d <= 8);
     const int q = (rank + (to[i] ? d : 0)) % C;
+    lastq[i] = last_own(q);
     ya[i] = tc::map_rank(ys + r, q);
     ma[i] = tc::map_rank(mb, q);
   }
@@ -2252,7 +2259,7 @@ trisolve64_kernel(const float2* __restrict__ LU, long long lda, int n,
       const unsigned yo = (unsigned)k * kBytes, mo = (unsigned)k * 8u;
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (to[i]) tc::store_async8(ya[i] + yo, y, ma[i] + mo);
+        if (to[i] && (dir || k < lastq[i])) tc::store_async8(ya[i] + yo, y, ma[i] + mo);
       if (g == 0) {
         ys[(size_t)k * kNB + r] = y;
         if (dir && k * kNB + r < n) xout[(size_t)k * kNB + r] = y;
@@ -2283,12 +2290,13 @@ trisolve64_kernel(const float2* __restrict__ LU, long long lda, int n,
     }
     if (inside(mn)) lblock(p, mn, kfirst);
     if (inside(mn + st * C)) lblock(o, mn + st * C, kfirst);
-    for (int s = 0; s < nk - 1; ++s) {
+    const int steps = dir ? nk - 1 : last;  // forward up to the last own block
+    for (int s = 0; s < steps; ++s) {
       const int k = kfirst + st * s;
       if (k % C == rank) {
         __syncthreads();  // this CTA's y_k
       } else {
-        ok = tc::mbar_wait_cluster(&mb[k], (unsigned)dir, &s_abort) && ok;
+        ok = tc::mbar_wait_cluster(&mb[k], dir && k < last ? 1u : 0u, &s_abort) && ok;
         if (!dir && t == 0) tc::mbar_expect_tx(&mb[k], kBytes);  // x_k, on the way back
       }
       const float2* yk = ys + (size_t)k * kNB;
@@ -2309,7 +2317,7 @@ trisolve64_kernel(const float2* __restrict__ LU, long long lda, int n,
         mn = next_own(m0);
         if (inside(mn)) dblock(d, mn);
       }
-      const bool more = s + 1 < nk - 1;
+      const bool more = s + 1 < steps;
       if (more && inside(mn)) lblock(p, mn, k + st);
       // the others, the second own block from o
       auto sub = [&](const float2 (&l)[16], int m) {
@@ -2329,14 +2337,9 @@ trisolve64_kernel(const float2* __restrict__ LU, long long lda, int n,
         sub(l, m);
       }
     }
-    // the last block of the direction has no readers there, but its message
-    // completes the phase before the barrier's next use
-    const int kl = dir ? 0 : nk - 1;
-    if (kl % C != rank) {
-      ok = tc::mbar_wait_cluster(&mb[kl], (unsigned)dir, &s_abort) && ok;
-      if (!dir && t == 0) tc::mbar_expect_tx(&mb[kl], kBytes);
-    }
   }
+  // x_0 has no readers, but must arrive before this CTA's shared memory goes
+  if (rank != 0) ok = tc::mbar_wait_cluster(&mb[0], last > 0 ? 1u : 0u, &s_abort) && ok;
   if (!ok) atomicExch(status, 1);
   cl.sync();  // no CTA leaves while another may still write its shared memory
 }
