@@ -2207,8 +2207,7 @@ int bem2d_debug_oz_update(bem2d_ctx* c, int M, int N, int K, void* C, int64_t ld
   if (!pack || !st) return rc;
   CUDA_TRY(c, cudaMemsetAsync(st, 0, sizeof(int), c->stream));
   if ((rc = launch_oz_zgemm(static_cast<double2*>(C), ldc, static_cast<const double2*>(A), lda,
-                            static_cast<const double2*>(B), ldb, M, N, K, 1, -1.0, nullptr, 0,
-                            pack, pb, st, c->stream, &c->launches)))
+                            static_cast<const double2*>(B), ldb, M, N, K, 1, -1.0, pack, pb, st, c->stream, &c->launches)))
     return fail(c, rc, "tensor-core update launch: %s", cudaGetErrorString(cudaGetLastError()));
   int h = 0;
   CUDA_TRY(c, cudaMemcpyAsync(&h, st, sizeof(int), cudaMemcpyDeviceToHost, c->stream));

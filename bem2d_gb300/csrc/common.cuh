@@ -522,14 +522,12 @@ int launch_tc_step(float2* A, long long lda, int M, int k0, int nb, int cl, int 
                    int max_ctas, int passes);
 
 // C = beta C + sign A B (complex128, column-major; C is M x N, A M x K, B K x
-// N; beta 0 or 1) on the tensor cores, FP64 accurate (lu_oz.cu).  piv (null:
-// none): entries (k, k) whose exponents scale inner index k.  pack:
+// N; beta 0 or 1) on the tensor cores, FP64 accurate (lu_oz.cu).  pack:
 // oz_pack_bytes(M, N) bytes.  Sets *status on a device-side wait timeout.
 size_t oz_pack_bytes(int M, int N);
 int launch_oz_zgemm(double2* C, long long ldc, const double2* A, long long lda, const double2* B,
-                    long long ldb, int M, int N, int K, int beta, double sign,
-                    const double2* piv, long long ldp, void* pack, size_t pack_bytes, int* status,
-                    cudaStream_t s, long long* launches);
+                    long long ldb, int M, int N, int K, int beta, double sign, void* pack,
+                    size_t pack_bytes, int* status, cudaStream_t s, long long* launches);
 
 // Complex128 panel of at most 64 columns (lu_zpanel.cu): columns [k0, k0 + nb)
 // of rows k0 .. n, interchanges on these columns only.  1: not possible here

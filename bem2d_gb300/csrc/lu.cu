@@ -1758,10 +1758,9 @@ static int update_sub(T* C, const T* Am, const T* Bm, long long ld, int M, int N
                       const LuWork& w, cudaStream_t s, long long* launches) {
   if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
   if constexpr (sizeof(T) == sizeof(double2)) {
-    // Am holds L: its diagonal block's pivots sit K rows above it in A
     if (w.pack && oz_pack_bytes(M, N) <= w.pack_bytes)
-      return launch_oz_zgemm(C, ld, Am, ld, Bm, ld, M, N, K, 1, -1.0, Am - K, ld, w.pack,
-                             w.pack_bytes, w.status, s, launches);
+      return launch_oz_zgemm(C, ld, Am, ld, Bm, ld, M, N, K, 1, -1.0, w.pack, w.pack_bytes,
+                             w.status, s, launches);
   }
   if constexpr (sizeof(T) == sizeof(float2)) {
     // tall and narrow updates (the columns inside an outer block), and short

@@ -17,13 +17,27 @@
 // collects the pairs of one order s + t (at most 8) over K = 64: at most 2^23,
 // exact in the FP32 accumulator.  Kept are the 36 pairs with s + t <= 7; what
 // is dropped is below 2^-52 of (largest entry of the row) x (largest of the
-// column) in the worst case and 2^-59 typically, where an FP64 sum of 64
-// products rounds at about 2^-51.  An entry's 53 bits survive whole while it
-// is within 2^-10 of its row's largest.
+// column) in the worst case and 2^-60 typically, where an FP64 sum of 64
+// products rounds at about 2^-51 of its largest.  An entry's 53 bits survive
+// whole while it is within 2^-10 of its row's largest.
 //
-// To keep rows and columns of very different size apart (graded meshes) the
-// LU scales inner index k by the pivot's exponent: A(:, k) 2^p_k, B(k, :)
-// 2^-p_k, so A is read as it was before the division by the pivot.
+// Rows and columns of very different size (graded meshes, unknowns in different
+// units) must not meet in that bound:
+//  - inner index k is scaled by the largest exponent of A(:, k) (colscale.cuh),
+//    which makes the digits independent of powers of two on the rows and
+//    columns of the matrix being factored.  (Scaled by the pivot's exponent, as
+//    if A were read before the division by the pivot, columns of a system 2^60
+//    apart left no correct digit in its solution.)
+//  - an entry of the product whose 64 terms are all below 2^-kOzSpan of (row's
+//    largest) x (column's largest) is summed in FP64 by the epilogue.  The pack
+//    kernel marks rows and columns whose own entries span more than that; where
+//    both are marked the terms' exponents are compared.  Disk, kite and random
+//    systems have no such entries, squares and L-shapes graded over 8 levels 1
+//    to 2 % of them in the updates behind a corner's panel.  Scales, marks and
+//    comparisons together cost nothing that can be measured (disk N = 160 1.132
+//    -> 1.127 ms, kite N = 2048 20.31 -> 20.33, N = 3001 21.1 -> 20.9, with one
+//    pack kernel for both operands instead of two), the sums 9 % of the solve
+//    on a graded square.
 //
 // Complex arithmetic as in lu_tc.cu: A' (rows 2i, 2i + 1 = re, im of row i)
 // times [B_r B_i]; re C_i = D1[2i] - D2[2i+1], im C_i = D2[2i] + D1[2i+1].
@@ -53,6 +67,7 @@
 
 #include <algorithm>
 
+#include "colscale.cuh"
 #include "common.cuh"
 #include "oz.cuh"
 
@@ -79,27 +94,55 @@ constexpr int kOzBBytes = kOzKSteps * kOzBStep;    // 32 KB
 constexpr int kOzBarOff = kOzABytes + kOzStages * kOzBBytes;  // 192 KB
 constexpr int kOzSmem = kOzBarOff + 256;
 constexpr unsigned kOzAcc = 2 * kOzBN * kOzS;      // 256 TMEM columns
+// exponents that a row's or column's entries, or an entry's terms, may span
+constexpr int kOzSpan = 10;
 
 // ---- packing -------------------------------------------------------------------
-// Exponent p_k of inner index k: that of the pivot, entry k of column k of
-// the factored block at piv (null: 0).
-__device__ __forceinline__ int oz_shift(const double2* piv, long long ldp, int k, int K) {
-  if (!piv || k >= K) return 0;
-  const double2 p = piv[(size_t)k * ldp + k];
-  const int f = max(expo(p.x), expo(p.y));
-  return f > 0 && f < 2047 ? f - 1023 : 0;
+// A row's or column's scale exponent er and whether its entries span more than
+// kOzSpan (a zero entry does), from the largest and smallest exponents.
+__device__ __forceinline__ int oz_scale_word(int er, int emin) {
+  const bool wide = er > kZero && er < kNaN && emin < er - kOzSpan;
+  return 2 * er + (wide ? 1 : 0);
 }
 
-// A (M x K) -> per row block of 64: [K-step][digit][128 x 16]; ea[i]: the
-// row's scale exponent.  Eight threads per complex row, thread c takes k = 8 c
-// .. 8 c + 7.
-__global__ void __launch_bounds__(512)
-oz_pack_a_kernel(const double2* __restrict__ A, long long lda, int M, int K, int ksteps,
-                 const double2* __restrict__ piv, long long ldp, unsigned char* __restrict__ Apk,
-                 int* __restrict__ ea) {
-  __shared__ int pk[kOzK], red[8][kOzBM];
+// Packs both operands; CTAs [0, mt) take a row block of A each, the others four
+// column blocks of B.
+//   A (M x K) -> per row block of 64: [K-step][digit][128 x 16]; ea[i]: the row's
+//   scale word.  Eight threads per complex row, thread c takes k = 8 c .. 8 c + 7.
+//   B (K x N) -> per block of 16 columns: [K-step][digit][32 x 16], rows 0..15 re
+//   and 16..31 im of the columns; eb[j].  Eight threads per column.
+// part, np: the columns' exponents (colscale.cuh), added to inner index k in A
+// and subtracted in B.
+// xa[i], xb[j]: the 64 exponents with their shifts as 16-bit integers (kOzNone:
+// zero), for oz_apart.
+constexpr int kOzPackThreads = 512;
+constexpr int kOzNone = -16000;  // two of them still fit 16 bits
+struct OzPack {
+  unsigned char *A, *B;  // digits
+  int *ea, *eb;          // scale words
+  uint4 *xa, *xb;        // exponents, kOzK of them per row / column
+  int* part;             // kOzK * kColParts partial maxima
+};
+
+__device__ __forceinline__ int oz_field(double2 v, int p) {
+  const int e = max(expo(v.x), expo(v.y));
+  return e == 0 ? kOzNone : e == 2047 ? kNaN : e + p;
+}
+
+__device__ __forceinline__ uint4 oz_pack_fields(const int (&x)[8]) {
+  unsigned w[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int a = min(max(x[2 * q], kOzNone), -kOzNone), b = min(max(x[2 * q + 1], kOzNone), -kOzNone);
+    w[q] = ((unsigned)a & 0xffffu) | ((unsigned)b << 16);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+__device__ __forceinline__ void oz_pack_a(const double2* __restrict__ A, long long lda, int M,
+                                          int K, int ksteps, const int* pk, int (*red)[kOzBM],
+                                          int (*low)[kOzBM], const OzPack& o) {
   const int il = threadIdx.x & 63, c = threadIdx.x >> 6, i = blockIdx.x * kOzBM + il;
-  if (threadIdx.x < kOzK) pk[threadIdx.x] = oz_shift(piv, ldp, threadIdx.x, K);
   double2 v[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
@@ -107,74 +150,101 @@ oz_pack_a_kernel(const double2* __restrict__ A, long long lda, int M, int K, int
     v[q] = i < M && k < K ? A[(size_t)k * lda + i] : make_double2(0.0, 0.0);
   }
   __syncthreads();
-  int emax = -10000;
+  int emax = -10000, emin = 100000, x[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
-    const int e = max(expo(v[q].x), expo(v[q].y));
-    if (e > 0) emax = max(emax, e == 2047 ? kNaN : e + pk[8 * c + q]);
+    x[q] = oz_field(v[q], pk[8 * c + q]);
+    emax = max(emax, x[q]);
+    if (8 * c + q < K) emin = min(emin, x[q]);
   }
+  if (i < M) o.xa[(size_t)i * 8 + c] = oz_pack_fields(x);
   red[c][il] = emax;
+  low[c][il] = emin;
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < 8; ++q) emax = max(emax, red[q][il]);
+  for (int q = 0; q < 8; ++q) {
+    emax = max(emax, red[q][il]);
+    emin = min(emin, low[q][il]);
+  }
   const int er = scale_of(emax);
-  if (c == 0 && i < M) ea[i] = er;
+  if (c == 0 && i < M) o.ea[i] = oz_scale_word(er, emin);
   if (c >= 2 * ksteps) return;
   const bool use = er > kZero && er < kNaN;
-  unsigned char* blk = Apk + ((size_t)blockIdx.x * ksteps + (c >> 1)) * kOzAStep;
+  unsigned char* blk = o.A + ((size_t)blockIdx.x * ksteps + (c >> 1)) * kOzAStep;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     long long f[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q)
       f[q] = fixed<kOzS>(!use ? 0.0 : h ? v[q].y : v[q].x, pk[8 * c + q], er);
-    Digits<kOzS> o;
-    digits<kOzS>(f, &o);
+    Digits<kOzS> d;
+    digits<kOzS>(f, &d);
 #pragma unroll
     for (int s = 0; s < kOzS; ++s)
       *reinterpret_cast<uint4*>(blk + s * kOzABlk + off(2 * il + h, c & 1)) =
-          make_uint4(o.w[s][0], o.w[s][1], o.w[s][2], o.w[s][3]);
+          make_uint4(d.w[s][0], d.w[s][1], d.w[s][2], d.w[s][3]);
   }
 }
 
-// B (K x N) -> per block of 16 columns: [K-step][digit][32 x 16], rows 0..15
-// re and 16..31 im of the columns.  Eight threads per column, thread c takes
-// k = 8 c .. 8 c + 7.
-__global__ void __launch_bounds__(128)
-oz_pack_b_kernel(const double2* __restrict__ B, long long ldb, int K, int N, int ksteps,
-                 const double2* __restrict__ piv, long long ldp, unsigned char* __restrict__ Bpk,
-                 int* __restrict__ eb) {
-  const int c = threadIdx.x & 7, jl = threadIdx.x >> 3, j = blockIdx.x * kOzBN + jl;
+__device__ __forceinline__ void oz_pack_b(const double2* __restrict__ B, long long ldb, int K,
+                                          int N, int ksteps, int nt, const int* pk,
+                                          const OzPack& o) {
+  const int c = threadIdx.x & 7, jl = threadIdx.x >> 3, j = nt * kOzBN + jl;
   double2 v[8];
-  int pk[8];
-  int emax = -10000;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int k = 8 * c + q;
     v[q] = (j < N && k < K) ? B[(size_t)j * ldb + k] : make_double2(0.0, 0.0);
-    pk[q] = -oz_shift(piv, ldp, k, K);
-    const int e = max(expo(v[q].x), expo(v[q].y));
-    if (e > 0) emax = max(emax, e == 2047 ? kNaN : e + pk[q]);
   }
+  __syncthreads();
+  int emax = -10000, emin = 100000, x[8];
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+  for (int q = 0; q < 8; ++q) {
+    x[q] = oz_field(v[q], -pk[8 * c + q]);
+    emax = max(emax, x[q]);
+    if (8 * c + q < K) emin = min(emin, x[q]);
+  }
+  if (j < N) o.xb[(size_t)j * 8 + c] = oz_pack_fields(x);
+#pragma unroll
+  for (int l = 4; l > 0; l >>= 1) {
+    emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, l));
+    emin = min(emin, __shfl_xor_sync(0xffffffffu, emin, l));
+  }
   const int er = scale_of(emax);
-  if (c == 0 && j < N) eb[j] = er;
-  if (c >= 2 * ksteps) return;
+  if (c == 0 && j < N) o.eb[j] = oz_scale_word(er, emin);
+  // blocks of 16 columns lie one after another: block nt + jl / 16, column jl % 16
+  if (c >= 2 * ksteps || j >= (N + kOzBN - 1) / kOzBN * kOzBN) return;
   const bool use = er > kZero && er < kNaN;
-  unsigned char* blk = Bpk + ((size_t)blockIdx.x * ksteps + (c >> 1)) * kOzBStep;
+  unsigned char* blk =
+      o.B + ((size_t)(nt + (jl >> 4)) * ksteps + (c >> 1)) * kOzBStep;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     long long f[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) f[q] = fixed<kOzS>(!use ? 0.0 : h ? v[q].y : v[q].x, pk[q], er);
-    Digits<kOzS> o;
-    digits<kOzS>(f, &o);
+    for (int q = 0; q < 8; ++q)
+      f[q] = fixed<kOzS>(!use ? 0.0 : h ? v[q].y : v[q].x, -pk[8 * c + q], er);
+    Digits<kOzS> d;
+    digits<kOzS>(f, &d);
 #pragma unroll
     for (int s = 0; s < kOzS; ++s)
-      *reinterpret_cast<uint4*>(blk + s * kOzBBlk + off(h * kOzBN + jl, c & 1)) =
-          make_uint4(o.w[s][0], o.w[s][1], o.w[s][2], o.w[s][3]);
+      *reinterpret_cast<uint4*>(blk + s * kOzBBlk + off(h * kOzBN + (jl & 15), c & 1)) =
+          make_uint4(d.w[s][0], d.w[s][1], d.w[s][2], d.w[s][3]);
   }
+}
+
+__global__ void __launch_bounds__(kOzPackThreads)
+oz_pack_kernel(const double2* __restrict__ A, long long lda, const double2* __restrict__ B,
+               long long ldb, int M, int N, int K, int ksteps, int mt,
+               int np, OzPack o) {
+  __shared__ int pk[kOzK], red[8][kOzBM], low[8][kOzBM];
+  if (threadIdx.x < kOzK) {
+    const int e = (int)threadIdx.x < K ? col_expo_max(o.part, np, K, threadIdx.x) : 0;
+    pk[threadIdx.x] = e > 0 ? 1023 - e : 0;
+  }
+  if ((int)blockIdx.x < mt)  // (the barrier that pk needs stands behind their loads)
+    oz_pack_a(A, lda, M, K, ksteps, pk, red, low, o);
+  else
+    oz_pack_b(B, ldb, K, N, ksteps, 4 * (blockIdx.x - mt), pk, o);
 }
 
 // ---- the product -----------------------------------------------------------------
@@ -189,12 +259,80 @@ __device__ __forceinline__ double oz_to_double(long long v) {
   return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
 }
 
-// C[M x N] = beta C + sign A B, beta 0 or 1, sign +-1.  grid: min(tiles, SMs).
+// A whole warp, lanes 2 r and 2 r + 1 on the real and imaginary part of a row's
+// eight entries (a: the row of A, k-th entry at a + k lda; er: its scale
+// exponent; c: the lane's component of column u at c + u cstep).  Of the lane's
+// columns in `cols` (eb[u], xb[8 u], k-th entry at b + u ldb + k) those whose sum
+// has all of its terms more than kOzSpan exponents below the scale exponents of
+// its row and column are finished here in FP64 and returned.
+//   The largest of 64 sums of two exponents is 32 add-maximum instructions on
+// pairs of 16-bit integers.  A sum takes the 32 lanes two terms each: 13 FP64
+// instructions of the warp; such entries come a row or two at a time, and the
+// lanes on their own would spend 128 on them (graded square N = 2064, combined
+// operator: solve 11.9 ms without these sums, 15.4 by lanes, 13.0 by warps).
+__device__ __noinline__ unsigned oz_apart(unsigned cols, int er, const int* __restrict__ eb,
+                                          const uint4* __restrict__ xa,
+                                          const uint4* __restrict__ xb,
+                                          const double2* __restrict__ a, long long lda,
+                                          const double2* __restrict__ b, long long ldb, int K,
+                                          double* c, long long cstep, int beta, double sign) {
+  const int lane = threadIdx.x & 31;
+  unsigned done = 0u;
+  if (cols) {
+    uint4 x[kOzK / 8];
+#pragma unroll
+    for (int q = 0; q < kOzK / 8; ++q) x[q] = __ldg(xa + q);
+    for (unsigned rest = cols; rest; rest &= rest - 1) {
+      const int u = __ffs(rest) - 1;
+      unsigned z = 0x80008000u;
+#pragma unroll
+      for (int q = 0; q < kOzK / 8; ++q) {
+        const uint4 y = __ldg(xb + 8 * u + q);
+        z = __viaddmax_s16x2(x[q].x, y.x, z);
+        z = __viaddmax_s16x2(x[q].y, y.y, z);
+        z = __viaddmax_s16x2(x[q].z, y.z, z);
+        z = __viaddmax_s16x2(x[q].w, y.w, z);
+      }
+      const int top = max((int)(short)(z & 0xffffu), (int)(short)(z >> 16));
+      if (top < er + (eb[u] >> 1) - kOzSpan) done |= 1u << u;
+    }
+  }
+  __syncwarp();
+  for (unsigned any = __reduce_or_sync(0xffffffffu, done); any; any &= any - 1) {
+    const int u = __ffs(any) - 1;
+    const double2* bu = b + (size_t)u * ldb;
+    for (unsigned rows = __ballot_sync(0xffffffffu, (done >> u) & 1u) & 0x55555555u; rows;
+         rows &= rows - 1) {
+      const int l = __ffs(rows) - 1;
+      const double2* al = a + ((l >> 1) - (lane >> 1));
+      double sr = 0.0, si = 0.0;
+#pragma unroll
+      for (int k = lane; k < kOzK; k += 32) {
+        if (k >= K) break;
+        const double2 x = al[(size_t)k * lda], y = bu[k];
+        sr = fma(x.x, y.x, fma(-x.y, y.y, sr));
+        si = fma(x.x, y.y, fma(x.y, y.x, si));
+      }
+      // real parts to lanes 0-15, imaginary ones to lanes 16-31
+      const bool up = lane & 16;
+      double s = (up ? si : sr) + __shfl_xor_sync(0xffffffffu, up ? sr : si, 16);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const double re = __shfl_sync(0xffffffffu, s, 0), im = __shfl_sync(0xffffffffu, s, 16);
+      if ((lane & ~1) == l)
+        c[u * cstep] = fma(sign, lane & 1 ? im : re, beta ? c[u * cstep] : 0.0);
+    }
+  }
+  return done;
+}
+
+// C[M x N] = beta C + sign A B, beta 0 or 1, sign +-1, from the packed operands
+// (A, M x K, and B, K x N, themselves only for oz_apart).  grid: min(tiles,
+// SMs).
 __global__ void __launch_bounds__(kOzThreads, 1)
-oz_zgemm_kernel(double2* __restrict__ C, long long ldc, const unsigned char* __restrict__ Apk,
-                const unsigned char* __restrict__ Bpk, const int* __restrict__ ea,
-                const int* __restrict__ eb, int M, int N, int ksteps, int ntiles, int tiles,
-                int beta, double sign, int* status) {
+oz_zgemm_kernel(double2* __restrict__ C, long long ldc, OzPack o, const double2* __restrict__ A,
+                long long lda, const double2* __restrict__ B, long long ldb, int M, int N, int K,
+                int ksteps, int ntiles, int tiles, int beta, double sign, int* status) {
   extern __shared__ __align__(1024) unsigned char sm[];
   unsigned long long* full = reinterpret_cast<unsigned long long*>(sm + kOzBarOff);
   unsigned long long* empty = full + kOzStages;
@@ -246,7 +384,7 @@ oz_zgemm_kernel(double2* __restrict__ C, long long ldc, const unsigned char* __r
           }
           mbar_expect_tx(afull, abytes);
           for (int k = 0; k < ksteps; ++k)
-            bulk_copy(sm + k * kOzAStep, Apk + (size_t)mt * abytes + (size_t)k * kOzAStep,
+            bulk_copy(sm + k * kOzAStep, o.A + (size_t)mt * abytes + (size_t)k * kOzAStep,
                       kOzAStep, afull);
           ++na;
           mt_prev = mt;
@@ -257,7 +395,7 @@ oz_zgemm_kernel(double2* __restrict__ C, long long ldc, const unsigned char* __r
           break;
         }
         mbar_expect_tx(&full[s], bbytes);
-        bulk_copy(sm + kOzABytes + s * kOzBBytes, Bpk + (size_t)nt * bbytes, bbytes, &full[s]);
+        bulk_copy(sm + kOzABytes + s * kOzBBytes, o.B + (size_t)nt * bbytes, bbytes, &full[s]);
       }
       if (!ok) {
         *s_abort = 1;
@@ -315,19 +453,26 @@ oz_zgemm_kernel(double2* __restrict__ C, long long ldc, const unsigned char* __r
     for (int tile = t0; tile < t1; ++tile, ++j) {
       const int mt = tile / ntiles, nt = tile - mt * ntiles;
       const int i = mt * kOzBM + (tl >> 1), n0 = nt * kOzBN + part * 8;
-      const int er = i < M ? __ldg(&ea[i]) : kZero;
+      const int ew = i < M ? __ldg(&o.ea[i]) : 2 * kZero, er = ew >> 1;
       const int nlim = i < M ? min(8, N - n0) : 0;
       double* pc = Cf + 2 * ((size_t)n0 * ldc + i) + cc;
       const long long cstep = 2 * ldc;
       double cv[8];
       int ec[8];
+      unsigned apart = 0u;  // marked columns, if the row is marked
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         cv[u] = u < nlim && beta ? pc[u * cstep] : 0.0;
-        ec[u] = n0 + u < N ? __ldg(&eb[n0 + u]) : kZero;
+        const int cw = n0 + u < N ? __ldg(&o.eb[n0 + u]) : 2 * kZero;
+        ec[u] = cw >> 1;
+        apart |= (unsigned)(ew & cw & 1) << u;
       }
+      if (__any_sync(0xffffffffu, apart != 0u))
+        apart = oz_apart(apart, er, o.eb + n0, o.xa + (size_t)i * 8, o.xb + (size_t)n0 * 8, A + i,
+                         lda, B + (size_t)n0 * ldb, ldb, K, pc, cstep, beta, sign);
       const int a = j & 1;
-      if (!mbar_wait(&acc_full[a], (unsigned)(j >> 1) & 1u, s_abort)) {
+      // (all lanes of a warp give up together: the rest of the loop needs them all)
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[a], (unsigned)(j >> 1) & 1u, s_abort))) {
         ok = false;
         break;
       }
@@ -376,7 +521,7 @@ oz_zgemm_kernel(double2* __restrict__ C, long long ldc, const unsigned char* __r
         } else {
           v = e < -3000 ? cv[u] : cv[u] + sign * ldexp(hi[u], e);
         }
-        pc[u * cstep] = v;
+        if (!((apart >> u) & 1u)) pc[u * cstep] = v;
       }
     }
     if (!ok) *s_abort = 1;
@@ -403,35 +548,51 @@ int oz_sms() {
 
 }  // namespace
 
-size_t oz_pack_bytes(int M, int N) {
+// The pack buffer's parts for an M x N product; returns its bytes.
+static size_t oz_parts(void* pack, int M, int N, OzPack* o) {
   const size_t mt = (size_t)(M + kOzBM - 1) / kOzBM, nt = (size_t)(N + kOzBN - 1) / kOzBN;
-  return up256(mt * kOzABytes) + up256(nt * kOzBBytes) + up256(sizeof(int) * (size_t)M) +
-         up256(sizeof(int) * (size_t)N);
+  char* p = static_cast<char*>(pack);
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    char* r = p ? p + at : nullptr;
+    at += up256(bytes);
+    return r;
+  };
+  o->A = reinterpret_cast<unsigned char*>(take(mt * kOzABytes));
+  o->B = reinterpret_cast<unsigned char*>(take(nt * kOzBBytes));
+  o->ea = reinterpret_cast<int*>(take(sizeof(int) * (size_t)M));
+  o->eb = reinterpret_cast<int*>(take(sizeof(int) * (size_t)N));
+  o->xa = reinterpret_cast<uint4*>(take(sizeof(uint4) * 8 * (size_t)M));
+  o->xb = reinterpret_cast<uint4*>(take(sizeof(uint4) * 8 * (size_t)N));
+  o->part = reinterpret_cast<int*>(take(sizeof(int) * kOzK * kColParts));
+  return at;
+}
+
+size_t oz_pack_bytes(int M, int N) {
+  OzPack o;
+  return oz_parts(nullptr, M, N, &o);
 }
 
 int launch_oz_zgemm(double2* C, long long ldc, const double2* A, long long lda, const double2* B,
-                    long long ldb, int M, int N, int K, int beta, double sign,
-                    const double2* piv, long long ldp, void* pack, size_t pack_bytes, int* status,
-                    cudaStream_t s, long long* launches) {
+                    long long ldb, int M, int N, int K, int beta, double sign, void* pack,
+                    size_t pack_bytes, int* status, cudaStream_t s, long long* launches) {
   static const cudaError_t attr = cudaFuncSetAttribute(
       oz_zgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOzSmem);
   if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
   if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
-  if (!pack || oz_pack_bytes(M, N) > pack_bytes) return BEM2D_ERR_ARG;
+  OzPack o;
+  if (!pack || oz_parts(pack, M, N, &o) > pack_bytes) return BEM2D_ERR_ARG;
   const int mt = (M + kOzBM - 1) / kOzBM, nt = (N + kOzBN - 1) / kOzBN;
-  unsigned char* Apk = static_cast<unsigned char*>(pack);
-  unsigned char* Bpk = Apk + up256((size_t)mt * kOzABytes);
-  int* ea = reinterpret_cast<int*>(Bpk + up256((size_t)nt * kOzBBytes));
-  int* eb = reinterpret_cast<int*>(reinterpret_cast<char*>(ea) + up256(sizeof(int) * (size_t)M));
   const int grid = std::min(mt * nt, oz_sms());
   for (int k = 0; k < K; k += kOzK) {
     const int kk = std::min(kOzK, K - k), ksteps = (kk + 15) / 16;
-    const double2* pv = piv ? piv + (size_t)k * ldp + k : nullptr;
-    oz_pack_a_kernel<<<mt, 8 * kOzBM, 0, s>>>(A + (size_t)k * lda, lda, M, kk, ksteps, pv, ldp, Apk,
-                                          ea);
-    oz_pack_b_kernel<<<nt, 128, 0, s>>>(B + k, ldb, kk, N, ksteps, pv, ldp, Bpk, eb);
-    oz_zgemm_kernel<<<grid, kOzThreads, kOzSmem, s>>>(C, ldc, Apk, Bpk, ea, eb, M, N, ksteps, nt,
-                                                      mt * nt, k == 0 ? beta : 1, sign, status);
+    const double2* a = A + (size_t)k * lda;
+    const double2* b = B + k;
+    const int np = launch_col_expo(a, lda, M, kk, o.part, s);
+    oz_pack_kernel<<<mt + (nt + 3) / 4, kOzPackThreads, 0, s>>>(a, lda, b, ldb, M, N, kk, ksteps,
+                                                               mt, np, o);
+    oz_zgemm_kernel<<<grid, kOzThreads, kOzSmem, s>>>(C, ldc, o, a, lda, b, ldb, M, N, kk, ksteps,
+                                                      nt, mt * nt, k == 0 ? beta : 1, sign, status);
     *launches += 3;
   }
   return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
