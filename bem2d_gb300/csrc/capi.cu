@@ -2234,7 +2234,7 @@ int bem2d_debug_tc_update(bem2d_ctx* c, int M, int N, int K, void* C, int64_t ld
                                 static_cast<const float2*>(B), ldb, M, N, K, pack, pb, st,
                                 c->stream)))
     return fail(c, rc, "tensor-core update launch: %s", cudaGetErrorString(cudaGetLastError()));
-  c->launches += 2;
+  c->launches += 3;
   int h = 0;
   CUDA_TRY(c, cudaMemcpyAsync(&h, st, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));

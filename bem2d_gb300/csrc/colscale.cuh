@@ -24,16 +24,15 @@ __device__ __forceinline__ int col_expo(float x) {
   return e == 255 ? 0 : e;
 }
 
-// part[p K + k]: largest exponent field in column k (blockIdx.x, K of them) of
-// A (M rows), p = blockIdx.y taking every gridDim.y-th block of 256 rows.
+// *out = largest exponent field of the rows of a column (M of them) in every np-th
+// block of 256 from block p on; 256 threads.
 template <typename T>
-__global__ void __launch_bounds__(256)
-col_expo_kernel(const T* __restrict__ A, long long lda, int M, int* __restrict__ part) {
+__device__ __forceinline__ void col_expo_part(const T* __restrict__ col, int M, int p, int np,
+                                              int* __restrict__ out) {
   __shared__ int red[8];
-  const T* col = A + (size_t)blockIdx.x * lda;
   int e = 0;
 #pragma unroll 4
-  for (int r = blockIdx.y * 256 + threadIdx.x; r < M; r += gridDim.y * 256) {
+  for (int r = p * 256 + threadIdx.x; r < M; r += np * 256) {
     const T v = col[r];
     e = max(e, max(col_expo(v.x), col_expo(v.y)));
   }
@@ -42,14 +41,27 @@ col_expo_kernel(const T* __restrict__ A, long long lda, int M, int* __restrict__
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < 8; ++w) e = max(e, red[w]);
-    part[blockIdx.y * gridDim.x + blockIdx.x] = e;
+    *out = e;
   }
 }
 
-// Launches it; returns the number of partial maxima per column.
+// part[p K + k]: part p (blockIdx.y) of column k (blockIdx.x, K of them) of A (M rows)
+template <typename T>
+__global__ void __launch_bounds__(256)
+col_expo_kernel(const T* __restrict__ A, long long lda, int M, int* __restrict__ part) {
+  col_expo_part(A + (size_t)blockIdx.x * lda, M, blockIdx.y, gridDim.y,
+                &part[blockIdx.y * gridDim.x + blockIdx.x]);
+}
+
+// Partial maxima per column of M rows.
+inline int col_expo_parts(int M) {
+  return M <= 1024 ? 1 : M >= 1024 * kColParts ? kColParts : (M + 1023) / 1024;
+}
+
+// Launches it; returns their number.
 template <typename T>
 int launch_col_expo(const T* A, long long lda, int M, int K, int* part, cudaStream_t s) {
-  const int np = M <= 1024 ? 1 : M >= 1024 * kColParts ? kColParts : (M + 1023) / 1024;
+  const int np = col_expo_parts(M);
   col_expo_kernel<T><<<dim3(K, np), 256, 0, s>>>(A, lda, M, part);
   return np;
 }
@@ -57,7 +69,9 @@ int launch_col_expo(const T* A, long long lda, int M, int K, int* part, cudaStre
 // largest exponent field of column k
 __device__ __forceinline__ int col_expo_max(const int* __restrict__ part, int np, int K, int k) {
   int e = 0;
-  for (int p = 0; p < np; ++p) e = max(e, __ldg(&part[p * K + k]));
+#pragma unroll
+  for (int p = 0; p < kColParts; ++p)  // all loads in flight at once
+    if (p < np) e = max(e, __ldg(&part[p * K + k]));
   return e;
 }
 

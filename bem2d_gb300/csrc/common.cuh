@@ -507,19 +507,33 @@ void launch_scatter_c64(int n, const float2* src, const int* perm, float2* dst, 
 // the first of them only (10 mantissa bits, a third of the tensor work).
 // Sets *status on a device-side wait timeout.
 // `pack` (tc_pack_bytes(M, N, K) bytes) holds the split, re-laid-out operands.
+// part: np partial maxima of the exponents of A's columns (colscale.cuh), over the
+// M rows or more; null: they are formed first, by one more launch.
 size_t tc_pack_bytes(int M, int N, int K);
+// The pack buffer's first bytes: the exponents of the panels of an outer block
+// (four slots of kColParts x 64 integers).
+constexpr size_t kPanelExpoBytes = 4 * 16 * 64 * sizeof(int);
+// Where an update's own exponents lie in the pack buffer.
+int* tc_update_part(void* pack);
 int launch_tc_cgemm_sub(float2* C, long long ldc, const float2* A, long long lda,
                         const float2* B, long long ldb, int M, int N, int K, void* pack,
                         size_t pack_bytes, int* status, cudaStream_t s, int max_ctas = 0,
-                        int passes = 3);
+                        int passes = 3, const int* part = nullptr, int np = 0);
 // What follows a complex64 panel of nb columns at k0 (ipiv[k0 ..]: its pivots;
 // null: no swaps): the row swaps on the columns [cl, k0) and [rs, cr), U12 =
 // L11^{-1} A12 on the latter and, with `update`, A22 -= L21 U12 there for the M
 // rows below the panel (pack: tc_pack_bytes(M, cr - rs, nb) bytes).  nb = 64
-// unless cr = rs.
+// unless cr = rs.  part: np partial maxima of the exponents of the panel's columns
+// (colscale.cuh), over the M rows or more.  ex: column exponents formed in the
+// same launch, for a later update.
+struct TcExpo {
+  const float2* A = nullptr;  // M x K, leading dimension lda
+  int M = 0, K = 0, np = 0;
+  int* part = nullptr;        // [np][K]
+};
 int launch_tc_step(float2* A, long long lda, int M, int k0, int nb, int cl, int rs, int cr,
-                   const int* ipiv, bool update, void* pack, int* status, cudaStream_t s,
-                   int max_ctas, int passes);
+                   const int* ipiv, bool update, const int* part, int np, const TcExpo& ex,
+                   void* pack, int* status, cudaStream_t s, int max_ctas, int passes);
 
 // C = beta C + sign A B (complex128, column-major; C is M x N, A M x K, B K x
 // N; beta 0 or 1) on the tensor cores, FP64 accurate (lu_oz.cu).  pack:

@@ -29,6 +29,7 @@ namespace cg = cooperative_groups;
 #include <climits>
 #include <mutex>
 
+#include "colscale.cuh"
 #include "common.cuh"
 #include "cplx.cuh"
 #include "tc.cuh"
@@ -843,6 +844,9 @@ panel_rows_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, 
 // us; with rank-1 updates and exchanges of all 64 columns 70 us, with cluster
 // barriers instead of asynchronous stores 109 us; in sub-blocks of 16 as long
 // for one panel, 2 % longer for many at once.
+// lexp (null: none): every CTA leaves the largest exponents of its part of L21's
+// columns there (colscale.cuh), read from Fin across its rows: 0.85 us (with a
+// warp reduce instruction per column 2.9 us, by a kernel of its own 5 us).
 constexpr int kWinMaxRows = 256;
 constexpr int kSub = 8;          // columns of a sub-block
 constexpr int kSubP = kSub / 2;   // 16-byte words of a candidate
@@ -872,7 +876,7 @@ __device__ __forceinline__ float2 crcp_fast(float2 a) {
 
 __global__ void __launch_bounds__(kWinMaxRows, 1)
 panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, int rpb,
-                 int* __restrict__ ipiv, int* info, int* status) {
+                 int* __restrict__ ipiv, int* info, int* status, int* __restrict__ lexp) {
   constexpr int kR = kNB - kSub;
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -895,6 +899,7 @@ panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, i
   __shared__ unsigned s_own[kNB / kSub];  // pivots of the sub-block held by this CTA
   __shared__ int s_ipiv[kNB];
   __shared__ int s_info;
+  __shared__ unsigned char s_exp[kWinMaxRows / 32][kNB];
   const int r0 = k0 + rank * rpb;
   const bool active = lr < max(min(rpb, n - r0), 0);
   unsigned label = active ? (unsigned)(r0 + lr) : 0xffffffffu;
@@ -1116,6 +1121,29 @@ panel_win_kernel(float2* __restrict__ A, long long lda, int n, int k0, int nb, i
   }
   if (active)
     for (int c = 0; c < nb; ++c) A[(size_t)(k0 + c) * lda + label] = Fin[(size_t)c * T + lr];
+  if (!lexp) return;
+  __syncwarp();
+  // this CTA's largest exponent in every column of L21 (nb = 64): lane l reads
+  // columns l and l + 32 of its warp's rows, starting at row l (other banks)
+  const unsigned below = __ballot_sync(0xffffffffu, active && label >= (unsigned)(k0 + kNB));
+  const unsigned mine = __funnelshift_r(below, below, ln);
+  float m0 = 0.f, m1 = 0.f;
+  const float2* f = Fin + (size_t)ln * T + 32 * lw;
+#pragma unroll 16
+  for (int i = 0; i < 32; ++i) {
+    const float2 a = f[(ln + i) & 31], b = f[32 * T + ((ln + i) & 31)];
+    const bool in = (mine >> i) & 1u;
+    m0 = in ? fmaxf(m0, fmaxf(fabsf(a.x), fabsf(a.y))) : m0;
+    m1 = in ? fmaxf(m1, fmaxf(fabsf(b.x), fabsf(b.y))) : m1;
+  }
+  s_exp[lw][ln] = (unsigned char)col_expo(m0);
+  s_exp[lw][ln + 32] = (unsigned char)col_expo(m1);
+  __syncthreads();
+  if (lr < kNB) {
+    int e = 0;
+    for (int k = 0; k < nw; ++k) e = max(e, (int)s_exp[k][lr]);
+    lexp[rank * kNB + lr] = e;
+  }
 }
 
 template <typename K, typename... Args>
@@ -1371,13 +1399,15 @@ __global__ void tslu_gather_kernel(const float2* __restrict__ S, long long lds, 
 // infc): ipiv[k0 + c] (LAPACK), and the rows that end beyond the pivots at
 // positions other than their own: moved[0] = count, then (position, row)
 // pairs.  Positions relative to k0 live in shared memory (2 H ints).  One
-// CTA of 1024 threads.
+// CTA of 1024 threads.  lexp (null: none): set to zero, for tslu_rows_kernel.
 __global__ void __launch_bounds__(1024)
 tslu_perm_kernel(int n, int k0, int nb, const int* __restrict__ candF, int Gc,
                  const int* __restrict__ ipc, const int* __restrict__ infc, int* __restrict__ ipiv,
-                 int* info, int* __restrict__ moved) {
+                 int* info, int* __restrict__ moved, int* __restrict__ lexp) {
   extern __shared__ int sh[];
   const int H = n - k0;
+  static_assert(kColParts * kNB == 1024, "");
+  if (lexp) lexp[threadIdx.x] = 0;
   int* pos = sh;       // [H] position of row k0 + i
   int* at = sh + H;    // [H] row at position k0 + i
   __shared__ int cw[kTsluMaxCand];
@@ -1441,19 +1471,20 @@ tslu_perm_kernel(int n, int k0, int nb, const int* __restrict__ candF, int Gc,
 // 8 as in the panels: the sub-block's triangle, then the columns right of it.
 // FP32 issue bounds it (2016 complex multiply-subtracts per row); 16384 x 64 take
 // 22 us, as a warp per row with lanes on columns (a shuffle per column, strided
-// loads) 41 us.
+// loads) 41 us.  lexp (null: none): the largest exponents of L21's columns, CTA b
+// adds its rows' to part b % kColParts.
 constexpr int kRowsCta = 128, kULd = kNB + 2;
 __global__ void __launch_bounds__(kRowsCta)
 tslu_rows_kernel(const float2* __restrict__ A, long long lda, int n, int k0, int nb,
                  const float2* __restrict__ Cf, int Gc, const int* __restrict__ moved,
-                 float2* __restrict__ P) {
+                 float2* __restrict__ P, int* __restrict__ lexp) {
   constexpr int kR = kNB - kSub;
   __shared__ __align__(16) float2 U[kNB][kULd];  // row c of U11
   __shared__ float2 dv[kNB];
   __shared__ float2 Xs[kSub][kRowsCta];
   __shared__ int src[kRowsCta];
   const int t = threadIdx.x, H = n - k0, i = blockIdx.x * kRowsCta + t;
-  src[t] = k0 + i;
+  src[t] = k0 + min(i, H - 1);  // beyond H: the last row once more, not stored
   for (int e = t; e < kNB * kNB; e += kRowsCta) {
     const int c = e / kNB, r = e - c * kNB;  // coalesced: consecutive rows of column c
     U[r][c] = c < nb && r < nb ? Cf[(size_t)c * Gc + r] : make_float2(0.f, 0.f);
@@ -1468,11 +1499,11 @@ tslu_rows_kernel(const float2* __restrict__ A, long long lda, int n, int k0, int
     if (q >= 0 && q < kRowsCta) src[q] = moved[2 + 2 * u];
   }
   __syncthreads();
-  if (i >= H) return;
   if (i < nb) {
     for (int c = 0; c < nb; ++c) P[(size_t)c * H + i] = Cf[(size_t)c * Gc + i];
     return;
   }
+  int* my = lexp ? lexp + (blockIdx.x % kColParts) * kNB : nullptr;
   const float2* row = A + (size_t)k0 * lda + src[t];
   float2 w[kSub], R[kR];
 #pragma unroll
@@ -1495,7 +1526,21 @@ tslu_rows_kernel(const float2* __restrict__ A, long long lda, int n, int k0, int
     }
 #pragma unroll
     for (int q = 0; q < kSub; ++q)
-      if (c0 + q < nb) P[(size_t)(c0 + q) * H + i] = w[q];
+      if (c0 + q < nb && i < H) P[(size_t)(c0 + q) * H + i] = w[q];
+    if (my) {  // (nb = 64: whole warps) four lanes per column, 8 of the warp's rows each
+      __syncwarp();
+      const int l = t & 31, q = l >> 2, r0 = t - l + 8 * (l & 3);
+      float m = 0.f;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {  // starting at row q: other banks
+        const float2 v = Xs[q][r0 + ((r + q) & 7)];
+        m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+      }
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+      if ((l & 3) == 0) atomicMax(&my[c0 + q], col_expo(m));
+      __syncwarp();
+    }
     const int ng = (kNB - c0) / kSub - 1;  // groups of 8 columns right
 #pragma unroll 1
     for (int q = 0; q < kSub; ++q) {
@@ -1522,8 +1567,9 @@ tslu_rows_kernel(const float2* __restrict__ A, long long lda, int n, int k0, int
 // Tournament-pivoted panel of columns k0 .. k0 + nb - 1 (rows k0 .. n - 1).
 // false: not applicable (taller than the tournament holds, scratch too
 // small, or the cluster launch refused); A and ipiv are then untouched.
+// lexp (null: none): kColParts partial maxima of the exponents of L21's columns.
 static bool tslu_panel(float2* A, long long lda, int n, int k0, int nb, const LuWork& w, int cmax,
-                       cudaStream_t s, long long* launches) {
+                       int* lexp, cudaStream_t s, long long* launches) {
   const int H = n - k0;
   if (H > kTsluMaxH || tslu_bytes(n) == 0 ||
       w.scratch_bytes < slots_region() + tslu_bytes(n))
@@ -1575,14 +1621,15 @@ static bool tslu_panel(float2* A, long long lda, int n, int k0, int nb, const Lu
   const int threads = win_threads(rpb);
   cudaMemsetAsync(ts.infc, 0, sizeof(int), s);
   if (launch_cluster(panel_win_kernel, C, threads, panel_win_smem(rpb), s, Cf, (long long)ld, Gf,
-                     0, nb, rpb, ts.ipc, ts.infc, w.status) != cudaSuccess) {
+                     0, nb, rpb, ts.ipc, ts.infc, w.status, (int*)nullptr) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   tslu_perm_kernel<<<1, 1024, sizeof(int) * 2 * (size_t)H, s>>>(n, k0, nb, candF, Gf, ts.ipc,
-                                                                ts.infc, w.ipiv, w.info, ts.moved);
+                                                                ts.infc, w.ipiv, w.info, ts.moved,
+                                                                 lexp);
   tslu_rows_kernel<<<(H + kRowsCta - 1) / kRowsCta, kRowsCta, 0, s>>>(A, lda, n, k0, nb, Cf, ld,
-                                                                      ts.moved, ts.P);
+                                                                      ts.moved, ts.P, lexp);
   cudaMemcpy2DAsync(A + (size_t)k0 * lda + k0, sizeof(float2) * lda, ts.P, sizeof(float2) * H,
                     sizeof(float2) * H, nb, cudaMemcpyDeviceToDevice, s);
   *launches += 2;  // + the cluster launch the caller counts
@@ -1753,9 +1800,11 @@ size_t lu_aux_bytes(int n, size_t elem) {
 // dimension ld inside the matrix being factored).  complex64 updates of at
 // least kTensorMinN rows and columns run on the tensor cores, the rest on the
 // CUDA cores in slices of K = 64.
+// part, np: as for launch_tc_cgemm_sub.
 template <typename T>
 static int update_sub(T* C, const T* Am, const T* Bm, long long ld, int M, int N, int K,
-                      const LuWork& w, cudaStream_t s, long long* launches) {
+                      const LuWork& w, cudaStream_t s, long long* launches,
+                      const int* part = nullptr, int np = 0) {
   if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
   if constexpr (sizeof(T) == sizeof(double2)) {
     if (w.pack && oz_pack_bytes(M, N) <= w.pack_bytes)
@@ -1769,11 +1818,11 @@ static int update_sub(T* C, const T* Am, const T* Bm, long long ld, int M, int N
         (N >= 4 * kTensorMinN && M >= kNB)) {
       ++*launches;
       if (w.pack && tc_pack_bytes(M, N, K) <= w.pack_bytes) {
-        ++*launches;  // + the packing kernel
+        *launches += part ? 1 : 2;  // + the packing kernel and the one for its scales
         return launch_tc_cgemm_sub(reinterpret_cast<float2*>(C), ld,
                                    reinterpret_cast<const float2*>(Am), ld,
                                    reinterpret_cast<const float2*>(Bm), ld, M, N, K, w.pack,
-                                   w.pack_bytes, w.status, s, w.tc_ctas, w.tc_passes)
+                                   w.pack_bytes, w.status, s, w.tc_ctas, w.tc_passes, part, np)
                    ? BEM2D_ERR_CUDA
                    : BEM2D_OK;
       }
@@ -1862,8 +1911,10 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
     w2.tc_ctas = w.aux_ctas;
   }
   bool far_pending = false;
+  static_assert(kOuterNB <= 4 * kNB && kPanelExpoBytes == sizeof(int) * 4 * kColParts * kNB, "");
   for (int K0 = 0; K0 < n; K0 += outer) {
   const int bend = std::min(n, K0 + outer);
+  int lparts[4] = {0, 0, 0, 0};  // parts of L's exponents of the block's panels in w.pack
   for (int k0 = K0; k0 < bend; k0 += kNB) {
     const int nb = std::min(kNB, n - k0);
     const int H = n - k0;
@@ -1875,6 +1926,12 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
     // portable) CTAs and kPanelRPT rows per thread.
     const int rows_target = sizeof(T) == sizeof(float2) ? kPanelThreads : 64;
     bool done = false;
+    // where the panel leaves the exponents of L21's columns
+    const int slot = (k0 - K0) / kNB;
+    int* lexp = nullptr;
+    if (sizeof(T) == sizeof(float2) && nb == kNB && H > nb && w.pack &&
+        w.pack_bytes >= tc_pack_bytes(H - nb, 1, nb))
+      lexp = static_cast<int*>(w.pack) + slot * kColParts * kNB;
     if constexpr (sizeof(T) == sizeof(double2)) {
       const int rc = launch_zpanel(A, lda, n, k0, nb, w, s, launches);
       if (rc < 0) return rc;
@@ -1891,9 +1948,10 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
         const int threads = win_threads(rpb);
         cudaError_t e = launch_cluster(panel_win_kernel, C, threads, panel_win_smem(rpb), s,
                                        reinterpret_cast<float2*>(A), lda, n, k0, nb, rpb,
-                                       w.ipiv, w.info, w.status);
+                                       w.ipiv, w.info, w.status, lexp);
         if (e == cudaSuccess) {
           done = true;
+          lparts[slot] = lexp ? C : 0;
           break;
         }
         cudaGetLastError();
@@ -1923,7 +1981,8 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
       // rows panel above: ~200 us per 64 columns for it up to 16 x 416 rows,
       // about as much for the tournament there; beyond, the grid panel: ~370 us)
       done = tslu_panel(reinterpret_cast<float2*>(A), lda, n, k0, nb, w,
-                        cluster16 ? kMaxClusterPanel : 8, s, launches);
+                        cluster16 ? kMaxClusterPanel : 8, lexp, s, launches);
+      if (done && lexp) lparts[slot] = kColParts;
     }
     for (int cmax : {cluster16 ? kMaxClusterPanel : 8, 8}) {
       if (done) break;
@@ -1962,9 +2021,14 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
       // block)
       const int cl = la ? K0 : 0, cr = la ? bend : n, c1 = k0 + nb, M = n - c1, N = cr - c1;
       const bool tc = N > 0 && w.pack && tc_pack_bytes(M, N, nb) <= w.pack_bytes;
+      if (lexp && !lparts[slot]) {  // panels that leave none
+        lparts[slot] = launch_col_expo(A + (size_t)k0 * lda + c1, lda, M, nb, lexp, s);
+        ++*launches;
+      }
       if (N > 0 || k0 > cl) {
-        if (launch_tc_step(reinterpret_cast<float2*>(A), lda, M, k0, nb, cl, c1, cr, w.ipiv, tc, w.pack,
-                           w.status, s, w.tc_ctas, w.tc_passes))
+        if (launch_tc_step(reinterpret_cast<float2*>(A), lda, M, k0, nb, cl, c1, cr, w.ipiv, tc,
+                           lexp, lparts[slot], TcExpo(), w.pack, w.status, s, w.tc_ctas,
+                           w.tc_passes))
           return BEM2D_ERR_CUDA;
         *launches += tc ? 2 : 1;
       }
@@ -1997,12 +2061,22 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
   // then A22 -= L21 U12 with K = the block width
   const int nc = n - bend;
   const bool stepped = sizeof(T) == sizeof(float2) && outer == kNB && !la;
+  TcExpo ex;  // the exponents of the block's L21, by the last step's launch
   if (nc > 0 && !stepped) {
     for (int j0 = K0; j0 < bend; j0 += kNB) {
-      const int r1 = j0 + kNB;
-      if (la && w.pack && tc_pack_bytes(bend - r1, nc, kNB) <= w.pack_bytes) {
+      const int r1 = j0 + kNB, slot = (j0 - K0) / kNB;
+      if (la && lparts[slot] && tc_pack_bytes(bend - r1, nc, kNB) <= w.pack_bytes) {
+        if (r1 >= bend && tc_pack_bytes(nc, 1, bend - K0) <= w.pack_bytes) {
+          ex.A = reinterpret_cast<const float2*>(A) + (size_t)K0 * lda + bend;
+          ex.M = nc;
+          ex.K = bend - K0;
+          ex.np = std::min(4, col_expo_parts(nc));  // CTAs of the step's size: few
+          ex.part = tc_update_part(w.pack);
+        }
         if (launch_tc_step(reinterpret_cast<float2*>(A), lda, bend - r1, j0, kNB, j0, bend, n,
-                           nullptr, r1 < bend, w.pack, w.status, s, w.tc_ctas, w.tc_passes))
+                           nullptr, r1 < bend,
+                           static_cast<const int*>(w.pack) + slot * kColParts * kNB, lparts[slot],
+                           ex, w.pack, w.status, s, w.tc_ctas, w.tc_passes))
           return BEM2D_ERR_CUDA;
         *launches += r1 < bend ? 2 : 1;
         continue;
@@ -2019,7 +2093,7 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
       const int next = std::min(n, bend + outer);
       int rc = update_sub(A + (size_t)bend * lda + bend, A + (size_t)K0 * lda + bend,
                           A + (size_t)bend * lda + K0, lda, nc, next - bend, bend - K0, w, s,
-                          launches);
+                          launches, ex.part, ex.np);
       if (rc) return rc;
       if (next < n) {
         if (cudaEventRecord(w.ev_u12, s) != cudaSuccess ||
@@ -2027,7 +2101,7 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
           return BEM2D_ERR_CUDA;
         rc = update_sub(A + (size_t)next * lda + bend, A + (size_t)K0 * lda + bend,
                         A + (size_t)next * lda + K0, lda, nc, n - next, bend - K0, w2, w.aux,
-                        launches);
+                        launches, ex.part, ex.np);  // (rewritten after ev_far only)
         if (rc) return rc;
         if (cudaEventRecord(w.ev_far, w.aux) != cudaSuccess) return BEM2D_ERR_CUDA;
         far_pending = true;
@@ -2959,6 +3033,38 @@ __global__ void identity_c64_kernel(int n, float2* __restrict__ X, long long ldx
   if (i < n) X[(size_t)i * ldx + i] = make_float2(1.f, 0.f);
 }
 
+// The exponents of every column k of LU (colscale.cuh), for all updates of the
+// inverse in one launch: ex[k] of the rows below k's 64-column block, ex[n + k]
+// of those below its outer block of ob columns, ex[2 n + k] and ex[3 n + k] of
+// those above them.
+__global__ void __launch_bounds__(256)
+inverse_expo_kernel(const float2* __restrict__ LU, long long lda, int n, int ob,
+                    int* __restrict__ ex) {
+  __shared__ int red[4][8];
+  const int k = blockIdx.x, b0 = k / kNB * kNB, b1 = b0 + kNB, q0 = k / ob * ob, q1 = q0 + ob;
+  int e[4] = {0, 0, 0, 0};
+#pragma unroll 4
+  for (int r = threadIdx.x; r < n; r += 256) {
+    const float2 v = LU[(size_t)k * lda + r];
+    const int x = max(col_expo(v.x), col_expo(v.y));
+    if (r >= b1) e[0] = max(e[0], x);
+    if (r >= q1) e[1] = max(e[1], x);
+    if (r < b0) e[2] = max(e[2], x);
+    if (r < q0) e[3] = max(e[3], x);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    e[i] = __reduce_max_sync(0xffffffffu, e[i]);
+    if ((threadIdx.x & 31) == 0) red[i][threadIdx.x >> 5] = e[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    int m = 0;
+    for (int w = 0; w < 8; ++w) m = max(m, red[threadIdx.x][w]);
+    ex[(size_t)threadIdx.x * n + k] = m;
+  }
+}
+
 int lu_inverse_c64(const float2* LU, long long lda, int n, const LuWork& w, float2* W,
                    long long ldw, cudaStream_t s, long long* launches) {
   if (n <= 0) return BEM2D_OK;
@@ -2967,11 +3073,20 @@ int lu_inverse_c64(const float2* LU, long long lda, int n, const LuWork& w, floa
   // outer blocks of kOuterNB rows where the packing buffer holds rank-256
   // operands (one pass over the rest of W per outer block, not per 64 rows)
   const int ob = tc_pack_bytes(n, n, kOuterNB) <= w.pack_bytes ? kOuterNB : kNB;
-  auto upd = [&](float2* C, const float2* Am, const float2* Bm, int M, int N, int K) -> int {
+  // the panels' scratch is free by now
+  int* ex = w.scratch_bytes >= sizeof(int) * 4 * (size_t)n ? static_cast<int*>(w.scratch) : nullptr;
+  if (ex) {
+    inverse_expo_kernel<<<n, 256, 0, s>>>(LU, lda, n, ob, ex);
+    ++*launches;
+  }
+  // set 0 .. 3 of the exponents, of the columns from k on
+  auto upd = [&](float2* C, const float2* Am, const float2* Bm, int M, int N, int K, int set,
+                 int k) -> int {
     if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
-    if (launch_tc_cgemm_sub(C, ldw, Am, lda, Bm, ldw, M, N, K, w.pack, w.pack_bytes, w.status, s))
+    if (launch_tc_cgemm_sub(C, ldw, Am, lda, Bm, ldw, M, N, K, w.pack, w.pack_bytes, w.status, s,
+                            0, 3, ex ? ex + (size_t)set * n + k : nullptr, 1))
       return BEM2D_ERR_CUDA;
-    *launches += 2;
+    *launches += ex ? 2 : 3;
     return BEM2D_OK;
   };
   if (cudaMemset2DAsync(W, sizeof(float2) * ldw, 0, sizeof(float2) * n, n, s) != cudaSuccess)
@@ -2988,10 +3103,11 @@ int lu_inverse_c64(const float2* LU, long long lda, int n, const LuWork& w, floa
                                                         W + k0, ldw, bs, nc);
       ++*launches;
       // the rest of this outer block's rows
-      if ((rc = upd(W + nc, LU + (size_t)k0 * lda + nc, W + k0, R1 - nc, nc, bs))) return rc;
+      if ((rc = upd(W + nc, LU + (size_t)k0 * lda + nc, W + k0, R1 - nc, nc, bs, 0, k0))) return rc;
     }
     // the rows below the outer block, columns 0 .. R1 - 1 (Y is zero beyond)
-    if ((rc = upd(W + R1, LU + (size_t)R0 * lda + R1, W + R0, n - R1, R1, R1 - R0))) return rc;
+    if ((rc = upd(W + R1, LU + (size_t)R0 * lda + R1, W + R0, n - R1, R1, R1 - R0, 1, R0)))
+      return rc;
   }
   const int nob = (n + ob - 1) / ob;
   for (int q = nob - 1; q >= 0; --q) {  // backward: W = U^{-1} Y
@@ -3001,9 +3117,9 @@ int lu_inverse_c64(const float2* LU, long long lda, int n, const LuWork& w, floa
       block_apply_kernel<<<(n + 15) / 16, 256, 0, s>>>(dinv + (size_t)(2 * kb + 1) * kNB * kNB,
                                                        W + k0, ldw, bs, n);
       ++*launches;
-      if ((rc = upd(W + R0, LU + (size_t)k0 * lda + R0, W + k0, k0 - R0, n, bs))) return rc;
+      if ((rc = upd(W + R0, LU + (size_t)k0 * lda + R0, W + k0, k0 - R0, n, bs, 2, k0))) return rc;
     }
-    if ((rc = upd(W, LU + (size_t)R0 * lda, W + R0, R0, n, R1 - R0))) return rc;
+    if ((rc = upd(W, LU + (size_t)R0 * lda, W + R0, R0, n, R1 - R0, 3, R0))) return rc;
   }
   return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
 }

@@ -29,6 +29,14 @@
 // All updates of the L-shape's LU, N = 16384: 51.4 -> 30.1 ms, their packing
 // (one kernel instead of two) 8.7 -> 3.9 ms; norm and condition number's, N =
 // 8192: 19 -> 12.4 ms.
+//   Inner index k is scaled first, by the largest exponent of A(:, k) and its
+// inverse on B(k, :) (colscale.cuh), so that powers of two on the rows and
+// columns of the matrix being factored do not meet in a column of U: without it
+// one row 2^40 heavier than the others pushed the rest of its 64-row block of U
+// below the split (refinement 3 -> 6 steps and 1e-8 in the solution; with 2^60
+// no convergence at n = 1500).  The panels leave these exponents behind, the last
+// step of an outer block forms those of its rank-256 update beside its own work:
+// kite N = 2048 5.02 -> 5.06 ms, L-shape N = 16384 128.4 -> 129.1 ms.
 //
 // Operands are packed once per update (pack_kernel): scaled, split into hi/lo
 // and laid out, per tile and per chunk of 32 along K, exactly as
@@ -62,6 +70,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "colscale.cuh"
 #include "common.cuh"
 #include "cplx.cuh"
 #include "tc.cuh"
@@ -122,6 +131,13 @@ __device__ __forceinline__ int scale_exp(float m) {
 }
 __device__ __forceinline__ float exp_float(int e) { return __int_as_float(e << 23); }
 
+// 2^t of an inner index for A, 2^-t for B from the exponent of A's column (see
+// colscale.cuh); t clamped to what the products of finite entries leave room for
+__device__ __forceinline__ float inner_scale(int e, bool is_a) {
+  const int t = e > 0 ? min(max(127 - e, -60), 100) : 0;
+  return exp_float(127 + (is_a ? t : -t));
+}
+
 // 8 values times sc, split into f16 hi and lo, 16 bytes each
 __device__ __forceinline__ void split8(const float (&v)[8], float sc, int passes,
                                        unsigned char* hi, unsigned char* lo) {
@@ -144,9 +160,11 @@ __device__ __forceinline__ void split8(const float (&v)[8], float sc, int passes
 // B (K x N complex) -> Bpk[nt][kc] = {hi, lo} chunks of kTcBpart bytes, each
 // with rows 0..127 = re and rows 128..255 = im of the tile's 128 columns;
 // isa, isb: exponent fields of the inverse scales.
+// part, np: the exponents of A's columns.
 struct TcPack {
   unsigned char *A, *B, *isa, *isb;
-  int nkc, passes;
+  const int* part;
+  int nkc, passes, np;
 };
 template <bool IS_A>
 __device__ __forceinline__ void pack_octet(const TcPack& pk, int r, int o, const float (&re)[8],
@@ -161,10 +179,12 @@ __device__ __forceinline__ void pack_octet(const TcPack& pk, int r, int o, const
 }
 // 32 rows of A from row 32 blk (a warp 32 rows x 8 k at a time) or 8 columns of
 // B from column 8 blk (a warp 8 columns x 32 k).  Each entry is read twice, for
-// the largest and for the split (the second time from L1).  256 threads.
+// the largest and for the split (the second time from L1).  256 threads; fk:
+// 32 nkc floats of shared memory for the inner indices' scales.
 template <bool IS_A>
 __device__ __forceinline__ void pack_block(const float2* __restrict__ P, long long ld, int lim,
-                                           int K, int blk, const TcPack& pk, float (*red)[32]) {
+                                           int K, int blk, const TcPack& pk, float (*red)[32],
+                                           float* fk) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // row of A, or column of B; first octet of k and octet step of this thread
   const int r = IS_A ? blk * 32 + lane : blk * 8 + (lane & 7);
@@ -172,13 +192,16 @@ __device__ __forceinline__ void pack_block(const float2* __restrict__ P, long lo
   const bool ok = r < lim;
   const float2* src = IS_A ? P + r : P + (size_t)r * ld;
   const long long st = IS_A ? ld : 1;
+  for (int k = threadIdx.x; k < pk.nkc * kTcBK; k += 256)
+    fk[k] = inner_scale(k < K ? col_expo_max(pk.part, pk.np, K, k) : 0, IS_A);
+  __syncthreads();
   float mx = 0.f;
   for (int o = o0; o < 4 * pk.nkc; o += os) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int k = 8 * o + j;
       const float2 v = ok && k < K ? src[k * st] : make_float2(0.f, 0.f);
-      mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+      mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)) * fk[k]);
     }
   }
   if (!IS_A) {
@@ -198,8 +221,8 @@ __device__ __forceinline__ void pack_block(const float2* __restrict__ P, long lo
     for (int j = 0; j < 8; ++j) {
       const int k = 8 * o + j;
       const float2 v = ok && k < K ? src[k * st] : make_float2(0.f, 0.f);
-      re[j] = v.x;
-      im[j] = v.y;
+      re[j] = v.x * fk[k];
+      im[j] = v.y * fk[k];
     }
     pack_octet<IS_A>(pk, r, o, re, im, sc);
   }
@@ -209,11 +232,12 @@ __device__ __forceinline__ void pack_block(const float2* __restrict__ P, long lo
 __global__ void __launch_bounds__(256)
 pack_kernel(const float2* __restrict__ A, long long lda, const float2* __restrict__ B,
             long long ldb, int M, int N, int K, int ab, TcPack pk) {
+  extern __shared__ float fk[];
   __shared__ float red[8][32];
   if ((int)blockIdx.x < ab)
-    pack_block<true>(A, lda, M, K, blockIdx.x, pk, red);
+    pack_block<true>(A, lda, M, K, blockIdx.x, pk, red, fk);
   else
-    pack_block<false>(B, ldb, N, K, blockIdx.x - ab, pk, red);
+    pack_block<false>(B, ldb, N, K, blockIdx.x - ab, pk, red, fk);
 }
 
 // ---- between a panel and its update ----------------------------------------
@@ -222,6 +246,8 @@ pack_kernel(const float2* __restrict__ A, long long lda, const float2* __restric
 // L21 U12 for the M rows below the panel, in one launch.  CTAs:
 //   [0, nright)  32 columns right of the panel each: swaps, U12, its pack;
 //   then nleft   32 columns left of it: swaps;
+//   then nexpo   a part of a column's exponents each, of the block that the
+//                update after this launch takes (ex);
 //   then         32 rows of L21 each: their pack.
 // The swaps are applied as the permutation they amount to: 128 threads each
 // follow one position (the panel's 64 rows; the other row of each swap) back
@@ -237,14 +263,20 @@ constexpr size_t kStepSmem = sizeof(float2) * (kNBs * kNBs + kNBs * kStepCols);
 
 __global__ void __launch_bounds__(256)
 tc_step_kernel(float2* __restrict__ A, long long lda, int M, int k0, int nb, int cl, int rs,
-               int cr, const int* __restrict__ ipiv, int nright, int nleft, bool packing, TcPack pk) {
+               int cr, const int* __restrict__ ipiv, int nright, int nleft, int nexpo, bool packing,
+               TcPack pk, TcExpo ex) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_ip[kNBs], s_src[kNBs], s_pos[kNBs], s_from[kNBs];
-  __shared__ float red[8][32];
+  __shared__ float red[8][32], fk[kNBs];
+  __shared__ int s_le[4][kNBs];
   const int t = threadIdx.x, c = t & 31, w = t >> 5;
   const int b = blockIdx.x;
   if (b >= nright + nleft) {
-    pack_block<true>(A + (size_t)k0 * lda + k0 + nb, lda, M, nb, b - nright - nleft, pk, red);
+    const int q = b - nright - nleft;
+    if (q < nexpo)
+      col_expo_part(ex.A + (size_t)(q % ex.K) * lda, ex.M, q / ex.K, ex.np, &ex.part[q]);
+    else
+      pack_block<true>(A + (size_t)k0 * lda + k0 + nb, lda, M, nb, q - nexpo, pk, red, fk);
     return;
   }
   const bool right = b < nright;
@@ -256,6 +288,13 @@ tc_step_kernel(float2* __restrict__ A, long long lda, int M, int k0, int nb, int
     s_ip[t] = ipiv && t < nb ? ipiv[k0 + t] : k0 + t;
     s_src[t] = k0 + t;
     s_pos[t] = -1;
+  }
+  // inner index t & 63's exponent: a quarter of the parts each, used when packing
+  int le = 0;
+  if (right && packing) {
+#pragma unroll
+    for (int p = 0; p < kColParts / 4; ++p)
+      if ((t >> 6) + 4 * p < pk.np) le = max(le, __ldg(&pk.part[((t >> 6) + 4 * p) * kNBs + (t & 63)]));
   }
   if (right) {  // nb = 64
 #pragma unroll
@@ -337,14 +376,19 @@ tc_step_kernel(float2* __restrict__ A, long long lda, int M, int k0, int nb, int
     if (cc < nc) A[(size_t)(cb + cc) * lda + k0 + r] = X[r * kStepCols + cc];
   }
   if (!packing) return;
+  s_le[t >> 6][t & 63] = le;
+  __syncthreads();
+  if (t < kNBs)
+    fk[t] = inner_scale(max(max(s_le[0][t], s_le[1][t]), max(s_le[2][t], s_le[3][t])), false);
+  __syncthreads();
   // pack: thread (column c, octet w)
   float re[8], im[8], mx = 0.f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const float2 v = X[(8 * w + j) * kStepCols + c];
-    re[j] = v.x;
-    im[j] = v.y;
-    mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+    re[j] = v.x * fk[8 * w + j];
+    im[j] = v.y * fk[8 * w + j];
+    mx = fmaxf(mx, fmaxf(fabsf(re[j]), fabsf(im[j])));
   }
   red[w][c] = mx;
   __syncthreads();
@@ -573,10 +617,18 @@ int num_sms() {
 
 }  // namespace
 
+// The pack buffer starts with the slots that panels leave L's exponents in, then
+// those that an update forms of its own.
+static size_t part_bytes(int K) { return align256(sizeof(int) * kColParts * (size_t)K); }
+
+int* tc_update_part(void* pack) {
+  return reinterpret_cast<int*>(static_cast<char*>(pack) + kPanelExpoBytes);
+}
+
 size_t tc_pack_bytes(int M, int N, int K) {
   const size_t nkc = (size_t)(K + kTcBK - 1) / kTcBK;
   const size_t mt = (size_t)(M + kTcBM - 1) / kTcBM, nt = (size_t)(N + kTcBN - 1) / kTcBN;
-  return align256(mt * nkc * kTcChunkA) + align256(nt * nkc * kTcChunkB) +
+  return kPanelExpoBytes + part_bytes(K) + align256(mt * nkc * kTcChunkA) + align256(nt * nkc * kTcChunkB) +
          align256(mt * kTcBM) + align256(nt * kTcBN);
 }
 
@@ -585,7 +637,9 @@ static TcPack pack_parts(void* pack, int M, int N, int K, int passes) {
   const int nkc = (K + kTcBK - 1) / kTcBK;
   const int mt = (M + kTcBM - 1) / kTcBM, nt = (N + kTcBN - 1) / kTcBN;
   TcPack pk;
-  pk.A = static_cast<unsigned char*>(pack);
+  pk.part = nullptr;
+  pk.np = 0;
+  pk.A = static_cast<unsigned char*>(pack) + kPanelExpoBytes + part_bytes(K);
   pk.B = pk.A + align256((size_t)mt * nkc * kTcChunkA);
   pk.isa = pk.B + align256((size_t)nt * nkc * kTcChunkB);
   pk.isb = pk.isa + align256((size_t)mt * kTcBM);
@@ -610,30 +664,42 @@ static int update_packed(float2* C, long long ldc, int M, int N, const TcPack& p
 int launch_tc_cgemm_sub(float2* C, long long ldc, const float2* A, long long lda,
                         const float2* B, long long ldb, int M, int N, int K, void* pack,
                         size_t pack_bytes, int* status, cudaStream_t s, int max_ctas,
-                        int passes) {
+                        int passes, const int* part, int np) {
   if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
   if (!pack || tc_pack_bytes(M, N, K) > pack_bytes) return BEM2D_ERR_ARG;
   if (passes != 1 && passes != 3) return BEM2D_ERR_ARG;
-  const TcPack pk = pack_parts(pack, M, N, K, passes);
+  TcPack pk = pack_parts(pack, M, N, K, passes);
+  if (!part) {
+    int* own = tc_update_part(pack);
+    np = launch_col_expo(A, lda, M, K, own, s);
+    part = own;
+  }
+  pk.part = part;
+  pk.np = np;
   const int ab = (M + kTcBM - 1) / kTcBM * (kTcBM / 32), bb = (N + kTcBN - 1) / kTcBN * (kTcBN / 8);
-  pack_kernel<<<ab + bb, 256, 0, s>>>(A, lda, B, ldb, M, N, K, ab, pk);
+  pack_kernel<<<ab + bb, 256, sizeof(float) * kTcBK * pk.nkc, s>>>(A, lda, B, ldb, M, N, K, ab, pk);
   return update_packed(C, ldc, M, N, pk, status, s, max_ctas);
 }
 
 int launch_tc_step(float2* A, long long lda, int M, int k0, int nb, int cl, int rs, int cr,
-                   const int* ipiv, bool update, void* pack, int* status, cudaStream_t s,
-                   int max_ctas, int passes) {
+                   const int* ipiv, bool update, const int* part, int np, const TcExpo& ex,
+                   void* pack, int* status, cudaStream_t s, int max_ctas, int passes) {
   static const cudaError_t attr = cudaFuncSetAttribute(
       tc_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepSmem);
   if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
   const int N = cr - rs;  // N > 0: nb = 64
   const int nright = (N + kStepCols - 1) / kStepCols, nleft = (k0 - cl + kStepCols - 1) / kStepCols;
   TcPack pk{};
-  if (update) pk = pack_parts(pack, M, N, nb, passes);
-  const int grid = nright + nleft + (update ? (M + 31) / 32 : 0);
+  if (update) {
+    pk = pack_parts(pack, M, N, nb, passes);
+    pk.part = part;
+    pk.np = np;
+  }
+  const int nexpo = ex.K * ex.np;
+  const int grid = nright + nleft + nexpo + (update ? (M + 31) / 32 : 0);
   if (grid == 0) return BEM2D_OK;
   tc_step_kernel<<<grid, 256, kStepSmem, s>>>(A, lda, M, k0, nb, cl, rs, cr, ipiv, nright, nleft,
-                                              update, pk);
+                                              nexpo, update, pk, ex);
   if (update)
     return update_packed(A + (size_t)rs * lda + k0 + nb, lda, M, N, pk, status, s, max_ctas);
   return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
