@@ -11,6 +11,7 @@
 
 #include "../../include/bem2d_gpu.h"
 #include "hankel_c.cuh"
+#include "per_device.h"
 
 namespace bem2d_gpu {
 
@@ -404,6 +405,37 @@ int launch_potential(const DevGeom& g, const NodeTable& t, int ng, int kernel, d
                      double ki, double eta, const double2* coef, int npts, const double* pts,
                      double2* out, double2* part, void* ck_tab, cudaStream_t s);
 size_t potential_part_bytes(int npts, int nodes);
+
+// ---- devices ----------------------------------------------------------------
+inline int current_device() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return dev;
+}
+// SMs of the current device
+inline int device_sms() {
+  static PerDevice<int> sms(0);
+  const int dev = current_device();
+  int v = dev < kMaxDevices ? sms[dev].load() : 0;
+  if (v > 0) return v;
+  if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) v = 0;
+  if (v < 1) return 1;
+  sms[dev] = v;
+  return v;
+}
+// Kernel KERN may take `bytes` of dynamic shared memory on the current device from
+// here on (one value per kernel); false if the device refuses.
+template <auto KERN>
+bool opt_in_smem(int bytes) {
+  static PerDevice<bool> ok(false);
+  static PerDeviceOnce once;
+  const int dev = current_device();
+  once(dev, [&] {
+    ok[dev] = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) ==
+              cudaSuccess;
+  });
+  return ok[dev];
+}
 
 // ---- context accessors (capi.cu) ------------------------------------------
 int ctx_device(const bem2d_ctx* c);

@@ -395,9 +395,15 @@ size_t hess_eigenvalues_work_bytes() { return sizeof(QrControl); }
 
 int launch_hess_eigenvalues(double2* H, int n, double2* w, int* status, void* work,
                             cudaStream_t s) {
-  static const bool big = cudaFuncSetAttribute(hess_eigenvalues_kernel,
-                                               cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                               1) == cudaSuccess;
+  static PerDevice<bool> non_portable(false);
+  static PerDeviceOnce attr;
+  const int dev = current_device();
+  attr(dev, [&] {
+    non_portable[dev] =
+        cudaFuncSetAttribute(hess_eigenvalues_kernel,
+                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  });
+  const bool big = non_portable[dev];
   cudaMemsetAsync(status, 0, sizeof(int), s);
   for (int C : {big ? 16 : 8, 8}) {
     cudaLaunchConfig_t cfg = {};

@@ -397,13 +397,6 @@ far_fp64_kernel(DevGeom g, NodeTable t, FarGroups fg, int ng, int cols, HankelTa
   }
 }
 
-static int far_sms() {
-  int dev = 0, v = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-  return std::max(v, 1);
-}
-
 template <int KERNEL, int NB, bool CK>
 static void launch_far_nb(const DevGeom& g, const NodeTable& t, const FarGroups& fg, int ng,
                           double k, double ki, double eta, double alpha, const HankelTab& tb,
@@ -414,7 +407,7 @@ static void launch_far_nb(const DevGeom& g, const NodeTable& t, const FarGroups&
   // columns per CTA: up to 40, fewer while the triangle of CTAs would not
   // give every SM a few (their cost is the staging of 32 + cols groups)
   int cols = 8 * kFarWarps;
-  while (cols > kFarWarps && (long long)rows * ((fg.n + cols - 1) / cols) / 2 < 8LL * far_sms())
+  while (cols > kFarWarps && (long long)rows * ((fg.n + cols - 1) / cols) / 2 < 8LL * device_sms())
     cols /= 2;
   const size_t per_col = sizeof(double) * ng * (4 + NB);
   const size_t fixed = sizeof(double) * ((size_t)(4 + NB) * ng * 32 +
@@ -494,7 +487,7 @@ int launch_far_fp64(const DevGeom& g, const NodeTable& t, const int2* grp, int n
 // (point, node) for the single layer; 40,000 points, 1,024 elements, 57.9 ->
 // 16.5 ms against one slice and direct evaluation.
 constexpr int kPotThreads = 128;
-constexpr int kPotCtas = 24 * 152;
+constexpr int kPotCtas = 24;  // per SM
 
 template <int KERNEL, bool CK>
 __global__ void __launch_bounds__(kPotThreads)
@@ -577,7 +570,7 @@ __global__ void potential_sum_kernel(int npts, int slices, const double2* __rest
 static int potential_slices(int npts, int nodes) {
   const int blocks = (npts + kPotThreads - 1) / kPotThreads;
   const int chunks = (nodes + kPotThreads - 1) / kPotThreads;
-  return std::max(1, std::min(chunks, (kPotCtas + blocks - 1) / blocks));
+  return std::max(1, std::min(chunks, (kPotCtas * device_sms() + blocks - 1) / blocks));
 }
 
 size_t potential_part_bytes(int npts, int nodes) {

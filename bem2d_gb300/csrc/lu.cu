@@ -27,7 +27,6 @@ namespace cg = cooperative_groups;
 #include <algorithm>
 #include <atomic>
 #include <climits>
-#include <mutex>
 
 #include "colscale.cuh"
 #include "common.cuh"
@@ -414,12 +413,7 @@ gemm_sub_kernel(const T* __restrict__ Am, long long lda, const T* __restrict__ B
 
 template <typename T>
 static int panel_blocks(int H) {
-  static const int nsm = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return std::max(v, 1);
-  }();
+  const int nsm = device_sms();
   // at least 64 rows per block: fewer blocks make the per-column barrier
   // and the pivot agreement cheaper; one block per SM at most
   return std::max(1, std::min(nsm, (H + 63) / 64));
@@ -1785,10 +1779,7 @@ constexpr int kLookaheadFreeSMs = 64;
 #endif
 bool lu_lookahead(int n) { return n >= BEM2D_LOOKAHEAD_MIN_N; }
 int lu_lookahead_ctas() {
-  int dev = 0, v = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-  return std::max(1, v - kLookaheadFreeSMs);
+  return std::max(1, device_sms() - kLookaheadFreeSMs);
 }
 
 size_t lu_aux_bytes(int n, size_t elem) {
@@ -1861,9 +1852,11 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
   cudaMemsetAsync(sl.base, 0, slots_bytes(sizeof(T)), s);
   // one-time function attributes; thread-safe (workers of a sweep factor
   // concurrently from several host threads)
-  static std::atomic<bool> cluster16{true};
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice<bool> c16(true);
+  static PerDeviceOnce attr;
+  const int dev = current_device();
+  std::atomic<bool>& cluster16 = c16[dev];
+  attr(dev, [&] {
     cudaFuncSetAttribute(panel_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(panel_cluster_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kClusterSmem);
@@ -2560,13 +2553,7 @@ static int lu_solve_wave(const TS* LU, long long lda, int n, const LuWork& w, co
   T* v = static_cast<T*>(w.scratch);
   T* ybuf = v + n;
   int* flags = reinterpret_cast<int*>(ybuf + (size_t)nk * kNB);
-  static const int nsm = [] {
-    int dev = 0, c = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-    return std::max(c, 1);
-  }();
-  const int G = std::min(nk, nsm);
+  const int G = std::min(nk, device_sms());
   const size_t smem = sizeof(T) * ((size_t)((nk + G - 1) / G) * kNB + 5 * kNB);
   if (smem > 48 * 1024) return BEM2D_ERR_ARG;
   cudaMemsetAsync(flags, 0, sizeof(int) * 2 * nk, s);
@@ -2594,9 +2581,11 @@ static int lu_solve_wave(const TS* LU, long long lda, int n, const LuWork& w, co
 template <typename T>
 static int lu_solve_cluster(const T* LU, long long lda, int n, const LuWork& w, const T* b, T* x,
                             cudaStream_t s, long long* launches) {
-  static std::atomic<int> cmax{kMaxCluster};
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice<int> largest(kMaxCluster);
+  static PerDeviceOnce attr;
+  const int dev = current_device();
+  std::atomic<int>& cmax = largest[dev];
+  attr(dev, [&] {
     cudaFuncSetAttribute(trisolve_cluster_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kClusterSmem);
     if (cudaFuncSetAttribute(trisolve_cluster_kernel<T>,
@@ -2624,9 +2613,11 @@ static int lu_solve_cluster(const T* LU, long long lda, int n, const LuWork& w, 
 
 static int lu_solve64(const float2* LU, long long lda, int n, const LuWork& w, const float2* b,
                       float2* x, cudaStream_t s, long long* launches) {
-  static std::atomic<int> cmax{kMaxCluster};
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice<int> largest(kMaxCluster);
+  static PerDeviceOnce attr;
+  const int dev = current_device();
+  std::atomic<int>& cmax = largest[dev];
+  attr(dev, [&] {
     cudaFuncSetAttribute(trisolve64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kClusterSmem);
     if (cudaFuncSetAttribute(trisolve64_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed,
@@ -2664,9 +2655,11 @@ int lu_solve(const T* LU, long long lda, int n, const LuWork& w, const T* b, T* 
 int lu_solve_mixed(const float2* LU, long long lda, int n, const LuWork& w, const double2* b,
                    double2* x, cudaStream_t s, long long* launches) {
   if (n >= kWaveMinN) return lu_solve_wave<double2, float2>(LU, lda, n, w, b, x, s, launches);
-  static std::atomic<int> cmax{kMaxCluster};
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice<int> largest(kMaxCluster);
+  static PerDeviceOnce attr;
+  const int dev = current_device();
+  std::atomic<int>& cmax = largest[dev];
+  attr(dev, [&] {
     cudaFuncSetAttribute(trisolve_cluster_kernel<double2, float2>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem);
     if (cudaFuncSetAttribute(trisolve_cluster_kernel<double2, float2>,
@@ -2773,9 +2766,11 @@ trisolve_h_cluster_kernel(const T* __restrict__ LU, long long lda, int n,
 template <typename T>
 int lu_solve_h(const T* LU, long long lda, int n, const LuWork& w, const T* b, T* x,
                cudaStream_t s, long long* launches) {
-  static std::atomic<int> cmax{kMaxCluster};
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice<int> largest(kMaxCluster);
+  static PerDeviceOnce attr;
+  const int dev = current_device();
+  std::atomic<int>& cmax = largest[dev];
+  attr(dev, [&] {
     cudaFuncSetAttribute(trisolve_h_cluster_kernel<T>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem);
     if (cudaFuncSetAttribute(trisolve_h_cluster_kernel<T>,
@@ -2820,8 +2815,8 @@ int lu_panel_timeout_probe(float2* A, long long lda, int n, const LuWork& w, uns
   cudaMemsetAsync(w.info, 0, sizeof(int), s);
   cudaMemsetAsync(w.status, 0, sizeof(int), s);
   cudaMemsetAsync(sl.base, 0, slots_bytes(sizeof(float2)), s);
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDeviceOnce attr;
+  attr(current_device(), [] {
     cudaFuncSetAttribute(panel_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          200 * 1024);
   });

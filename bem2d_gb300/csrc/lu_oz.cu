@@ -536,16 +536,6 @@ oz_zgemm_kernel(double2* __restrict__ C, long long ldc, OzPack o, const double2*
 
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
-int oz_sms() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v > 0 ? v : 1;
-  }();
-  return n;
-}
-
 }  // namespace
 
 // The pack buffer's parts for an M x N product; returns its bytes.
@@ -576,14 +566,12 @@ size_t oz_pack_bytes(int M, int N) {
 int launch_oz_zgemm(double2* C, long long ldc, const double2* A, long long lda, const double2* B,
                     long long ldb, int M, int N, int K, int beta, double sign, void* pack,
                     size_t pack_bytes, int* status, cudaStream_t s, long long* launches) {
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      oz_zgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOzSmem);
-  if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
+  if (!opt_in_smem<oz_zgemm_kernel>(kOzSmem)) return BEM2D_ERR_CUDA;
   if (M <= 0 || N <= 0 || K <= 0) return BEM2D_OK;
   OzPack o;
   if (!pack || oz_parts(pack, M, N, &o) > pack_bytes) return BEM2D_ERR_ARG;
   const int mt = (M + kOzBM - 1) / kOzBM, nt = (N + kOzBN - 1) / kOzBN;
-  const int grid = std::min(mt * nt, oz_sms());
+  const int grid = std::min(mt * nt, device_sms());
   for (int k = 0; k < K; k += kOzK) {
     const int kk = std::min(kOzK, K - k), ksteps = (kk + 15) / 16;
     const double2* a = A + (size_t)k * lda;

@@ -605,16 +605,6 @@ tc_cgemm_sub_kernel(float2* __restrict__ C, long long ldc, const unsigned char* 
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
-int num_sms() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v > 0 ? v : 1;
-  }();
-  return n;
-}
-
 }  // namespace
 
 // The pack buffer starts with the slots that panels leave L's exponents in, then
@@ -651,11 +641,9 @@ static TcPack pack_parts(void* pack, int M, int N, int K, int passes) {
 // The update of packed operands.
 static int update_packed(float2* C, long long ldc, int M, int N, const TcPack& pk, int* status,
                          cudaStream_t s, int max_ctas) {
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      tc_cgemm_sub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-  if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
+  if (!opt_in_smem<tc_cgemm_sub_kernel>(kTcSmem)) return BEM2D_ERR_CUDA;
   const int mt = (M + kTcBM - 1) / kTcBM, nt = (N + kTcBN - 1) / kTcBN;
-  const int grid = std::min(mt * nt, max_ctas > 0 ? max_ctas : num_sms());
+  const int grid = std::min(mt * nt, max_ctas > 0 ? max_ctas : device_sms());
   tc_cgemm_sub_kernel<<<grid, kTcThreads, kTcSmem, s>>>(C, ldc, pk.A, pk.B, pk.isa, pk.isb, M, N,
                                                         pk.nkc, mt, nt, pk.passes, status);
   return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
@@ -684,9 +672,7 @@ int launch_tc_cgemm_sub(float2* C, long long ldc, const float2* A, long long lda
 int launch_tc_step(float2* A, long long lda, int M, int k0, int nb, int cl, int rs, int cr,
                    const int* ipiv, bool update, const int* part, int np, const TcExpo& ex,
                    void* pack, int* status, cudaStream_t s, int max_ctas, int passes) {
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      tc_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepSmem);
-  if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
+  if (!opt_in_smem<tc_step_kernel>((int)kStepSmem)) return BEM2D_ERR_CUDA;
   const int N = cr - rs;  // N > 0: nb = 64
   const int nright = (N + kStepCols - 1) / kStepCols, nleft = (k0 - cl + kStepCols - 1) / kStepCols;
   TcPack pk{};

@@ -22,7 +22,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <mutex>
 
 #include "common.cuh"
 #include "cplx.cuh"
@@ -306,9 +305,11 @@ panel_update_kernel(double2* __restrict__ A, long long lda, int n, int kb, int j
 // available, having changed nothing.
 int launch_zpanel(double2* A, long long lda, int n, int k0, int nb, const LuWork& w,
                   cudaStream_t s, long long* launches) {
-  static std::atomic<int> max_cluster{kZMaxC};
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice<int> largest(kZMaxC);
+  static PerDeviceOnce attr;
+  const int dev = current_device();
+  std::atomic<int>& max_cluster = largest[dev];
+  attr(dev, [&] {
     bool ok = true;
     for (auto k : {panel16_kernel<1, 1>, panel16_kernel<1, 2>, panel16_kernel<1, 4>,
                    panel16_kernel<2, 1>})

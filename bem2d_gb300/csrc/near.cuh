@@ -307,16 +307,6 @@ static size_t near_table_bytes(const DevRules& r, int nb) {
   return sizeof(double) * (size_t)(nb > 1 ? 4 + kNearBasis : 5) * (cs + ct);
 }
 
-static int near_sms() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v > 0 ? v : 1;
-  }();
-  return n;
-}
-
 template <int KERNEL, bool MIXED, bool CK, int NB>
 static void launch_near_k(const DevGeom& g, const DevRules& r, const NearPair* pairs, int npairs,
                           double k, double ki, double eta, double alpha, double beta,
@@ -332,7 +322,7 @@ static void launch_near_k(const DevGeom& g, const DevRules& r, const NearPair* p
   // Two are enough in the mixed path, where every block copies the e^{ix} table
   // (kite N = 2048: 414 us with 8 warps, 427 with 2).
   int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (96 * 1024 - 1024) / per_warp));
-  while (wpb > 1 && (npairs + wpb - 1) / wpb < (MIXED ? 2 : 8) * near_sms()) wpb /= 2;
+  while (wpb > 1 && (npairs + wpb - 1) / wpb < (MIXED ? 2 : 8) * device_sms()) wpb /= 2;
   const size_t smem = 1024 + per_warp * wpb;
   const int blocks = (npairs + wpb - 1) / wpb;
   auto fn = near_kernel<KERNEL, MIXED, CK, NB>;

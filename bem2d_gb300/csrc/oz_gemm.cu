@@ -351,7 +351,7 @@ void pack_a(const T* A, long long lda, int n, int ks, unsigned char* dst, int* e
 int splits(int n, int m) {
   const long long tiles = (long long)((n + kGM - 1) / kGM) * ((m + kGN - 1) / kGN);
   const int chunks = (n + 16 * kGChunk - 1) / (16 * kGChunk);
-  return (int)std::max<long long>(1, std::min<long long>((2 * 152 + tiles - 1) / tiles, chunks / 2));
+  return (int)std::max<long long>(1, std::min<long long>((2 * device_sms() + tiles - 1) / tiles, chunks / 2));
 }
 
 }  // namespace
@@ -392,23 +392,15 @@ void launch_oz_pack(bool herm, int S, const T* A, long long lda, int n, void* ds
 template <int S, typename T>
 static int gemm_t(const void* Apk, int n, const T* B, long long ldb, int m, T* C, long long ldc,
                   void* work, int* status, cudaStream_t s) {
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      oz_gemm_kernel<S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<S>::kSmem);
-  if (attr != cudaSuccess) return BEM2D_ERR_CUDA;
+  if (!opt_in_smem<oz_gemm_kernel<S, T>>(Cfg<S>::kSmem)) return BEM2D_ERR_CUDA;
   const int ks = (n + 15) / 16, mt = (n + kGM - 1) / kGM, nt = (m + kGN - 1) / kGN, nz = splits(n, m);
   const unsigned char* ap = static_cast<const unsigned char*>(Apk);
   const int* ea = reinterpret_cast<const int*>(ap + up256((size_t)mt * ks * S * kGA));
   unsigned char* bp = static_cast<unsigned char*>(work);
   int* eb = reinterpret_cast<int*>(bp + up256((size_t)nt * ks * S * kGB));
   T* P = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(eb) + up256(sizeof(int) * (size_t)m));
-  static const int sms = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return std::max(v, 1);
-  }();
   const int units = mt * nt * nz;
-  oz_gemm_kernel<S, T><<<std::min(units, sms), kGThreads, Cfg<S>::kSmem, s>>>(
+  oz_gemm_kernel<S, T><<<std::min(units, device_sms()), kGThreads, Cfg<S>::kSmem, s>>>(
       nz > 1 ? P : C, nz > 1 ? n : ldc, (long long)n * m, ap, bp, ea, eb, n, m, ks, nt, nz, units,
       status);
   if (nz > 1)
