@@ -1025,6 +1025,17 @@ static int attach_lookahead(bem2d_ctx* c, LuWork& w, int n) {
   return BEM2D_OK;
 }
 
+// The packing buffer of a complex128 factorisation; without room for it the
+// updates run on the CUDA cores.
+static void attach_pack64(bem2d_ctx* c, LuWork& w, int n) {
+  int rc = 0;
+  w.pack_bytes = lu_pack_bytes(n, sizeof(double2));
+  w.pack = ws(c, "lu_pack", w.pack_bytes, &rc);
+  if (w.pack) return;
+  w.pack_bytes = 0;
+  cudaGetLastError();
+}
+
 // Solve with device-resident A (lda) and b; x written to device memory.
 // A32pre: a complex64 copy of A already in the "lu32" workspace (mixed
 // assembly writes it); otherwise A is converted here.
@@ -1064,9 +1075,7 @@ static int solve_dev(bem2d_ctx* c, int n, const double2* A, long long lda, const
     if (!LU) return rc;
     CUDA_TRY(c, cudaMemcpy2DAsync(LU, sizeof(double2) * n, A, sizeof(double2) * lda,
                                   sizeof(double2) * n, n, cudaMemcpyDeviceToDevice, c->stream));
-    w.pack_bytes = lu_pack_bytes(n, sizeof(double2));
-    w.pack = ws(c, "lu_pack", w.pack_bytes, &rc);
-    if (!w.pack) return rc;
+    attach_pack64(c, w, n);
     int t = tic(c, BEM2D_PHASE_LU);
     if ((rc = lu_factor<double2>(LU, n, n, w, c->stream, &c->launches)))
       return fail(c, rc, "LU launch failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1961,15 +1970,16 @@ int bem2d_l2_norm_cond_prec(bem2d_ctx* c, int n, const void* A, int64_t lda, dou
   w.dinv = aux;
   w.perm = reinterpret_cast<int*>(aux + (lu_aux_bytes(n, esz) - 256 - sizeof(int) * (size_t)n));
   const int tl = tic(c, BEM2D_PHASE_LU);
-  w.pack_bytes = lu_pack_bytes(n, esz);
-  w.pack = ws(c, "lu_pack", w.pack_bytes, &rc);
-  if (!w.pack) return rc;
   if (mixed) {
+    w.pack_bytes = lu_pack_bytes(n, esz);
+    w.pack = ws(c, "lu_pack", w.pack_bytes, &rc);
+    if (!w.pack) return rc;
     if ((rc = attach_lookahead(c, w, n))) return rc;
     launch_to_c64(dA, la, static_cast<float2*>(LU), n, n, n, c->stream);
     ++c->launches;
     rc = lu_factor<float2>(static_cast<float2*>(LU), n, n, w, c->stream, &c->launches);
   } else {
+    attach_pack64(c, w, n);
     CUDA_TRY(c, cudaMemcpy2DAsync(LU, sizeof(double2) * n, dA, sizeof(double2) * la,
                                   sizeof(double2) * n, n, cudaMemcpyDeviceToDevice, c->stream));
     rc = lu_factor<double2>(static_cast<double2*>(LU), n, n, w, c->stream, &c->launches);
