@@ -1457,25 +1457,43 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
   int* dmap = static_cast<int*>(ws(c, "nr_map", sizeof(int) * 2 * nang, &rc));
   double* dthc = static_cast<double*>(ws(c, "nr_thc", sizeof(double) * nang, &rc));
   if (!Qalt || !Walt || !dmap || !dthc) return rc;
-  // the products with A and A^H: digits packed once, on the tensor cores;
-  // without room for the two packed copies, on the CUDA cores
+  // the products with A and A^H on the tensor cores: all digits packed once;
+  // where the two packed copies do not fit, a quarter of the rows at a time, and
+  // so on; without room for 64 rows, on the CUDA cores
   size_t zwork_bytes = 0;
-  for (int m = 1; m <= nang; ++m)
-    zwork_bytes = std::max(zwork_bytes, oz_gemm_work_bytes(n, m, digits, sizeof(T)));
-  const size_t pa = oz_gemm_a_bytes(n, digits);
-  char* oz = static_cast<char*>(ws(c, "nr_oz", 2 * pa + 256, &rc));
-  void* zwork = oz ? ws(c, LzNames<T>::Z, zwork_bytes, &rc) : nullptr;
-  int* oz_status = reinterpret_cast<int*>(oz + 2 * pa);
-  if (oz && zwork) {
-    launch_oz_pack(false, digits, dA, la, n, oz, c->stream);
-    launch_oz_pack(true, digits, dA, la, n, oz + pa, c->stream);
-    CUDA_TRY(c, cudaMemsetAsync(oz_status, 0, sizeof(int), c->stream));
-    c->launches += 4;
-    CHECK_LAUNCH(c);
-  } else {
+  void* zwork = nullptr;
+  char* oz = nullptr;
+  int* oz_status = nullptr;
+  int oz_rows = n;
+  for (;;) {
+    zwork_bytes = 0;
+    for (int m = 1; m <= nang; ++m)
+      zwork_bytes = std::max(zwork_bytes, oz_gemm_work_bytes(oz_rows, n, m, digits, sizeof(T)));
+    if (oz_rows < n)  // the last rows may split K further
+      for (int m = 1; m <= nang; ++m)
+        zwork_bytes = std::max(zwork_bytes, oz_gemm_work_bytes((n - 1) % oz_rows + 1, n, m, digits,
+                                                               sizeof(T)));
+    const size_t pa = oz_gemm_a_bytes(oz_rows, n, digits) * (oz_rows >= n ? 2 : 1);
+    zwork = ws(c, LzNames<T>::Z, zwork_bytes, &rc);
+    oz = zwork ? static_cast<char*>(ws(c, "nr_oz", pa + 256, &rc)) : nullptr;
+    if (oz) {
+      oz_status = reinterpret_cast<int*>(oz + pa);
+      break;
+    }
     cudaGetLastError();
     rc = 0;
-    oz = nullptr;
+    if (oz_rows <= 64) break;
+    oz_rows = std::max(64, oz_rows / 4 / 64 * 64);
+  }
+  if (oz) {
+    if (oz_rows >= n) {
+      launch_oz_pack(false, digits, dA, la, 0, n, n, oz, c->stream);
+      launch_oz_pack(true, digits, dA, la, 0, n, n, oz + oz_gemm_a_bytes(n, n, digits), c->stream);
+      c->launches += 4;
+    }
+    CUDA_TRY(c, cudaMemsetAsync(oz_status, 0, sizeof(int), c->stream));
+    CHECK_LAUNCH(c);
+  } else {
     zwork_bytes = 0;
     for (int m = 1; m <= nang; ++m)
       zwork_bytes = std::max(zwork_bytes, zgemm_work_bytes(n, m, sizeof(T)));
@@ -1525,10 +1543,9 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
   for (int j = 0; j < mmax; ++j) {
     const T* Qj = Q + (size_t)j * n;
     if (oz) {
-      if ((rc = launch_oz_gemm_pair(digits, oz, oz + pa, n, Qj, qs, na, Y1, Y2, n, zwork,
-                                    oz_status, c->stream)))
+      if ((rc = launch_oz_gemm_pair(digits, dA, la, oz_rows, oz, n, Qj, qs, na, Y1, Y2, n, zwork,
+                                    oz_status, c->stream, &c->launches)))
         return fail(c, rc, "product launch: %s", cudaGetErrorString(cudaGetLastError()));
-      c->launches += 2;
     } else {
       launch_zgemm(false, dA, la, n, Qj, qs, na, Y1, n, zwork, zwork_bytes, c->stream);
       launch_zgemm(true, dA, la, n, Qj, qs, na, Y2, n, zwork, zwork_bytes, c->stream);

@@ -40,18 +40,21 @@ void launch_split_ff(const double2* A, long long lda, int n, float2* hi, float2*
 
 // Products with an n x n matrix through exact digit products on the tensor
 // cores (oz_gemm.cu): S digits, 8 or 7 for complex128 (FP64 and better than
-// float-float accuracy), 4 for complex64 (FP32).  launch_oz_pack packs A or
-// A^H (herm) once into oz_gemm_a_bytes(n, S); launch_oz_gemm_pair forms C1 = A
-// B and C2 = A^H B (B n x m, ldb) with oz_gemm_work_bytes(n, m, S, sizeof(T)) of
-// work.  Sets *status on a device-side wait timeout.
-size_t oz_gemm_a_bytes(int n, int S);
-size_t oz_gemm_work_bytes(int n, int m, int S, size_t elem);
+// float-float accuracy), 4 for complex64 (FP32).  launch_oz_pack packs `rows`
+// rows from r0 of A or A^H (herm) into oz_gemm_a_bytes(rows, n, S).
+// launch_oz_gemm_pair forms C1 = A B and C2 = A^H B (B n x m, ldb) with
+// oz_gemm_work_bytes(rows, n, m, S, sizeof(T)) of work: rows >= n: Apk holds all of
+// A packed, then all of A^H; otherwise `rows` rows (a multiple of 64) are packed
+// into Apk at a time.  Sets *status on a device-side wait timeout.
+size_t oz_gemm_a_bytes(int rows, int n, int S);
+size_t oz_gemm_work_bytes(int rows, int n, int m, int S, size_t elem);
 template <typename T>
-void launch_oz_pack(bool herm, int S, const T* A, long long lda, int n, void* dst, cudaStream_t s);
+void launch_oz_pack(bool herm, int S, const T* A, long long lda, int r0, int rows, int n, void* dst,
+                    cudaStream_t s);
 template <typename T>
-int launch_oz_gemm_pair(int S, const void* Apk, const void* Ahpk, int n, const T* B, long long ldb,
-                        int m, T* C1, T* C2, long long ldc, void* work, int* status,
-                        cudaStream_t s);
+int launch_oz_gemm_pair(int S, const T* A, long long lda, int rows, void* Apk, int n, const T* B,
+                        long long ldb, int m, T* C1, T* C2, long long ldc, void* work, int* status,
+                        cudaStream_t s, long long* launches);
 // C (rows x m, ldc) = A (rows x k, lda) B (k x m, ldb), complex128
 void launch_zgemm_rect(const double2* A, long long lda, int rows, int k, const double2* B,
                        long long ldb, int m, double2* C, long long ldc, cudaStream_t s);

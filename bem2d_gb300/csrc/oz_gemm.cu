@@ -1,6 +1,8 @@
 // C = op(A) B for the numerical range's block Lanczos on the tensor cores:
 // exact products of 8-bit digits (see lu_oz.cu for the splitting), A n x n
-// packed once for all products of a scan, B n x m packed per product.
+// packed once for all products of a scan, or, where its digits (8 S n^2 bytes for
+// A and A^H) do not fit, a block of rows at a time in every product; B n x m
+// packed per product.
 //
 // S digits (template): 8 where the products were FP64 (complex128 Lanczos), 7
 // where they were float-float (error about 2^-51 of row maximum x column
@@ -340,46 +342,54 @@ __global__ void oz_reduce_kernel(const T* __restrict__ P, long long cz, int nz, 
 
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
+// rows of A (first at A), or columns (HERM), n entries each
 template <int S, typename T, bool HERM>
-void pack_a(const T* A, long long lda, int n, int ks, unsigned char* dst, int* ex, cudaStream_t s) {
-  row_expo_kernel<T, HERM><<<HERM ? (n + 7) / 8 : (n + 31) / 32, 256, 0, s>>>(A, lda, n, n, ex);
+void pack_a(const T* A, long long lda, int rows, int n, int ks, unsigned char* dst, int* ex,
+            cudaStream_t s) {
+  row_expo_kernel<T, HERM>
+      <<<HERM ? (rows + 7) / 8 : (rows + 31) / 32, 256, 0, s>>>(A, lda, rows, n, ex);
   pack_digits_kernel<S, T, HERM, HERM, false, kGM>
-      <<<dim3((n + kGM - 1) / kGM, ks), 2 * kGM, 0, s>>>(A, lda, n, n, ex, dst);
+      <<<dim3((rows + kGM - 1) / kGM, ks), 2 * kGM, 0, s>>>(A, lda, rows, n, ex, dst);
 }
 
-// K splits: about two units per SM, at least two chunks each
-int splits(int n, int m) {
-  const long long tiles = (long long)((n + kGM - 1) / kGM) * ((m + kGN - 1) / kGN);
+// K splits of a rows x m product: about two units per SM, at least two chunks each
+int splits(int rows, int n, int m) {
+  const long long tiles = (long long)((rows + kGM - 1) / kGM) * ((m + kGN - 1) / kGN);
   const int chunks = (n + 16 * kGChunk - 1) / (16 * kGChunk);
   return (int)std::max<long long>(1, std::min<long long>((2 * device_sms() + tiles - 1) / tiles, chunks / 2));
 }
 
 }  // namespace
 
-size_t oz_gemm_a_bytes(int n, int S) {
-  const size_t ks = (size_t)(n + 15) / 16, mt = (size_t)(n + kGM - 1) / kGM;
-  return up256(mt * ks * S * kGA) + up256(sizeof(int) * (size_t)n);
+size_t oz_gemm_a_bytes(int rows, int n, int S) {
+  const size_t ks = (size_t)(n + 15) / 16, mt = (size_t)(rows + kGM - 1) / kGM;
+  return up256(mt * ks * S * kGA) + up256(sizeof(int) * (size_t)rows);
 }
 
-size_t oz_gemm_work_bytes(int n, int m, int S, size_t elem) {
+// the packed B, and the partial sums of a K split
+static size_t b_bytes(int n, int m, int S) {
   const size_t ks = (size_t)(n + 15) / 16, nt = (size_t)(m + kGN - 1) / kGN;
-  const int z = splits(n, m);
-  return up256(nt * ks * S * kGB) + up256(sizeof(int) * (size_t)m) +
-         (z > 1 ? elem * (size_t)z * n * m : 0);
+  return up256(nt * ks * S * kGB) + up256(sizeof(int) * (size_t)m);
+}
+size_t oz_gemm_work_bytes(int rows, int n, int m, int S, size_t elem) {
+  const int z = splits(rows, n, m);
+  return b_bytes(n, m, S) + (z > 1 ? elem * (size_t)z * rows * m : 0);
 }
 
 template <typename T>
-void launch_oz_pack(bool herm, int S, const T* A, long long lda, int n, void* dst, cudaStream_t s) {
+void launch_oz_pack(bool herm, int S, const T* A, long long lda, int r0, int rows, int n, void* dst,
+                    cudaStream_t s) {
   const int ks = (n + 15) / 16;
   unsigned char* d = static_cast<unsigned char*>(dst);
-  const size_t mt = (size_t)(n + kGM - 1) / kGM;
+  const size_t mt = (size_t)(rows + kGM - 1) / kGM;
+  A += herm ? (size_t)r0 * lda : (size_t)r0;
   int* ex = reinterpret_cast<int*>(d + up256(mt * ks * S * kGA));
   auto pack = [&](auto digits) {
     constexpr int D = decltype(digits)::value;
     if (herm)
-      pack_a<D, T, true>(A, lda, n, ks, d, ex, s);
+      pack_a<D, T, true>(A, lda, rows, n, ks, d, ex, s);
     else
-      pack_a<D, T, false>(A, lda, n, ks, d, ex, s);
+      pack_a<D, T, false>(A, lda, rows, n, ks, d, ex, s);
   };
   if constexpr (sizeof(T) == sizeof(float2))
     pack(std::integral_constant<int, 4>());
@@ -390,22 +400,23 @@ void launch_oz_pack(bool herm, int S, const T* A, long long lda, int n, void* ds
 }
 
 template <int S, typename T>
-static int gemm_t(const void* Apk, int n, const T* B, long long ldb, int m, T* C, long long ldc,
-                  void* work, int* status, cudaStream_t s) {
+static int gemm_t(const void* Apk, int rows, int n, int m, T* C, long long ldc, void* work,
+                  int* status, cudaStream_t s) {
   if (!opt_in_smem<oz_gemm_kernel<S, T>>(Cfg<S>::kSmem)) return BEM2D_ERR_CUDA;
-  const int ks = (n + 15) / 16, mt = (n + kGM - 1) / kGM, nt = (m + kGN - 1) / kGN, nz = splits(n, m);
+  const int ks = (n + 15) / 16, mt = (rows + kGM - 1) / kGM, nt = (m + kGN - 1) / kGN,
+            nz = splits(rows, n, m);
   const unsigned char* ap = static_cast<const unsigned char*>(Apk);
   const int* ea = reinterpret_cast<const int*>(ap + up256((size_t)mt * ks * S * kGA));
   unsigned char* bp = static_cast<unsigned char*>(work);
   int* eb = reinterpret_cast<int*>(bp + up256((size_t)nt * ks * S * kGB));
-  T* P = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(eb) + up256(sizeof(int) * (size_t)m));
+  T* P = reinterpret_cast<T*>(bp + b_bytes(n, m, S));
   const int units = mt * nt * nz;
   oz_gemm_kernel<S, T><<<std::min(units, device_sms()), kGThreads, Cfg<S>::kSmem, s>>>(
-      nz > 1 ? P : C, nz > 1 ? n : ldc, (long long)n * m, ap, bp, ea, eb, n, m, ks, nt, nz, units,
-      status);
+      nz > 1 ? P : C, nz > 1 ? rows : ldc, (long long)rows * m, ap, bp, ea, eb, rows, m, ks, nt, nz,
+      units, status);
   if (nz > 1)
-    oz_reduce_kernel<T><<<dim3((n + 255) / 256, m), 256, 0, s>>>(P, (long long)n * m, nz, n, m, C,
-                                                                 ldc);
+    oz_reduce_kernel<T><<<dim3((rows + 255) / 256, m), 256, 0, s>>>(P, (long long)rows * m, nz, rows,
+                                                                    m, C, ldc);
   return cudaPeekAtLastError() == cudaSuccess ? BEM2D_OK : BEM2D_ERR_CUDA;
 }
 
@@ -420,14 +431,27 @@ static void pack_b(const T* B, long long ldb, int n, int m, void* work, cudaStre
 }
 
 template <typename T>
-int launch_oz_gemm_pair(int S, const void* Apk, const void* Ahpk, int n, const T* B, long long ldb,
-                        int m, T* C1, T* C2, long long ldc, void* work, int* status,
-                        cudaStream_t s) {
+int launch_oz_gemm_pair(int S, const T* A, long long lda, int rows, void* Apk, int n, const T* B,
+                        long long ldb, int m, T* C1, T* C2, long long ldc, void* work, int* status,
+                        cudaStream_t s, long long* launches) {
   auto both = [&](auto digits) {
     constexpr int D = decltype(digits)::value;
     pack_b<D, T>(B, ldb, n, m, work, s);
-    const int rc = gemm_t<D, T>(Apk, n, B, ldb, m, C1, ldc, work, status, s);
-    return rc ? rc : gemm_t<D, T>(Ahpk, n, B, ldb, m, C2, ldc, work, status, s);
+    *launches += 2;
+    for (int r0 = 0; r0 < n; r0 += rows) {
+      const int r = std::min(rows, n - r0);
+      for (int herm = 0; herm < 2; ++herm) {
+        char* pk = static_cast<char*>(Apk) + (rows >= n ? herm * oz_gemm_a_bytes(n, n, D) : 0);
+        if (rows < n) {
+          launch_oz_pack<T>(herm != 0, D, A, lda, r0, r, n, pk, s);
+          *launches += 2;
+        }
+        const int rc = gemm_t<D, T>(pk, r, n, m, (herm ? C2 : C1) + r0, ldc, work, status, s);
+        if (rc) return rc;
+        *launches += splits(r, n, m) > 1 ? 2 : 1;
+      }
+    }
+    return (int)BEM2D_OK;
   };
   if constexpr (sizeof(T) == sizeof(float2))
     return both(std::integral_constant<int, 4>());
@@ -436,9 +460,11 @@ int launch_oz_gemm_pair(int S, const void* Apk, const void* Ahpk, int n, const T
 }
 
 #define BEM2D_OZ_INST(T)                                                                         \
-  template void launch_oz_pack<T>(bool, int, const T*, long long, int, void*, cudaStream_t);     \
-  template int launch_oz_gemm_pair<T>(int, const void*, const void*, int, const T*, long long,   \
-                                      int, T*, T*, long long, void*, int*, cudaStream_t);
+  template void launch_oz_pack<T>(bool, int, const T*, long long, int, int, int, void*,          \
+                                  cudaStream_t);                                                 \
+  template int launch_oz_gemm_pair<T>(int, const T*, long long, int, void*, int, const T*,       \
+                                      long long, int, T*, T*, long long, void*, int*,            \
+                                      cudaStream_t, long long*);
 BEM2D_OZ_INST(double2)
 BEM2D_OZ_INST(float2)
 #undef BEM2D_OZ_INST
