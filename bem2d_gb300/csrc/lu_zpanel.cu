@@ -321,11 +321,13 @@ int launch_zpanel(double2* A, long long lda, int n, int k0, int nb, const LuWork
     }
   });
   const int kend = k0 + nb;
+  // this panel's own limit: another thread's refused launch must not make a block
+  // too tall whose predecessors are already factored
+  int cmax = max_cluster;
   for (int kb = k0; kb < kend; kb += kZW) {
     const int bw = std::min(kZW, kend - kb), H = n - kb;
     // rows of a CTA: the fewest that 16 CTAs hold, in whole warps
     for (;;) {
-      const int cmax = max_cluster;
       const int rpb = std::max(32, ((H + cmax - 1) / cmax + 31) / 32 * 32);
       if (rpb > 2 * kZThreads) return kb == k0 ? 1 : BEM2D_ERR_CUDA;
       const int C = (H + rpb - 1) / rpb;
@@ -353,7 +355,7 @@ int launch_zpanel(double2* A, long long lda, int n, int k0, int nb, const LuWork
       if (e == cudaSuccess) break;
       cudaGetLastError();
       if (cmax <= 8) return kb == k0 ? 1 : BEM2D_ERR_CUDA;
-      max_cluster = 8;
+      cmax = max_cluster = 8;
     }
     const int others = nb - bw;
     if (others > 0)
