@@ -131,8 +131,9 @@ panel16_kernel(double2* __restrict__ A, long long lda, int n, int kb, int w, int
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (label[r] == 0xffffffffu || label[r] < kc || t != c % TPR) continue;
-      const long long b = __double_as_longlong(cabs1(a[r][c / TPR]));
-      if (b > 0x7ff0000000000000ll) continue;  // NaN
+      const unsigned long long b =
+          (unsigned long long)__double_as_longlong(cabs1(a[r][c / TPR]));
+      if (b > 0x7ff0000000000000ull) continue;  // NaN, whose sign bit may be set
       const unsigned h = (unsigned)(b >> 32), l = (unsigned)b;
       if (h > k.hi || (h == k.hi && (l > k.lo || (l == k.lo && label[r] < k.label))))
         k = ZKey{h, l, label[r]};
