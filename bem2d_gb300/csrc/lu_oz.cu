@@ -126,7 +126,7 @@ struct OzPack {
 
 __device__ __forceinline__ int oz_field(double2 v, int p) {
   const int e = max(expo(v.x), expo(v.y));
-  return e == 0 ? kOzNone : e == 2047 ? kNaN : e + p;
+  return is_zero(v) ? kOzNone : e == 2047 ? kNaN : e + p;
 }
 
 __device__ __forceinline__ uint4 oz_pack_fields(const int (&x)[8]) {

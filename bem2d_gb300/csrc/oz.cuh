@@ -34,8 +34,15 @@ __device__ __forceinline__ void mma(unsigned d, unsigned a, unsigned b, unsigned
       "l"(desc(a)), "l"(desc(b)), "r"(idesc), "r"(acc));
 }
 
-// exponent field of a double (0: zero or subnormal, 2047: not finite)
-__device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 2047; }
+// exponent field of a double (0: zero or subnormal, 2047: not finite), and the
+// exponent that goes with the mantissa: subnormals have that of the smallest
+// normal numbers
+__device__ __forceinline__ int expo_field(double x) { return (__double2hiint(x) >> 20) & 2047; }
+__device__ __forceinline__ int expo(double x) { return max(expo_field(x), 1); }
+__device__ __forceinline__ bool is_zero(double2 v) {
+  const int h = __double2hiint(v.x) | __double2hiint(v.y);
+  return ((h & 0x7fffffff) | __double2loint(v.x) | __double2loint(v.y)) == 0;
+}
 
 __device__ __forceinline__ int scale_of(int emax) {
   return emax > 50000 ? kNaN : emax <= -5000 ? kZero : emax;
@@ -43,18 +50,17 @@ __device__ __forceinline__ int scale_of(int emax) {
 
 // x 2^p as a fixed-point integer F, |F| < 2^(8 S - 1): x 2^p = F 2^(erow -
 // 1022 - (8 S - 1)), erow the largest exponent field plus p of the row, whose
-// largest entry has |F| >= 2^(8 S - 2).  Rounded to nearest (S = 8: toward
-// zero, below 2^-62 of the row's largest).  Subnormals count as zero.
+// largest entry has |F| >= 2^(8 S - 2) if it is normal.  Rounded to nearest (S =
+// 8: toward zero, below 2^-62 of the row's largest).
 template <int S>
 __device__ __forceinline__ long long fixed(double x, int p, int erow) {
-  const int e = expo(x);
-  if (e == 0) return 0;
   const long long b = __double_as_longlong(x);
-  const long long m = (b & 0xfffffffffffffll) | 0x10000000000000ll;
+  const int e = expo(x);
+  const long long m = (b & 0xfffffffffffffll) | (expo_field(x) ? 0x10000000000000ll : 0ll);
   const int d = erow - (e + p) + 54 - 8 * S;  // shift to the right
   long long f;
   if (d <= 0)
-    f = m << -d;
+    f = m << min(-d, 63);  // at most 10 for the entries of a scaled row
   else if (S == 8)
     f = d < 53 ? m >> d : 0;
   else

@@ -74,7 +74,7 @@ row_expo_kernel(const T* __restrict__ src, long long ld, int rows, int K, int* _
     for (int k = TRANS ? a : b; k < K; k += TRANS ? 32 : 8) {
       const double2 v = widen(src[TRANS ? (size_t)r * ld + k : (size_t)k * ld + r]);
       const int f = max(expo(v.x), expo(v.y));
-      if (f > 0) e = max(e, f == 2047 ? kNaN : f);
+      if (!is_zero(v)) e = max(e, f == 2047 ? kNaN : f);
     }
   }
   if (TRANS) {
