@@ -1787,6 +1787,14 @@ size_t lu_aux_bytes(int n, size_t elem) {
   return sizeof(int) * (size_t)n + 2 * nk * kNB * kNB * elem + 256;
 }
 
+// Updates large enough for the tensor cores on their own account: at least
+// kTensorMinN rows and columns, or tall and narrow ones (the columns inside an
+// outer block), or short wide ones (the rows of an outer block right of it).
+static bool tensor_sized(int M, int N) {
+  return (M >= kTensorMinN && N >= kTensorMinN) || (M >= 4 * kTensorMinN && N >= kNB) ||
+         (N >= 4 * kTensorMinN && M >= kNB);
+}
+
 // C -= Am Bm (M x N, inner dimension K; all three column-major with leading
 // dimension ld inside the matrix being factored).  complex64 updates of at
 // least kTensorMinN rows and columns run on the tensor cores, the rest on the
@@ -1803,10 +1811,7 @@ static int update_sub(T* C, const T* Am, const T* Bm, long long ld, int M, int N
                              w.status, s, launches);
   }
   if constexpr (sizeof(T) == sizeof(float2)) {
-    // tall and narrow updates (the columns inside an outer block), and short
-    // wide ones (the rows of an outer block right of it) too
-    if ((M >= kTensorMinN && N >= kTensorMinN) || (M >= 4 * kTensorMinN && N >= kNB) ||
-        (N >= 4 * kTensorMinN && M >= kNB)) {
+    if (tensor_sized(M, N)) {
       ++*launches;
       if (w.pack && tc_pack_bytes(M, N, K) <= w.pack_bytes) {
         *launches += part ? 1 : 2;  // + the packing kernel and the one for its scales
@@ -2018,10 +2023,13 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
         lparts[slot] = launch_col_expo(A + (size_t)k0 * lda + c1, lda, M, nb, lexp, s);
         ++*launches;
       }
+      // (one product per term only where the work is worth it: small updates cost
+      // no less with one than with three)
+      const int passes = tensor_sized(M, N) ? w.tc_passes : 3;
       if (N > 0 || k0 > cl) {
         if (launch_tc_step(reinterpret_cast<float2*>(A), lda, M, k0, nb, cl, c1, cr, w.ipiv, tc,
                            lexp, lparts[slot], TcExpo(), w.pack, w.status, s, w.tc_ctas,
-                           w.tc_passes))
+                           passes))
           return BEM2D_ERR_CUDA;
         *launches += tc ? 2 : 1;
       }
@@ -2069,7 +2077,8 @@ int lu_factor(T* A, long long lda, int n, const LuWork& w, cudaStream_t s,
         if (launch_tc_step(reinterpret_cast<float2*>(A), lda, bend - r1, j0, kNB, j0, bend, n,
                            nullptr, r1 < bend,
                            static_cast<const int*>(w.pack) + slot * kColParts * kNB, lparts[slot],
-                           ex, w.pack, w.status, s, w.tc_ctas, w.tc_passes))
+                           ex, w.pack, w.status, s, w.tc_ctas,
+                           tensor_sized(bend - r1, nc) ? w.tc_passes : 3))
           return BEM2D_ERR_CUDA;
         *launches += r1 < bend ? 2 : 1;
         continue;
