@@ -326,6 +326,7 @@ struct Staged {
   bool has_ff = false;
   NearPair* pairs;
   int npairs;
+  bool far = true;  // whether any pair is left to the far-field kernels
   // FP64 far field: runs of consecutive unknowns of one element
   const int2* grp = nullptr;
   int ngrp = 0, nb = 1;
@@ -481,6 +482,9 @@ static int stage(bem2d_ctx* c, const bem2d_geometry* g, const bem2d_quad* q, boo
   if (pairs) {
     const std::vector<NearPair> np = near_pairs(g, groups);
     st->npairs = (int)np.size();
+    long long left = (long long)groups.size() * groups.size();
+    for (const NearPair& p : np) left -= p.rule == RULE_G3_PAIR ? 2 : 1;
+    st->far = left > 0;
     st->pairs = static_cast<NearPair*>(ws(c, "pairs", sizeof(NearPair) * np.size(), &rc));
     if (!st->pairs) return rc;
     if (!np.empty())
@@ -540,14 +544,16 @@ static int check_k(bem2d_ctx* c, double k_re, double k_im) {
 static int assemble_dev(bem2d_ctx* c, const Staged& st, int kernel, double k, double eta,
                         double alpha, double beta, double2* A, long long ld, double ki = 0.0) {
   int t = tic(c, BEM2D_PHASE_FAR);
-  int rc = 0;
-  void* ck_tab = ki != 0.0 ? ws(c, "hankel_tab", hankel_tab_bytes(), &rc) : nullptr;
-  if (rc) return rc;
-  if (launch_far_fp64(st.g, st.t, st.grp, st.ngrp, st.nb, st.r.ng, kernel, k, ki, eta, alpha, A,
-                      ld, ck_tab, c->stream) != BEM2D_OK)
-    return fail(c, BEM2D_ERR_NOMEM, "device table for the far-field kernel");
+  if (st.far) {  // (a complex wavenumber's table takes longer than a few elements do)
+    int rc = 0;
+    void* ck_tab = ki != 0.0 ? ws(c, "hankel_tab", hankel_tab_bytes(), &rc) : nullptr;
+    if (rc) return rc;
+    if (launch_far_fp64(st.g, st.t, st.grp, st.ngrp, st.nb, st.r.ng, kernel, k, ki, eta, alpha, A,
+                        ld, ck_tab, c->stream) != BEM2D_OK)
+      return fail(c, BEM2D_ERR_NOMEM, "device table for the far-field kernel");
+    c->launches += ki != 0.0 ? 2 : 1;
+  }
   toc(c, t);
-  c->launches += ki != 0.0 ? 2 : 1;
   CHECK_LAUNCH(c);
   t = tic(c, BEM2D_PHASE_NEAR);
   if (ki != 0.0)
