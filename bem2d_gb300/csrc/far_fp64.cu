@@ -15,21 +15,6 @@
 
 namespace bem2d_gpu {
 
-// Direct evaluation outside the table's octaves.
-__device__ __noinline__ void hankel_direct(double d, double kr, double ki, double* h0r,
-                                           double* h0i, double* h1r, double* h1i) {
-  if (ki == 0.0) {
-    hankel01_d(kr * d, h0r, h0i, h1r, h1i);
-    return;
-  }
-  cd h0, h1;
-  hankel01_c(cd{kr * d, ki * d}, &h0, &h1);
-  *h0r = h0.re;
-  *h0i = h0.im;
-  *h1r = h1.re;
-  *h1i = h1.im;
-}
-
 // ---- table -------------------------------------------------------------------
 // One half-warp per interval: lane l evaluates Chebyshev point l, the
 // discrete Chebyshev sums a_j = (2/16) sum_l f_l cos(j theta_l), j <= 6, are
