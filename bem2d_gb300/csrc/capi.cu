@@ -1455,9 +1455,11 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
   for (int a = 0; a < nang; ++a) slot_angle[a] = a;
   int na = nang;
   // between two GPU steps the host resolves one tridiagonal per angle: 0.3 ms
-  // a step for 360 angles on one core, shared by up to 8 here
-  HostPool pool(std::min(7, std::max(0, std::min(nang / 16 - 1,
-                                                 (int)std::thread::hardware_concurrency() - 1))));
+  // a step for 360 angles on one core, shared by up to 8 here; not for the few
+  // steps of a small matrix (n = 5, 360 angles: 2.5 ms alone, 3.5 with threads)
+  const int share = mmax < 16 ? 0 : nang / 16 - 1;
+  HostPool pool(
+      std::min(7, std::max(0, std::min(share, (int)std::thread::hardware_concurrency() - 1))));
   T* Qalt = static_cast<T*>(ws(c, LzNames<T>::Q2, sizeof(T) * (size_t)qs * nang, &rc));
   T* Walt = static_cast<T*>(ws(c, LzNames<T>::W2, sizeof(T) * (size_t)n * nang, &rc));
   int* dmap = static_cast<int*>(ws(c, "nr_map", sizeof(int) * 2 * nang, &rc));
@@ -1471,7 +1473,13 @@ static int numrange_lanczos(bem2d_ctx* c, int n, const T* dA, long long la, int 
   char* oz = nullptr;
   int* oz_status = nullptr;
   int oz_rows = n;
-  for (;;) {
+  // Few small products: the digits' extra launches cost more than they save.  One
+  // angle, mixed: n = 33 2.47 ms with digits, 2.17 without, n = 65 3.60 / 3.28, n =
+  // 100 4.00 / 3.96, n = 130 4.69 / 5.03; 8 angles: n = 17 1.89 / 1.65, n = 33 2.90
+  // / 2.85, n = 65 4.34 / 4.77.  FP64, one angle: n = 17 1.67 / 1.54, n = 33 2.55 /
+  // 2.54, n = 65 3.73 / 4.45; 8 angles: n = 17 1.85 / 2.50.
+  const bool few = (long long)n * (nang + 3) < (digits == 8 ? 132 : 400);
+  for (; !few;) {
     zwork_bytes = 0;
     for (int m = 1; m <= nang; ++m)
       zwork_bytes = std::max(zwork_bytes, oz_gemm_work_bytes(oz_rows, n, m, digits, sizeof(T)));
