@@ -2343,13 +2343,6 @@ namespace bem2d_gpu {
 // Eigenvalues of the Hermitian M (N x N, device, overwritten): `count`
 // ascending from the smallest or descending from the largest, into out
 // (host or device, count doubles).
-static int sm_count(const bem2d_ctx* c) {
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess)
-    sms = 0;
-  return std::max(sms, 1);
-}
-
 static int spectra_run(bem2d_ctx* c, double2* M, int N, int count, int descending, double* out) {
   int rc = 0;
   void* work = ws(c, "sp_work", spectra_work_bytes(N), &rc);
@@ -2357,7 +2350,7 @@ static int spectra_run(bem2d_ctx* c, double2* M, int N, int count, int descendin
   const bool odev = is_device_ptr(out);
   double* dout = odev ? out : static_cast<double*>(ws(c, "sp_out", sizeof(double) * count, &rc));
   if (!dout) return rc;
-  c->launches += launch_tridiag_eigs(M, N, count, descending, work, dout, sm_count(c), c->stream);
+  c->launches += launch_tridiag_eigs(M, N, count, descending, work, dout, device_sms(), c->stream);
   CHECK_LAUNCH(c);
   if (!odev)
     CUDA_TRY(c, cudaMemcpyAsync(out, dout, sizeof(double) * count, cudaMemcpyDeviceToHost,
@@ -2404,7 +2397,7 @@ int bem2d_singular_values(bem2d_ctx* c, int n, const void* A, int64_t lda, doubl
   if (!M) return rc;
   CUDA_TRY(c, cudaMemcpy2DAsync(M, sizeof(double2) * n, dA, sizeof(double2) * la,
                                 sizeof(double2) * n, n, cudaMemcpyDeviceToDevice, c->stream));
-  const int sms = sm_count(c);
+  const int sms = device_sms();
   void* work = ws(c, "sp_work", bidiag_work_bytes(n, sms), &rc);
   if (!work) return rc;
   const bool odev = is_device_ptr(s);
@@ -2442,10 +2435,7 @@ int bem2d_eigenvalues(bem2d_ctx* c, int n, const void* A, int64_t lda, void* w) 
   if (!dw) return rc;
   CUDA_TRY(c, cudaMemcpy2DAsync(H, sizeof(double2) * n, dA, sizeof(double2) * la,
                                 sizeof(double2) * n, n, cudaMemcpyDeviceToDevice, c->stream));
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
-      sms < 1)
-    sms = 1;
+  const int sms = device_sms();
   const long long nl = launch_eigenvalues(H, n, work, dw, sms, c->stream);
   if (nl < 0)
     return fail(c, BEM2D_ERR_CUDA, "QR launch: %s", cudaGetErrorString(cudaGetLastError()));
@@ -2488,10 +2478,7 @@ int bem2d_eigenvectors(bem2d_ctx* c, int n, const void* A, int64_t lda, void* w,
   if (!dw || !X) return rc;
   CUDA_TRY(c, cudaMemcpy2DAsync(H, sizeof(double2) * n, dA, sizeof(double2) * la,
                                 sizeof(double2) * n, n, cudaMemcpyDeviceToDevice, c->stream));
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
-      sms < 1)
-    sms = 1;
+  const int sms = device_sms();
   const long long nl = launch_eigenvalues(H, n, work, dw, sms, c->stream, Z);
   if (nl < 0)
     return fail(c, BEM2D_ERR_CUDA, "QR launch: %s", cudaGetErrorString(cudaGetLastError()));

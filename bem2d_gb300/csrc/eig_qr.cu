@@ -276,8 +276,8 @@ hess_eigenvalues_kernel(double2* __restrict__ H, long long ld, int n, double2* _
         for (int v = tid; v < mm * mm; v += kQrCta) S[v % mm][v / mm] = at(base + v % mm, base + v / mm);
         __syncthreads();
         if (lw == 0) {
-          // entries below the subdiagonal are not zero in memory (bulges of
-          // earlier sweeps are cleared, reflectors are not stored there)
+          // entries below the subdiagonal are zero in memory (bulges are
+          // cleared, reflectors are not stored there)
           const bool good = small_eigs(S, mm, s_w);
           if (ln == 0) s_defl = good ? 1 : 0;
         }

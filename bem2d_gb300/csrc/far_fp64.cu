@@ -109,7 +109,7 @@ size_t hankel_tab_bytes() { return kHtBytes; }
 // shared, an orientation adds its normal factor n . (x - y), a basis function
 // its weight.  Measured against one direct evaluation (hankel01_d, ~175
 // instructions) per entry and node pair: kite N = 2048 31.2 -> 7.5 ms; 801
-// elements of PolBasis(2), N = 2403, 32.3 -> 2.0 ms; disk N = 160 2.1 -> 0.15
+// elements of PolBasis(2), N = 2403, 32.3 -> 1.24 ms; disk N = 160 2.1 -> 0.15
 // ms; complex wavenumber, N = 512, 113.6 -> 1.5 ms (hankel01_c sums up to 105
 // complex square roots per evaluation).
 //

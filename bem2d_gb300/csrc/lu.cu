@@ -1170,7 +1170,7 @@ static cudaError_t launch_cluster(K kern, int C, int threads, size_t smem, cudaS
 //      factored with partial pivoting by the register-window cluster kernel:
 //      its nb pivot rows are the panel's, its top nb rows are L11 \ U11;
 //   3. every other row a of the panel becomes L21 = a U11^{-1} (substitution
-//      across the columns, one warp per row), and the panel is written back
+//      across the columns, a thread per row), and the panel is written back
 //      in pivot order; the pivot sequence is returned as LAPACK row
 //      interchanges (ipiv), so the rest of the factorisation is unchanged.
 // One exchange between CTAs per panel instead of one per column.  The pivots

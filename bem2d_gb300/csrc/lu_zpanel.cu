@@ -15,8 +15,8 @@
 //                     block, U = L11^{-1} A (a warp per column)
 //   panel_update_kernel  A -= L U on the panel's columns right of the block,
 //                     spread over the whole chip
-// Measured: kite N = 2048, panels 24.7 -> 11.3 ms (4.4 us a column instead of
-// 12) against one cluster kernel with 64 columns in shared memory.
+// Measured: kite N = 2048, panels 24.7 -> 9.3 ms (panel16_kernel 7.4 of them, 3.6
+// us a column; one cluster kernel with 64 columns in shared memory: 12).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

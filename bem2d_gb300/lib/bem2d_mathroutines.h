@@ -75,7 +75,7 @@ void InPolygon(const pGeometry polygon, const std::vector<Point>& testpoints,
 
 // Solver precision of SolveSystem / SoundSoftScattering::Solve:
 // 0 = complex128 LU (default), 1 = complex64 LU + FP64 refinement,
-// 2 = as 1 with one tensor-core product per term in the LU's updates (10
+// 2 = as 1 with one tensor-core product per term in the LU's large updates (10
 // mantissa bits, as TF32 holds).
 void SetSolverPrecision(int precision);
 int GetSolverPrecision();

@@ -78,9 +78,9 @@ extern "C" {
 /* ---- solver precision -------------------------------------------------- */
 #define BEM2D_PREC_FP64 0  /* complex128 LU, FP64 throughout                 */
 #define BEM2D_PREC_MIXED 1 /* complex64 LU + FP64 iterative refinement      */
-/* As BEM2D_PREC_MIXED, with the LU's tensor-core trailing updates as one
- * product per term (operands rounded to 10 mantissa bits, as TF32 holds; a
- * third of the tensor work).  The factor is then accurate to about
+/* As BEM2D_PREC_MIXED, with the LU's large trailing updates (256 rows and
+ * columns or more) as one product per term (operands rounded to 10 mantissa
+ * bits, as TF32 holds; a third of the tensor work).  The factor is then accurate to about
  * 1e-3 relative instead of 1e-6, so refinement contracts the error by about
  * cond(A) 1e-3 per step: for systems with cond(A) up to ~100; beyond that
  * GMRES-IR takes over (see bem2d_solve_system).  Accepted by
